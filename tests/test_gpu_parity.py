@@ -12,7 +12,7 @@ of the last bit and are counted, not failed (``Parity.ok``).
 import pytest
 import torch
 
-from ayla_b200 import _lib, gemm_op, gemm_op_compiler, swiglu_op, swiglu_op_compiler
+from ayla_b200 import _lib, gemm_act_op, gemm_op, gemm_op_compiler, swiglu_op, swiglu_op_compiler
 from ayla_b200.gemm_jit import gemm_jit_compiler
 from oracle import gemm_oracle as O
 from tests.conftest import load_golden_cases
@@ -351,6 +351,35 @@ def test_fused_activation_epilogue(activation, device_state):
             assert int(status.item()) == 0
             want = O.act_ref32(activation, O.gemm_ref32(operation, *tensors))
             assert_parity(out.cpu(), want, f"{activation} {operation} {batch}x{m}x{n}x{k} {cfg}")
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("activation", ["sigmoid", "silu", "gelu", "gelu_tanh"])
+def test_activations_at_every_16_bit_value(activation, dtype):
+    """act(x @ I) over every finite value of the type (bf16 from 2^-100 up: its square and cube must not
+    leave fp32's range at the bottom), against the function in double precision.  The bound is half an ulp
+    for the one rounding, plus the relative error of the fp32 evaluation: 2^z with |z| <= 130 carries z's
+    own rounding (130 * 2^-24 * ln 2 < 6e-6, three times that for the cubic argument of gelu_tanh), GELU's
+    polynomial 3e-6 down to x = -6 and less than 6e-9 absolutely below, where 6 * Phi(-6) is 5.9e-9;
+    results under 2^-100 may be flushed."""
+    values = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(TD[dtype])
+    values = values[torch.isfinite(values)]
+    if dtype == "bfloat16":
+        values = torch.where(values.float().abs() < 2.0 ** -100, torch.zeros_like(values), values)
+    x = torch.cat([values, values.new_zeros(-values.numel() % 64)]).view(-1, 64)
+    out = torch.full_like(x, float("nan"), device=DEV)
+    gemm_act_op("mm", activation, dtype)(x.to(DEV), torch.eye(64, dtype=TD[dtype], device=DEV), out)
+    x64 = x.double()
+    want = {"sigmoid": lambda t: torch.special.expit(t), "silu": lambda t: t * torch.special.expit(t),
+            "gelu": lambda t: 0.5 * t * torch.special.erfc(-t * 0.5 ** 0.5),
+            "gelu_tanh": lambda t: t * torch.special.expit(2 * (2 / torch.pi) ** 0.5 * (t + 0.044715 * t ** 3)),
+            }[activation](x64)
+    got = out.cpu().double()
+    half_ulp = 0.5 * O._ulp(want.float(), TD[dtype]).double()
+    relative = {"gelu": 3e-6, "gelu_tanh": 2e-5}.get(activation, 7e-6)
+    bound = 1.001 * half_ulp + relative * want.abs() + (6e-9 if activation == "gelu" else 2.0 ** -100)
+    bad = ~((got - want).abs() <= bound)
+    assert not bad.any(), [(x64[bad][i].item(), got[bad][i].item(), want[bad][i].item()) for i in range(min(5, int(bad.sum())))]
 
 
 @pytest.mark.parametrize("activation", ["none", "sigmoid", "silu"])
