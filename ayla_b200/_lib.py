@@ -27,6 +27,7 @@ EXPORTS = (
     "ayla_b200_gemm_act_rowmul",
     "ayla_b200_gemm_static_scratch",
     "ayla_b200_swiglu",
+    "ayla_b200_rms_factors",
     "ayla_b200_default_config",
     "ayla_b200_config_valid",
     "ayla_b200_workspace_bytes",
@@ -127,6 +128,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_gemm_static_scratch.restype = i32
         lib.ayla_b200_swiglu.argtypes = [i32, vp, vp, vp, vp, i64, i64, i64, cfgp, vp, vp]
         lib.ayla_b200_swiglu.restype = i32
+        lib.ayla_b200_rms_factors.argtypes = [i32, vp, vp, i64, i64, ctypes.c_float, vp]
+        lib.ayla_b200_rms_factors.restype = i32
         lib.ayla_b200_default_config.argtypes = [i32, i32, i64, i64, i64, i64, cfgp]
         lib.ayla_b200_default_config.restype = i32
         lib.ayla_b200_config_valid.argtypes = [cfgp, i32, i32, i64, i64, i64, i64]
@@ -307,6 +310,11 @@ def swiglu(dtype: str, x_ptr: int, wg_ptr: int, wu_ptr: int, out_ptr: int, m: in
     check(load().ayla_b200_swiglu(
         DTYPE_CODES[dtype], x_ptr, wg_ptr, wu_ptr, out_ptr, m, n, k,
         ctypes.byref(cfg) if cfg is not None else None, status_ptr or None, stream or None))
+
+
+def rms_factors(dtype: str, x_ptr: int, factors_ptr: int, rows: int, k: int, eps: float, stream: int) -> None:
+    """One factor per row, ``rsqrt(mean(row ** 2) + eps)``, in the operands' type."""
+    check(load().ayla_b200_rms_factors(DTYPE_CODES[dtype], x_ptr, factors_ptr, rows, k, eps, stream or None))
 
 
 def set_launch_overlap(enabled: bool) -> None:

@@ -17,6 +17,7 @@
 #include <unordered_map>
 
 #include "kernel_registry.h"
+#include "rms_factors.h"
 
 namespace ayla_b200 {
 namespace {
@@ -1033,6 +1034,20 @@ int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate, const void* w
   if (rc) return rc;
   return launch_plan(plan, c, pr, dtype == AYLA_B200_BF16 ? 1 : 0, nullptr, w_up, out, m, n, nullptr, 0,
                      status, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int ayla_b200_rms_factors(int dtype, const void* x, void* factors, int64_t rows, int64_t k, float eps, void* stream) {
+  const int rc = check_shape(AYLA_B200_OP_MM, dtype, 1, rows, 8, k);
+  if (rc) return rc;
+  if (x == nullptr || factors == nullptr) return fail(AYLA_B200_E_INVALID, "x and factors must be non-null");
+  if (!aligned16(x) || (reinterpret_cast<uintptr_t>(factors) & 1) != 0) {
+    return fail(AYLA_B200_E_UNSUPPORTED, "x must be 16-byte aligned and factors 2-byte aligned");
+  }
+  const cudaError_t err =
+      launch_rms_factors(x, factors, static_cast<int>(rows), static_cast<int>(k), eps, dtype == AYLA_B200_BF16 ? 1 : 0,
+                         g_launch_overlap.load(), reinterpret_cast<cudaStream_t>(stream));
+  if (err != cudaSuccess) return fail(AYLA_B200_E_CUDA, "kernel launch failed: %s", cudaGetErrorString(err));
+  return AYLA_B200_OK;
 }
 
 // The listing covers the variants without the activation epilogue; each of them except the

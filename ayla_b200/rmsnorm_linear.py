@@ -10,9 +10,13 @@ are never written to or read back from memory.  The reference lists epilogue fus
 
 from __future__ import annotations
 
+from functools import cache
+
 import torch
 
+from . import _lib
 from .gemm_jit import _SHORT_DTYPES, _TORCH_DTYPES, gemm_act_rowmul_op
+from .torch_custom_call import DEFAULT_NAMESPACE, _library
 
 _DTYPE_NAMES = {torch_dtype: name for name, torch_dtype in _TORCH_DTYPES.items() if name in _SHORT_DTYPES}
 
@@ -21,6 +25,32 @@ def fold_norm_weight(weight: torch.Tensor, norm_weight: torch.Tensor) -> torch.T
     """``W * g`` along the input features, computed in fp32 and rounded once: ``weight`` is
     ``[out_features, in_features]``, ``norm_weight`` is ``[in_features]``."""
     return (weight.float() * norm_weight.float()).to(weight.dtype)
+
+
+@cache
+def _row_factors_op(dtype: str) -> torch._ops.OpOverload:
+    """Torch op ``(x, eps, factors) -> ()`` writing ``factors[r, 0] = rsqrt(mean(x[r] ** 2) + eps)``."""
+    name = f"rms_row_factors_{_SHORT_DTYPES[dtype]}"
+
+    def cuda_impl(x: torch.Tensor, eps: float, factors: torch.Tensor) -> None:
+        if x.dim() != 2:
+            raise ValueError(f"{name}: expected a rank-2 tensor, got shape {tuple(x.shape)}")
+        if x.dtype != _TORCH_DTYPES[dtype] or factors.dtype != x.dtype:
+            raise ValueError(f"{name}: expected dtype {_TORCH_DTYPES[dtype]}, got {x.dtype} and {factors.dtype}")
+        if not (x.is_contiguous() and factors.is_contiguous()):
+            raise ValueError(f"{name}: all tensors must be contiguous")
+        if factors.device != x.device or factors.numel() != x.shape[0]:
+            raise ValueError(f"{name}: factors must hold one element per row of x on its device")
+        with torch.cuda.device(x.device):
+            _lib.init(x.device.index)
+            _lib.rms_factors(dtype, x.data_ptr(), factors.data_ptr(), x.shape[0], x.shape[1], eps,
+                             torch.cuda.current_stream().cuda_stream)
+
+    lib = _library(DEFAULT_NAMESPACE)
+    lib.define(f"{name}(Tensor arg0, float eps, Tensor(a1!) arg1) -> ()")
+    lib.impl(name, cuda_impl, "CUDA")
+    lib.impl(name, lambda x, eps, factors: None, "Meta")
+    return getattr(getattr(torch.ops, DEFAULT_NAMESPACE), name).default
 
 
 def rms_norm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float = 1e-5, activation: str = "none",
@@ -36,6 +66,8 @@ def rms_norm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float = 1
     tokens = x.shape[0]
     if out is None:
         out = torch.empty(tokens, folded_weight.shape[0], dtype=x.dtype, device=x.device)
-    factors = torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + eps).to(x.dtype)
-    gemm_act_rowmul_op("mm", activation, _DTYPE_NAMES[x.dtype])(x, folded_weight, factors, out)
+    dtype = _DTYPE_NAMES[x.dtype]
+    factors = torch.empty(tokens, 1, dtype=x.dtype, device=x.device)
+    _row_factors_op(dtype)(x, eps, factors)
+    gemm_act_rowmul_op("mm", activation, dtype)(x, folded_weight, factors, out)
     return out

@@ -219,6 +219,15 @@ AYLA_B200_API int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate,
                      void* stream);
 
 /*
+ * factors[r] = 1 / sqrt(mean(x[r,:]^2) + eps) over the rows of x[rows,k], computed in fp32 and rounded
+ * once to the operands' type: the row factors ayla_b200_gemm_act_rowmul applies for an RMS norm whose
+ * weight vector is folded into the projection.  x must be 16-byte aligned, k a multiple of 8.  No
+ * counterpart in the reference.
+ */
+AYLA_B200_API int ayla_b200_rms_factors(int dtype, const void* x, void* factors, int64_t rows, int64_t k, float eps,
+                                        void* stream);
+
+/*
  * The schedule ayla_b200_gemm uses when cfg == NULL.  Counterpart of
  * select_gemm_schedule's fallback (ayla/gemm_jit.py:225-264).
  */

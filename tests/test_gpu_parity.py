@@ -484,6 +484,37 @@ def test_rms_norm_linear_matches_the_unfused_form():
                                                                                 dtype=torch.bfloat16))
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("rows, k", [(1, 8), (9, 248), (7, 2040), (5, 2048), (3, 4096), (2, 8184), (2, 8200), (1, 65536)])
+def test_rms_row_factors(rows, k, dtype):
+    """Either side of each choice of threads per row, against double precision: half an ulp for the one
+    rounding, and k * 2^-24 relative for the fp32 sum (halved by the root) with 2^-22 for rsqrt."""
+    from ayla_b200.rmsnorm_linear import _row_factors_op
+
+    torch.manual_seed(rows * k)
+    x = (torch.randn(rows, k) * torch.linspace(0.1, 4.0, rows).view(-1, 1)).to(TD[dtype])
+    factors = torch.full((rows + 1, 1), float("nan"), dtype=TD[dtype], device=DEV)
+    _row_factors_op(dtype)(x.to(DEV), 1e-5, factors[:rows])
+    want = torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-5)
+    bound = 0.5 * O._ulp(want.float(), TD[dtype]).double() + want * (0.5 * k * 2.0 ** -24 + 2.0 ** -22)
+    assert ((factors[:rows].cpu().double() - want).abs() <= bound).all()
+    assert torch.isnan(factors[rows])
+
+
+def test_rms_norm_linear_refuses_what_the_projection_refuses():
+    from ayla_b200.rmsnorm_linear import rms_norm_linear
+
+    x = torch.randn(16, 264, device=DEV).bfloat16()
+    w = torch.randn(64, 264, device=DEV).bfloat16()
+    for bad_x, bad_w in ((x[:, :256], w[:, :256].contiguous()), (x.view(2, 8, 264), w), (x[:0], w), (x, w[:, :256]),
+                         (x.view(-1)[4:].narrow(0, 0, 15 * 264).view(15, 264), w),
+                         (x[:, :260].contiguous(), w[:, :260].contiguous())):
+        with pytest.raises(ValueError):
+            rms_norm_linear(bad_x, bad_w)
+    y = x.clone().requires_grad_()
+    assert torch.equal(rms_norm_linear(y, w), rms_norm_linear(x, w))
+
+
 def test_gemm_act_mul_op_matches_the_oracle():
     from ayla_b200 import gemm_act_mul_op
 
