@@ -26,6 +26,8 @@ EXPORTS = (
     "ayla_b200_gemm_act_mul",
     "ayla_b200_gemm_act_rowmul",
     "ayla_b200_gemm_static_scratch",
+    "ayla_b200_gemm_packed",
+    "ayla_b200_packed_preferred",
     "ayla_b200_swiglu",
     "ayla_b200_rms_factors",
     "ayla_b200_default_config",
@@ -126,6 +128,10 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_gemm_act_rowmul.restype = i32
         lib.ayla_b200_gemm_static_scratch.argtypes = [i32, i32, vp, vp, vp, vp, i64, i64, i64, i64, cfgp, vp, vp]
         lib.ayla_b200_gemm_static_scratch.restype = i32
+        lib.ayla_b200_gemm_packed.argtypes = [i32, i32, vp, vp, vp, vp, i64, i64, i64, i64, vp, vp]
+        lib.ayla_b200_gemm_packed.restype = i32
+        lib.ayla_b200_packed_preferred.argtypes = [i32, i64, i64, i64, i64]
+        lib.ayla_b200_packed_preferred.restype = i32
         lib.ayla_b200_swiglu.argtypes = [i32, vp, vp, vp, vp, i64, i64, i64, cfgp, vp, vp]
         lib.ayla_b200_swiglu.restype = i32
         lib.ayla_b200_rms_factors.argtypes = [i32, vp, vp, i64, i64, ctypes.c_float, vp]
@@ -284,6 +290,19 @@ def gemm_act_rowmul(op: str, dtype: str, activation: str, bias_ptr: int, a_ptr: 
         OP_CODES[op], DTYPE_CODES[dtype], ACT_CODES[activation], bias_ptr or None, a_ptr, bt_ptr, row_mul_ptr or None,
         out_ptr, batch, m, n, k, ctypes.byref(cfg) if cfg is not None else None, workspace_ptr or None,
         workspace_size, status_ptr or None, stream or None))
+
+
+def packed_preferred(op: str, batch: int, m: int, n: int, k: int) -> bool:
+    """Whether ``gemm_packed`` is the faster way to run the problem."""
+    return bool(load().ayla_b200_packed_preferred(OP_CODES[op], batch, m, n, k))
+
+
+def gemm_packed(op: str, dtype: str, bias_ptr: int, a_ptr: int, bt_ptr: int, out_ptr: int, batch: int, m: int,
+                n: int, k: int, status_ptr: int, stream: int) -> None:
+    """``gemm`` through the kernel for ``n`` and ``k`` of at most 128 (see ``include/ayla_b200.h``)."""
+    check(load().ayla_b200_gemm_packed(
+        OP_CODES[op], DTYPE_CODES[dtype], bias_ptr or None, a_ptr, bt_ptr, out_ptr, batch, m, n, k,
+        status_ptr or None, stream or None))
 
 
 STATIC_SCRATCH_BYTES = 8 << 20

@@ -17,6 +17,7 @@
 #include <unordered_map>
 
 #include "kernel_registry.h"
+#include "packed_gemm.h"
 #include "rms_factors.h"
 
 namespace ayla_b200 {
@@ -772,6 +773,11 @@ int ayla_b200_init(int device) {
       }
     }
     if (rc) break;
+    err = init_packed_gemm();
+    if (err != cudaSuccess) {
+      rc = fail(AYLA_B200_E_CUDA, "cudaFuncSetAttribute for the packed kernel: %s", cudaGetErrorString(err));
+      break;
+    }
     {
       // Resolve the built-in scratch array here as well, with `device` current: the query loads the
       // library's device image if nothing has yet, which is better done at set-up than inside the
@@ -904,6 +910,8 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   ayla_b200_config c;
   if (cfg != nullptr) {
     c = *cfg;
+  } else if (activation == AYLA_B200_ACT_NONE && mul == nullptr && packed_preferred(batch, m, n, k, ds->sm_count)) {
+    return ayla_b200_gemm_packed(op, dtype, bias, a, bt, out, batch, m, n, k, status, stream);
   } else {
     default_config(batch, m, n, k, ds->sm_count, &c);
   }
@@ -930,6 +938,54 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   if (rc) return rc;
   return launch_plan(plan, c, pr, dtype == AYLA_B200_BF16 ? 1 : 0, bias, nullptr, out, m, n, workspace,
                      workspace_bytes, status, reinterpret_cast<cudaStream_t>(stream), activation, mul, mul_per_row);
+}
+
+int ayla_b200_gemm_packed(int op, int dtype, const void* bias, const void* a, const void* bt, void* out,
+                          int64_t batch, int64_t m, int64_t n, int64_t k, uint32_t* status, void* stream) {
+  int rc = check_shape(op, dtype, batch, m, n, k);
+  if (rc) return rc;
+  if (a == nullptr || bt == nullptr || out == nullptr) {
+    return fail(AYLA_B200_E_INVALID, "a, bt and out must be non-null");
+  }
+  if (op == AYLA_B200_OP_ADDMM && bias == nullptr) {
+    return fail(AYLA_B200_E_INVALID, "addmm needs a bias pointer");
+  }
+  if (!aligned16(a) || !aligned16(bt) || !aligned16(out)) {
+    return fail(AYLA_B200_E_UNSUPPORTED, "a, bt and out must be 16-byte aligned");
+  }
+  if (n > kPackedMaxN || k > kPackedMaxK || batch * ceil_div(m, 128) > 0x7FFFFFFF) {
+    return fail(AYLA_B200_E_UNSUPPORTED, "the packed kernel takes n <= %d and k <= %d, got n=%lld k=%lld", kPackedMaxN,
+                kPackedMaxK, (long long)n, (long long)k);
+  }
+  DeviceState* ds = nullptr;
+  int dev = -1;
+  rc = current_device_state(&ds, &dev);
+  if (rc) return rc;
+  PackedProblem pr = {};
+  pr.a = a;
+  pr.b = bt;
+  pr.bias = op == AYLA_B200_OP_ADDMM ? bias : nullptr;
+  pr.out = out;
+  pr.batch = batch;
+  pr.m = m;
+  pr.n = n;
+  pr.k = k;
+  pr.is_bf16 = dtype == AYLA_B200_BF16 ? 1 : 0;
+  pr.idesc_base = make_idesc(pr.is_bf16, 128, 0);
+  pr.status = status;
+  pr.timeout_ns = static_cast<unsigned long long>(g_timeout_ns.load());
+  pr.debug_flags = g_debug_flags.load();
+  pr.sm_count = ds->sm_count;
+  pr.overlap = g_launch_overlap.load();
+  pr.stream = reinterpret_cast<cudaStream_t>(stream);
+  const cudaError_t err = launch_packed_gemm(pr);
+  if (err != cudaSuccess) return fail(AYLA_B200_E_CUDA, "kernel launch failed: %s", cudaGetErrorString(err));
+  return AYLA_B200_OK;
+}
+
+int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k) {
+  if (check_shape(op, AYLA_B200_BF16, batch, m, n, k) != AYLA_B200_OK) return 0;
+  return packed_preferred(batch, m, n, k, 148) ? 1 : 0;
 }
 
 int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const void* a, const void* bt,

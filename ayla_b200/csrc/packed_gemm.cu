@@ -1,0 +1,427 @@
+// out[b, m, n] = [bias[n] +] sum_k a[b, m, k] * b[b, n, k] for n, k <= 128: window attention, pointwise
+// convolutions, any product whose work is reading a and writing out.
+//
+// What bounds these is memory, and on the way to it the fixed cost of a tile.  The general kernel spends some
+// 0.8 us of one SM on a tile however little it holds (one CTA per SM, half of the epilogue warps idle at 64
+// columns), and its TMA boxes are 64 elements deep: rows of 24 elements take four times as long as rows of 64.
+// Here
+//  * a unit is one 128-row accumulator: 128 rows of one matrix, or two or four small matrices side by side (their
+//    rows stacked in A, their columns in B; the products of one matrix's rows with another's columns are computed
+//    along and dropped, a tcgen05.mma of 128 rows takes the same 39 cycles up to 32 columns);
+//  * operands come through cp.async in 16-byte pieces, which read the contiguous rows as one stream whatever
+//    their length and put each piece where the swizzle wants it;
+//  * the accumulator leaves through shared memory as one contiguous run of 16-byte pieces;
+//  * two to four CTAs share an SM and hide each other's waits; inside one, the next unit's loads run under the
+//    MMAs and the epilogue.
+// us per launch (graph replay, operands past L2), general kernel -> this one: bmm 8192 x 56x32x56 45.9 -> 22.4
+// (110 MB: 16.8 at the copy peak), 8192 x 16x16x16 44.9 -> 7.1, mm 200704x96x24 37.3 -> 16.3 (7.4 at the peak),
+// 153718x32x16 18.5 -> 6.2.  What is left is latency: with two or three units per CTA a unit takes some 5000 cycles
+// from its load to its last store, over half of them in the epilogue's chain of TMEM load, conversion, staging and
+// copy.  Measured and left out: 256 threads per CTA (bmm 22.4 -> 35.8), a third ring slot (25.6, it costs a resident
+// CTA), two accumulators per CTA with the MMAs of a unit under the epilogue of the one before (25.5: half the CTAs
+// find room in TMEM).
+#include "packed_gemm.h"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "gemm_sm100.cuh"
+
+namespace ayla_b200 {
+namespace {
+
+constexpr int kThreads = 128;     // a warp per quarter of the accumulator's rows
+constexpr int kStages = 2;
+constexpr int kMaxCtasPerSm = 4;  // each may hold 128 of the 512 TMEM columns
+constexpr int kRows = 128;        // accumulator rows
+
+struct PackedParams {
+  const uint8_t* a;
+  const uint8_t* b;
+  const void* bias;
+  uint8_t* out;
+  int units, row_tiles, batch, m, n;
+  int matrices;   // small matrices per unit (1, 2 or 4)
+  int slot_rows;  // accumulator rows each of them has
+  int k_chunks;   // 16-byte pieces of one operand row
+  int k_blocks;   // 64-deep blocks of an operand in shared memory
+  int narrow;     // operand rows of 128 >> narrow bytes per block (a depth of at most 64 >> narrow)
+  int mma_n;      // accumulator columns
+  int shared_b;   // 1: every unit multiplies by the same B, loaded once
+  int tmem_cols;
+  uint32_t idesc;
+  uint32_t staging_pitch;
+  int load_rows;     // operand rows the CTA loads at a time: each thread keeps to one piece of its row
+  int load_threads;  // load_rows * k_chunks
+  FastDiv div_k_chunks, div_n_chunks, div_row_tiles;
+  unsigned* status;
+  unsigned long long timeout_ns;
+  int debug_flags;
+};
+
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+
+// Offset of 16-byte piece `c` of row `row` in an operand tile of 64-deep blocks of `block_bytes`, in the
+// 128-, 64- or 32-byte swizzle (rows of 128 >> narrow bytes, a single block where narrow > 0).
+__device__ __forceinline__ uint32_t piece_offset(int row, int c, uint32_t block_bytes, int narrow) {
+  const int swizzle = (row >> narrow) & (7 >> narrow);
+  return static_cast<uint32_t>(c >> 3) * block_bytes + (static_cast<uint32_t>(row) << (7 - narrow)) +
+         static_cast<uint32_t>(((c & 7) ^ swizzle) << 4);
+}
+
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr, int narrow) {
+  // As umma_smem_desc_sw128, with eight rows 1024 >> narrow bytes apart and layout type 2, 4 or 6.
+  uint64_t d = umma_smem_desc_sw128(smem_addr);
+  d &= ~((static_cast<uint64_t>(0x3FFF) << 32) | (static_cast<uint64_t>(7) << 61));
+  d |= static_cast<uint64_t>(64 >> narrow) << 32;
+  d |= static_cast<uint64_t>(2 + 2 * narrow) << 61;
+  return d;
+}
+
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  return pack2(lo, hi, BF16 ? 1 : 0);
+}
+
+template <bool BF16>
+__global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(const PackedParams p) {
+#if defined(__CUDA_ARCH_FEAT_SM100_ALL) || defined(__CUDA_ARCH_FEAT_SM101_ALL)
+  extern __shared__ __align__(1024) uint8_t packed_smem[];
+  const int narrow = p.narrow;
+  const uint32_t a_block = static_cast<uint32_t>(kRows * 128) >> narrow;
+  const uint32_t a_bytes = static_cast<uint32_t>(p.k_blocks) * a_block;
+  const uint32_t b_block = static_cast<uint32_t>(p.mma_n * 128) >> narrow;
+  const uint32_t b_bytes = static_cast<uint32_t>(p.k_blocks) * b_block;
+  const int b_copies = p.shared_b ? 1 : kStages;
+  uint8_t* smem_b = packed_smem + kStages * a_bytes;
+  uint8_t* smem_staging = smem_b + b_copies * b_bytes;
+  float* smem_bias = reinterpret_cast<float*>(smem_staging + kRows * p.staging_pitch);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_bias + kPackedMaxN);
+  const uint32_t bar_done = smem_u32(bars);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int tid = static_cast<int>(threadIdx.x);
+  const int warp = tid >> 5, lane = tid & 31;
+  const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    if ((smem_u32(packed_smem) & 1023u) != 0) bw.give_up(ST_BAD_SMEM_ALIGN);
+    mbar_init(bar_done, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc<1>(smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
+    tmem_relinquish<1>();
+  }
+  // A depth that is an odd number of pieces is read one piece further by the MMAs: zero in both operands.
+  if ((p.k_chunks & 1) != 0) {
+    for (int i = tid; i < kStages * kRows; i += kThreads) {
+      const int s = i / kRows, row = i % kRows;
+      *reinterpret_cast<uint4*>(packed_smem + s * a_bytes + piece_offset(row, p.k_chunks, a_block, narrow)) =
+          make_uint4(0, 0, 0, 0);
+    }
+    for (int s = 0; s < b_copies; ++s) {
+      for (int row = tid; row < p.mma_n; row += kThreads) {
+        *reinterpret_cast<uint4*>(smem_b + s * b_bytes + piece_offset(row, p.k_chunks, b_block, narrow)) =
+            make_uint4(0, 0, 0, 0);
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (p.bias != nullptr && tid < p.n) smem_bias[tid] = load_elem(p.bias, tid, BF16 ? 1 : 0);
+
+  const int first = static_cast<int>(blockIdx.x), stride = static_cast<int>(gridDim.x);
+  const int count = (p.units - first + stride - 1) / stride;  // the grid is no larger than `units`
+
+  // Loads of this CTA's i-th unit into ring slot `s`: one commit group per unit, empty past the last.
+  const int load_row = p.div_k_chunks.div(tid);
+  const int load_c = tid - load_row * p.k_chunks;
+  const bool loads = tid < p.load_threads;
+  auto load_operand = [&](uint32_t dst, const uint8_t* src, int rows, uint32_t block_bytes, int rows_per_matrix,
+                          int gap) {
+    src += static_cast<uint32_t>(tid) * 16u;
+    const uint32_t step = static_cast<uint32_t>(p.load_threads) * 16u;
+    int slot_row = load_row, left = rows_per_matrix - load_row;  // rows of this matrix still ahead
+    for (int row = load_row; row < rows; row += p.load_rows) {
+      while (left <= 0) {
+        left += rows_per_matrix;
+        slot_row += gap;
+      }
+      cp_async_16(dst + piece_offset(slot_row, load_c, block_bytes, narrow), src);
+      src += step;
+      slot_row += p.load_rows;
+      left -= p.load_rows;
+    }
+  };
+  auto load_unit = [&](int i, int s) {
+    if (i < count && loads) {
+      const int unit = first + i * stride;
+      int first_matrix, matrices, row0, rows;  // rows: of A, over all of the unit's matrices
+      if (p.matrices == 1) {
+        first_matrix = p.div_row_tiles.div(unit);
+        matrices = 1;
+        row0 = (unit - first_matrix * p.row_tiles) * kRows;
+        rows = min(kRows, p.m - row0);
+      } else {
+        first_matrix = unit * p.matrices;
+        matrices = min(p.matrices, p.batch - first_matrix);
+        row0 = 0;
+        rows = matrices * p.m;
+      }
+      load_operand(smem_u32(packed_smem) + static_cast<uint32_t>(s) * a_bytes,
+                   p.a + (static_cast<size_t>(first_matrix) * p.m + row0) * p.k_chunks * 16, rows, a_block,
+                   p.matrices == 1 ? kRows : p.m, p.slot_rows - p.m);
+      if (!p.shared_b || i == 0) {
+        load_operand(smem_u32(smem_b) + (p.shared_b ? 0u : static_cast<uint32_t>(s) * b_bytes),
+                     p.b + static_cast<size_t>(first_matrix) * p.n * p.k_chunks * 16, matrices * p.n, b_block,
+                     kPackedMaxN, 0);
+      }
+    }
+    cp_async_commit();
+  };
+
+  // Rows of this warp's accumulator quarter: matrix `my_matrix` of the unit, from its row `my_row` on.
+  const int warps_per_slot = p.slot_rows / 32;
+  const int my_matrix = warp / warps_per_slot;
+  const int my_row = (warp % warps_per_slot) * 32;
+  const int n_chunks = p.n >> 3;
+  uint8_t* staging = smem_staging + warp * 32 * p.staging_pitch;
+  // This lane's first piece of the warp's staged rows, and the steps to the one 32 pieces on.
+  const int out_row = p.div_n_chunks.div(lane), out_c = lane - out_row * n_chunks;
+  const int out_row_step = p.div_n_chunks.div(32), out_c_step = 32 - out_row_step * n_chunks;
+  const uint32_t out_offset = static_cast<uint32_t>(out_row) * p.staging_pitch + static_cast<uint32_t>(out_c) * 16u;
+  const uint32_t out_step =
+      static_cast<uint32_t>(out_row_step) * p.staging_pitch + static_cast<uint32_t>(out_c_step) * 16u;
+  const uint32_t out_wrap = p.staging_pitch - static_cast<uint32_t>(n_chunks) * 16u;
+
+  auto epilogue = [&](int i) {
+    const int unit = first + i * stride;
+    int matrix, row0;
+    if (p.matrices == 1) {
+      matrix = p.div_row_tiles.div(unit);
+      row0 = (unit - matrix * p.row_tiles) * kRows + my_row;
+    } else {
+      matrix = unit * p.matrices + my_matrix;
+      row0 = my_row;
+    }
+    const int rows = matrix < p.batch ? min(32, p.m - row0) : 0;
+    if (rows <= 0) return;
+    const uint32_t t = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) +
+                       static_cast<uint32_t>(p.matrices > 1 ? my_matrix * p.n : 0);
+    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
+      uint32_t r[32];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c0 + j < n_chunks) tmem_ld_32x8(t + (c0 + j) * 8, r + 8 * j);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c0 + j < n_chunks) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
+          if (p.bias != nullptr) {
+            const float4* b4 = reinterpret_cast<const float4*>(smem_bias + (c0 + j) * 8);
+            const float4 lo = b4[0], hi = b4[1];
+            v[0] += lo.x;
+            v[1] += lo.y;
+            v[2] += lo.z;
+            v[3] += lo.w;
+            v[4] += hi.x;
+            v[5] += hi.y;
+            v[6] += hi.z;
+            v[7] += hi.w;
+          }
+          *reinterpret_cast<uint4*>(staging + lane * p.staging_pitch + (c0 + j) * 16) =
+              make_uint4(pack_pair<BF16>(v[0], v[1]), pack_pair<BF16>(v[2], v[3]), pack_pair<BF16>(v[4], v[5]),
+                         pack_pair<BF16>(v[6], v[7]));
+        }
+      }
+    }
+    __syncwarp();
+    // The rows follow one another in `out` without a gap.
+    uint8_t* dst = p.out + ((static_cast<size_t>(matrix) * p.m + row0) * n_chunks + lane) * 16;
+    const int pieces = rows * n_chunks;
+    int c = out_c;
+    const uint8_t* src = staging + out_offset;
+    for (int j = lane; j < pieces; j += 128) {
+      uint4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j + 32 * u < pieces) x[u] = *reinterpret_cast<const uint4*>(src);
+        src += out_step;
+        c += out_c_step;
+        if (c >= n_chunks) {
+          c -= n_chunks;
+          src += out_wrap;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j + 32 * u < pieces) *reinterpret_cast<uint4*>(dst + 512 * u) = x[u];
+      }
+      dst += 2048;
+    }
+  };
+
+#pragma unroll
+  for (int s = 0; s < kStages; ++s) load_unit(s, s);
+
+  int slot = 0;
+  for (int i = 0; i < count; ++i) {
+    // Groups are committed in the order of the units: all but the kStages - 1 newest are in.
+    cp_async_wait<kStages - 1>();
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
+    __syncthreads();  // the unit's operands are in; everyone is done with the accumulator and the staging rows
+    if (warp == 0) {
+      tc_fence_after_sync();
+      if (elect_one() && (p.debug_flags & 1) == 0) {
+        const uint64_t desc_a = operand_desc(smem_u32(packed_smem) + static_cast<uint32_t>(slot) * a_bytes, narrow);
+        const uint64_t desc_b =
+            operand_desc(smem_u32(smem_b) + (p.shared_b ? 0u : static_cast<uint32_t>(slot) * b_bytes), narrow);
+        const int steps = (p.k_chunks + 1) >> 1;
+        for (int ks = 0; ks < steps; ++ks) {
+          const uint32_t kb = static_cast<uint32_t>(ks >> 2), in_block = 2u * static_cast<uint32_t>(ks & 3);
+          umma_f16<1>(tmem_base, desc_a + kb * (a_block >> 4) + in_block, desc_b + kb * (b_block >> 4) + in_block,
+                      p.idesc, ks > 0 ? 1u : 0u);
+        }
+        umma_commit_1cta(bar_done);
+      }
+      __syncwarp();
+      bw.wait(bar_done, static_cast<uint32_t>(i) & 1u, ST_TIMEOUT_FULL);
+    }
+    __syncthreads();
+    tc_fence_after_sync();
+    load_unit(i + kStages, slot);  // the MMAs have read the slot
+    if (++slot == kStages) slot = 0;
+    epilogue(i);
+  }
+
+  cp_async_wait<0>();
+  if (bw.aborted()) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // MMAs still in flight
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after_sync();
+    tmem_dealloc<1>(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+  }
+#endif
+}
+
+constexpr int kSmemPerSm = 233472, kSmemPerCta = 232448, kCtaReserve = 1024;
+
+// As many matrices to a unit as its quarters of 32 rows and its columns hold.
+int matrices_per_unit(int64_t batch, int64_t m, int64_t n) {
+  int matrices = 1;
+  while (batch > 1 && matrices < 4 && m * matrices * 2 <= kRows && n * matrices * 2 <= kPackedMaxN) matrices *= 2;
+  return matrices;
+}
+
+}  // namespace
+
+cudaError_t init_packed_gemm() {
+  const cudaError_t err = cudaFuncSetAttribute(reinterpret_cast<const void*>(&packed_gemm_kernel<false>),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+  if (err != cudaSuccess) return err;
+  return cudaFuncSetAttribute(reinterpret_cast<const void*>(&packed_gemm_kernel<true>),
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+}
+
+// Where this kernel is the faster one (us, general -> packed; 88 shapes of up to 128 columns and a depth of up to
+// 128 measured):
+//  * from one 128-row tile per SM on; below, both are a launch and one pass (bmm 8 x 1024x64x64 2.8 -> 3.5);
+//  * matrices that share an accumulator: 574 x 15x16x32 5.4 -> 2.6, 1024 x 64x64x64 8.7 -> 7.3;
+//  * rows shorter than the general kernel's 64-deep boxes: 200704x96x48 21.6 -> 15.5.  Not with rows of exactly 32
+//    against more than 64 columns of a bmm, whose outputs dominate: 512 x 128x128x32 7.8 -> 9.1;
+//  * few columns: 1698 x 118x24x104 17.4 -> 14.5, 100352x48x96 11.1 -> 9.8; with more columns and a depth of 64 and
+//    above two CTAs or one fit an SM and the general kernel wins: 89 x 509x128x64 6.3 -> 8.6, 1412 x 61x128x72
+//    19.5 -> 28.0;
+//  * rows that start in the middle of a 32-byte sector cost the general kernel's TMA loads twice, which one B for
+//    all units makes up for up to 96 columns: 153121x88x72 29.0 -> 16.1.
+bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count) {
+  if (n > kPackedMaxN || k > kPackedMaxK) return false;
+  const int64_t tiles = batch * ((m + kRows - 1) / kRows);
+  if (tiles < sm_count || tiles > 0x7FFFFFFF) return false;
+  if (matrices_per_unit(batch, m, n) > 1 || n <= 48) return true;
+  if (k < 64) return k != 32 || n <= 64 || batch == 1;
+  return batch == 1 && k % 16 != 0 && n <= 96;
+}
+
+cudaError_t launch_packed_gemm(const PackedProblem& pr) {
+  PackedParams p = {};
+  p.a = static_cast<const uint8_t*>(pr.a);
+  p.b = static_cast<const uint8_t*>(pr.b);
+  p.bias = pr.bias;
+  p.out = static_cast<uint8_t*>(pr.out);
+  p.batch = static_cast<int>(pr.batch);
+  p.m = static_cast<int>(pr.m);
+  p.n = static_cast<int>(pr.n);
+  p.k_chunks = static_cast<int>(pr.k / 8);
+  p.k_blocks = static_cast<int>((pr.k + 63) / 64);
+  p.matrices = matrices_per_unit(pr.batch, pr.m, pr.n);
+  p.slot_rows = kRows / p.matrices;
+  p.row_tiles = (p.m + kRows - 1) / kRows;
+  p.units = p.matrices == 1 ? p.batch * p.row_tiles : (p.batch + p.matrices - 1) / p.matrices;
+  p.mma_n = (p.n * p.matrices + 15) / 16 * 16;
+  p.shared_b = p.batch == 1 ? 1 : 0;
+  p.narrow = pr.k <= 16 ? 2 : pr.k <= 32 ? 1 : 0;
+  p.idesc = pr.idesc_base | (static_cast<uint32_t>(p.mma_n >> 3) << 17);
+  // An odd number of 16-byte pieces per staging row: eight lanes writing a piece of eight rows meet eight banks.
+  p.staging_pitch = 16u * static_cast<uint32_t>((p.n / 8) | 1);
+  p.load_rows = kThreads / p.k_chunks;
+  p.load_threads = p.load_rows * p.k_chunks;
+  p.div_k_chunks = FastDiv::make(static_cast<uint32_t>(p.k_chunks));
+  p.div_n_chunks = FastDiv::make(static_cast<uint32_t>(p.n / 8));
+  p.div_row_tiles = FastDiv::make(static_cast<uint32_t>(p.row_tiles));
+  p.status = pr.status;
+  p.timeout_ns = pr.timeout_ns;
+  p.debug_flags = pr.debug_flags;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < p.mma_n) p.tmem_cols *= 2;
+
+  const int a_bytes = (p.k_blocks * kRows * 128) >> p.narrow, b_bytes = (p.k_blocks * p.mma_n * 128) >> p.narrow;
+  const int fixed = kRows * static_cast<int>(p.staging_pitch) + kPackedMaxN * 4 + 64;
+  const int smem = kStages * a_bytes + (p.shared_b ? 1 : kStages) * b_bytes + fixed;
+  int ctas = kSmemPerSm / (smem + kCtaReserve);
+  if (ctas > kMaxCtasPerSm) ctas = kMaxCtasPerSm;
+  const int64_t room = static_cast<int64_t>(ctas) * pr.sm_count;
+
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.units < room ? p.units : room));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = pr.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pr.overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, pr.is_bf16 ? packed_gemm_kernel<true> : packed_gemm_kernel<false>, p);
+}
+
+}  // namespace ayla_b200

@@ -230,7 +230,11 @@ class GemmLauncher:
         index = device.index if device.index is not None else torch.cuda.current_device()
         with torch.cuda.device(index):
             _lib.init(index)
-        need = _lib.workspace_bytes(self.config, operation, batch, m, n, k)
+        # Many small or thin products run on a kernel of their own, which the library takes for them where it is
+        # given no schedule.
+        self._packed = (activation == "none" and not gated and
+                        _lib.packed_preferred(operation, batch, m, n, k))
+        need = 0 if self._packed else _lib.workspace_bytes(self.config, operation, batch, m, n, k)
         self._ws_bytes = need
         self.workspace = torch.zeros(need, dtype=torch.uint8, device=device) if need else None
         self.status = _lib.StatusWord()
@@ -247,7 +251,7 @@ class GemmLauncher:
         lib = _lib.load()
         self._entry = lib.ayla_b200_gemm_act_rowmul if gated == "row" else lib.ayla_b200_gemm_act_mul
         self._head = (_lib.OP_CODES[operation], _lib.DTYPE_CODES[dtype], _lib.ACT_CODES[activation])
-        self._tail = (batch, m, n, k, ctypes.byref(self.config), self._ws_ptr or None,
+        self._tail = (batch, m, n, k, None if self._packed else ctypes.byref(self.config), self._ws_ptr or None,
                       self.workspace.numel() if self.workspace is not None else 0, self._status_ptr)
         self._has_bias = operation == "addmm"
         self._device_index = index

@@ -207,6 +207,21 @@ AYLA_B200_API int ayla_b200_gemm_static_scratch(int op, int dtype, const void* b
                                                 uint32_t* status, void* stream);
 
 /*
+ * ayla_b200_gemm through the kernel for few columns and a shallow depth (n <= 128, k <= 128; otherwise
+ * AYLA_B200_E_UNSUPPORTED): needs no schedule and no workspace.  Several small matrices of a bmm share
+ * one 128-row accumulator.
+ */
+AYLA_B200_API int ayla_b200_gemm_packed(int op, int dtype, const void* bias, const void* a, const void* bt, void* out,
+                                        int64_t batch, int64_t m, int64_t n, int64_t k, uint32_t* status,
+                                        void* stream);
+
+/*
+ * 1 where ayla_b200_gemm_packed is the faster way to run the problem, else 0: there ayla_b200_gemm takes
+ * it by itself when cfg == NULL.
+ */
+AYLA_B200_API int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k);
+
+/*
  * out[M,N] = silu(x[M,K] @ w_gate[N,K]^T) * (x @ w_up[N,K]^T), both products kept
  * in fp32 until one final rounding.  One kernel, one pass over x; the
  * intermediates never reach HBM.  New op; its precedent is the reference's fused
@@ -228,7 +243,7 @@ AYLA_B200_API int ayla_b200_rms_factors(int dtype, const void* x, void* factors,
                                         void* stream);
 
 /*
- * The schedule ayla_b200_gemm uses when cfg == NULL.  Counterpart of
+ * The schedule ayla_b200_gemm uses when cfg == NULL (and ayla_b200_packed_preferred() is 0).  Counterpart of
  * select_gemm_schedule's fallback (ayla/gemm_jit.py:225-264).
  */
 AYLA_B200_API int ayla_b200_default_config(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,

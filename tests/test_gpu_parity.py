@@ -515,6 +515,73 @@ def test_rms_norm_linear_refuses_what_the_projection_refuses():
     assert torch.equal(rms_norm_linear(y, w), rms_norm_linear(x, w))
 
 
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize(
+    "operation, batch, m, n, k",
+    [
+        # one matrix per accumulator: one row, row tiles with remainders, every operand swizzle, odd depths in
+        # 16-byte pieces, the most columns and depth, several units per CTA
+        ("mm", 1, 1, 8, 8), ("addmm", 1, 129, 24, 24), ("mm", 1, 257, 128, 128), ("addmm", 1, 300, 120, 40),
+        ("mm", 1, 128, 104, 120), ("addmm", 1, 90001, 16, 16), ("mm", 1, 150003, 96, 72),
+        ("bmm", 3, 65, 128, 72), ("bmm", 2, 200, 56, 16), ("bmm", 700, 100, 40, 104), ("bmm", 1, 70, 32, 48),
+        # two and four, the last unit partly filled
+        ("bmm", 5, 64, 64, 128), ("bmm", 3, 33, 40, 8), ("bmm", 2049, 56, 32, 56), ("bmm", 3, 8, 48, 32),
+        ("bmm", 7, 32, 32, 16), ("bmm", 6, 1, 8, 24), ("bmm", 4001, 17, 24, 40),
+    ])
+def test_packed_kernel_equals_the_general_one(operation, batch, m, n, k, dtype):
+    """Both add the same products in the same order in fp32 and round once: every bit is the same."""
+    _lib.init(0)
+    g = torch.Generator(device=DEV).manual_seed(m * n + k)
+    lead = (batch,) if operation == "bmm" else ()
+    a = torch.randn(*lead, m, k, device=DEV, generator=g).to(TD[dtype])
+    bt = torch.randn(*lead, n, k, device=DEV, generator=g).to(TD[dtype])
+    bias = torch.randn(n, device=DEV, generator=g).to(TD[dtype])
+    guard = 64
+    out = torch.full((batch * m * n + guard,), 7.0, dtype=TD[dtype], device=DEV)
+    want = torch.empty(*lead, m, n, dtype=TD[dtype], device=DEV)
+    status = _lib.StatusWord()
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.gemm_packed(operation, dtype, bias.data_ptr(), a.data_ptr(), bt.data_ptr(), out.data_ptr(), batch, m, n, k,
+                     status.ptr, stream)
+    _lib.gemm(operation, dtype, bias.data_ptr(), a.data_ptr(), bt.data_ptr(), want.data_ptr(), batch, m, n, k,
+              _lib.Config.from_dict(dict(tile_n=64)), 0, 0, status.ptr, stream)
+    torch.cuda.synchronize()
+    assert status.peek() == 0
+    assert torch.equal(out[:-guard].view_as(want), want)
+    assert bool((out[-guard:] == 7.0).all())
+
+
+def test_packed_kernel_through_the_ops_and_its_limits():
+    a = torch.randn(300, 32, 24, device=DEV).half()
+    bt = torch.randn(300, 16, 24, device=DEV).half()
+    out = torch.empty(300, 32, 16, device=DEV, dtype=torch.float16)
+    gemm_op("bmm", "float16")(a, bt, out)
+    launcher = gemm_op_compiler("bmm", "float16")._launcher((a, bt, out))
+    assert launcher._packed
+    assert_parity(out.cpu(), O.bmm_ref32(a.cpu(), bt.cpu()), "packed bmm through the op")
+    with pytest.raises(ValueError, match="n <= 128"):
+        _lib.gemm_packed("mm", "float16", 0, a.data_ptr(), bt.data_ptr(), out.data_ptr(), 1, 8, 136, 64, 0, 0)
+    # Infinities and NaN stay in their own matrix.
+    a[7, 3, 5] = float("inf")
+    bt[9, 2, 1] = float("nan")
+    gemm_op("bmm", "float16")(a, bt, out)
+    bad = ~torch.isfinite(out)
+    assert bool(bad[7, 3].all()) and bool(bad[9, :, 2].all()) and int(bad.sum()) == 16 + 32
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(30)
+        lib.ayla_b200_debug_set_flags(1)
+        launcher(a, bt, out)            # the MMAs are withheld: the wait for them runs out
+        torch.cuda.synchronize()
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    with pytest.raises(RuntimeError, match="timed out"):
+        launcher(a, bt, out)
+    launcher(a, bt, out)
+    launcher.check_status()
+
+
 def test_gemm_act_mul_op_matches_the_oracle():
     from ayla_b200 import gemm_act_mul_op
 
