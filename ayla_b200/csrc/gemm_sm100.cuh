@@ -770,6 +770,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       cluster_arrive_relaxed();
       cluster_wait();
     }
+    if (CG == 1 && csk > 0) cluster_arrive_relaxed();  // the exit barrier, see the teardown
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
     if (is_leader) {
@@ -893,6 +894,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       cluster_arrive_relaxed();
       cluster_wait();
     }
+    if (CG == 1 && csk > 0) cluster_arrive_relaxed();
   } else {
     // ---------------------------------------------------------------- epilogue
     // Eight warps: warp w may read TMEM lanes [32 * (w % 4), +32), so two warps share
@@ -1189,6 +1191,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #ifdef AYLA_B200_TRACE
           if (stamps != nullptr && warp == 2 && lane == 0) trace_stamp(stamps, 15);
 #endif
+          if constexpr (CG == 1) cluster_arrive_relaxed();  // the exit barrier: this warp has sent all it sends
           // The partials of this CTA's columns have all landed when the inbox barrier completes.
           bw.wait(bar_inbox, 0, ST_TIMEOUT_INBOX);
 #ifdef AYLA_B200_TRACE
@@ -1538,6 +1541,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
+  // No CTA of a k-split cluster leaves while another may still send into its inbox.  In the ordinary course its own
+  // inbox barrier has told it that all sends are in; a CTA whose waits ran out has given up on that, and a peer that
+  // gives up later would write into the shared memory of a CTA that has left.  Every warp arrived when it had sent.
+  if (CG == 1 && csk > 0) cluster_wait();
   if constexpr (CG == 2) {
     // The leader's MMAs write the peer's TMEM and both CTAs' barriers: neither
     // CTA may free TMEM or exit before both are done.  Nothing is published by this meeting:

@@ -864,6 +864,31 @@ def test_timed_out_split_k_launch_is_reported_by_the_next_call_without_the_debug
     assert_parity(out, O.mm_ref32(a, bt), "k-split launch after a reported timeout")
 
 
+@pytest.mark.parametrize("config", [
+    dict(tile_n=64, cta_group=1, split_k=2), dict(tile_n=128, cta_group=1, split_k=4),
+    dict(tile_n=64, cta_group=2, split_k=2), dict(tile_n=16, cta_group=1, swap_ab=1, split_k=4, group_m=1)])
+def test_timed_out_cluster_split_leaves_the_context_usable(config, device_state):
+    """A cluster k-split whose loads are withheld: every CTA gives up in its own time, and none leaves while
+    another may still send partial sums into its shared memory."""
+    m, n, k = (8 if config.get("swap_ab") else 512), 1024, 2048
+    g = torch.Generator().manual_seed(4)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+    config = dict(config, cluster_split=1)
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(20)
+        lib.ayla_b200_debug_set_flags(1)
+        _, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    assert status & 0xFF != 0
+    out, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    assert status == 0
+    assert_parity(out, O.mm_ref32(a, bt), f"after a timed-out cluster split {config}")
+
+
 def test_random_shapes_through_the_public_ops():
     """Schedule selection on shapes nobody measured: transferred table entries (trimmed tiles, 192-wide
     tiles, cluster k-splits, eviction hints) and the default heuristic must all stay correct on ragged
