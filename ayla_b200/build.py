@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -46,6 +47,31 @@ def _newest_header() -> float:
 
 
 TRACE_LIB_PATH = LIB_DIR / "libayla_b200_trace.so"
+
+
+DISPATCH_SOURCE = CSRC / "torch_dispatch.cpp"
+DISPATCH_PATH = LIB_DIR / "_torch_dispatch.so"
+
+
+def build_dispatch(verbose: bool = False, force: bool = False) -> Path:
+    if not force and DISPATCH_PATH.exists() and DISPATCH_PATH.stat().st_mtime >= DISPATCH_SOURCE.stat().st_mtime:
+        return DISPATCH_PATH
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    LIB_DIR.mkdir(exist_ok=True)
+    includes = [*include_paths(), "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[f"-isystem{path}" for path in includes], str(DISPATCH_SOURCE), "-o", str(DISPATCH_PATH),
+           *[f"-L{path}" for path in library_paths()],
+           "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or proc.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
+    if proc.returncode != 0:
+        raise RuntimeError(f"building {DISPATCH_PATH.name} failed")
+    return DISPATCH_PATH
 
 
 def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, trace: bool = False) -> Path:
@@ -89,6 +115,8 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
         or not lib_path.exists()
         or lib_path.stat().st_mtime < max(os.stat(o).st_mtime for o in objects)
     )
+    if not trace:
+        build_dispatch(verbose, force)
     if relink:
         cmd = [
             nvcc, "-shared", "-o", str(lib_path), *objects,

@@ -137,10 +137,18 @@ int encode_map(CUtensorMap* out, const void* ptr, uint64_t d0, uint64_t d1, uint
   const cuuint64_t strides[2] = {d0 * 2, d0 * d1 * 2};
   const cuuint32_t box[3] = {b0, b1, b2};
   const cuuint32_t elem_strides[3] = {1, 1, 1};
-  const CUresult r = g_encode_tiled(
-      out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box,
-      elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return g_encode_tiled(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box,
+                          elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread's first CUDA call may be this one, which wants a current context: selecting the current
+    // device makes its primary context current.
+    int device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     return fail(AYLA_B200_E_CUDA,
                 "cuTensorMapEncodeTiled failed (%d) for ptr=%p dims=[%llu,%llu,%llu] box=[%u,%u,%u]",

@@ -286,6 +286,24 @@ class GemmLauncher:
         if self._debug:
             self.check_status()
 
+    def native_call(self) -> dict[str, object] | None:
+        """What the compiled dispatcher needs to repeat this launch on its home stream; ``None`` where every launch
+        is to be checked (``AYLA_B200_DEBUG``)."""
+        if self._debug:
+            return None
+        import ctypes
+
+        op, dtype, activation = self._head
+        return {
+            "entry": ctypes.cast(self._entry, ctypes.c_void_p).value, "swiglu": False,
+            "op": op, "dtype": dtype, "activation": activation,
+            "has_bias": self._has_bias, "gated": bool(self.gated),
+            "batch": self.batch, "m": self.m, "n": self.n, "k": self.k,
+            "config": 0 if self._packed else ctypes.addressof(self.config),
+            "workspace": self._ws_ptr, "workspace_bytes": self._ws_bytes,
+            "status": self._status_ptr, "home_stream": self._home_stream or 0, "device": self._device_index,
+        }
+
     def _tail_for_stream(self, stream: int) -> tuple:
         """The call arguments with the workspace that belongs to ``stream`` (allocated on first use)."""
         entry = self._per_stream.get(stream)

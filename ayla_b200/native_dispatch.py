@@ -1,0 +1,55 @@
+"""The compiled CUDA kernels of the torch ops (``csrc/torch_dispatch.cpp``).
+
+An op registered here runs without entering Python whenever its shapes have been specialised; everything else
+-- an unseen shape, refused operands, a reported timeout, another stream's workspace -- goes to the Python
+fallback it was registered with.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import importlib.util
+from collections.abc import Callable
+from functools import cache
+from pathlib import Path
+from types import ModuleType
+
+import torch
+
+from . import _lib
+
+_PATH = Path(__file__).resolve().parent / "lib" / "_torch_dispatch.so"
+
+
+@cache
+def load() -> ModuleType:
+    if not _PATH.exists():
+        raise ImportError(f"{_PATH} not found: build it with `python -m ayla_b200.build`")
+    spec = importlib.util.spec_from_file_location("_torch_dispatch", _PATH)
+    assert spec is not None and spec.loader is not None
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+def register(namespace: str, name: str, compiler) -> None:
+    """Register the CUDA kernel of ``namespace::name``, backed by a ``ShapeSpecializingJITCompiler`` whose
+    operands are the op's arguments."""
+    [dtype] = {spec.dtype for spec in compiler.signature}
+    dispatcher = None
+
+    def fallback(*tensors: torch.Tensor) -> None:
+        compiler(*tensors)
+        launcher = compiler._launcher(tensors)
+        native_call: Callable[[], dict | None] | None = getattr(launcher, "native_call", None)
+        fields = native_call() if native_call is not None else None
+        if fields is not None:
+            dispatcher.insert(list(tensors), launcher, fields)
+
+    dispatcher = load().register_op(namespace, name, len(compiler.signature), dtype, fallback)
+
+
+def register_rms_factors(namespace: str, name: str, dtype: str, torch_dtype: torch.dtype, fallback) -> None:
+    """Register the CUDA kernel of the row-factors op ``(x, eps, factors) -> ()``."""
+    entry = ctypes.cast(_lib.load().ayla_b200_rms_factors, ctypes.c_void_p).value
+    load().register_rms_factors(namespace, name, entry, _lib.DTYPE_CODES[dtype], torch_dtype, fallback)

@@ -14,7 +14,7 @@ from functools import cache
 
 import torch
 
-from . import _lib
+from . import _lib, native_dispatch
 from .gemm_jit import _SHORT_DTYPES, _TORCH_DTYPES, gemm_act_rowmul_op
 from .torch_custom_call import DEFAULT_NAMESPACE, _library
 
@@ -48,7 +48,7 @@ def _row_factors_op(dtype: str) -> torch._ops.OpOverload:
 
     lib = _library(DEFAULT_NAMESPACE)
     lib.define(f"{name}(Tensor arg0, float eps, Tensor(a1!) arg1) -> ()")
-    lib.impl(name, cuda_impl, "CUDA")
+    native_dispatch.register_rms_factors(DEFAULT_NAMESPACE, name, dtype, _TORCH_DTYPES[dtype], cuda_impl)
     lib.impl(name, lambda x, eps, factors: None, "Meta")
     return getattr(getattr(torch.ops, DEFAULT_NAMESPACE), name).default
 

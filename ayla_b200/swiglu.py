@@ -44,6 +44,21 @@ class SwigluLauncher:
         if self._debug:
             self.check_status()
 
+    def native_call(self) -> dict[str, object] | None:
+        """What the compiled dispatcher needs to repeat this launch; ``None`` where every launch is to be checked."""
+        if self._debug:
+            return None
+        import ctypes
+
+        return {
+            "entry": ctypes.cast(_lib.load().ayla_b200_swiglu, ctypes.c_void_p).value, "swiglu": True,
+            "op": 0, "dtype": _lib.DTYPE_CODES[self.dtype], "activation": 0, "has_bias": False, "gated": False,
+            "batch": 1, "m": self.m, "n": self.n, "k": self.k,
+            "config": ctypes.addressof(self.config) if self.config is not None else 0,
+            "workspace": 0, "workspace_bytes": 0,
+            "status": self._status_ptr, "home_stream": 0, "device": self._device_index,
+        }
+
     def _report_timeout(self) -> None:
         code = self.status.peek()
         self.status.clear()
