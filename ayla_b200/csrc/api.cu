@@ -47,6 +47,7 @@ struct Registry {
     append_variants_trans(entries, &count);
     append_variants_swiglu(entries, &count);
     base_count = count;
+    append_variants_swiglu_trans(entries, &count);
     append_variants_act_cg1(entries, &count);
     append_variants_act_cg2(entries, &count);
     append_variants_act_trans(entries, &count);
@@ -291,14 +292,15 @@ constexpr size_t kCounterBytes = static_cast<size_t>(kMaxSplitKTiles) * 4;
 int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t rows, int64_t cols,
               int64_t k, int sm_count, Plan* plan, int activation = 0) {
   const int transposed = c.swap_ab ? 1 : 0;
-  const int tile_n = (epilogue == EPI_SWIGLU) ? 256 : c.tile_n;
+  const bool swiglu_cols = epilogue == EPI_SWIGLU && !c.swap_ab;
+  const int tile_n = swiglu_cols ? 256 : c.tile_n;
   const int lean = (c.split_k <= 1 && c.stream_k == 0) ? 1 : 0;
   const KernelEntry* e = registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, lean);
   if (e == nullptr) {
     return fail(AYLA_B200_E_UNSUPPORTED, "no kernel variant tile_n=%d cta_group=%d epilogue=%d swap=%d",
                 tile_n, c.cta_group, epilogue, transposed);
   }
-  const int out_tile_n = (epilogue == EPI_SWIGLU) ? 128 : tile_n;
+  const int out_tile_n = swiglu_cols ? 128 : tile_n;
   plan->kernel = e;
   plan->tile_rows = (c.swap_ab && c.tile_rows > 0) ? c.tile_rows : 128;
   plan->m_tiles = static_cast<int>(ceil_div(rows, c.swap_ab ? plan->tile_rows : 128 * c.cta_group));
@@ -553,6 +555,45 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count
   if (ceil_div(m, 128 * c->cta_group) > c->group_m) c->l2_hint_b = 2;
 }
 
+// The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
+// leave 32 of them working at n = 4096): 64 output columns per tile, M on the narrow accumulator, k split across
+// a cluster, all in one wave.  False where no such schedule exists; where one does it measured the faster (us,
+// row-major -> swapped: 8x1024x4096 25.0 -> 6.5, 8x4096x4096 26.7 -> 13.0, 64x8192x4096 30.4 -> 24.3,
+// 128x4096x4096 27.9 -> 17.9, 512x1024x4096 23.5 -> 15.6, 1024x1024x4096 24.1 -> 21.9; in more than one wave it
+// loses: 64x14336x4096 41.7 -> 42.6, 769x1472x3008 20.0 -> 29.4).
+bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b200_config* c) {
+  // us per k-block and per cluster exchange, fitted to the same measurements.
+  struct Width { int tile_n; double per_kb, exchange2, exchange4; };
+  static const Width kWidths[4] = {{16, 0.160, 0.9, 1.4}, {32, 0.170, 0.9, 1.4}, {64, 0.20, 1.5, 3.0}, {128, 0.28, 2.7, 4.6}};
+  const int64_t k_blocks = ceil_div(k, 64), row_tiles = ceil_div(n, 64);
+  double best = 1e300;
+  for (const Width& w : kWidths) {
+    const int64_t tiles = row_tiles * ceil_div(m, w.tile_n);
+    for (int split = 1; split <= 4; split *= 2) {
+      if (tiles * split > sm_count || (split > 1 && k_blocks < 4 * split)) break;
+      const double cost = static_cast<double>(ceil_div(k_blocks, split)) * w.per_kb +
+                          (split == 1 ? 0.0 : split == 2 ? w.exchange2 : w.exchange4);
+      if (cost < best && static_cast<int64_t>(split - 1) * ceil_div(k_blocks, split) < k_blocks) {
+        best = cost;
+        c->tile_n = w.tile_n;
+        c->split_k = split;
+      }
+    }
+  }
+  if (best == 1e300) return false;
+  c->swap_ab = 1;
+  c->cta_group = 1;
+  c->group_m = 1;
+  c->tile_rows = 64;
+  c->cluster_split = c->split_k > 1 ? 1 : 0;
+  c->l2_hint_a = 2;
+  c->l2_hint_b = 1;
+  // The weights' first blocks are asked into L2 under the preceding launch's tail (8x4096x4096 13.6 -> 13.0).
+  const int64_t share = k_blocks / c->split_k / 2;
+  c->early_prefetch = m > 64 ? 0 : static_cast<int>(share < 8 ? share : 8);
+  return true;
+}
+
 int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, int is_bf16,
                 const void* bias, const void* b2_operand, void* out, int64_t out_rows,
                 int64_t out_cols, void* workspace, size_t workspace_bytes, uint32_t* status,
@@ -560,7 +601,9 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
   const KernelEntry& e = *plan.kernel;
   LaunchArgs la;
   memset(&la, 0, sizeof(la));
-  int b_box_rows = (e.epilogue == EPI_SWIGLU) ? 128 : e.tile_n / e.cta_group;
+  const bool swiglu_cols = e.epilogue == EPI_SWIGLU && !e.transposed_out;
+  const bool swiglu_rows = e.epilogue == EPI_SWIGLU && e.transposed_out;
+  int b_box_rows = swiglu_cols ? 128 : e.tile_n / e.cta_group;
   int b_stage_rows = e.tile_n / e.cta_group;  // rows of the column operand one CTA receives per stage
   int a_box_rows = plan.tile_rows;
   // An operand that fits in a single tile is loaded with a box of just its own rows (rounded
@@ -572,7 +615,7 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
     const int rows8 = static_cast<int>(ceil_div(pr.rows, 8) * 8);
     const int cols8 = static_cast<int>(ceil_div(pr.cols, 8) * 8);
     if (plan.m_tiles == 1 && rows8 < a_box_rows) a_box_rows = rows8;
-    if (plan.n_tiles == 1 && e.epilogue != EPI_SWIGLU && plan.narrow_from_tile == 0x7FFFFFFF && cols8 < b_box_rows) {
+    if (plan.n_tiles == 1 && !swiglu_cols && plan.narrow_from_tile == 0x7FFFFFFF && cols8 < b_box_rows) {
       b_box_rows = cols8;
       b_stage_rows = cols8;
     }
@@ -582,7 +625,8 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
   rc = encode_map(&la.tm_b, pr.col_operand, pr.k, pr.cols, pr.batch, 64, b_box_rows, 1);
   if (rc) return rc;
   if (e.epilogue == EPI_SWIGLU) {
-    rc = encode_map(&la.tm_b2, b2_operand, pr.k, pr.cols, pr.batch, 64, b_box_rows, 1);
+    rc = swiglu_rows ? encode_map(&la.tm_b2, b2_operand, pr.k, pr.rows, pr.batch, 64, a_box_rows, 1)
+                     : encode_map(&la.tm_b2, b2_operand, pr.k, pr.cols, pr.batch, 64, b_box_rows, 1);
     if (rc) return rc;
   } else {
     la.tm_b2 = la.tm_b;
@@ -672,7 +716,7 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
   p.mul_per_row = mul_per_row;
   // One stage receives this CTA's rows of the row operand and its share of the column
   // operand; the leader of a pair counts both CTAs' bytes.
-  p.stage_tx = static_cast<uint32_t>((a_box_rows + b_stage_rows) * 128 * e.cta_group);
+  p.stage_tx = static_cast<uint32_t>((a_box_rows * (swiglu_rows ? 2 : 1) + b_stage_rows) * 128 * e.cta_group);
   if (plan.slabs > 0) {
     const size_t need = workspace_bytes_for(plan);
     if (workspace == nullptr || workspace_bytes < need) {
@@ -1071,30 +1115,36 @@ int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate, const void* w
   int dev = -1;
   rc = current_device_state(&ds, &dev);
   if (rc) return rc;
+  bool swapped = false;
   ayla_b200_config c;
   if (cfg != nullptr) {
     c = *cfg;
   } else {
     memset(&c, 0, sizeof(c));
-    c.cta_group = (m >= 256) ? 2 : 1;
-    c.group_m = 8;
-    c.l2_hint_a = 2;  // x is re-read by every column tile,
-    c.l2_hint_b = 1;  // the weights stream through once
+    swapped = swapped_swiglu_config(m, n, k, ds->sm_count, &c);
+    if (!swapped) {
+      c.cta_group = (m >= 256) ? 2 : 1;
+      c.group_m = 8;
+      c.l2_hint_a = 2;  // x is re-read by every column tile,
+      c.l2_hint_b = 1;  // the weights stream through once
+    }
   }
-  c.tile_n = 256;
-  c.split_k = 1;
-  c.swap_ab = 0;
-  rc = check_config(c, true);
-  if (rc) return rc;
+  if (!swapped) {
+    c.tile_n = 256;
+    c.split_k = 1;
+    c.swap_ab = 0;
+    rc = check_config(c, true);
+    if (rc) return rc;
+  }
   Problem pr;
-  pr.rows = m;
-  pr.cols = n;
+  pr.rows = swapped ? n : m;
+  pr.cols = swapped ? m : n;
   pr.k = k;
   pr.batch = 1;
-  pr.row_operand = x;
-  pr.col_operand = w_gate;
+  pr.row_operand = swapped ? w_gate : x;
+  pr.col_operand = swapped ? x : w_gate;
   Plan plan{};
-  rc = make_plan(c, EPI_SWIGLU, 1, m, n, k, ds->sm_count, &plan);
+  rc = make_plan(c, EPI_SWIGLU, 1, pr.rows, pr.cols, k, ds->sm_count, &plan);
   if (rc) return rc;
   return launch_plan(plan, c, pr, dtype == AYLA_B200_BF16 ? 1 : 0, nullptr, w_up, out, m, n, nullptr, 0,
                      status, reinterpret_cast<cudaStream_t>(stream));

@@ -170,7 +170,11 @@ struct GemmTraits {
   static constexpr int STAGES = STAGES_;
   static constexpr int BM = 128;                // rows per CTA
   static constexpr int BK = 64;                 // one 128-byte swizzle atom of 16-bit elements
-  static constexpr int OUT_BN = (EPI == EPI_SWIGLU) ? BN / 2 : BN;  // output tile width
+  // SwiGLU: row-major, gate and up share the accumulator's columns (2 x 128); swapped, its rows (2 x 64),
+  // `tm_a` then being the gate and `tm_b2` the up weight.
+  static constexpr bool SWIGLU_COLS = EPI == EPI_SWIGLU && !TRANS_OUT;
+  static constexpr bool SWIGLU_ROWS = EPI == EPI_SWIGLU && TRANS_OUT;
+  static constexpr int OUT_BN = SWIGLU_COLS ? BN / 2 : BN;  // output tile width
   static constexpr int B_ROWS = BN / CTA_GROUP; // B rows this CTA loads per stage
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = B_ROWS * BK * 2;
@@ -191,7 +195,9 @@ struct GemmTraits {
                                                              : 512;
   static constexpr int EPI_WARPS = 8;
   static constexpr int STORE_BUF_BYTES = 32 * 128;  // 32 rows x 64 columns of 16-bit
-  static constexpr int STORE_BYTES = TRANS_OUT ? 0 : EPI_WARPS * STORE_BUF_BYTES;
+  // Swapped SwiGLU: where the epilogue warps of the up rows leave 32 columns for those of the gate rows.
+  static constexpr int UP_BUF_BYTES = 32 * 64 * 4;
+  static constexpr int STORE_BYTES = SWIGLU_ROWS ? 2 * UP_BUF_BYTES : TRANS_OUT ? 0 : EPI_WARPS * STORE_BUF_BYTES;
   static constexpr int BIAS_BYTES = (EPI == EPI_BIAS && !TRANS_OUT) ? 2 * BN * 4 : 0;
   static constexpr int MISC_BYTES = 256;
 #ifdef AYLA_B200_TRACE
@@ -205,7 +211,7 @@ struct GemmTraits {
   static constexpr int THREADS = 64 + EPI_WARPS * 32 + 32;
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N extent");
   static_assert(B_BYTES % 1024 == 0, "B slab must keep the 1024-byte swizzle alignment");
-  static_assert(EPI != EPI_SWIGLU || (BN == 256 && !TRANS_OUT), "SwiGLU uses the 2x128 layout");
+  static_assert(!SWIGLU_COLS || BN == 256, "row-major SwiGLU uses the 2x128 layout");
   static_assert(TRANS_OUT || BN >= 64, "the TMA-store epilogue writes 64-column boxes");
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared-memory limit");
   static_assert((2 * STAGES + 2 * ACC_BUFS + 1) * 8 + 16 <= MISC_BYTES, "barrier area too small");
@@ -563,7 +569,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
   // Cluster split-K: the cluster holds `csk` CTAs (CTA pairs when CG == 2), one per k-split
   // of the cluster's tile.
-  const int csk = (T::EPI != EPI_SWIGLU && !T::LEAN) ? p.cluster_split : 0;
+  const int csk = (!T::SWIGLU_COLS && !T::LEAN) ? p.cluster_split : 0;
   constexpr int group = T::KB_PER_SLOT;  // k-blocks per ring slot
   const int n_stages = p.stages;         // ring slots in use
 
@@ -670,16 +676,17 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       if (bw.aborted()) break;
       // A narrow unit needs only the first half of each CTA's B slab; the full box is
       // still loaded (its tail is ignored by the narrower MMA).
-      const int b_row = (T::EPI == EPI_SWIGLU)
+      const int b_row = T::SWIGLU_COLS
                             ? w.n0
                             : w.n0 + static_cast<int>(cta_rank) * (w.is_narrow ? T::B_ROWS / 2 : T::B_ROWS);
-      const int b_batch = (T::EPI == EPI_SWIGLU) ? 0 : w.batch;
+      const int b_batch = T::SWIGLU_COLS ? 0 : w.batch;
       const CUtensorMap* tm_b_mine = &tm_b;
-      if constexpr (T::EPI == EPI_SWIGLU && CG == 2) tm_b_mine = is_leader ? &tm_b : &tm_b2;
+      if constexpr (T::SWIGLU_COLS && CG == 2) tm_b_mine = is_leader ? &tm_b : &tm_b2;
       auto prefetch_l2 = [&](int kb) {
         tma_prefetch_l2_3d(&tm_a, kb * T::BK, w.m0, w.batch);
         tma_prefetch_l2_3d(tm_b_mine, kb * T::BK, b_row, b_batch);
-        if constexpr (T::EPI == EPI_SWIGLU && CG == 1) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, b_row, 0);
+        if constexpr (T::SWIGLU_COLS && CG == 1) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, b_row, 0);
+        if constexpr (T::SWIGLU_ROWS) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, w.m0, 0);
       };
       const int pf = p.l2_prefetch;
       if (!dependency_met) {
@@ -693,10 +700,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           for (int i = 0; i < p.early_prefetch && w.kb0 + i < w.kb1; ++i) {
             if (((slot_count + static_cast<uint32_t>(i / group)) & 1u) != prod_id) continue;
             const int kb = w.kb0 + i;
-            if (p.early_operands & 1) tma_prefetch_l2_3d(&tm_a, kb * T::BK, w.m0, w.batch);
+            if (p.early_operands & 1) {
+              tma_prefetch_l2_3d(&tm_a, kb * T::BK, w.m0, w.batch);
+              if constexpr (T::SWIGLU_ROWS) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, w.m0, 0);
+            }
             if (p.early_operands & 2) {
               tma_prefetch_l2_3d(tm_b_mine, kb * T::BK, b_row, b_batch);
-              if constexpr (T::EPI == EPI_SWIGLU && CG == 1) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, b_row, 0);
+              if constexpr (T::SWIGLU_COLS && CG == 1) tma_prefetch_l2_3d(&tm_b2, kb * T::BK, b_row, 0);
             }
           }
         }
@@ -739,7 +749,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 const uint32_t sb = sa + T::A_BYTES;
                 const int k0 = (kb + g) * T::BK;
                 tma_load_3d<CG>(sa, &tm_a, full_bar, k0, w.m0, w.batch, pol_a);
-                if constexpr (T::EPI == EPI_SWIGLU && CG == 1) {
+                // Rows [0, 64) of the slab = gate, [64, 128) = up.
+                if constexpr (T::SWIGLU_ROWS) tma_load_3d<CG>(sa + T::A_BYTES / 2, &tm_b2, full_bar, k0, w.m0, 0, pol_a);
+                if constexpr (T::SWIGLU_COLS && CG == 1) {
                   // Accumulator columns [0,128) = gate, [128,256) = up.
                   tma_load_3d<CG>(sb, &tm_b, full_bar, k0, b_row, 0, pol_b);
                   tma_load_3d<CG>(sb + T::B_BYTES / 2, &tm_b2, full_bar, k0, b_row, 0, pol_b);
@@ -905,6 +917,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int wsub = (warp - 2) >> 2;                // 0 / 1: which 64-column groups
     const int epi_tid = (warp - 2) * 32 + lane;      // 0..255
     const int row_in_tile = q * 32 + lane;
+    const bool up_rows = T::SWIGLU_ROWS && q >= 2;  // this warp's accumulator rows belong to the up weight
     const int is_bf16 = p.is_bf16;
     const int act = T::ACT ? p.act : static_cast<int>(ACT_NONE);
     uint8_t* my_store = smem_store + (warp - 2) * T::STORE_BUF_BYTES;
@@ -953,7 +966,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // Rows of the tile that exist: the matrix may end inside it, and the swapped form may
       // give a tile fewer than 128 rows.
       const int row_end = T::TRANS_OUT ? min(p.m, w.m0 + p.tile_rows) : p.m;
-      const bool rows_live = (w.m0 + q * 32) < row_end;
+      // Swapped SwiGLU: the warps of one chunk meet at a barrier, so they go through it together.
+      const bool rows_live = T::SWIGLU_ROWS || (w.m0 + q * 32) < row_end;
       const int unit_chunks = w.is_narrow ? CHUNKS32 / 2 : CHUNKS32;
       const int unit_groups = (unit_chunks + 1) / 2;
 
@@ -1029,6 +1043,22 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       auto finish_chunk = [&](float (&v)[32], int c32) {
         if constexpr (T::TRANS_OUT) {
           // Kernel rows are output columns: out[batch][col][row].
+          if constexpr (T::SWIGLU_ROWS) {
+            // The up rows' warps hand their values to the gate rows' (both of the same chunk and half of the
+            // epilogue warps); the second meeting frees the buffer for the next chunk.
+            float* up = reinterpret_cast<float*>(smem_store + wsub * T::UP_BUF_BYTES) + (row_in_tile & 63);
+            if (up_rows) {
+#pragma unroll
+              for (int j = 0; j < CHUNK_COLS; ++j) up[j * 64] = v[j];
+            }
+            named_bar_sync(4 + wsub, 128);
+            if (!up_rows) {
+#pragma unroll
+              for (int j = 0; j < CHUNK_COLS; ++j) v[j] = silu_mul(v[j], up[j * 64]);
+            }
+            named_bar_sync(4 + wsub, 128);
+            if (up_rows) return;
+          }
           const int row = w.m0 + row_in_tile;
           float bias_v = 0.0f;
           if constexpr (T::EPI == EPI_BIAS) {
@@ -1119,7 +1149,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         // owner's inbox barrier with its bytes; an owner waits for that barrier alone, adds
         // the S partials in split order and stores.  Nobody waits for a sender's stores but
         // their receiver.
-        if constexpr (T::EPI != EPI_SWIGLU) {
+        if constexpr (!T::SWIGLU_COLS) {
           const int slice_cols = BN / csk;
           const int slice_shift = __ffs(slice_cols) - 1;
           const int slice_c4 = slice_cols >> 2;
@@ -1304,6 +1334,21 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
               const int col = w.n0 + csk_rank * slice_cols + c4 * 4;
               if (col < p.n) {
                 float v4[4] = {sum.x, sum.y, sum.z, sum.w};
+                if constexpr (T::SWIGLU_ROWS) {
+                  // The up partials are in the exchange area as well, 64 rows further on.
+                  float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
+                  for (int s = 0; s < csk; ++s) {
+                    const float4 x = mine[(s * slice_c4 + c4) * 128 + row_in_tile + 64];
+                    up.x += x.x;
+                    up.y += x.y;
+                    up.z += x.z;
+                    up.w += x.w;
+                  }
+                  v4[0] = silu_mul(v4[0], up.x);
+                  v4[1] = silu_mul(v4[1], up.y);
+                  v4[2] = silu_mul(v4[2], up.z);
+                  v4[3] = silu_mul(v4[3], up.w);
+                }
                 if constexpr (T::TRANS_OUT) {
                   float bias_v = 0.0f;
                   if constexpr (T::EPI == EPI_BIAS) bias_v = load_elem(p.bias, row, is_bf16);
@@ -1342,10 +1387,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           // This warp's 64-column groups, software-pipelined over 32-column chunks: the
           // TMEM load of the next chunk is in flight while this one is converted,
           // staged and stored.
-          constexpr int REGS = (T::EPI == EPI_SWIGLU) ? 64 : 32;
+          constexpr int REGS = T::SWIGLU_COLS ? 64 : 32;
           uint32_t ra[REGS], rb[REGS];
           auto issue = [&](int c32, uint32_t (&r)[REGS]) {
-            if constexpr (T::EPI == EPI_SWIGLU) {
+            if constexpr (T::SWIGLU_COLS) {
               tmem_ld_32x32(t_acc + c32 * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
               tmem_ld_32x32(t_acc + T::OUT_BN + c32 * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
             } else {
@@ -1358,7 +1403,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              if constexpr (T::EPI == EPI_SWIGLU) {
+              if constexpr (T::SWIGLU_COLS) {
                 v[j] = silu_mul(__uint_as_float(r[j]), __uint_as_float(r[32 + j]));
               } else {
                 v[j] = __uint_as_float(r[j]);

@@ -93,6 +93,7 @@ void append_variants_cg1(KernelEntry* out, int* count);
 void append_variants_cg2(KernelEntry* out, int* count);
 void append_variants_trans(KernelEntry* out, int* count);
 void append_variants_swiglu(KernelEntry* out, int* count);
+void append_variants_swiglu_trans(KernelEntry* out, int* count);
 void append_variants_act_cg1(KernelEntry* out, int* count);
 void append_variants_act_cg2(KernelEntry* out, int* count);
 void append_variants_act_trans(KernelEntry* out, int* count);

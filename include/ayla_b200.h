@@ -227,7 +227,8 @@ AYLA_B200_API int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, i
  * intermediates never reach HBM.  New op; its precedent is the reference's fused
  * matmul+sigmoid op (ayla/gemm_collection/auto_matmul_4096_wgmma256_wg_sigmoid.py:22-142)
  * and its silu/mul lowerings (ayla/passes/lower_to_ptx_template.py:296-315, :62-81).
- * Only cfg->cta_group, group_m, grid_ctas and the L2 hints are used.
+ * Only cfg->cta_group, group_m, grid_ctas and the L2 hints are used.  cfg == NULL chooses, for products too
+ * small to fill the GPU, a form with the weights on the row side and k split across a cluster.
  */
 AYLA_B200_API int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate, const void* w_up, void* out,
                      int64_t m, int64_t n, int64_t k, const ayla_b200_config* cfg, uint32_t* status,

@@ -516,6 +516,24 @@ def test_rms_norm_linear_refuses_what_the_projection_refuses():
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("m, n, k", [
+    (1, 8, 8), (5, 72, 136), (16, 200, 520), (20, 136, 1032),     # 16 and 32 columns; no split, two, four
+    (64, 264, 1032), (49, 1032, 520), (130, 1000, 1000),          # 64
+    (100, 4104, 520), (128, 1032, 2056), (300, 1160, 2056)])      # 128, and several column tiles
+def test_swapped_swiglu(m, n, k, dtype):
+    """Shapes that run with the weights on the row side: remainders of the 64 weight rows per tile, of the
+    columns and of the depth, every width and cluster split."""
+    g = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g).to(TD[dtype])
+    gate, up = ((torch.randn(n, k, generator=g) * k ** -0.5).to(TD[dtype]) for _ in range(2))
+    guard = 128
+    out = torch.full((m * n + guard,), 7.0, dtype=TD[dtype], device=DEV)
+    swiglu_op(dtype)(x.to(DEV), gate.to(DEV), up.to(DEV), out[:-guard].view(m, n))
+    assert_parity(out[:-guard].view(m, n).cpu(), O.swiglu_ref32(x, gate, up), f"swiglu {m}x{n}x{k}")
+    assert bool((out[-guard:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize(
     "operation, batch, m, n, k",
     [
