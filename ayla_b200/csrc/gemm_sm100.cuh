@@ -45,6 +45,7 @@ enum : unsigned {
   ST_TIMEOUT_ACC_FULL = 4,   // epilogue waited for a finished accumulator
   ST_BAD_SMEM_ALIGN = 5,
   ST_TIMEOUT_INBOX = 6,      // epilogue waited for the other k-splits' partial sums (cluster split-K)
+  ST_TIMEOUT_GATE = 7,       // epilogue waited for its box of the gate operand
 };
 
 // Division of a non-negative 32-bit value by a divisor fixed at launch: q = (n * mul) >> (32 + shift),
@@ -153,7 +154,8 @@ __device__ __forceinline__ void trace_stamp(long long* stamps, int slot) {
 #define AYLA_TRACE_END(slot)
 #endif
 
-template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, bool ACT_ = false, bool LEAN_ = false>
+template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, bool ACT_ = false, bool LEAN_ = false,
+          bool GATED_ = false>
 struct GemmTraits {
   // LEAN: the kernel is compiled without the k-split epilogues (workspace and cluster forms) and
   // serves the launches that do not split k.  The unused code is never executed, yet it costs a
@@ -193,13 +195,19 @@ struct GemmTraits {
                                    : TMEM_COLS_NEEDED <= 128 ? 128
                                    : TMEM_COLS_NEEDED <= 256 ? 256
                                                              : 512;
-  static constexpr int EPI_WARPS = 8;
+  // GATED: the launch multiplies by a gate operand shaped like the output.  Each epilogue warp has one 64-column
+  // group of the tile: its box of the gate is loaded into its staging rows while the MMAs run, multiplied in place
+  // and stored from there.  (A thread reading its own row of the gate from global memory touches 16 bytes of 32
+  // lines per instruction: 10 us of an SM per 128 x 256 tile with eight warps, 8.5 with sixteen, 5.4 this way.)
+  // One staging box per warp; at 256 columns the sixteen of them cost a ring slot.
+  static constexpr bool GATED = GATED_;
+  static constexpr int EPI_WARPS = GATED ? BN / 16 : 8;
   static constexpr int STORE_BUF_BYTES = 32 * 128;  // 32 rows x 64 columns of 16-bit
   // Swapped SwiGLU: where the epilogue warps of the up rows leave 32 columns for those of the gate rows.
   static constexpr int UP_BUF_BYTES = 32 * 64 * 4;
   static constexpr int STORE_BYTES = SWIGLU_ROWS ? 2 * UP_BUF_BYTES : TRANS_OUT ? 0 : EPI_WARPS * STORE_BUF_BYTES;
   static constexpr int BIAS_BYTES = (EPI == EPI_BIAS && !TRANS_OUT) ? 2 * BN * 4 : 0;
-  static constexpr int MISC_BYTES = 256;
+  static constexpr int MISC_BYTES = GATED ? 384 : 256;
 #ifdef AYLA_B200_TRACE
   static constexpr int TRACE_BYTES = 40 * 8;  // the CTA's timeline stamps, copied out at exit
 #else
@@ -212,9 +220,11 @@ struct GemmTraits {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N extent");
   static_assert(B_BYTES % 1024 == 0, "B slab must keep the 1024-byte swizzle alignment");
   static_assert(!SWIGLU_COLS || BN == 256, "row-major SwiGLU uses the 2x128 layout");
+  static_assert(!GATED || (ACT && LEAN && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
   static_assert(TRANS_OUT || BN >= 64, "the TMA-store epilogue writes 64-column boxes");
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared-memory limit");
-  static_assert((2 * STAGES + 2 * ACC_BUFS + 1) * 8 + 16 <= MISC_BYTES, "barrier area too small");
+  static_assert((2 * STAGES + 2 * ACC_BUFS + 1) * 8 + 16 + (GATED ? EPI_WARPS * 8 : 0) <= MISC_BYTES,
+                "barrier area too small");
 };
 
 // A wait that gives up: polls the barrier, and every few thousand polls checks a
@@ -536,6 +546,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * T::ACC_BUFS + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* last_flag = tmem_slot + 2;
+  const uint32_t bar_gate = bar_inbox + 24;  // GATED: one per epilogue warp, behind the inbox barrier and four words
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -591,6 +602,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       mbar_init(bar_acc_empty + b * 8, T::EPI_WARPS * CG);
     }
     mbar_init(bar_inbox, 1);
+    if constexpr (T::GATED) {
+      prefetch_tensormap(&tm_b2);
+      for (int i = 0; i < T::EPI_WARPS; ++i) mbar_init(bar_gate + i * 8, 1);
+    }
     // The inbox is used once per launch (one tile per cluster): announce its bytes now, before any
     // CTA of the cluster can send.
     if (csk > 0) mbar_arrive_expect_tx(bar_inbox, p.inbox_tx);
@@ -914,8 +929,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // scheduler is latency-bound on its own dependent instruction stream; two hide
     // each other's TMEM-load, conversion and store latencies.
     const int q = warp & 3;                          // TMEM lane quarter
-    const int wsub = (warp - 2) >> 2;                // 0 / 1: which 64-column groups
-    const int epi_tid = (warp - 2) * 32 + lane;      // 0..255
+    const int wsub = (warp - 2) >> 2;                // which 64-column groups: 0 / 1; GATED: the group
+    const int epi_tid = (warp - 2) * 32 + lane;
     const int row_in_tile = q * 32 + lane;
     const bool up_rows = T::SWIGLU_ROWS && q >= 2;  // this warp's accumulator rows belong to the up weight
     const int is_bf16 = p.is_bf16;
@@ -923,6 +938,9 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     uint8_t* my_store = smem_store + (warp - 2) * T::STORE_BUF_BYTES;
     uint32_t acc = 0, acc_phase = 0;
     uint32_t bias_buf = 0;
+    uint32_t gate_phase = 0;
+    const uint32_t my_gate_bar = bar_gate + (warp - 2) * 8;
+    const uint64_t gate_policy = make_policy(0);
     constexpr int CHUNKS32 = T::OUT_BN / 32 > 0 ? T::OUT_BN / 32 : 1;  // 32-column chunks
     constexpr int CHUNK_COLS = T::OUT_BN < 32 ? T::OUT_BN : 32;
     constexpr int EPI_THREADS = T::EPI_WARPS * 32;
@@ -951,6 +969,15 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           bdst[c] = (col < p.n) ? load_elem(p.bias, col, is_bf16) : 0.0f;
         }
         named_bar_sync(1, EPI_THREADS);
+      }
+
+      // Ask for this warp's box of the gate as soon as its last bulk store has read the staging rows.
+      const bool gate_live = T::GATED && wsub < (w.is_narrow ? CHUNKS32 / 4 : CHUNKS32 / 2) &&
+                             w.m0 + q * 32 < p.m && w.n0 + wsub * 64 < p.n;
+      if (gate_live && lane == 0) {
+        tma_store_wait_read<0>();
+        mbar_arrive_expect_tx(my_gate_bar, T::STORE_BUF_BYTES);
+        tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, gate_policy);
       }
 
       AYLA_TRACE_WAIT(tr_wait, bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL))
@@ -1383,7 +1410,54 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           release_accumulator();
         }
       } else if (!split_k) {
-        if constexpr (!T::TRANS_OUT) {
+        if constexpr (T::GATED) {
+          if (!gate_live) {
+            release_accumulator();
+          } else {
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+              const int c32 = 2 * wsub + half;
+              uint32_t r[32];
+              tmem_ld_32x32(t_acc + c32 * 32, r);
+              tmem_ld_wait();
+              if (half == 1) release_accumulator();
+              float v[32];
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+              if constexpr (T::EPI == EPI_BIAS) {
+                const float4* b4 = reinterpret_cast<const float4*>(smem_bias + bias_buf * BN + c32 * 32);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const float4 b = b4[j];
+                  v[4 * j + 0] += b.x;
+                  v[4 * j + 1] += b.y;
+                  v[4 * j + 2] += b.z;
+                  v[4 * j + 3] += b.w;
+                }
+              }
+              apply_act_chunk<32>(v, act);
+              if (half == 0) bw.wait(my_gate_bar, gate_phase, ST_TIMEOUT_GATE);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                uint4* at = reinterpret_cast<uint4*>(my_store + lane * 128 + (((half * 4 + j) ^ (lane & 7)) << 4));
+                const uint4 g = *at;
+                const float2 g0 = unpack2(g.x, is_bf16), g1 = unpack2(g.y, is_bf16);
+                const float2 g2 = unpack2(g.z, is_bf16), g3 = unpack2(g.w, is_bf16);
+                *at = make_uint4(pack2(v[8 * j + 0] * g0.x, v[8 * j + 1] * g0.y, is_bf16),
+                                 pack2(v[8 * j + 2] * g1.x, v[8 * j + 3] * g1.y, is_bf16),
+                                 pack2(v[8 * j + 4] * g2.x, v[8 * j + 5] * g2.y, is_bf16),
+                                 pack2(v[8 * j + 6] * g3.x, v[8 * j + 7] * g3.y, is_bf16));
+              }
+            }
+            gate_phase ^= 1;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_3d(&tm_d, smem_u32(my_store), w.n0 + wsub * 64, w.m0 + q * 32, w.batch);
+              tma_store_commit();
+            }
+          }
+        } else if constexpr (!T::TRANS_OUT) {
           // This warp's 64-column groups, software-pipelined over 32-column chunks: the
           // TMEM load of the next chunk is in flight while this one is converted,
           // staged and stored.

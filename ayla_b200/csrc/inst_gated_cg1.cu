@@ -1,0 +1,15 @@
+// Row-major-output variants for a gate operand shaped like the output, one CTA per 128-row tile.
+#include "kernel_registry.h"
+
+namespace ayla_b200 {
+void append_variants_gated_cg1(KernelEntry* out, int* count) {
+  out[(*count)++] = make_entry<64, 1, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<128, 1, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<192, 1, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<256, 1, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<64, 1, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<128, 1, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<192, 1, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<256, 1, EPI_BIAS, false, true, true, true>();
+}
+}  // namespace ayla_b200

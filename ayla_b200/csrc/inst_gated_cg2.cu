@@ -1,0 +1,15 @@
+// Row-major-output variants for a gate operand shaped like the output, a CTA pair per 256-row tile.
+#include "kernel_registry.h"
+
+namespace ayla_b200 {
+void append_variants_gated_cg2(KernelEntry* out, int* count) {
+  out[(*count)++] = make_entry<64, 2, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<128, 2, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<192, 2, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<256, 2, EPI_PLAIN, false, true, true, true>();
+  out[(*count)++] = make_entry<64, 2, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<128, 2, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<192, 2, EPI_BIAS, false, true, true, true>();
+  out[(*count)++] = make_entry<256, 2, EPI_BIAS, false, true, true, true>();
+}
+}  // namespace ayla_b200

@@ -21,7 +21,8 @@ struct LaunchArgs {
 struct KernelEntry {
   int tile_n, cta_group, epilogue, transposed_out, stages, smem_bytes;
   int kb_per_slot;  // k-blocks one ring slot holds
-  int activation;  // 1 = the variant whose epilogue applies the launch's activation
+  int activation;  // 1 = the variant whose epilogue applies the launch's activation, 2 = the same for
+                   // launches with a gate operand shaped like the output
   int lean;        // 1 = the variant without the k-split epilogues
   const void* func;
   cudaError_t (*launch)(const LaunchArgs&);
@@ -29,9 +30,9 @@ struct KernelEntry {
 
 constexpr int kMaxSmem = 232448;
 
-template <int BN, int CG, int EPI, bool TR>
+template <int BN, int CG, int EPI, bool TR, bool GATED = false>
 constexpr int max_stages() {
-  using T1 = GemmTraits<BN, CG, EPI, TR, 1>;
+  using T1 = GemmTraits<BN, CG, EPI, TR, 1, GATED, GATED, GATED>;
   const int fixed = T1::STORE_BYTES + T1::BIAS_BYTES + T1::MISC_BYTES;
   const int s = (kMaxSmem - fixed) / T1::SLOT_BYTES;
 #ifdef AYLA_B200_STAGE_CAP
@@ -70,9 +71,9 @@ cudaError_t launch_variant(const LaunchArgs& a) {
   return cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<T>, a.tm_a, a.tm_b, a.tm_b2, a.tm_d, a.p);
 }
 
-template <int BN, int CG, int EPI, bool TR, bool ACT = false, bool LEAN = false>
+template <int BN, int CG, int EPI, bool TR, bool ACT = false, bool LEAN = false, bool GATED = false>
 KernelEntry make_entry() {
-  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR>(), ACT, LEAN>;
+  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED>(), ACT, LEAN, GATED>;
   KernelEntry e;
   e.tile_n = BN;
   e.cta_group = CG;
@@ -81,7 +82,7 @@ KernelEntry make_entry() {
   e.stages = T::STAGES;
   e.smem_bytes = T::SMEM_BYTES;
   e.kb_per_slot = T::KB_PER_SLOT;
-  e.activation = ACT ? 1 : 0;
+  e.activation = GATED ? 2 : ACT ? 1 : 0;
   e.lean = LEAN ? 1 : 0;
   e.func = reinterpret_cast<const void*>(&gemm_sm100_kernel<T>);
   e.launch = &launch_variant<T>;
@@ -102,6 +103,8 @@ void append_variants_lean_cg2(KernelEntry* out, int* count);
 void append_variants_lean_trans(KernelEntry* out, int* count);
 void append_variants_lean_act_cg1(KernelEntry* out, int* count);
 void append_variants_lean_act_cg2(KernelEntry* out, int* count);
+void append_variants_gated_cg1(KernelEntry* out, int* count);
+void append_variants_gated_cg2(KernelEntry* out, int* count);
 void append_variants_lean_act_trans(KernelEntry* out, int* count);
 
 }  // namespace ayla_b200

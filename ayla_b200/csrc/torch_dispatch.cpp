@@ -104,7 +104,8 @@ class Dispatcher {
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(l->device)).stream();
     if (l->workspace_bytes != 0 && reinterpret_cast<uintptr_t>(stream) != l->home_stream) return false;
     const void* p[kMaxOperands];
-    for (size_t i = 0; i < operands_; ++i) p[i] = args[i].toTensor().const_data_ptr();
+    for (size_t i = 0; i + 1 < operands_; ++i) p[i] = args[i].toTensor().const_data_ptr();
+    p[operands_ - 1] = args[operands_ - 1].toTensor().mutable_data_ptr();  // the last operand is written
     if (l->swiglu) {
       return reinterpret_cast<SwigluFn>(l->entry)(l->dtype, p[0], p[1], p[2], const_cast<void*>(p[3]), l->m, l->n,
                                                   l->k, l->config, l->status, stream) == 0;

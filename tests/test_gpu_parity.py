@@ -419,6 +419,38 @@ def test_gated_activation_epilogue(activation, device_state):
             assert_parity(out.cpu(), want, f"{activation}*mul {operation} {batch}x{m}x{n}x{k} {cfg}")
 
 
+@pytest.mark.parametrize("cta_group", [1, 2])
+@pytest.mark.parametrize("tile_n", [64, 128, 192, 256])
+def test_gated_tiles(tile_n, cta_group, device_state):
+    """The kernels that load the gate through their staging rows: every tile width, many units per CTA (few
+    CTAs asked for), a half-width last wave, ragged rows and columns, a bias, batches."""
+    status, workspace = device_state
+    g = torch.Generator().manual_seed(tile_n + cta_group)
+    for operation, batch, m, n, k, grid, tail in (("mm", 1, 1000, 1096, 200, 6, 0), ("addmm", 1, 333, 520, 72, 4, 0),
+                                                  ("bmm", 3, 200, 264, 136, 2, 0), ("mm", 1, 1500, 776, 64, 16, 2)):
+        if tail and tile_n % 128 != 0:
+            continue
+        lead = (batch,) if operation == "bmm" else ()
+        a = torch.randn(*lead, m, k, generator=g).bfloat16()
+        bt = (torch.randn(*lead, n, k, generator=g) * k ** -0.5).bfloat16()
+        mul = torch.randn(*lead, m, n, generator=g).bfloat16()
+        tensors = (a, bt) if operation != "addmm" else (torch.randn(n, generator=g).bfloat16(), a, bt)
+        dev, gate = [t.to(DEV) for t in tensors], mul.to(DEV)
+        out = torch.full((batch * m * n + 64,), 7.0, dtype=torch.bfloat16, device=DEV)
+        config = _lib.Config.from_dict(dict(tile_n=tile_n, cta_group=cta_group, grid_ctas=grid, split_tail=tail))
+        status.zero_()
+        for _ in range(2):
+            _lib.gemm_act_mul(operation, "bfloat16", "silu", dev[0].data_ptr() if operation == "addmm" else 0,
+                              dev[-2].data_ptr(), dev[-1].data_ptr(), gate.data_ptr(), out.data_ptr(), batch, m, n, k,
+                              config, workspace.data_ptr(), workspace.numel(), status.data_ptr(),
+                              torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        want = O.act_ref32("silu", O.gemm_ref32(operation, *tensors)) * mul.float()
+        assert_parity(out[:-64].view(*lead, m, n).cpu(), want, f"{operation} {batch}x{m}x{n}x{k} {config.to_dict()}")
+        assert bool((out[-64:] == 7.0).all())
+
+
 def test_row_factor_epilogue(device_state):
     """act([bias +] a @ bt.T) * row_mul[:, None] through the bulk-store, transposed, workspace split-K
     and cluster split-K epilogues."""
