@@ -519,10 +519,16 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count
                                    {128, 1, 0.62}, {64, 2, 0.50}, {64, 1, 0.40}};
   double best_cost = 1e300;
   for (const Shape& sh : kShapes) {
-    if (sh.cta_group == 2 && (m <= 128 || k_blocks <= 4)) continue;  // shallow K: pairing only adds set-up
+    if (sh.cta_group == 2 && m <= 128) continue;
     if (sh.tile_n > 64 && n * 2 <= sh.tile_n) continue;
     const int64_t ctas = sm_count / sh.cta_group;
     const int64_t tiles = batch * ceil_div(m, 128 * sh.cta_group) * ceil_div(n, sh.tile_n);
+    // Shallow K: below two waves pairing only adds set-up, and a matrix of less than one pair's rows gains nothing
+    // from it; from there on it halves what the SMs read of B, and that traffic bounds them (us, single -> pair: bmm
+    // 16 x 2000x2000x128 28.0 -> 26.1, 128 x 256x1024x80 18.3 -> 16.7, 37 x 1500x704x96 20.7 -> 19.7, addmm
+    // 12095x5824x256 44.2 -> 41.4, the same with a GELU 73.2 -> 74.8; mm 1000x1000x256 5.4 -> 5.5, bmm
+    // 100 x 129x1000x64 12.4 -> 13.1).
+    if (sh.cta_group == 2 && k_blocks <= 4 && (m < 256 || tiles < 2 * ctas)) continue;
     const double tile_cost = (sh.tile_n / 256.0) / sh.eff * static_cast<double>(k_blocks);
     const double launch_cost = 6.0 + sh.tile_n / 64.0;
     for (int split = 1; split <= 16; split *= 2) {
