@@ -14,6 +14,7 @@
 //   warps 2..9  epilogue      : TMEM -> registers -> (bias | activation | SiLU*up) -> round ->
 //                               swizzled shared -> TMA store   (or direct stores for the
 //                               transposed form and narrow cluster slices)
+// (kernels for gated launches have one epilogue warp per 64 columns and lane quarter instead of eight)
 // The accumulator is double buffered in TMEM so the epilogue of one tile runs
 // under the main loop of the next.  CTAs are persistent and walk a static,
 // M-grouped raster over (batch, m-tile, n-tile, k-split) work units.
