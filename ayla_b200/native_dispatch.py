@@ -17,6 +17,8 @@ from types import ModuleType
 import torch
 
 from . import _lib
+from .jit_compiler import ShapeSpecializingJITCompiler
+from .torch_custom_call import OperandKind
 
 _PATH = Path(__file__).resolve().parent / "lib" / "_torch_dispatch.so"
 
@@ -32,9 +34,22 @@ def load() -> ModuleType:
     return module
 
 
-def register(namespace: str, name: str, compiler) -> None:
-    """Register the CUDA kernel of ``namespace::name``, backed by a ``ShapeSpecializingJITCompiler`` whose
-    operands are the op's arguments."""
+_MAX_OPERANDS = 5  # kMaxOperands of the compiled dispatcher
+
+
+def serves(launcher, kinds: list[OperandKind]) -> bool:
+    """Whether the compiled dispatcher can stand in for ``launcher``: a per-shape dispatcher itself (a subclass
+    may do something else on a call), whose operands are the op's arguments, all of one dtype, the last one
+    written."""
+    if type(launcher) is not ShapeSpecializingJITCompiler:
+        return False
+    signature = launcher.signature
+    return (len(signature) <= _MAX_OPERANDS and len({spec.dtype for spec in signature}) == 1 and
+            kinds == [OperandKind.R] * (len(signature) - 1) + [OperandKind.RW])
+
+
+def register(namespace: str, name: str, compiler: ShapeSpecializingJITCompiler) -> None:
+    """Register the CUDA kernel of ``namespace::name``, backed by a compiler that ``serves`` accepts."""
     [dtype] = {spec.dtype for spec in compiler.signature}
     dispatcher = None
 

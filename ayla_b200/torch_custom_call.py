@@ -4,8 +4,8 @@ Same surface as the reference's glue (ayla/torch_custom_call.py:40-43, :64-80,
 :83-155): ``OperandKind`` marks each launcher operand as read-only input (R),
 caller-allocated in/out tensor (RW, rendered ``Tensor(aN!)`` in the schema) or
 op-allocated result (RESULT); the op gets a CUDA implementation that calls the
-launcher (a compiled one for the per-shape dispatchers, ``native_dispatch``) and a Meta implementation that only allocates, so tracing never
-launches a kernel.
+launcher -- a compiled one where ``native_dispatch`` can serve it, i.e. for per-shape dispatchers that write
+into a caller's tensor -- and a Meta implementation that only allocates, so tracing never launches a kernel.
 """
 
 from __future__ import annotations
@@ -87,7 +87,6 @@ def make_torch_custom_call(
     infer_result_shapes: Callable[..., list[tuple[int, ...]]] | None = None,
 ) -> torch._ops.OpOverload:
     from . import native_dispatch
-    from .jit_compiler import ShapeSpecializingJITCompiler
 
     kinds = list(signature_mapping)
     op_name = name or launcher.name
@@ -123,9 +122,9 @@ def make_torch_custom_call(
     def meta_impl(*inputs: torch.Tensor):
         return pack(new_results(inputs))
 
-    if result_positions or not isinstance(launcher, ShapeSpecializingJITCompiler):
-        lib.impl(op_name, cuda_impl, "CUDA")
-    else:
+    if native_dispatch.serves(launcher, kinds):
         native_dispatch.register(namespace, op_name, launcher)
+    else:
+        lib.impl(op_name, cuda_impl, "CUDA")
     lib.impl(op_name, meta_impl, "Meta")
     return getattr(getattr(torch.ops, namespace), op_name).default

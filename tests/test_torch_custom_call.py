@@ -1,8 +1,11 @@
 """Custom-op glue on the meta device -- mirrors the reference's
 tests/test_torch_custom_call.py:8-53."""
 
+import pytest
 import torch
 
+from ayla_b200 import native_dispatch
+from ayla_b200.jit_compiler import OpTemplate, ShapeSpecializingJITCompiler
 from ayla_b200.torch_custom_call import OperandKind, TensorSpec, make_schema, make_torch_custom_call
 
 
@@ -54,3 +57,31 @@ def test_dynamic_m_op_infers_its_result_on_meta():
     rhs = torch.empty((256, 64), dtype=torch.bfloat16, device="meta")
     out = op(lhs, rhs)
     assert out.shape == (3, 256) and out.dtype == torch.bfloat16 and out.device.type == "meta"
+
+
+class _Counting(ShapeSpecializingJITCompiler):
+    def __call__(self, *tensors):
+        raise AssertionError("Meta dispatch must not launch the kernel")
+
+
+_BF16, _F32 = torch.bfloat16, torch.float32
+
+
+@pytest.mark.parametrize("name, cls, dtypes, written", [
+    ("mixed_dtypes", ShapeSpecializingJITCompiler, (_BF16, _F32), 1),
+    ("six_operands", ShapeSpecializingJITCompiler, (_BF16,) * 6, 5),
+    ("first_written", ShapeSpecializingJITCompiler, (_BF16,) * 3, 0),
+    ("subclass", _Counting, (_BF16,) * 3, 2),
+    ("plain", ShapeSpecializingJITCompiler, (_BF16,) * 5, 4),
+])
+def test_per_shape_dispatchers_of_any_signature_become_ops(name, cls, dtypes, written, monkeypatch):
+    """Only a signature that the compiled dispatcher handles goes to it; the others keep the Python one."""
+    compiled = []
+    register = native_dispatch.register
+    monkeypatch.setattr(native_dispatch, "register", lambda *args: (compiled.append(args[1]), register(*args)))
+    compiler = cls(OpTemplate(name, tuple(TensorSpec(dtype, (None, None)) for dtype in dtypes)), lambda bound, device: None)
+    kinds = [OperandKind.RW if i == written else OperandKind.R for i in range(len(dtypes))]
+    op = make_torch_custom_call(compiler, kinds, namespace="ayla_b200_signatures_test")
+    assert op(*[torch.empty(4, 8, dtype=dtype, device="meta") for dtype in dtypes]) is None
+    assert torch._C._dispatch_has_kernel_for_dispatch_key(f"ayla_b200_signatures_test::{name}", "CUDA")
+    assert compiled == (["plain"] if name == "plain" else [])
