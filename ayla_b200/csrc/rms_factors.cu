@@ -29,10 +29,11 @@ __device__ __forceinline__ float square_sum(uint4 v, bool is_bf16, float sum) {
 constexpr int kThreads = 256;
 constexpr int kUnroll = 4;  // 16-byte loads a thread has in flight
 
-// ROW_THREADS threads (one to eight warps) share a row.
+// ROW_THREADS threads (one to eight warps) share a row.  x is read through L2 (ld.global.cg), not as read-only data:
+// this launch may begin while the one that writes x still runs, so x does change during the kernel's lifetime.
 template <int ROW_THREADS>
 __global__ void __launch_bounds__(kThreads)
-rms_factors_kernel(const uint4* __restrict__ x, void* __restrict__ factors, int rows, int chunks, float k, float eps,
+rms_factors_kernel(const uint4* x, void* factors, int rows, int chunks, float k, float eps,
                    int is_bf16) {
   grid_launch_dependents();
   grid_dependency_wait();
@@ -46,11 +47,11 @@ rms_factors_kernel(const uint4* __restrict__ x, void* __restrict__ factors, int 
     for (; c + (kUnroll - 1) * ROW_THREADS < chunks; c += kUnroll * ROW_THREADS) {
       uint4 v[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) v[u] = __ldg(src + c + u * ROW_THREADS);
+      for (int u = 0; u < kUnroll; ++u) v[u] = __ldcg(src + c + u * ROW_THREADS);
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) part[u] = square_sum(v[u], is_bf16 != 0, part[u]);
     }
-    for (; c < chunks; c += ROW_THREADS) part[0] = square_sum(__ldg(src + c), is_bf16 != 0, part[0]);
+    for (; c < chunks; c += ROW_THREADS) part[0] = square_sum(__ldcg(src + c), is_bf16 != 0, part[0]);
     sum = (part[0] + part[1]) + (part[2] + part[3]);
   }
 #pragma unroll

@@ -533,6 +533,38 @@ def test_rms_row_factors(rows, k, dtype):
     assert torch.isnan(factors[rows])
 
 
+@pytest.mark.parametrize("m, k", [(256, 1024), (2048, 512), (40, 8192)])
+def test_rms_norm_linear_behind_the_launch_that_writes_its_input(m, k):
+    """x is rewritten by a GEMM directly in front of every call: with launches overlapping, the row factors and
+    the projection are those of the new x, bit for bit what serialised launches give."""
+    from ayla_b200.rmsnorm_linear import rms_norm_linear
+
+    g = torch.Generator().manual_seed(k)
+    sources = [(torch.randn(m, 128, generator=g) * 4.0 ** (i % 4)).bfloat16().to(DEV) for i in range(6)]
+    up = (torch.randn(k, 128, generator=g) * 128 ** -0.5).bfloat16().to(DEV)
+    weight = (torch.randn(192, k, generator=g) * k ** -0.5).bfloat16().to(DEV)
+    x = torch.empty(m, k, dtype=torch.bfloat16, device=DEV)
+    mm = gemm_op("mm", "bfloat16")
+
+    def chain():
+        outs = []
+        for source in sources * 4:
+            mm(source, up, x)
+            outs.append(rms_norm_linear(x, weight))
+        torch.cuda.synchronize()
+        return torch.stack(outs)
+
+    try:
+        _lib.set_launch_overlap(False)
+        serial = chain()
+    finally:
+        _lib.set_launch_overlap(True)
+    assert torch.equal(chain(), serial)
+    x32 = O.gemm_ref32("mm", sources[-1].cpu(), up.cpu()).bfloat16().float()
+    factors = torch.rsqrt(x32.pow(2).mean(-1, keepdim=True) + 1e-5).bfloat16().float()
+    assert_parity(serial[-1].cpu(), (x32 @ weight.cpu().float().T) * factors, f"rms_norm_linear {m}x192x{k}")
+
+
 def test_rms_norm_linear_refuses_what_the_projection_refuses():
     from ayla_b200.rmsnorm_linear import rms_norm_linear
 
