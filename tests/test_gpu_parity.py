@@ -360,7 +360,8 @@ def test_activations_at_every_16_bit_value(activation, dtype):
     leave fp32's range at the bottom), against the function in double precision.  The bound is half an ulp
     for the one rounding, plus the relative error of the fp32 evaluation: 2^z with |z| <= 130 carries z's
     own rounding (130 * 2^-24 * ln 2 < 6e-6, three times that for the cubic argument of gelu_tanh), GELU's
-    polynomial 3e-6 down to x = -6 and less than 6e-9 absolutely below, where 6 * Phi(-6) is 5.9e-9;
+    polynomial 3e-6 down to x = -5 and less than 6e-9 absolutely below (5e-6 of 5 * Phi(-5) = 1.4e-6 down to
+    x = -6, where x * Phi(x) itself is 5.9e-9);
     results under 2^-100 may be flushed."""
     values = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(TD[dtype])
     values = values[torch.isfinite(values)]
@@ -380,6 +381,27 @@ def test_activations_at_every_16_bit_value(activation, dtype):
     bound = 1.001 * half_ulp + relative * want.abs() + (6e-9 if activation == "gelu" else 2.0 ** -100)
     bad = ~((got - want).abs() <= bound)
     assert not bad.any(), [(x64[bad][i].item(), got[bad][i].item(), want[bad][i].item()) for i in range(min(5, int(bad.sum())))]
+
+
+@pytest.mark.parametrize("activation, at_minus_infinity", [("relu", 0.0), ("sigmoid", 0.0), ("silu", float("nan")),
+                                                           ("gelu", float("nan")), ("gelu_tanh", float("nan"))])
+@pytest.mark.parametrize("m", [16, 256])
+def test_activations_of_infinities_and_nan(activation, at_minus_infinity, m):
+    """The formulas of the framework's own activations at the ends: x * sigmoid(x) and 0.5 x (1 + erf or tanh) are
+    0 * inf at minus infinity.  (relu is max(x, 0) on the fp32 sum, whose result for a NaN is 0.)"""
+    def run(rows):
+        a = torch.zeros(m, 8).half()
+        for i, row in enumerate(rows):
+            a[i] = torch.tensor(row).half()
+        out = torch.empty(m, 128, dtype=torch.float16, device=DEV)
+        gemm_act_op("mm", activation, "float16")(a.to(DEV), torch.ones(128, 8).half().to(DEV), out)
+        return out.cpu()[:len(rows)]
+
+    top, nan, inf = 1.0 if activation == "sigmoid" else float("inf"), float("nan"), float("inf")
+    got = run([[inf] + [0.0] * 7, [-inf] + [0.0] * 7, [nan] + [0.0] * 7, [65504.0] * 8, [-65504.0] * 8])
+    want = torch.tensor([top, at_minus_infinity, 0.0 if activation == "relu" else nan, top, 0.0]).half()
+    assert torch.equal(got.nan_to_num(nan=7.0, posinf=8.0, neginf=9.0),
+                       want[:, None].expand(5, 128).nan_to_num(nan=7.0, posinf=8.0, neginf=9.0)), got[:, 0]
 
 
 @pytest.mark.parametrize("activation", ["none", "sigmoid", "silu"])
