@@ -982,10 +982,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         named_bar_sync(1, EPI_THREADS);
       }
 
-      // Ask for this warp's box of the gate as soon as its last bulk store has read the staging rows.
+      // Ask for this warp's box of the gate as soon as its last bulk store has read the staging rows.  Not after an
+      // abort: the box before may still be on its way, its barrier's phase open.
       const bool gate_live = T::GATED && wsub < (w.is_narrow ? CHUNKS32 / 4 : CHUNKS32 / 2) &&
                              w.m0 + q * 32 < p.m && w.n0 + wsub * 64 < p.n;
-      if (gate_live && lane == 0) {
+      if (gate_live && lane == 0 && !bw.aborted()) {
         tma_store_wait_read<0>();
         mbar_arrive_expect_tx(my_gate_bar, T::STORE_BUF_BYTES);
         tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, gate_policy);

@@ -993,6 +993,40 @@ def test_timed_out_cluster_split_leaves_the_context_usable(config, device_state)
     assert_parity(out, O.mm_ref32(a, bt), f"after a timed-out cluster split {config}")
 
 
+@pytest.mark.parametrize("config", [dict(tile_n=64, cta_group=1, grid_ctas=3), dict(tile_n=256, cta_group=1, grid_ctas=2),
+                                    dict(tile_n=128, cta_group=2, grid_ctas=4), dict(tile_n=256, cta_group=2, grid_ctas=4)])
+def test_timed_out_gated_launch_leaves_the_context_usable(config, device_state):
+    """A gated launch whose operands never come, with several units per CTA: its gate boxes do come, and after
+    the abort none is asked for again.  The next launch is correct."""
+    status, workspace = device_state
+    m, n, k = 700, 1024, 256
+    g = torch.Generator().manual_seed(8)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+    mul = torch.randn(m, n, generator=g).bfloat16()
+    da, dbt, dmul = a.to(DEV), bt.to(DEV), mul.to(DEV)
+    out = torch.zeros(m, n, dtype=torch.bfloat16, device=DEV)
+
+    def launch():
+        status.zero_()
+        _lib.gemm_act_mul("mm", "bfloat16", "sigmoid", 0, da.data_ptr(), dbt.data_ptr(), dmul.data_ptr(), out.data_ptr(),
+                          1, m, n, k, _lib.Config.from_dict(config), workspace.data_ptr(), workspace.numel(),
+                          status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return int(status.item())
+
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(20)
+        lib.ayla_b200_debug_set_flags(1)
+        assert launch() & 0xFF in (2, 4)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    assert launch() == 0
+    assert_parity(out.cpu(), O.act_ref32("sigmoid", O.gemm_ref32("mm", a, bt)) * mul.float(), f"after a timeout {config}")
+
+
 def test_random_shapes_through_the_public_ops():
     """Schedule selection on shapes nobody measured: transferred table entries (trimmed tiles, 192-wide
     tiles, cluster k-splits, eviction hints) and the default heuristic must all stay correct on ragged
