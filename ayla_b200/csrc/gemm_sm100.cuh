@@ -1672,9 +1672,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
-  // No CTA of a k-split cluster leaves while another may still send into its inbox.  In the ordinary course its own
-  // inbox barrier has told it that all sends are in; a CTA whose waits ran out has given up on that, and a peer that
-  // gives up later would write into the shared memory of a CTA that has left.  Every warp arrived when it had sent.
+  // No CTA of a k-split cluster leaves while sends into its inbox are under way.  In the ordinary course its own
+  // inbox barrier has told it that all of them are in; a CTA whose waits ran out has given up on that, and a peer that
+  // gives up later would write into the shared memory of a CTA that has left.  Every warp arrives when it has issued
+  // its sends (pairs meet below), so from here on what is to come is on its way.
   if (CG == 1 && csk > 0) cluster_wait();
   if constexpr (CG == 2) {
     // The leader's MMAs write the peer's TMEM and both CTAs' barriers: neither
@@ -1688,6 +1689,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc<CG>(tmem_base, T::TMEM_COLS);
+  }
+  // The sends are asynchronous: having been issued, they still have to land, which the inbox barrier counts (an
+  // aborted epilogue sends all its parts as well).  A CTA that gave up on it stays until then, or for a bounded time.
+  if (csk > 0 && threadIdx.x == 0 && bw.aborted()) {
+    for (int i = 0; i < 64 && !mbar_try_wait(bar_inbox, 0); ++i) __nanosleep(2000);
   }
 #ifdef AYLA_B200_TRACE
   if (stamps != nullptr && threadIdx.x == 32) {

@@ -993,6 +993,26 @@ def test_timed_out_cluster_split_leaves_the_context_usable(config, device_state)
     assert_parity(out, O.mm_ref32(a, bt), f"after a timed-out cluster split {config}")
 
 
+@pytest.mark.parametrize("m, n, k", [(8, 1024, 2048), (100, 1024, 1024), (60, 4096, 512)])
+def test_timed_out_swapped_swiglu_leaves_the_context_usable(m, n, k, device_state):
+    """The SwiGLU form of few rows, its k split across a cluster or (the last) not split, with its loads withheld."""
+    g = torch.Generator().manual_seed(m)
+    x = torch.randn(m, k, generator=g).bfloat16()
+    gate, up = ((torch.randn(n, k, generator=g) * k ** -0.5).bfloat16() for _ in range(2))
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(20)
+        lib.ayla_b200_debug_set_flags(1)
+        _, status = run_abi("swiglu", "bfloat16", (x, gate, up), None, device_state)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    assert status & 0xFF != 0
+    out, status = run_abi("swiglu", "bfloat16", (x, gate, up), None, device_state)
+    assert status == 0
+    assert_parity(out.cpu(), O.swiglu_ref32(x, gate, up), f"after a timed-out launch {m}x{n}x{k}")
+
+
 @pytest.mark.parametrize("config", [dict(tile_n=64, cta_group=1, grid_ctas=3), dict(tile_n=256, cta_group=1, grid_ctas=2),
                                     dict(tile_n=128, cta_group=2, grid_ctas=4), dict(tile_n=256, cta_group=2, grid_ctas=4)])
 def test_timed_out_gated_launch_leaves_the_context_usable(config, device_state):
