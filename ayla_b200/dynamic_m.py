@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import torch
 
-from .gemm_jit import GemmLauncher, select_gemm_schedule
+from .gemm_jit import GemmLauncher, packed_serves, select_gemm_schedule
 from .jit_compiler import OpTemplate, ShapeSpecializingJITCompiler
 from .torch_custom_call import DEFAULT_NAMESPACE, OperandKind, TensorSpec, make_torch_custom_call
 
@@ -31,7 +31,7 @@ def make_dynamic_m_matmul(n: int, k: int, *, name: str | None = None, namespace:
         schedule = select_gemm_schedule("mm", "bfloat16", m, n, k)
         if schedule is None:
             raise ValueError(f"{name}: no schedule for mm {m}x{n}x{k}")
-        return GemmLauncher("mm", "bfloat16", 1, m, n, k, schedule, device)
+        return GemmLauncher("mm", "bfloat16", 1, m, n, k, schedule, device, packed=packed_serves("mm", 1, m, n, k, device))
 
     compiler = ShapeSpecializingJITCompiler(template, compile_specialization)
     return make_torch_custom_call(

@@ -145,7 +145,8 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
 
     An exact table hit has empty ``adaptations``; a schedule transferred from a
     nearby measured shape names that shape; otherwise the library's shape-aware
-    default is returned with ``source_shape`` ``None``.
+    default is returned with ``source_shape`` ``None``.  It is a schedule of the general
+    kernel: plain products that ``packed_serves`` run on the packed kernel, which takes none.
     """
     if min(batch, m, n, k) <= 0 or operation not in _OPERATIONS:
         return None
@@ -199,6 +200,18 @@ def _fallback_schedule(operation: str, dtype: str, m: int, n: int, k: int,
     )
 
 
+def packed_serves(operation: str, batch: int, m: int, n: int, k: int, device: torch.device,
+                  activation: str = "none", gated: bool | str = False) -> bool:
+    """Whether the ops run a product of these extents on the packed kernel (few columns, a shallow depth, rows
+    enough to fill the GPU) instead of the general one with ``select_gemm_schedule``'s schedule."""
+    if activation != "none" or gated:
+        return False
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    with torch.cuda.device(index):
+        _lib.init(index)  # the rule goes by the device's SM count
+        return _lib.packed_preferred(operation, batch, m, n, k)
+
+
 class GemmLauncher:
     """One specialised ``(operation, dtype, shape, device)`` launch.
 
@@ -216,11 +229,14 @@ class GemmLauncher:
     counters that launch may have left dirty are cleared first, so the call after the
     error is correct again.  ``check_status()`` does the same after a synchronise, and
     ``AYLA_B200_DEBUG=1`` calls it after every launch.
+
+    It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the launch goes to the
+    packed kernel instead, and ``seed`` and ``config`` are not used.
     """
 
     def __init__(self, operation: str, dtype: str, batch: int, m: int, n: int, k: int,
                  seed: GemmScheduleSeed, device: torch.device, activation: str = "none",
-                 gated: bool | str = False):
+                 gated: bool | str = False, packed: bool = False):
         assert seed.builder_config is not None
         self.operation, self.dtype, self.activation, self.gated = operation, dtype, activation, gated
         self.batch, self.m, self.n, self.k = batch, m, n, k
@@ -230,10 +246,7 @@ class GemmLauncher:
         index = device.index if device.index is not None else torch.cuda.current_device()
         with torch.cuda.device(index):
             _lib.init(index)
-        # Many small or thin products run on a kernel of their own, which the library takes for them where it is
-        # given no schedule.
-        self._packed = (activation == "none" and not gated and
-                        _lib.packed_preferred(operation, batch, m, n, k))
+        self._packed = packed  # the library takes that kernel where it is given no schedule
         need = 0 if self._packed else _lib.workspace_bytes(self.config, operation, batch, m, n, k)
         self._ws_bytes = need
         self.workspace = torch.zeros(need, dtype=torch.uint8, device=device) if need else None
@@ -393,7 +406,9 @@ def gemm_jit_compiler(operation: str, dtype: str, activation: str = "none",
         schedule = select_gemm_schedule(operation, dtype, m, n, k, *batch)
         if schedule is None:
             raise ValueError(f"{bound.name}: no schedule for {operation} {lead}x{m}x{n}x{k}")
-        return GemmLauncher(operation, dtype, batch[0] if batch else 1, m, n, k, schedule, device, activation, gated)
+        count = batch[0] if batch else 1
+        return GemmLauncher(operation, dtype, count, m, n, k, schedule, device, activation, gated,
+                            packed_serves(operation, count, m, n, k, device, activation, gated))
 
     return ShapeSpecializingJITCompiler(template, compile_specialization)
 

@@ -311,3 +311,32 @@ def test_a_schedule_is_not_transferred_to_a_shape_where_its_tiles_are_mostly_pad
     # whatever the table holds near it, a 64-column output never gets a schedule wider than it needs twice over
     seed = gemm_jit.select_gemm_schedule("mm", "bfloat16", 401536, 64, 512)
     assert seed is not None and gemm_jit._column_padding({**gemm_jit._DEFAULTS, **seed.builder_config}, 401536, 64) < 0.34
+
+
+@pytest.mark.parametrize("activation, gated, packed", [("none", False, True), ("relu", False, False), ("none", True, False)])
+def test_only_plain_ops_ask_for_the_packed_kernel(activation, gated, packed, monkeypatch):
+    """A launcher runs the schedule it is given; it is the op's specialisation that prefers the packed kernel."""
+    import contextlib
+    import types
+
+    from ayla_b200 import _lib, gemm_jit
+
+    class Status:
+        ptr = 16
+
+    monkeypatch.setattr(torch.cuda, "device", lambda index: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index=None: types.SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(_lib, "init", lambda index: None)
+    monkeypatch.setattr(_lib, "StatusWord", Status)
+    monkeypatch.delenv("AYLA_B200_DEBUG", raising=False)
+    m, n, k = 65536, 32, 32
+    compiler = gemm_jit.gemm_jit_compiler("mm", "bfloat16", activation, gated)
+    shapes = [(m, k), (n, k)] + [(m, n)] * (2 if gated else 1)
+    launcher = compiler._compile_fn(compiler._template.specialize(shapes), torch.device("cpu"))
+    assert launcher._packed is packed and (launcher.native_call()["config"] == 0) is packed
+    captured = {**gemm_jit._DEFAULTS, "tile_n": 64}
+    seed = gemm_jit.GemmScheduleSeed(captured, gemm_jit._builder_config(captured), (), None)
+    given = gemm_jit.GemmLauncher("mm", "bfloat16", 1, m, n, k, seed, torch.device("cpu"), activation, gated)
+    assert not given._packed and given.native_call()["config"] != 0 and given.config.tile_n == 64

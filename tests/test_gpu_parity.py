@@ -686,6 +686,26 @@ def test_packed_kernel_through_the_ops_and_its_limits():
     launcher.check_status()
 
 
+def test_a_launcher_runs_the_schedule_it_is_given():
+    """Also where the ops would take the packed kernel: the schedule's workspace is there, its result right, and the
+    record for repeated calls carries it."""
+    from ayla_b200.gemm_jit import GemmLauncher, GemmScheduleSeed, _DEFAULTS, packed_serves
+
+    m, n, k = 20000, 32, 128
+    assert packed_serves("mm", 1, m, n, k, torch.device(DEV))
+    assert not packed_serves("mm", 1, m, n, k, torch.device(DEV), activation="relu")
+    captured = {**_DEFAULTS, "tile_n": 64, "cta_group": 1, "split_k": 2}
+    seed = GemmScheduleSeed(captured, {key: int(captured[key]) for key in _lib.Config.FIELDS}, (), (m, n, k))
+    launcher = GemmLauncher("mm", "bfloat16", 1, m, n, k, seed, torch.device(DEV))
+    assert launcher.workspace is not None and launcher.native_call()["config"] != 0
+    a = torch.randn(m, k, device=DEV).bfloat16()
+    bt = (torch.randn(n, k, device=DEV) * k ** -0.5).bfloat16()
+    out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    launcher(a, bt, out)
+    launcher.check_status()
+    assert_parity(out.cpu(), O.mm_ref32(a.cpu(), bt.cpu()), "explicit schedule")
+
+
 def test_gemm_act_mul_op_matches_the_oracle():
     from ayla_b200 import gemm_act_mul_op
 
