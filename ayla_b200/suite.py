@@ -17,7 +17,7 @@ import statistics
 import torch
 
 from . import _lib
-from .gemm_jit import select_gemm_schedule
+from .gemm_jit import packed_serves, select_gemm_schedule
 
 L2_BYTES = 126e6
 SWEEP_M = (1, 8, 16, 32, 64, 128, 256, 512, 1024, 2048, 4096, 8192, 16384)
@@ -61,6 +61,15 @@ def time_interleaved(fns: dict, launches: int, rounds: int = 9) -> dict:
     return {name: statistics.median(vals) for name, vals in samples.items()}
 
 
+def op_schedule(operation: str, dtype: str, batch: int, m: int, n: int, k: int) -> tuple[_lib.Config | None, str]:
+    """What the op runs for these extents, as ``_lib.gemm`` takes it, and where it comes from; no schedule where
+    that is the packed kernel."""
+    if packed_serves(operation, batch, m, n, k, torch.device("cuda")):
+        return None, "packed kernel"
+    seed = select_gemm_schedule(operation, dtype, m, n, k, batch)
+    return _lib.Config.from_dict(seed.builder_config), "table" if seed.source_shape is not None else "default"
+
+
 def measure_gemm(operation: str, dtype: str, batch: int, m: int, n: int, k: int, peaks: dict,
                  cfg: dict | None = None, rounds: int = 9, with_torch: bool = True) -> dict:
     dev = "cuda"
@@ -77,11 +86,10 @@ def measure_gemm(operation: str, dtype: str, batch: int, m: int, n: int, k: int,
         sets.append((bias, a, bt, out))
     source = "explicit"
     if cfg is None:
-        seed = select_gemm_schedule(operation, dtype, m, n, k, batch)
-        cfg = dict(seed.builder_config)
-        source = "table" if seed.source_shape is not None else "default"
-    config = _lib.Config.from_dict(cfg)
-    need = _lib.workspace_bytes(config, operation, batch, m, n, k)
+        config, source = op_schedule(operation, dtype, batch, m, n, k)
+    else:
+        config = _lib.Config.from_dict(cfg)
+    need = _lib.workspace_bytes(config, operation, batch, m, n, k) if config is not None else 0
     ws = torch.zeros(max(need, 16), dtype=torch.uint8, device=dev)
 
     def ours(i, stream):
@@ -108,7 +116,8 @@ def measure_gemm(operation: str, dtype: str, batch: int, m: int, n: int, k: int,
     ms = times["ours"]
     row = {
         "op": operation, "dtype": dtype, "batch": batch, "m": m, "n": n, "k": k,
-        "schedule": {key: val for key, val in config.to_dict().items() if val}, "schedule_source": source,
+        "schedule": {key: val for key, val in config.to_dict().items() if val} if config is not None else {},
+        "schedule_source": source,
         "operand_copies": copies, "launches_per_graph": launches, "rounds": rounds,
         "ms": ms, "tflops": flops / ms / 1e9, "gbs": nbytes / ms / 1e6,
         "frac_tensor_peak": flops / ms / 1e9 / peaks["bf16"], "frac_hbm_peak": nbytes / ms / 1e6 / peaks["hbm"],

@@ -232,7 +232,7 @@ def run_case(args) -> None:
     """Launch one config ``--launches`` times and exit (random inputs, nothing checked): the
     command profiled with ncu."""
     from ayla_b200 import _lib
-    from ayla_b200.gemm_jit import select_gemm_schedule
+    from ayla_b200.suite import op_schedule
 
     if args.case in CASES:
         op, batch, m, n, k = CASES[args.case]
@@ -263,8 +263,8 @@ def run_case(args) -> None:
         bias = torch.randn(n, device=dev).to(td)
         out = torch.empty((*lead, m, n), device=dev, dtype=td)
         if cfg is None:
-            cfg = _lib.Config.from_dict(select_gemm_schedule(op, args.dtype, m, n, k, batch).builder_config)
-        need = _lib.workspace_bytes(cfg, op, batch, m, n, k)
+            cfg, _ = op_schedule(op, args.dtype, batch, m, n, k)
+        need = _lib.workspace_bytes(cfg, op, batch, m, n, k) if cfg is not None else 0
         ws = torch.zeros(max(need, 16), dtype=torch.uint8, device=dev)
         for _ in range(args.launches):
             if args.torch:
@@ -321,8 +321,7 @@ def run_timeline(args) -> None:
             raise SystemExit("--timeline needs the trace build: python -m ayla_b200.build --trace")
         os.environ["AYLA_B200_LIB"] = str(_build.TRACE_LIB_PATH)
     from ayla_b200 import _lib
-    from ayla_b200.gemm_jit import select_gemm_schedule
-    from ayla_b200.suite import _copies
+    from ayla_b200.suite import _copies, op_schedule
 
     if args.case in CASES:
         op, batch, m, n, k = CASES[args.case]
@@ -335,9 +334,11 @@ def run_timeline(args) -> None:
     dev = "cuda:0"
     _lib.init(0)
     td = torch.bfloat16 if args.dtype == "bfloat16" else torch.float16
-    schedule = json.loads(args.schedule) if args.schedule else dict(
-        select_gemm_schedule(op, args.dtype, m, n, k, batch).builder_config)
-    cfg = _lib.Config.from_dict(schedule)
+    cfg = _lib.Config.from_dict(json.loads(args.schedule)) if args.schedule else op_schedule(
+        op, args.dtype, batch, m, n, k)[0]
+    if cfg is None:
+        raise SystemExit("the op runs the packed kernel here, which leaves no stamps: give a --schedule to see the general one")
+    schedule = cfg.to_dict()
     if _lib.workspace_bytes(cfg, op, batch, m, n, k) > 0:
         raise SystemExit("this schedule reduces through workspace slabs; the stamps need the workspace")
     lead = (batch,) if op == "bmm" else ()

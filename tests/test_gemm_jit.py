@@ -340,3 +340,16 @@ def test_only_plain_ops_ask_for_the_packed_kernel(activation, gated, packed, mon
     seed = gemm_jit.GemmScheduleSeed(captured, gemm_jit._builder_config(captured), (), None)
     given = gemm_jit.GemmLauncher("mm", "bfloat16", 1, m, n, k, seed, torch.device("cpu"), activation, gated)
     assert not given._packed and given.native_call()["config"] != 0 and given.config.tile_n == 64
+
+
+@pytest.mark.parametrize("packed", [True, False])
+def test_the_suite_times_the_kernel_the_ops_run(packed, monkeypatch):
+    from ayla_b200 import suite
+
+    monkeypatch.setattr(suite, "packed_serves", lambda *args: packed)
+    config, source = suite.op_schedule("mm", "bfloat16", 1, 65536, 32, 32)
+    if packed:
+        assert config is None and source == "packed kernel"
+    else:
+        assert config.to_dict() == select_gemm_schedule("mm", "bfloat16", 65536, 32, 32).builder_config
+        assert source in ("table", "default")
