@@ -15,6 +15,7 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
+#include <vector>
 
 #include "kernel_registry.h"
 #include "packed_gemm.h"
@@ -35,30 +36,28 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
-constexpr int kMaxVariants = 128;
 constexpr int kMaxDevices = 64;
 
 struct Registry {
-  KernelEntry entries[kMaxVariants];
-  int count = 0;
+  std::vector<KernelEntry> entries;
   Registry() {
-    append_variants_cg1(entries, &count);
-    append_variants_cg2(entries, &count);
-    append_variants_trans(entries, &count);
-    append_variants_swiglu(entries, &count);
-    base_count = count;
-    append_variants_swiglu_trans(entries, &count);
-    append_variants_act_cg1(entries, &count);
-    append_variants_act_cg2(entries, &count);
-    append_variants_act_trans(entries, &count);
-    append_variants_lean_cg1(entries, &count);
-    append_variants_lean_cg2(entries, &count);
-    append_variants_lean_trans(entries, &count);
-    append_variants_lean_act_cg1(entries, &count);
-    append_variants_lean_act_cg2(entries, &count);
-    append_variants_lean_act_trans(entries, &count);
-    append_variants_gated_cg1(entries, &count);
-    append_variants_gated_cg2(entries, &count);
+    append_variants_cg1(&entries);
+    append_variants_cg2(&entries);
+    append_variants_trans(&entries);
+    append_variants_swiglu(&entries);
+    base_count = static_cast<int>(entries.size());
+    append_variants_swiglu_trans(&entries);
+    append_variants_act_cg1(&entries);
+    append_variants_act_cg2(&entries);
+    append_variants_act_trans(&entries);
+    append_variants_lean_cg1(&entries);
+    append_variants_lean_cg2(&entries);
+    append_variants_lean_trans(&entries);
+    append_variants_lean_act_cg1(&entries);
+    append_variants_lean_act_cg2(&entries);
+    append_variants_lean_act_trans(&entries);
+    append_variants_gated_cg1(&entries);
+    append_variants_gated_cg2(&entries);
   }
   int base_count = 0;  // the variants without the activation epilogue come first
   // `lean` asks for the variant without the k-split epilogues; where there is none the full
@@ -66,8 +65,7 @@ struct Registry {
   const KernelEntry* find(int tile_n, int cta_group, int epilogue, int transposed, int activation = 0,
                           int lean = 0) const {
     const KernelEntry* full = nullptr;
-    for (int i = 0; i < count; ++i) {
-      const KernelEntry& e = entries[i];
+    for (const KernelEntry& e : entries) {
       if (e.tile_n == tile_n && e.cta_group == cta_group && e.epilogue == epilogue &&
           e.transposed_out == transposed && e.activation == activation) {
         if (e.lean == lean) return &e;
@@ -79,7 +77,7 @@ struct Registry {
 };
 
 const Registry& registry() {
-  static const Registry r;
+  static const Registry& r = *new Registry;  // kept for good: threads may launch while the process exits
   return r;
 }
 
@@ -831,11 +829,11 @@ int ayla_b200_init(int device) {
       g_encode_tiled = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fn);
     }
     const Registry& reg = registry();
-    for (int i = 0; i < reg.count; ++i) {
+    for (size_t i = 0; i < reg.entries.size(); ++i) {
       const KernelEntry& e = reg.entries[i];
       err = cudaFuncSetAttribute(e.func, cudaFuncAttributeMaxDynamicSharedMemorySize, e.smem_bytes);
       if (err != cudaSuccess) {
-        rc = fail(AYLA_B200_E_CUDA, "cudaFuncSetAttribute(smem=%d) for variant %d: %s", e.smem_bytes, i,
+        rc = fail(AYLA_B200_E_CUDA, "cudaFuncSetAttribute(smem=%d) for variant %zu: %s", e.smem_bytes, i,
                   cudaGetErrorString(err));
         break;
       }

@@ -3,14 +3,14 @@
 #include "kernel_registry.h"
 
 namespace ayla_b200 {
-void append_variants_lean_cg1(KernelEntry* out, int* count) {
-  out[(*count)++] = make_entry<64, 1, EPI_PLAIN, false, false, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_PLAIN, false, false, true>();
-  out[(*count)++] = make_entry<192, 1, EPI_PLAIN, false, false, true>();
-  out[(*count)++] = make_entry<256, 1, EPI_PLAIN, false, false, true>();
-  out[(*count)++] = make_entry<64, 1, EPI_BIAS, false, false, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_BIAS, false, false, true>();
-  out[(*count)++] = make_entry<192, 1, EPI_BIAS, false, false, true>();
-  out[(*count)++] = make_entry<256, 1, EPI_BIAS, false, false, true>();
+void append_variants_lean_cg1(std::vector<KernelEntry>* out) {
+  out->push_back(make_entry<64, 1, EPI_PLAIN, false, false, true>());
+  out->push_back(make_entry<128, 1, EPI_PLAIN, false, false, true>());
+  out->push_back(make_entry<192, 1, EPI_PLAIN, false, false, true>());
+  out->push_back(make_entry<256, 1, EPI_PLAIN, false, false, true>());
+  out->push_back(make_entry<64, 1, EPI_BIAS, false, false, true>());
+  out->push_back(make_entry<128, 1, EPI_BIAS, false, false, true>());
+  out->push_back(make_entry<192, 1, EPI_BIAS, false, false, true>());
+  out->push_back(make_entry<256, 1, EPI_BIAS, false, false, true>());
 }
 }  // namespace ayla_b200

@@ -3,14 +3,14 @@
 #include "kernel_registry.h"
 
 namespace ayla_b200 {
-void append_variants_lean_trans(KernelEntry* out, int* count) {
-  out[(*count)++] = make_entry<16, 1, EPI_PLAIN, true, false, true>();
-  out[(*count)++] = make_entry<32, 1, EPI_PLAIN, true, false, true>();
-  out[(*count)++] = make_entry<64, 1, EPI_PLAIN, true, false, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_PLAIN, true, false, true>();
-  out[(*count)++] = make_entry<16, 1, EPI_BIAS, true, false, true>();
-  out[(*count)++] = make_entry<32, 1, EPI_BIAS, true, false, true>();
-  out[(*count)++] = make_entry<64, 1, EPI_BIAS, true, false, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_BIAS, true, false, true>();
+void append_variants_lean_trans(std::vector<KernelEntry>* out) {
+  out->push_back(make_entry<16, 1, EPI_PLAIN, true, false, true>());
+  out->push_back(make_entry<32, 1, EPI_PLAIN, true, false, true>());
+  out->push_back(make_entry<64, 1, EPI_PLAIN, true, false, true>());
+  out->push_back(make_entry<128, 1, EPI_PLAIN, true, false, true>());
+  out->push_back(make_entry<16, 1, EPI_BIAS, true, false, true>());
+  out->push_back(make_entry<32, 1, EPI_BIAS, true, false, true>());
+  out->push_back(make_entry<64, 1, EPI_BIAS, true, false, true>());
+  out->push_back(make_entry<128, 1, EPI_BIAS, true, false, true>());
 }
 }  // namespace ayla_b200

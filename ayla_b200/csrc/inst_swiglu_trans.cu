@@ -3,14 +3,14 @@
 #include "kernel_registry.h"
 
 namespace ayla_b200 {
-void append_variants_swiglu_trans(KernelEntry* out, int* count) {
-  out[(*count)++] = make_entry<16, 1, EPI_SWIGLU, true>();
-  out[(*count)++] = make_entry<32, 1, EPI_SWIGLU, true>();
-  out[(*count)++] = make_entry<64, 1, EPI_SWIGLU, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_SWIGLU, true>();
-  out[(*count)++] = make_entry<16, 1, EPI_SWIGLU, true, false, true>();
-  out[(*count)++] = make_entry<32, 1, EPI_SWIGLU, true, false, true>();
-  out[(*count)++] = make_entry<64, 1, EPI_SWIGLU, true, false, true>();
-  out[(*count)++] = make_entry<128, 1, EPI_SWIGLU, true, false, true>();
+void append_variants_swiglu_trans(std::vector<KernelEntry>* out) {
+  out->push_back(make_entry<16, 1, EPI_SWIGLU, true>());
+  out->push_back(make_entry<32, 1, EPI_SWIGLU, true>());
+  out->push_back(make_entry<64, 1, EPI_SWIGLU, true>());
+  out->push_back(make_entry<128, 1, EPI_SWIGLU, true>());
+  out->push_back(make_entry<16, 1, EPI_SWIGLU, true, false, true>());
+  out->push_back(make_entry<32, 1, EPI_SWIGLU, true, false, true>());
+  out->push_back(make_entry<64, 1, EPI_SWIGLU, true, false, true>());
+  out->push_back(make_entry<128, 1, EPI_SWIGLU, true, false, true>());
 }
 }  // namespace ayla_b200

@@ -5,6 +5,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "gemm_sm100.cuh"
 
 namespace ayla_b200 {
@@ -90,21 +92,21 @@ KernelEntry make_entry() {
 }
 
 // Each instantiation unit contributes its variants.
-void append_variants_cg1(KernelEntry* out, int* count);
-void append_variants_cg2(KernelEntry* out, int* count);
-void append_variants_trans(KernelEntry* out, int* count);
-void append_variants_swiglu(KernelEntry* out, int* count);
-void append_variants_swiglu_trans(KernelEntry* out, int* count);
-void append_variants_act_cg1(KernelEntry* out, int* count);
-void append_variants_act_cg2(KernelEntry* out, int* count);
-void append_variants_act_trans(KernelEntry* out, int* count);
-void append_variants_lean_cg1(KernelEntry* out, int* count);
-void append_variants_lean_cg2(KernelEntry* out, int* count);
-void append_variants_lean_trans(KernelEntry* out, int* count);
-void append_variants_lean_act_cg1(KernelEntry* out, int* count);
-void append_variants_lean_act_cg2(KernelEntry* out, int* count);
-void append_variants_gated_cg1(KernelEntry* out, int* count);
-void append_variants_gated_cg2(KernelEntry* out, int* count);
-void append_variants_lean_act_trans(KernelEntry* out, int* count);
+void append_variants_cg1(std::vector<KernelEntry>* out);
+void append_variants_cg2(std::vector<KernelEntry>* out);
+void append_variants_trans(std::vector<KernelEntry>* out);
+void append_variants_swiglu(std::vector<KernelEntry>* out);
+void append_variants_swiglu_trans(std::vector<KernelEntry>* out);
+void append_variants_act_cg1(std::vector<KernelEntry>* out);
+void append_variants_act_cg2(std::vector<KernelEntry>* out);
+void append_variants_act_trans(std::vector<KernelEntry>* out);
+void append_variants_lean_cg1(std::vector<KernelEntry>* out);
+void append_variants_lean_cg2(std::vector<KernelEntry>* out);
+void append_variants_lean_trans(std::vector<KernelEntry>* out);
+void append_variants_lean_act_cg1(std::vector<KernelEntry>* out);
+void append_variants_lean_act_cg2(std::vector<KernelEntry>* out);
+void append_variants_gated_cg1(std::vector<KernelEntry>* out);
+void append_variants_gated_cg2(std::vector<KernelEntry>* out);
+void append_variants_lean_act_trans(std::vector<KernelEntry>* out);
 
 }  // namespace ayla_b200
