@@ -51,26 +51,33 @@ TRACE_LIB_PATH = LIB_DIR / "libayla_b200_trace.so"
 
 DISPATCH_SOURCE = CSRC / "torch_dispatch.cpp"
 DISPATCH_PATH = LIB_DIR / "_torch_dispatch.so"
+DISPATCH_STAMP = BUILD_DIR / "torch_dispatch.stamp"
 
 
 def build_dispatch(verbose: bool = False, force: bool = False) -> Path:
-    if not force and DISPATCH_PATH.exists() and DISPATCH_PATH.stat().st_mtime >= DISPATCH_SOURCE.stat().st_mtime:
-        return DISPATCH_PATH
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
 
-    LIB_DIR.mkdir(exist_ok=True)
-    includes = [*include_paths(), "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
+    includes = [*include_paths("cuda"), sysconfig.get_paths()["include"]]
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            *[f"-isystem{path}" for path in includes], str(DISPATCH_SOURCE), "-o", str(DISPATCH_PATH),
            *[f"-L{path}" for path in library_paths()],
            "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    # What it was built for: another torch or Python may not load it, or worse, load it.
+    stamp = "\n".join([torch.__version__, sys.version, *cmd])
+    if (not force and DISPATCH_PATH.exists() and DISPATCH_STAMP.exists() and DISPATCH_STAMP.read_text() == stamp
+            and DISPATCH_PATH.stat().st_mtime >= DISPATCH_SOURCE.stat().st_mtime):
+        return DISPATCH_PATH
+    LIB_DIR.mkdir(exist_ok=True)
+    BUILD_DIR.mkdir(exist_ok=True)
+    DISPATCH_STAMP.unlink(missing_ok=True)
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or proc.returncode != 0:
         sys.stderr.write(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
     if proc.returncode != 0:
         raise RuntimeError(f"building {DISPATCH_PATH.name} failed")
+    DISPATCH_STAMP.write_text(stamp)
     return DISPATCH_PATH
 
 

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import warnings
 from collections.abc import Callable
 from functools import cache
 from pathlib import Path
@@ -24,14 +25,20 @@ _PATH = Path(__file__).resolve().parent / "lib" / "_torch_dispatch.so"
 
 
 @cache
-def load() -> ModuleType:
-    if not _PATH.exists():
-        raise ImportError(f"{_PATH} not found: build it with `python -m ayla_b200.build`")
-    spec = importlib.util.spec_from_file_location("_torch_dispatch", _PATH)
-    assert spec is not None and spec.loader is not None
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
-    return module
+def load() -> ModuleType | None:
+    """The compiled dispatcher.  ``None``, with a warning, where it is missing or does not load (it is built for one
+    torch and one Python): the ops keep their Python implementation then, which launches the same kernels at some
+    8 us of host time more per call."""
+    try:
+        spec = importlib.util.spec_from_file_location("_torch_dispatch", _PATH)
+        assert spec is not None and spec.loader is not None
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except (ImportError, OSError) as error:
+        warnings.warn(f"the compiled op dispatcher cannot be used, calls go through Python: {error}; "
+                      "build it with `python -m ayla_b200.build`", RuntimeWarning, stacklevel=2)
+        return None
 
 
 _MAX_OPERANDS = 5  # kMaxOperands of the compiled dispatcher
@@ -40,12 +47,12 @@ _MAX_OPERANDS = 5  # kMaxOperands of the compiled dispatcher
 def serves(launcher, kinds: list[OperandKind]) -> bool:
     """Whether the compiled dispatcher can stand in for ``launcher``: a per-shape dispatcher itself (a subclass
     may do something else on a call), whose operands are the op's arguments, all of one dtype, the last one
-    written."""
+    written -- and it is there to do so."""
     if type(launcher) is not ShapeSpecializingJITCompiler:
         return False
     signature = launcher.signature
     return (len(signature) <= _MAX_OPERANDS and len({spec.dtype for spec in signature}) == 1 and
-            kinds == [OperandKind.R] * (len(signature) - 1) + [OperandKind.RW])
+            kinds == [OperandKind.R] * (len(signature) - 1) + [OperandKind.RW] and load() is not None)
 
 
 def register(namespace: str, name: str, compiler: ShapeSpecializingJITCompiler) -> None:

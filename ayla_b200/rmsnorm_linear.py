@@ -48,7 +48,10 @@ def _row_factors_op(dtype: str) -> torch._ops.OpOverload:
 
     lib = _library(DEFAULT_NAMESPACE)
     lib.define(f"{name}(Tensor arg0, float eps, Tensor(a1!) arg1) -> ()")
-    native_dispatch.register_rms_factors(DEFAULT_NAMESPACE, name, dtype, _TORCH_DTYPES[dtype], cuda_impl)
+    if native_dispatch.load() is not None:
+        native_dispatch.register_rms_factors(DEFAULT_NAMESPACE, name, dtype, _TORCH_DTYPES[dtype], cuda_impl)
+    else:
+        lib.impl(name, cuda_impl, "CUDA")
     lib.impl(name, lambda x, eps, factors: None, "Meta")
     return getattr(getattr(torch.ops, DEFAULT_NAMESPACE), name).default
 

@@ -1,6 +1,8 @@
 """Custom-op glue on the meta device -- mirrors the reference's
 tests/test_torch_custom_call.py:8-53."""
 
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -85,3 +87,61 @@ def test_per_shape_dispatchers_of_any_signature_become_ops(name, cls, dtypes, wr
     assert op(*[torch.empty(4, 8, dtype=dtype, device="meta") for dtype in dtypes]) is None
     assert torch._C._dispatch_has_kernel_for_dispatch_key(f"ayla_b200_signatures_test::{name}", "CUDA")
     assert compiled == (["plain"] if name == "plain" else [])
+
+
+_WITHOUT_THE_EXTENSION = """
+import sys, warnings
+from pathlib import Path
+import torch
+from ayla_b200 import native_dispatch
+path = Path(sys.argv[1])
+if sys.argv[2] == "broken":
+    path.write_bytes(b"not a shared object")
+native_dispatch._PATH = path
+with warnings.catch_warnings(record=True) as caught:
+    warnings.simplefilter("always")
+    from ayla_b200 import gemm_op, swiglu_op
+    from ayla_b200.rmsnorm_linear import rms_norm_linear
+    def empty(*shape):
+        return torch.empty(*shape, dtype=torch.bfloat16, device="meta")
+    assert gemm_op("mm", "bfloat16")(empty(8, 64), empty(16, 64), empty(8, 16)) is None
+    assert swiglu_op("bfloat16")(empty(8, 64), empty(16, 64), empty(16, 64), empty(8, 16)) is None
+    assert rms_norm_linear(empty(8, 64), empty(16, 64)).shape == (8, 16)
+assert sum("go through Python" in str(w.message) for w in caught) == 1, [str(w.message) for w in caught]
+for name in ("jit_mm_bf16", "swiglu_bf16", "rms_row_factors_bf16"):
+    assert torch._C._dispatch_has_kernel_for_dispatch_key("ayla::" + name, "CUDA")
+"""
+
+
+@pytest.mark.parametrize("state", ["missing", "broken"])
+def test_ops_without_the_compiled_dispatcher(state, tmp_path):
+    """A missing or unloadable extension is reported once; the ops keep their Python implementation."""
+    import subprocess
+    import sys
+
+    subprocess.run([sys.executable, "-c", _WITHOUT_THE_EXTENSION, str(tmp_path / "_torch_dispatch.so"), state],
+                   check=True, cwd=Path(__file__).resolve().parent.parent)
+
+
+def test_the_compiled_dispatcher_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    import types
+
+    from ayla_b200 import build
+
+    (tmp_path / "source.cpp").write_text("")
+    for name, path in (("DISPATCH_SOURCE", "source.cpp"), ("DISPATCH_PATH", "out.so"), ("DISPATCH_STAMP", "stamp")):
+        monkeypatch.setattr(build, name, tmp_path / path)
+    built = []
+
+    def compile_it(cmd, **kwargs):
+        built.append(cmd)
+        (tmp_path / "out.so").write_text("")
+        return types.SimpleNamespace(returncode=0, stdout="", stderr="")
+
+    monkeypatch.setattr(build.subprocess, "run", compile_it)
+    build.build_dispatch()
+    build.build_dispatch()
+    assert len(built) == 1
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    build.build_dispatch()
+    assert len(built) == 2
