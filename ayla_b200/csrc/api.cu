@@ -463,6 +463,17 @@ int current_device_state(DeviceState** out, int* device) {
   return AYLA_B200_OK;
 }
 
+// For queries, which need no device: the current device's SM count where it has been set up, else a B200's.
+int current_sm_count() {
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
+      g_devices[dev].ready.load(std::memory_order_acquire)) {
+    return g_devices[dev].sm_count;
+  }
+  (void)cudaGetLastError();
+  return 148;
+}
+
 void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count,
                     ayla_b200_config* c) {
   memset(c, 0, sizeof(*c));
@@ -864,15 +875,7 @@ int ayla_b200_default_config(int op, int dtype, int64_t batch, int64_t m, int64_
   if (cfg_out == nullptr) return fail(AYLA_B200_E_INVALID, "cfg_out is null");
   const int rc = check_shape(op, dtype, batch, m, n, k);
   if (rc) return rc;
-  int sm_count = 148;
-  int dev = -1;
-  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
-      g_devices[dev].ready.load(std::memory_order_acquire)) {
-    sm_count = g_devices[dev].sm_count;
-  } else {
-    (void)cudaGetLastError();
-  }
-  default_config(batch, m, n, k, sm_count, cfg_out);
+  default_config(batch, m, n, k, current_sm_count(), cfg_out);
   return AYLA_B200_OK;
 }
 
@@ -1052,7 +1055,7 @@ int ayla_b200_gemm_packed(int op, int dtype, const void* bias, const void* a, co
 
 int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k) {
   if (check_shape(op, AYLA_B200_BF16, batch, m, n, k) != AYLA_B200_OK) return 0;
-  return packed_preferred(batch, m, n, k, 148) ? 1 : 0;
+  return packed_preferred(batch, m, n, k, current_sm_count()) ? 1 : 0;
 }
 
 int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const void* a, const void* bt,

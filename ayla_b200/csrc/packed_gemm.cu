@@ -335,11 +335,28 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
 
 constexpr int kSmemPerSm = 233472, kSmemPerCta = 232448, kCtaReserve = 1024;
 
-// As many matrices to a unit as its quarters of 32 rows and its columns hold.
-int matrices_per_unit(int64_t batch, int64_t m, int64_t n) {
-  int matrices = 1;
-  while (batch > 1 && matrices < 4 && m * matrices * 2 <= kRows && n * matrices * 2 <= kPackedMaxN) matrices *= 2;
-  return matrices;
+// How a problem lies in shared memory and how many CTAs of it an SM holds.
+struct Footprint {
+  int matrices;  // small matrices per unit: as many as the accumulator's quarters of 32 rows and its columns hold
+  int mma_n, narrow, k_blocks;
+  int staging_pitch;
+  int smem, ctas;
+};
+
+Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
+  Footprint f;
+  f.matrices = 1;
+  while (batch > 1 && f.matrices < 4 && m * f.matrices * 2 <= kRows && n * f.matrices * 2 <= kPackedMaxN) f.matrices *= 2;
+  f.mma_n = static_cast<int>((n * f.matrices + 15) / 16 * 16);
+  f.narrow = k <= 16 ? 2 : k <= 32 ? 1 : 0;
+  f.k_blocks = static_cast<int>((k + 63) / 64);
+  // An odd number of 16-byte pieces per staging row: eight lanes writing a piece of eight rows meet eight banks.
+  f.staging_pitch = 16 * static_cast<int>((n / 8) | 1);
+  const int a_bytes = (f.k_blocks * kRows * 128) >> f.narrow, b_bytes = (f.k_blocks * f.mma_n * 128) >> f.narrow;
+  f.smem = kStages * a_bytes + (batch == 1 ? 1 : kStages) * b_bytes + kRows * f.staging_pitch + kPackedMaxN * 4 + 64;
+  f.ctas = kSmemPerSm / (f.smem + kCtaReserve);
+  if (f.ctas > kMaxCtasPerSm) f.ctas = kMaxCtasPerSm;
+  return f;
 }
 
 }  // namespace
@@ -352,27 +369,45 @@ cudaError_t init_packed_gemm() {
                               cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
 }
 
-// Where this kernel is the faster one (us, general -> packed; 88 shapes of up to 128 columns and a depth of up to
-// 128 measured):
-//  * from one 128-row tile per SM on; below, both are a launch and one pass (bmm 8 x 1024x64x64 2.8 -> 3.5);
-//  * matrices that share an accumulator: 574 x 15x16x32 5.4 -> 2.6, 1024 x 64x64x64 8.7 -> 7.3;
-//  * rows shorter than the general kernel's 64-deep boxes: 200704x96x48 21.6 -> 15.5.  Not with rows of exactly 32
-//    against more than 64 columns of a bmm, whose outputs dominate: 512 x 128x128x32 7.8 -> 9.1;
-//  * few columns: 1698 x 118x24x104 17.4 -> 14.5, 100352x48x96 11.1 -> 9.8; with more columns and a depth of 64 and
-//    above two CTAs or one fit an SM and the general kernel wins: 89 x 509x128x64 6.3 -> 8.6, 1412 x 61x128x72
-//    19.5 -> 28.0;
-//  * rows that start in the middle of a 32-byte sector cost the general kernel's TMA loads twice, which one B for
-//    all units makes up for up to 96 columns: 153121x88x72 29.0 -> 16.1.
+// Where this kernel is the faster one.  1276 shapes of up to 128 columns and a depth of up to 128 were timed on both
+// (graph replay, operands past L2): by this rule the geometric mean is 0.739 of the general kernel's time, ten shapes
+// are slower by 3 to 10 %, 39 that this kernel would do in less than 0.9 stay with the general one; choosing the
+// faster one every time would give 0.732.  What it goes by (us, general -> packed):
+//  * a 128-row tile for every SM; below, both are a launch and one pass (bmm 8 x 1024x64x64 2.8 -> 3.5).
+//  * Small matrices that share an accumulator gain most (1024 x 64x64x64 8.7 -> 7.3, 574 x 15x16x32 5.4 -> 2.6), as
+//    long as two CTAs fit an SM or four matrices a unit (7467 x 17x48x104, one CTA: 42.5 -> 47.9).
+//  * Otherwise resident CTAs hide a unit's chain of load, MMA and epilogue: with one per SM nothing does (512 x
+//    128x72x104 8.4 -> 10.3), four always do up to 64 columns, and with three or two it takes an advantage besides:
+//    few columns, or rows that start in the middle of a 32-byte sector, which cost the general kernel's TMA loads
+//    twice (200 x 500x56x72 10.1 -> 9.1, but 200 x 500x48x128 9.1 -> 10.0 and 200 x 500x128x56 9.3 -> 12.9), or one B
+//    for all units (162131x72x48 0.60 of the general time, 4252 x 85x112x48 1.46).
+//  * A second round of units that fills less than a third of the resident CTAs is a round all the same (512 x
+//    128x72x56, 1.15 rounds: 7.6 -> 8.2); so is a first one that leaves half of them without work, at a depth where
+//    the general kernel is quick (19815x64x48 1.09, 170 x 110x64x56 1.10).
+//  * A product of one 16-byte piece in depth with shared B, in a single round (60000x64x8 8.6 -> 10.8; 131072x64x8, in
+//    two, 16.0 -> 13.7).
 bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count) {
   if (n > kPackedMaxN || k > kPackedMaxK) return false;
   const int64_t tiles = batch * ((m + kRows - 1) / kRows);
   if (tiles < sm_count || tiles > 0x7FFFFFFF) return false;
-  if (matrices_per_unit(batch, m, n) > 1 || n <= 48) return true;
-  if (k < 64) return k != 32 || n <= 64 || batch == 1;
-  return batch == 1 && k % 16 != 0 && n <= 96;
+  const Footprint f = footprint(batch, m, n, k);
+  if (f.matrices > 1) return f.matrices == 4 || f.ctas >= 2;
+  if (f.ctas < 2) return false;
+  const bool shared_b = batch == 1, mid_sector = k % 16 != 0;
+  if (n <= 32) return shared_b || f.ctas >= 3 || mid_sector;
+  const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);
+  if (shared_b && k < 16 && n > 40) return rounds >= 1.35;
+  if (k > 32 && rounds < 0.5) return false;
+  const bool settled = rounds <= 0.95 || rounds >= 1.35;
+  if (f.ctas >= 4) return n <= 64 || mid_sector || settled;
+  if (!settled) return false;
+  if (f.ctas == 3) return n <= 64 || (shared_b ? rounds >= 1.35 : mid_sector || (k <= 32 && rounds >= 2.0));
+  if (mid_sector) return n <= 64 || (shared_b && (n <= 96 || rounds >= 1.35));
+  return shared_b && n <= 64 && rounds >= 1.35;
 }
 
 cudaError_t launch_packed_gemm(const PackedProblem& pr) {
+  const Footprint f = footprint(pr.batch, pr.m, pr.n, pr.k);
   PackedParams p = {};
   p.a = static_cast<const uint8_t*>(pr.a);
   p.b = static_cast<const uint8_t*>(pr.b);
@@ -382,17 +417,16 @@ cudaError_t launch_packed_gemm(const PackedProblem& pr) {
   p.m = static_cast<int>(pr.m);
   p.n = static_cast<int>(pr.n);
   p.k_chunks = static_cast<int>(pr.k / 8);
-  p.k_blocks = static_cast<int>((pr.k + 63) / 64);
-  p.matrices = matrices_per_unit(pr.batch, pr.m, pr.n);
+  p.k_blocks = f.k_blocks;
+  p.matrices = f.matrices;
   p.slot_rows = kRows / p.matrices;
   p.row_tiles = (p.m + kRows - 1) / kRows;
   p.units = p.matrices == 1 ? p.batch * p.row_tiles : (p.batch + p.matrices - 1) / p.matrices;
-  p.mma_n = (p.n * p.matrices + 15) / 16 * 16;
+  p.mma_n = f.mma_n;
   p.shared_b = p.batch == 1 ? 1 : 0;
-  p.narrow = pr.k <= 16 ? 2 : pr.k <= 32 ? 1 : 0;
+  p.narrow = f.narrow;
   p.idesc = pr.idesc_base | (static_cast<uint32_t>(p.mma_n >> 3) << 17);
-  // An odd number of 16-byte pieces per staging row: eight lanes writing a piece of eight rows meet eight banks.
-  p.staging_pitch = 16u * static_cast<uint32_t>((p.n / 8) | 1);
+  p.staging_pitch = static_cast<uint32_t>(f.staging_pitch);
   p.load_rows = kThreads / p.k_chunks;
   p.load_threads = p.load_rows * p.k_chunks;
   p.div_k_chunks = FastDiv::make(static_cast<uint32_t>(p.k_chunks));
@@ -404,17 +438,12 @@ cudaError_t launch_packed_gemm(const PackedProblem& pr) {
   p.tmem_cols = 32;
   while (p.tmem_cols < p.mma_n) p.tmem_cols *= 2;
 
-  const int a_bytes = (p.k_blocks * kRows * 128) >> p.narrow, b_bytes = (p.k_blocks * p.mma_n * 128) >> p.narrow;
-  const int fixed = kRows * static_cast<int>(p.staging_pitch) + kPackedMaxN * 4 + 64;
-  const int smem = kStages * a_bytes + (p.shared_b ? 1 : kStages) * b_bytes + fixed;
-  int ctas = kSmemPerSm / (smem + kCtaReserve);
-  if (ctas > kMaxCtasPerSm) ctas = kMaxCtasPerSm;
-  const int64_t room = static_cast<int64_t>(ctas) * pr.sm_count;
+  const int64_t room = static_cast<int64_t>(f.ctas) * pr.sm_count;
 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.units < room ? p.units : room));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.dynamicSmemBytes = static_cast<size_t>(f.smem);
   cfg.stream = pr.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

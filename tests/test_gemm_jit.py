@@ -353,3 +353,20 @@ def test_the_suite_times_the_kernel_the_ops_run(packed, monkeypatch):
     else:
         assert config.to_dict() == select_gemm_schedule("mm", "bfloat16", 65536, 32, 32).builder_config
         assert source in ("table", "default")
+
+
+@pytest.mark.parametrize("operation, batch, m, n, k, packed", [
+    # The ops' shapes it is made for.
+    ("bmm", 8192, 56, 32, 56, True), ("mm", 1, 200704, 96, 24, True), ("bmm", 1024, 64, 64, 64, True),
+    ("bmm", 574, 15, 16, 32, True), ("mm", 1, 153121, 88, 72, True), ("bmm", 200, 500, 56, 72, True),
+    # Measured slower on it: a unit of two matrices at one CTA per SM, ...
+    ("bmm", 7467, 17, 48, 104, False), ("bmm", 3375, 41, 56, 120, False), ("bmm", 2668, 47, 40, 112, False),
+    # ... wide outputs at two CTAs, aligned rows at two CTAs, ...
+    ("bmm", 200, 500, 128, 56, False), ("bmm", 4252, 85, 112, 48, False), ("mm", 1, 229347, 128, 48, False),
+    ("bmm", 200, 500, 48, 128, False), ("bmm", 244, 1728, 16, 128, False),
+    # ... a thin second round, a thin first one, a depth of one piece, fewer tiles than SMs.
+    ("bmm", 512, 128, 72, 56, False), ("mm", 1, 21325, 64, 64, False), ("mm", 1, 60000, 64, 8, False),
+    ("bmm", 8, 1024, 64, 64, False),
+])
+def test_the_packed_kernel_is_preferred_where_it_measured_faster(operation, batch, m, n, k, packed):
+    assert _lib.packed_preferred(operation, batch, m, n, k) is packed
