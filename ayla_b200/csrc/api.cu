@@ -474,7 +474,32 @@ int current_sm_count() {
   return 148;
 }
 
-void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count,
+// Whether the tiles chosen for a product of at most four k-blocks are better run by CTA pairs, which read half as much
+// of B.  170 shapes timed in both forms: with this rule the paired ones take 0.946 of the time without an activation
+// (the slowest 1.05), the others would take 1.035.  us, single -> pair:
+//  * from two waves of 256-wide tiles on, and of 128-wide ones of three or four k-blocks (mm 8216x4976x104 29.1 -> 24.1,
+//    15515x1592x128 14.8 -> 14.1, addmm 12010x552x192 8.8 -> 8.6; in one wave pairing only adds set-up: mm
+//    1236x6728x192 7.5 -> 7.7, 3755x816x192 5.1 -> 5.3; 128-wide tiles of two k-blocks: mm 2437x1696x96 5.0 -> 5.3);
+//  * from one wave on where rows start in the middle of a 32-byte sector, so that B's are read twice (addmm
+//    10684x280x216 8.7 -> 7.3, mm 9609x552x120 7.7 -> 6.6);
+//  * not where 256-row tiles add much padding to the rows (bmm 28 x 1873x1576x128, 7 %: 40.5 -> 46.6; 82 x
+//    1335x1064x128, 9 %: 58.5 -> 72.8), more of which a deeper or misaligned product bears (bmm 26 x 830x1264x256, 14 %:
+//    21.4 -> 19.6);
+//  * behind an activation less: the padding rows pass through it too (bmm 26 x 830x1264x256 with SiLU 1.12), and from
+//    four waves on its epilogue bounds the launch in either form (GELU: 0.96 to 1.06, 1.007 in the mean).
+bool shallow_pairs_pay(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_n, int activation, int sm_count) {
+  const int64_t k_blocks = ceil_div(k, 64);
+  if (k_blocks > 4 || m < 256 || tile_n < 128) return false;
+  const bool mid_sector = k % 16 != 0;
+  const int64_t row_tiles = ceil_div(m, 128);
+  const double growth = static_cast<double>(2 * ceil_div(m, 256)) / static_cast<double>(row_tiles);
+  if (growth > (activation == AYLA_B200_ACT_NONE && (k_blocks >= 3 || mid_sector) ? 1.2 : 1.03)) return false;
+  const double waves = static_cast<double>(batch * row_tiles * ceil_div(n, tile_n)) / sm_count;
+  if (activation > AYLA_B200_ACT_RELU && waves >= 4.0) return false;
+  return mid_sector ? waves >= 1.0 : waves >= 2.0 && (tile_n == 256 || k_blocks >= 3);
+}
+
+void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, int sm_count,
                     ayla_b200_config* c) {
   memset(c, 0, sizeof(*c));
   c->cta_group = 1;
@@ -528,16 +553,10 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count
                                    {128, 1, 0.62}, {64, 2, 0.50}, {64, 1, 0.40}};
   double best_cost = 1e300;
   for (const Shape& sh : kShapes) {
-    if (sh.cta_group == 2 && m <= 128) continue;
+    if (sh.cta_group == 2 && (m <= 128 || k_blocks <= 4)) continue;  // shallow K: see shallow_pairs_pay
     if (sh.tile_n > 64 && n * 2 <= sh.tile_n) continue;
     const int64_t ctas = sm_count / sh.cta_group;
     const int64_t tiles = batch * ceil_div(m, 128 * sh.cta_group) * ceil_div(n, sh.tile_n);
-    // Shallow K: below two waves pairing only adds set-up, and a matrix of less than one pair's rows gains nothing
-    // from it; from there on it halves what the SMs read of B, and that traffic bounds them (us, single -> pair: bmm
-    // 16 x 2000x2000x128 28.0 -> 26.1, 128 x 256x1024x80 18.3 -> 16.7, 37 x 1500x704x96 20.7 -> 19.7, addmm
-    // 12095x5824x256 44.2 -> 41.4, the same with a GELU 73.2 -> 74.8; mm 1000x1000x256 5.4 -> 5.5, bmm
-    // 100 x 129x1000x64 12.4 -> 13.1).
-    if (sh.cta_group == 2 && k_blocks <= 4 && (m < 256 || tiles < 2 * ctas)) continue;
     const double tile_cost = (sh.tile_n / 256.0) / sh.eff * static_cast<double>(k_blocks);
     const double launch_cost = 6.0 + sh.tile_n / 64.0;
     for (int split = 1; split <= 16; split *= 2) {
@@ -571,6 +590,11 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count
         c->cluster_split = cluster ? 1 : 0;
       }
     }
+  }
+  if (c->cta_group == 1 && c->split_k == 1 && shallow_pairs_pay(batch, m, n, k, c->tile_n, activation, sm_count)) {
+    c->cta_group = 2;
+    const int64_t pairs = sm_count / 2, tiles = batch * ceil_div(m, 256) * ceil_div(n, c->tile_n), rest = tiles % pairs;
+    c->split_tail = tiles > pairs && rest != 0 && rest * 2 <= pairs ? 2 : 0;
   }
   // bt is streamed (evict-first) only while every row tile that needs a column tile's slab runs
   // in the same raster group; with more row tiles than that it is read again later and is kept.
@@ -872,10 +896,18 @@ int ayla_b200_init(int device) {
 
 int ayla_b200_default_config(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                              ayla_b200_config* cfg_out) {
+  return ayla_b200_default_config_act(op, dtype, AYLA_B200_ACT_NONE, batch, m, n, k, cfg_out);
+}
+
+int ayla_b200_default_config_act(int op, int dtype, int activation, int64_t batch, int64_t m, int64_t n, int64_t k,
+                                 ayla_b200_config* cfg_out) {
   if (cfg_out == nullptr) return fail(AYLA_B200_E_INVALID, "cfg_out is null");
   const int rc = check_shape(op, dtype, batch, m, n, k);
   if (rc) return rc;
-  default_config(batch, m, n, k, current_sm_count(), cfg_out);
+  if (activation < AYLA_B200_ACT_NONE || activation > AYLA_B200_ACT_GELU_TANH) {
+    return fail(AYLA_B200_E_INVALID, "unknown activation %d", activation);
+  }
+  default_config(batch, m, n, k, activation, current_sm_count(), cfg_out);
   return AYLA_B200_OK;
 }
 
@@ -982,7 +1014,7 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   } else if (activation == AYLA_B200_ACT_NONE && mul == nullptr && packed_preferred(batch, m, n, k, ds->sm_count)) {
     return ayla_b200_gemm_packed(op, dtype, bias, a, bt, out, batch, m, n, k, status, stream);
   } else {
-    default_config(batch, m, n, k, ds->sm_count, &c);
+    default_config(batch, m, n, k, activation, ds->sm_count, &c);
   }
   rc = check_config(c, false);
   if (rc) return rc;
@@ -1080,7 +1112,7 @@ int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const voi
   if (cfg != nullptr) {
     c = *cfg;
   } else {
-    default_config(batch, m, n, k, ds->sm_count, &c);
+    default_config(batch, m, n, k, AYLA_B200_ACT_NONE, ds->sm_count, &c);
   }
   rc = check_config(c, false);
   if (rc) return rc;

@@ -140,12 +140,13 @@ def measured_gemm_configs(operation: str, dtype: str, m: int, n: int, k: int,
 
 
 def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
-                         batch: int = 1) -> GemmScheduleSeed | None:
+                         batch: int = 1, activation: str = "none") -> GemmScheduleSeed | None:
     """The schedule a launch of this shape uses, or ``None`` if the shape is unsupported.
 
     An exact table hit has empty ``adaptations``; a schedule transferred from a
     nearby measured shape names that shape; otherwise the library's shape-aware
-    default is returned with ``source_shape`` ``None``.  It is a schedule of the general
+    default, which takes the fused ``activation`` into account, is returned with
+    ``source_shape`` ``None``.  It is a schedule of the general
     kernel: plain products that ``packed_serves`` run on the packed kernel, which takes none.
     """
     if min(batch, m, n, k) <= 0 or operation not in _OPERATIONS:
@@ -180,17 +181,17 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
                                             (*seed.adaptations, f"measured in {other}"), seed.source_shape,
                                             seed.source_percentage_of_torch)
                 return seed
-    return _fallback_schedule(operation, dtype, m, n, k, batch)
+    return _fallback_schedule(operation, dtype, m, n, k, batch, activation)
 
 
 def _fallback_schedule(operation: str, dtype: str, m: int, n: int, k: int,
-                       batch: int = 1) -> GemmScheduleSeed | None:
-    """Unmeasured schedule from the library's heuristic (ayla_b200_default_config)."""
+                       batch: int = 1, activation: str = "none") -> GemmScheduleSeed | None:
+    """Unmeasured schedule from the library's heuristic (ayla_b200_default_config_act)."""
     if not _shape_supported(m, n, k, batch) or dtype not in _SHORT_DTYPES:
         return None
     if operation not in _OPERATIONS or (operation != "bmm" and batch != 1):
         return None
-    captured = {**_DEFAULTS, **_lib.default_config(operation, dtype, batch, m, n, k).to_dict()}
+    captured = {**_DEFAULTS, **_lib.default_config(operation, dtype, batch, m, n, k, activation).to_dict()}
     return GemmScheduleSeed(
         captured,
         _builder_config(captured),
@@ -403,10 +404,10 @@ def gemm_jit_compiler(operation: str, dtype: str, activation: str = "none",
             raise ValueError(f"{bound.name}: the row factors must be {(*lead, m, 1)}, got {tuple(mul)}")
         if gated is True and tuple(mul) != tuple(out):
             raise ValueError(f"{bound.name}: mul must have the shape of out {tuple(out)}, got {tuple(mul)}")
-        schedule = select_gemm_schedule(operation, dtype, m, n, k, *batch)
+        count = batch[0] if batch else 1
+        schedule = select_gemm_schedule(operation, dtype, m, n, k, count, activation)
         if schedule is None:
             raise ValueError(f"{bound.name}: no schedule for {operation} {lead}x{m}x{n}x{k}")
-        count = batch[0] if batch else 1
         return GemmLauncher(operation, dtype, count, m, n, k, schedule, device, activation, gated,
                             packed_serves(operation, count, m, n, k, device, activation, gated))
 

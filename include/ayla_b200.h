@@ -250,6 +250,10 @@ AYLA_B200_API int ayla_b200_rms_factors(int dtype, const void* x, void* factors,
 AYLA_B200_API int ayla_b200_default_config(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                              ayla_b200_config* cfg_out);
 
+/* The same for ayla_b200_gemm_act and its relatives, whose epilogue's cost enters into the choice. */
+AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation, int64_t batch, int64_t m,
+                                               int64_t n, int64_t k, ayla_b200_config* cfg_out);
+
 /*
  * 0 if `cfg` can run the given problem, else an error code (message in
  * ayla_b200_last_error).  Counterpart of _legal (ayla/gemm_jit.py:115-138).

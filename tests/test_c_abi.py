@@ -151,3 +151,21 @@ def test_gemm_rejects_bad_arguments_before_touching_the_device():
     assert lib.ayla_b200_swiglu(1, one, one, None, one, 64, 64, 64, None, None, None) == _lib.E_INVALID
     with pytest.raises(ValueError, match="multiple of 8"):
         _lib.check(lib.ayla_b200_gemm(0, 1, None, one, one, one, 1, 64, 65, 64, None, None, 0, None, None))
+
+
+@pytest.mark.parametrize("op, batch, m, n, k, tile_n, plain, gelu", [
+    # Tiles of a shallow product: the width that the cost model picks for single CTAs, paired where that measured
+    # faster -- wide tiles of two waves and more, rows that start inside a sector; not behind a GELU of many waves ...
+    ("mm", 1, 12095, 5824, 256, 256, 2, 1), ("addmm", 1, 10351, 3728, 224, 256, 2, 1), ("mm", 1, 8216, 4976, 104, 256, 2, 1),
+    ("mm", 1, 11696, 520, 88, 128, 2, 2),
+    # ... not 128-wide tiles of two k-blocks, a single wave, or rows that pairs would pad ...
+    ("addmm", 1, 10600, 520, 64, 128, 1, 1), ("mm", 1, 1667, 3912, 96, 128, 1, 1), ("bmm", 28, 1873, 1576, 128, 256, 1, 1),
+    ("bmm", 53, 310, 528, 128, 128, 1, 1), ("mm", 1, 3755, 816, 192, 128, 1, 1),
+    # ... and never another width than single CTAs would take (22.5 us as 256 wide, 26.2 as 128-wide pairs; 6.5 and 7.9).
+    ("addmm", 1, 12751, 3104, 64, 256, 2, 1), ("addmm", 1, 824, 4232, 88, 128, 2, 1),
+])
+def test_shallow_products_are_paired_where_it_measured_faster(op, batch, m, n, k, tile_n, plain, gelu):
+    for activation, pairing in (("none", plain), ("gelu", gelu)):
+        cfg = _lib.default_config(op, "bfloat16", batch, m, n, k, activation)
+        assert (cfg.tile_n, cfg.cta_group) == (tile_n, pairing), (activation, cfg.to_dict())
+        assert _lib.config_valid(cfg, op, "bfloat16", batch, m, n, k)
