@@ -32,6 +32,7 @@ EXPORTS = (
     "ayla_b200_rms_factors",
     "ayla_b200_default_config",
     "ayla_b200_default_config_act",
+    "ayla_b200_swiglu_default_config",
     "ayla_b200_config_valid",
     "ayla_b200_workspace_bytes",
     "ayla_b200_workspace_counter_bytes",
@@ -141,6 +142,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_default_config.restype = i32
         lib.ayla_b200_default_config_act.argtypes = [i32, i32, i32, i64, i64, i64, i64, cfgp]
         lib.ayla_b200_default_config_act.restype = i32
+        lib.ayla_b200_swiglu_default_config.argtypes = [i32, i64, i64, i64, cfgp]
+        lib.ayla_b200_swiglu_default_config.restype = i32
         lib.ayla_b200_config_valid.argtypes = [cfgp, i32, i32, i64, i64, i64, i64]
         lib.ayla_b200_config_valid.restype = i32
         lib.ayla_b200_workspace_bytes.argtypes = [cfgp, i32, i64, i64, i64, i64]
@@ -235,6 +238,12 @@ def default_config(op: str, dtype: str, batch: int, m: int, n: int, k: int, acti
     cfg = Config()
     check(load().ayla_b200_default_config_act(OP_CODES[op], DTYPE_CODES[dtype], ACT_CODES[activation], batch, m, n, k,
                                               ctypes.byref(cfg)))
+    return cfg
+
+
+def swiglu_default_config(dtype: str, m: int, n: int, k: int) -> Config:
+    cfg = Config()
+    check(load().ayla_b200_swiglu_default_config(DTYPE_CODES[dtype], m, n, k, ctypes.byref(cfg)))
     return cfg
 
 

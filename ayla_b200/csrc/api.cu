@@ -603,20 +603,25 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
 
 // The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
 // leave 32 of them working at n = 4096): 64 output columns per tile, M on the narrow accumulator, k split across
-// a cluster, all in one wave.  False where no such schedule exists; where one does it measured the faster (us,
-// row-major -> swapped: 8x1024x4096 25.0 -> 6.5, 8x4096x4096 26.7 -> 13.0, 64x8192x4096 30.4 -> 24.3,
+// a cluster, all in one wave.  False where no such schedule exists; where one does it measured the faster in 168
+// shapes (us, row-major -> swapped: 8x1024x4096 25.0 -> 6.5, 8x4096x4096 26.7 -> 13.0, 64x8192x4096 30.4 -> 24.3,
 // 128x4096x4096 27.9 -> 17.9, 512x1024x4096 23.5 -> 15.6, 1024x1024x4096 24.1 -> 21.9; in more than one wave it
-// loses: 64x14336x4096 41.7 -> 42.6, 769x1472x3008 20.0 -> 29.4).
+// loses: 64x14336x4096 41.7 -> 42.6, 769x1472x3008 20.0 -> 29.4).  A 128-wide accumulator that no cluster shares is
+// written out by its one CTA in 4 us and more (see the swapped form's stores), which only a deep product earns back:
+// 740x1504x896, 14 k-blocks, 9.3 -> 10.4, 595x1024x2112, 33, 15.6 -> 17.6, 381x3136x3208, 51, 25.1 -> 29.2, but
+// 337x2672x4288, 67, 25.9 -> 23.3, 68x5232x11720, 184, 92.4 -> 72.8.
 bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b200_config* c) {
   // us per k-block and per cluster exchange, fitted to the same measurements.
   struct Width { int tile_n; double per_kb, exchange2, exchange4; };
   static const Width kWidths[4] = {{16, 0.160, 0.9, 1.4}, {32, 0.170, 0.9, 1.4}, {64, 0.20, 1.5, 3.0}, {128, 0.28, 2.7, 4.6}};
   const int64_t k_blocks = ceil_div(k, 64), row_tiles = ceil_div(n, 64);
   double best = 1e300;
+  memset(c, 0, sizeof(*c));
   for (const Width& w : kWidths) {
     const int64_t tiles = row_tiles * ceil_div(m, w.tile_n);
     for (int split = 1; split <= 4; split *= 2) {
       if (tiles * split > sm_count || (split > 1 && k_blocks < 4 * split)) break;
+      if (w.tile_n == 128 && split == 1 && k_blocks < 60) continue;
       const double cost = static_cast<double>(ceil_div(k_blocks, split)) * w.per_kb +
                           (split == 1 ? 0.0 : split == 2 ? w.exchange2 : w.exchange4);
       if (cost < best && static_cast<int64_t>(split - 1) * ceil_div(k_blocks, split) < k_blocks) {
@@ -638,6 +643,18 @@ bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b
   const int64_t share = k_blocks / c->split_k / 2;
   c->early_prefetch = m > 64 ? 0 : static_cast<int>(share < 8 ? share : 8);
   return true;
+}
+
+ayla_b200_config row_major_swiglu_config(int64_t m) {
+  ayla_b200_config c;
+  memset(&c, 0, sizeof(c));
+  c.tile_n = 256;
+  c.cta_group = (m >= 256) ? 2 : 1;
+  c.split_k = 1;
+  c.group_m = 8;
+  c.l2_hint_a = 2;  // x is re-read by every column tile,
+  c.l2_hint_b = 1;  // the weights stream through once
+  return c;
 }
 
 int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, int is_bf16,
@@ -911,6 +928,14 @@ int ayla_b200_default_config_act(int op, int dtype, int activation, int64_t batc
   return AYLA_B200_OK;
 }
 
+int ayla_b200_swiglu_default_config(int dtype, int64_t m, int64_t n, int64_t k, ayla_b200_config* cfg_out) {
+  if (cfg_out == nullptr) return fail(AYLA_B200_E_INVALID, "cfg_out is null");
+  const int rc = check_shape(AYLA_B200_OP_MM, dtype, 1, m, n, k);
+  if (rc) return rc;
+  if (!swapped_swiglu_config(m, n, k, current_sm_count(), cfg_out)) *cfg_out = row_major_swiglu_config(m);
+  return AYLA_B200_OK;
+}
+
 int ayla_b200_config_valid(const ayla_b200_config* cfg, int op, int dtype, int64_t batch, int64_t m,
                            int64_t n, int64_t k) {
   if (cfg == nullptr) return fail(AYLA_B200_E_INVALID, "cfg is null");
@@ -1165,21 +1190,10 @@ int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate, const void* w
   int dev = -1;
   rc = current_device_state(&ds, &dev);
   if (rc) return rc;
-  bool swapped = false;
   ayla_b200_config c;
-  if (cfg != nullptr) {
-    c = *cfg;
-  } else {
-    memset(&c, 0, sizeof(c));
-    swapped = swapped_swiglu_config(m, n, k, ds->sm_count, &c);
-    if (!swapped) {
-      c.cta_group = (m >= 256) ? 2 : 1;
-      c.group_m = 8;
-      c.l2_hint_a = 2;  // x is re-read by every column tile,
-      c.l2_hint_b = 1;  // the weights stream through once
-    }
-  }
+  const bool swapped = cfg == nullptr && swapped_swiglu_config(m, n, k, ds->sm_count, &c);
   if (!swapped) {
+    c = cfg != nullptr ? *cfg : row_major_swiglu_config(m);
     c.tile_n = 256;
     c.split_k = 1;
     c.swap_ab = 0;

@@ -255,6 +255,13 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
                                                int64_t n, int64_t k, ayla_b200_config* cfg_out);
 
 /*
+ * The schedule ayla_b200_swiglu uses when cfg == NULL: row-major (swap_ab == 0), or with the weights on the row
+ * side (swap_ab == 1), a form that cannot be asked for by a cfg.
+ */
+AYLA_B200_API int ayla_b200_swiglu_default_config(int dtype, int64_t m, int64_t n, int64_t k,
+                                                  ayla_b200_config* cfg_out);
+
+/*
  * 0 if `cfg` can run the given problem, else an error code (message in
  * ayla_b200_last_error).  Counterpart of _legal (ayla/gemm_jit.py:115-138).
  */

@@ -169,3 +169,18 @@ def test_shallow_products_are_paired_where_it_measured_faster(op, batch, m, n, k
         cfg = _lib.default_config(op, "bfloat16", batch, m, n, k, activation)
         assert (cfg.tile_n, cfg.cta_group) == (tile_n, pairing), (activation, cfg.to_dict())
         assert _lib.config_valid(cfg, op, "bfloat16", batch, m, n, k)
+
+
+@pytest.mark.parametrize("m, n, k, tile_n, split", [
+    (8, 1024, 4096, 16, 4), (8, 4096, 4096, 16, 2), (128, 4096, 4096, 128, 2), (512, 1024, 4096, 128, 2),
+    # Unshared 128-wide accumulators: deep products only.
+    (1024, 1024, 4096, 128, 1), (337, 2672, 4288, 128, 1), (68, 5232, 11720, 128, 1),
+    (740, 1504, 896, 0, 0), (595, 1024, 2112, 0, 0), (381, 3136, 3208, 0, 0), (142, 3632, 656, 0, 0),
+    (64, 14336, 4096, 0, 0), (8192, 14336, 4096, 0, 0),
+])
+def test_swiglu_of_few_rows_is_swapped_where_it_measured_faster(m, n, k, tile_n, split):
+    cfg = _lib.swiglu_default_config("bfloat16", m, n, k)
+    if tile_n == 0:
+        assert (cfg.swap_ab, cfg.tile_n, cfg.split_k, cfg.cta_group) == (0, 256, 1, 2 if m >= 256 else 1)
+    else:
+        assert (cfg.swap_ab, cfg.tile_n, cfg.split_k, cfg.cluster_split) == (1, tile_n, split, int(split > 1))
