@@ -5,7 +5,10 @@ import threading
 import pytest
 import torch
 
-from ayla_b200 import _lib, gemm_act_mul_op, gemm_op, gemm_op_compiler, swiglu_op
+from ayla_b200 import _lib, gemm_act_mul_op, gemm_jit, gemm_op, gemm_op_compiler, swiglu_op
+from ayla_b200.gemm_jit import _DEFAULTS, GemmLauncher, GemmScheduleSeed
+from ayla_b200.jit_compiler import ShapeSpecializingJITCompiler
+from ayla_b200.rmsnorm_linear import rms_norm_linear
 from oracle import gemm_oracle as O
 from tests.test_gpu_parity import assert_parity
 
@@ -22,8 +25,9 @@ def _mm(m, n, k, seed=0):
 
 
 @pytest.mark.parametrize("op", ["mm", "addmm", "bmm", "gated", "swiglu"])
-def test_repeated_calls_on_new_operands(op):
-    """Every operand layout: the first call specialises in Python, later ones, on other buffers, do not."""
+def test_repeated_calls_on_new_operands(op, monkeypatch):
+    """Every operand layout: the first call specialises in Python, later ones, on other buffers, do not enter it."""
+    monkeypatch.delenv("AYLA_B200_DEBUG", raising=False)
     g = torch.Generator().manual_seed(3)
     for seed in range(3):
         a = torch.randn(40, 136, generator=g).bfloat16()
@@ -42,6 +46,48 @@ def test_repeated_calls_on_new_operands(op):
         out = torch.full(want.shape, float("nan"), dtype=torch.bfloat16, device=DEV)
         assert call(*[t.to(DEV) for t in args], out) is None
         assert_parity(out.cpu(), want, f"{op} call {seed}")
+        monkeypatch.setattr(ShapeSpecializingJITCompiler, "_launcher", _no_python)
+
+
+def _no_python(*args, **kwargs):
+    raise AssertionError("a repeated call entered Python")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_repeated_row_factors_do_not_enter_python(dtype, monkeypatch):
+    weight = torch.randn(64, 264, device=DEV).to(dtype)
+    for seed in range(3):
+        x = torch.randn(24, 264, generator=torch.Generator().manual_seed(seed)).to(dtype)
+        out = rms_norm_linear(x.to(DEV), weight)
+        factors = torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-5).to(dtype).float()
+        assert_parity(out.cpu(), (x.float() @ weight.cpu().float().T) * factors, f"call {seed}")
+        monkeypatch.setattr(_lib, "rms_factors", _no_python)
+        monkeypatch.setattr(ShapeSpecializingJITCompiler, "_launcher", _no_python)
+
+
+def test_another_streams_k_split_launch_enters_python(monkeypatch):
+    """Only the stream that a workspace belongs to is served without Python."""
+    monkeypatch.delenv("AYLA_B200_DEBUG", raising=False)
+    m, n, k = 128, 192, 8192
+    a, bt, want = _mm(m, n, k, 6)
+    a, bt = a.to(DEV), bt.to(DEV)
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    captured = {**_DEFAULTS, "tile_n": 64, "cta_group": 1, "split_k": 4}
+    seed = GemmScheduleSeed(captured, {key: int(captured[key]) for key in _lib.Config.FIELDS}, (), None)
+    monkeypatch.setattr(gemm_jit, "select_gemm_schedule", lambda *args: seed)
+    op = gemm_op("mm", "bfloat16", "ayla_b200_k_split_test")
+    op(a, bt, out)
+    calls = []
+    launch = GemmLauncher.__call__
+    monkeypatch.setattr(GemmLauncher, "__call__", lambda self, *tensors: (calls.append(1), launch(self, *tensors))[1])
+    op(a, bt, out)
+    assert calls == []
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        op(a, bt, out)
+    torch.cuda.synchronize()
+    assert calls == [1]
+    assert_parity(out.cpu(), want, "another stream")
 
 
 def test_refusals_come_from_python_after_a_specialised_call():
@@ -65,8 +111,6 @@ def test_refusals_come_from_python_after_a_specialised_call():
 def test_streams_threads_and_timeouts_of_a_k_split_shape():
     """A launch with a workspace: another stream gets its own from Python, threads share the record, and a
     launch that timed out is reported by the next call."""
-    from ayla_b200.gemm_jit import GemmLauncher
-
     m, n, k = 128, 256, 8192
     a, bt, want = _mm(m, n, k, 5)
     a, bt = a.to(DEV), bt.to(DEV)
