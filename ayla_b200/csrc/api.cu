@@ -607,9 +607,11 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
 // shapes (us, row-major -> swapped: 8x1024x4096 25.0 -> 6.5, 8x4096x4096 26.7 -> 13.0, 64x8192x4096 30.4 -> 24.3,
 // 128x4096x4096 27.9 -> 17.9, 512x1024x4096 23.5 -> 15.6, 1024x1024x4096 24.1 -> 21.9; in more than one wave it
 // loses: 64x14336x4096 41.7 -> 42.6, 769x1472x3008 20.0 -> 29.4).  A 128-wide accumulator that no cluster shares is
-// written out by its one CTA in 4 us and more (see the swapped form's stores), which only a deep product earns back:
-// 740x1504x896, 14 k-blocks, 9.3 -> 10.4, 595x1024x2112, 33, 15.6 -> 17.6, 381x3136x3208, 51, 25.1 -> 29.2, but
-// 337x2672x4288, 67, 25.9 -> 23.3, 68x5232x11720, 184, 92.4 -> 72.8.
+// written out by its one CTA in 4 us and more, two bytes at a time, which only a deep product earns back.  Against
+// pairs (256 rows and more): 740x1504x896, 14 k-blocks, 9.3 -> 10.4, 595x1024x2112, 33, 15.6 -> 17.6, but
+// 659x896x2432, 38, 16.0 -> 15.2, 374x2944x3200, 50, 21.9 -> 20.7; against single CTAs: 109x6080x960, 15, 10.5 ->
+// 11.4, but 150x3304x1664, 26, 14.0 -> 12.8; with rows that start inside a 32-byte sector 381x3136x3208, 51,
+// 25.1 -> 29.2, but 68x5232x11720, 184, 92.4 -> 72.8.
 bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b200_config* c) {
   // us per k-block and per cluster exchange, fitted to the same measurements.
   struct Width { int tile_n; double per_kb, exchange2, exchange4; };
@@ -621,7 +623,7 @@ bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b
     const int64_t tiles = row_tiles * ceil_div(m, w.tile_n);
     for (int split = 1; split <= 4; split *= 2) {
       if (tiles * split > sm_count || (split > 1 && k_blocks < 4 * split)) break;
-      if (w.tile_n == 128 && split == 1 && k_blocks < 60) continue;
+      if (w.tile_n == 128 && split == 1 && k_blocks < (k % 16 != 0 ? 60 : m < 256 ? 20 : 36)) continue;
       const double cost = static_cast<double>(ceil_div(k_blocks, split)) * w.per_kb +
                           (split == 1 ? 0.0 : split == 2 ? w.exchange2 : w.exchange4);
       if (cost < best && static_cast<int64_t>(split - 1) * ceil_div(k_blocks, split) < k_blocks) {

@@ -369,21 +369,24 @@ cudaError_t init_packed_gemm() {
                               cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
 }
 
-// Where this kernel is the faster one.  1276 shapes of up to 128 columns and a depth of up to 128 were timed on both
-// (graph replay, operands past L2): by this rule the geometric mean is 0.739 of the general kernel's time, ten shapes
-// are slower by 3 to 10 %, 39 that this kernel would do in less than 0.9 stay with the general one; choosing the
-// faster one every time would give 0.732.  What it goes by (us, general -> packed):
+// Where this kernel is the faster one.  1606 shapes of up to 128 columns and a depth of up to 128 were timed on both
+// (graph replay, operands past L2): by this rule the geometric mean is 0.726 of the general kernel's time, 22 shapes
+// are slower by 3 to 14 %, 20 that this kernel would do in less than 0.9 stay with the general one; choosing the
+// faster one every time would give 0.722.  What it goes by (us, general -> packed; or packed over general):
 //  * a 128-row tile for every SM; below, both are a launch and one pass (bmm 8 x 1024x64x64 2.8 -> 3.5).
 //  * Small matrices that share an accumulator gain most (1024 x 64x64x64 8.7 -> 7.3, 574 x 15x16x32 5.4 -> 2.6), as
 //    long as two CTAs fit an SM or four matrices a unit (7467 x 17x48x104, one CTA: 42.5 -> 47.9).
 //  * Otherwise resident CTAs hide a unit's chain of load, MMA and epilogue: with one per SM nothing does (512 x
-//    128x72x104 8.4 -> 10.3), four always do up to 64 columns, and with three or two it takes an advantage besides:
-//    few columns, or rows that start in the middle of a 32-byte sector, which cost the general kernel's TMA loads
-//    twice (200 x 500x56x72 10.1 -> 9.1, but 200 x 500x48x128 9.1 -> 10.0 and 200 x 500x128x56 9.3 -> 12.9), or one B
-//    for all units (162131x72x48 0.60 of the general time, 4252 x 85x112x48 1.46).
+//    128x72x104 8.4 -> 10.3), with four nearly every product gains, and with three or two it takes an advantage
+//    besides: few columns, rows that start in the middle of a 32-byte sector, which cost the general kernel's TMA
+//    loads twice (200 x 500x56x72 10.1 -> 9.1, but 200 x 500x48x128 9.1 -> 10.0 and 200 x 500x128x56 9.3 -> 12.9),
+//    or one B for all units (162131x72x48 0.60, but 4252 x 85x112x48 1.46), for aligned rows at two CTAs from the third
+//    round on (159590x40x80, 4.2 rounds, 0.53; 42849x48x96, 1.1, 1.14) or with output rows that start inside a sector
+//    (70938x120x48 0.85, 72817x112x48 1.16).
 //  * A second round of units that fills less than a third of the resident CTAs is a round all the same (512 x
-//    128x72x56, 1.15 rounds: 7.6 -> 8.2); so is a first one that leaves half of them without work, at a depth where
-//    the general kernel is quick (19815x64x48 1.09, 170 x 110x64x56 1.10).
+//    128x72x56, 1.15 rounds: 7.6 -> 8.2), and so is a first one that leaves half of them without work (19815x64x48 1.09,
+//    170 x 110x64x56 1.10); up to a depth of 40 the general kernel's 64-deep boxes cost it more than that (37 x
+//    473x56x40 0.81, 512 x 128x48x40 0.83).
 //  * A product of one 16-byte piece in depth with shared B, in a single round (60000x64x8 8.6 -> 10.8; 131072x64x8, in
 //    two, 16.0 -> 13.7).
 bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count) {
@@ -396,14 +399,17 @@ bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_cou
   const bool shared_b = batch == 1, mid_sector = k % 16 != 0;
   if (n <= 32) return shared_b || f.ctas >= 3 || mid_sector;
   const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);
-  if (shared_b && k < 16 && n > 40) return rounds >= 1.35;
-  if (k > 32 && rounds < 0.5) return false;
+  if (k >= 48 && rounds < 0.5) return false;
+  if (f.ctas >= 4) return !(shared_b && k < 16 && n > 40 && n <= 64 && rounds > 0.5 && rounds < 1.35);
   const bool settled = rounds <= 0.95 || rounds >= 1.35;
-  if (f.ctas >= 4) return n <= 64 || mid_sector || settled;
-  if (!settled) return false;
-  if (f.ctas == 3) return n <= 64 || (shared_b ? rounds >= 1.35 : mid_sector || (k <= 32 && rounds >= 2.0));
-  if (mid_sector) return n <= 64 || (shared_b && (n <= 96 || rounds >= 1.35));
-  return shared_b && n <= 64 && rounds >= 1.35;
+  if (f.ctas == 3) {
+    if (n <= 64) return settled || k < 48;
+    if (shared_b) return rounds >= 1.35 || (mid_sector && k < 48);
+    return settled && (mid_sector || (n <= 80 && rounds >= 1.35) || (k <= 32 && rounds >= 2.0));
+  }
+  if (!shared_b) return n <= 64 ? settled && mid_sector : k < 64 && rounds <= 0.95;
+  if (mid_sector) return (k > 64 && n <= 96) || (settled && (n <= 96 || rounds >= 1.35 || k < 64));
+  return n <= 64 ? rounds >= 2.4 : k < 64 && n % 16 != 0 && rounds >= 1.35;
 }
 
 cudaError_t launch_packed_gemm(const PackedProblem& pr) {

@@ -175,6 +175,7 @@ def test_shallow_products_are_paired_where_it_measured_faster(op, batch, m, n, k
     (8, 1024, 4096, 16, 4), (8, 4096, 4096, 16, 2), (128, 4096, 4096, 128, 2), (512, 1024, 4096, 128, 2),
     # Unshared 128-wide accumulators: deep products only.
     (1024, 1024, 4096, 128, 1), (337, 2672, 4288, 128, 1), (68, 5232, 11720, 128, 1),
+    (374, 2944, 3200, 128, 1), (150, 3304, 1664, 128, 1),
     (740, 1504, 896, 0, 0), (595, 1024, 2112, 0, 0), (381, 3136, 3208, 0, 0), (142, 3632, 656, 0, 0),
     (64, 14336, 4096, 0, 0), (8192, 14336, 4096, 0, 0),
 ])

@@ -359,11 +359,12 @@ def test_the_suite_times_the_kernel_the_ops_run(packed, monkeypatch):
     # The ops' shapes it is made for.
     ("bmm", 8192, 56, 32, 56, True), ("mm", 1, 200704, 96, 24, True), ("bmm", 1024, 64, 64, 64, True),
     ("bmm", 574, 15, 16, 32, True), ("mm", 1, 153121, 88, 72, True), ("bmm", 200, 500, 56, 72, True),
+    ("bmm", 37, 473, 56, 40, True), ("mm", 1, 159590, 40, 80, True), ("mm", 1, 70938, 120, 48, True),
     # Measured slower on it: a unit of two matrices at one CTA per SM, ...
     ("bmm", 7467, 17, 48, 104, False), ("bmm", 3375, 41, 56, 120, False), ("bmm", 2668, 47, 40, 112, False),
     # ... wide outputs at two CTAs, aligned rows at two CTAs, ...
     ("bmm", 200, 500, 128, 56, False), ("bmm", 4252, 85, 112, 48, False), ("mm", 1, 229347, 128, 48, False),
-    ("bmm", 200, 500, 48, 128, False), ("bmm", 244, 1728, 16, 128, False),
+    ("bmm", 200, 500, 48, 128, False), ("bmm", 244, 1728, 16, 128, False), ("mm", 1, 72817, 112, 48, False),
     # ... a thin second round, a thin first one, a depth of one piece, fewer tiles than SMs.
     ("bmm", 512, 128, 72, 56, False), ("mm", 1, 21325, 64, 64, False), ("mm", 1, 60000, 64, 8, False),
     ("bmm", 8, 1024, 64, 64, False),
