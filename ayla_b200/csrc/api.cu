@@ -485,8 +485,8 @@ int current_sm_count() {
 //  * not where 256-row tiles add much padding to the rows (bmm 28 x 1873x1576x128, 7 %: 40.5 -> 46.6; 82 x
 //    1335x1064x128, 9 %: 58.5 -> 72.8), more of which a deeper or misaligned product bears (bmm 26 x 830x1264x256, 14 %:
 //    21.4 -> 19.6);
-//  * behind an activation less: the padding rows pass through it too (bmm 26 x 830x1264x256 with SiLU 1.12), and from
-//    four waves on its epilogue bounds the launch in either form (GELU: 0.96 to 1.06, 1.007 in the mean).
+//  * behind an activation only without padding: its rows pass through the epilogue too (bmm 26 x 830x1264x256 with
+//    SiLU 1.12).  There pairs take 0.96 of the time with SiLU and GELU, 0.99 with sigmoid and GELU-tanh, 0.81 to 1.04.
 bool shallow_pairs_pay(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_n, int activation, int sm_count) {
   const int64_t k_blocks = ceil_div(k, 64);
   if (k_blocks > 4 || m < 256 || tile_n < 128) return false;
@@ -495,7 +495,6 @@ bool shallow_pairs_pay(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_
   const double growth = static_cast<double>(2 * ceil_div(m, 256)) / static_cast<double>(row_tiles);
   if (growth > (activation == AYLA_B200_ACT_NONE && (k_blocks >= 3 || mid_sector) ? 1.2 : 1.03)) return false;
   const double waves = static_cast<double>(batch * row_tiles * ceil_div(n, tile_n)) / sm_count;
-  if (activation > AYLA_B200_ACT_RELU && waves >= 4.0) return false;
   return mid_sector ? waves >= 1.0 : waves >= 2.0 && (tile_n == 256 || k_blocks >= 3);
 }
 

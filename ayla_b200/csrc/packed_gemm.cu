@@ -404,7 +404,7 @@ bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_cou
   const bool settled = rounds <= 0.95 || rounds >= 1.35;
   if (f.ctas == 3) {
     if (n <= 64) return settled || k < 48;
-    if (shared_b) return rounds >= 1.35 || (mid_sector && k < 48);
+    if (shared_b) return rounds >= 1.25 || (mid_sector && k < 48);
     return settled && (mid_sector || (n <= 80 && rounds >= 1.35) || (k <= 32 && rounds >= 2.0));
   }
   if (!shared_b) return n <= 64 ? settled && mid_sector : k < 64 && rounds <= 0.95;
