@@ -56,19 +56,21 @@ DISPATCH_STAMP = BUILD_DIR / "torch_dispatch.stamp"
 
 def build_dispatch(verbose: bool = False, force: bool = False) -> Path:
     import torch
+
+    nvcc = _nvcc()
+    # What it was built for: another torch or Python may not load it, or worse, load it.
+    stamp = "\n".join([torch.__version__, torch.__file__, sys.version, nvcc])
+    if (not force and DISPATCH_PATH.exists() and DISPATCH_STAMP.exists() and DISPATCH_STAMP.read_text() == stamp
+            and DISPATCH_PATH.stat().st_mtime >= DISPATCH_SOURCE.stat().st_mtime):
+        return DISPATCH_PATH
     from torch.utils.cpp_extension import include_paths, library_paths
 
-    includes = [*include_paths("cuda"), sysconfig.get_paths()["include"]]
+    includes = [*include_paths(), str(Path(nvcc).resolve().parent.parent / "include"), sysconfig.get_paths()["include"]]
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            *[f"-isystem{path}" for path in includes], str(DISPATCH_SOURCE), "-o", str(DISPATCH_PATH),
            *[f"-L{path}" for path in library_paths()],
            "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
-    # What it was built for: another torch or Python may not load it, or worse, load it.
-    stamp = "\n".join([torch.__version__, sys.version, *cmd])
-    if (not force and DISPATCH_PATH.exists() and DISPATCH_STAMP.exists() and DISPATCH_STAMP.read_text() == stamp
-            and DISPATCH_PATH.stat().st_mtime >= DISPATCH_SOURCE.stat().st_mtime):
-        return DISPATCH_PATH
     LIB_DIR.mkdir(exist_ok=True)
     BUILD_DIR.mkdir(exist_ok=True)
     DISPATCH_STAMP.unlink(missing_ok=True)

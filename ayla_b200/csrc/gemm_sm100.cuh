@@ -438,8 +438,8 @@ __device__ __forceinline__ void store_elem(void* base, long long i, float v, int
 // its subnormal handling and a guarded division cost 40 instructions and more per element; the forms
 // below take two special-function results (one for GELU) and a handful of multiply-adds, the
 // polynomial two elements per instruction.  addmm 8192 x 3072 x 768 fp16, us per launch, library
-// functions -> these forms: gelu 52.5 -> 37.9, gelu_tanh 46.6 -> 38.6, silu 39.3 -> 37.5, sigmoid
-// 38.7 -> 37.2 (no activation: 31).
+// functions -> these forms: gelu 52.5 -> 38.7, gelu_tanh 46.6 -> 39.5, silu 39.3 -> 37.7, sigmoid
+// 38.7 -> 36.6 (no activation: 32.4).
 enum : int { ACT_NONE = 0, ACT_RELU = 1, ACT_SIGMOID = 2, ACT_SILU = 3, ACT_GELU = 4, ACT_GELU_TANH = 5 };
 
 // 1 / (1 + 2^-z): flushing a subnormal 2^-z to zero moves the result by less than 2^-126.

@@ -80,8 +80,8 @@ rms_factors_kernel(const uint4* x, void* factors, int rows, int chunks, float k,
 
 cudaError_t launch_rms_factors(const void* x, void* factors, int rows, int k, float eps, int is_bf16, int overlap,
                                cudaStream_t stream) {
-  // As few threads to a row as leave each at least kUnroll loads, so that a block's fixed cost (launch, reduction)
-  // is shared by as many rows as possible: 2400 rows of 8192 with one warp a row 9.0 us, with eight 7.4;
+  // The most threads to a row that still have kUnroll loads each; fewer on short rows, so that a block's fixed cost
+  // (launch, reduction) is shared by several: 2400 rows of 8192 with one warp a row 9.0 us, with eight 7.4;
   // 2300 rows of 1024 with eight warps a row 3.5 us, with one 2.1.
   const int chunks = k / 8;
   const int row_threads = chunks >= 256 * kUnroll ? 256 : chunks >= 128 * kUnroll ? 128 : chunks >= 64 * kUnroll ? 64 : 32;
