@@ -628,6 +628,7 @@ def test_swapped_swiglu(m, n, k, dtype):
         ("mm", 1, 1, 8, 8), ("addmm", 1, 129, 24, 24), ("mm", 1, 257, 128, 128), ("addmm", 1, 300, 120, 40),
         ("mm", 1, 128, 104, 120), ("addmm", 1, 90001, 16, 16), ("mm", 1, 150003, 96, 72),
         ("bmm", 3, 65, 128, 72), ("bmm", 2, 200, 56, 16), ("bmm", 700, 100, 40, 104), ("bmm", 1, 70, 32, 48),
+        ("mm", 1, 70938, 120, 48), ("addmm", 1, 100001, 40, 80), ("bmm", 84, 286, 112, 48), ("bmm", 37, 473, 56, 40),
         # two and four, the last unit partly filled
         ("bmm", 5, 64, 64, 128), ("bmm", 3, 33, 40, 8), ("bmm", 2049, 56, 32, 56), ("bmm", 3, 8, 48, 32),
         ("bmm", 7, 32, 32, 16), ("bmm", 6, 1, 8, 24), ("bmm", 4001, 17, 24, 40),
