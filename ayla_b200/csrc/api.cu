@@ -56,6 +56,8 @@ struct Registry {
     append_variants_lean_act_cg1(&entries);
     append_variants_lean_act_cg2(&entries);
     append_variants_lean_act_trans(&entries);
+    append_variants_paired_cg1(&entries);
+    append_variants_paired_cg2(&entries);
     append_variants_gated_cg1(&entries);
     append_variants_gated_cg2(&entries);
   }
@@ -295,11 +297,15 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   const bool swiglu_cols = epilogue == EPI_SWIGLU && !c.swap_ab;
   const int tile_n = swiglu_cols ? 256 : c.tile_n;
   const int lean = (c.split_k <= 1 && c.stream_k == 0) ? 1 : 0;
+  // `activation` 3: one that is more than a comparison, for which those launches have kernels with sixteen epilogue
+  // warps (see GemmTraits::PAIRED; with a comparison or a row factor alone eight do as well or better: RMS norm and
+  // projection 4096x6144x4096 172 against 173 us).
   // `activation` 2: a gate operand shaped like the output, for which the launches without a k-split have kernels of
   // their own (us per launch, before -> with them: 16384x2048x256 71.4 -> 38.1, 6983x1472x1312 43.8 -> 32.2,
   // 1024x4096x512 15.3 -> 12.0, 64x8192x1024 10.4 -> 8.9); the k-split and swapped forms load it directly.
   const KernelEntry* e = nullptr;
   if (activation == 2 && lean == 1) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 2, 1);
+  if (activation == 3 && lean == 1) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 3, 1);
   if (e == nullptr) e = registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, lean);
   if (e == nullptr) {
     return fail(AYLA_B200_E_UNSUPPORTED, "no kernel variant tile_n=%d cta_group=%d epilogue=%d swap=%d",
@@ -1062,7 +1068,10 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   const int epi = (op == AYLA_B200_OP_ADDMM) ? EPI_BIAS : EPI_PLAIN;
   Plan plan{};
   rc = make_plan(c, epi, batch, pr.rows, pr.cols, k, ds->sm_count, &plan,
-                 (mul != nullptr && mul_per_row == 0) ? 2 : (activation != 0 || mul != nullptr) ? 1 : 0);
+                 (mul != nullptr && mul_per_row == 0)  ? 2
+                 : activation > AYLA_B200_ACT_RELU       ? 3
+                 : activation != 0 || mul != nullptr     ? 1
+                                                         : 0);
   if (rc) return rc;
   return launch_plan(plan, c, pr, dtype == AYLA_B200_BF16 ? 1 : 0, bias, nullptr, out, m, n, workspace,
                      workspace_bytes, status, reinterpret_cast<cudaStream_t>(stream), activation, mul, mul_per_row);

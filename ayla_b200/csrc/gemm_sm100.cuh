@@ -14,7 +14,8 @@
 //   warps 2..9  epilogue      : TMEM -> registers -> (bias | activation | SiLU*up) -> round ->
 //                               swizzled shared -> TMA store   (or direct stores for the
 //                               transposed form and narrow cluster slices)
-// (kernels for gated launches have one epilogue warp per 64 columns and lane quarter instead of eight)
+// (kernels for gated launches have one epilogue warp per 64 columns and lane quarter instead of eight, those with an
+// activation sixteen, two to each 64 columns)
 // The accumulator is double buffered in TMEM so the epilogue of one tile runs
 // under the main loop of the next.  CTAs are persistent and walk a static,
 // M-grouped raster over (batch, m-tile, n-tile, k-split) work units.
@@ -155,7 +156,7 @@ __device__ __forceinline__ void trace_stamp(long long* stamps, int slot) {
 #define AYLA_TRACE_END(slot)
 #endif
 
-template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, bool ACT_ = false, bool LEAN_ = false,
+template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, int ACT_ = 0, bool LEAN_ = false,
           bool GATED_ = false>
 struct GemmTraits {
   // LEAN: the kernel is compiled without the k-split epilogues (workspace and cluster forms) and
@@ -165,7 +166,7 @@ struct GemmTraits {
   // ACT: the epilogue applies the activation named in the launch parameters.  A separate set of
   // instantiations, so that the plain kernels carry none of that code (compiled in as a run-time
   // branch it cost the output-bound bmm 5 %).
-  static constexpr bool ACT = ACT_;
+  static constexpr bool ACT = ACT_ != 0;
   static constexpr int BN = BN_;                // MMA N (accumulator columns)
   static constexpr int CTA_GROUP = CTA_GROUP_;
   static constexpr int EPI = EPI_;
@@ -202,11 +203,18 @@ struct GemmTraits {
   // lines per instruction: 10 us of an SM per 128 x 256 tile with eight warps, 8.5 with sixteen, 5.4 this way.)
   // One staging box per warp; at 256 columns the sixteen of them cost a ring slot.
   static constexpr bool GATED = GATED_;
-  static constexpr int EPI_WARPS = GATED ? BN / 16 : 8;
+  // PAIRED (ACT_ 2): sixteen epilogue warps, two to a 64-column group and lane quarter, one staging box between them.
+  // For the activations that are more than a comparison: a GELU takes 4000 cycles of an SM's multiply-adds per 128 x 256 tile, and with eight warps they came
+  // on top of the 5000 that loads from TMEM, staging and stores take; with sixteen they run under them.  us per launch,
+  // eight -> sixteen: addmm 12095x5824x256 + GELU fp16 81.4 -> 78.3, mm 16384x2048x512 + SiLU 44.3 -> 42.6, addmm
+  // 8192x3072x768 + GELU 45.3 -> 44.1 (the power cap takes back more than half of the cycles saved).  Without one
+  // there is nothing to hide (bmm 54x553x1880x64 31.0 -> 32.2, mm 2589x6016x320 15.2 -> 15.7).
+  static constexpr bool PAIRED = ACT_ == 2;
+  static constexpr int EPI_WARPS = GATED ? BN / 16 : PAIRED ? 16 : 8;
   static constexpr int STORE_BUF_BYTES = 32 * 128;  // 32 rows x 64 columns of 16-bit
   // Swapped SwiGLU: where the epilogue warps of the up rows leave 32 columns for those of the gate rows.
   static constexpr int UP_BUF_BYTES = 32 * 64 * 4;
-  static constexpr int STORE_BYTES = SWIGLU_ROWS ? 2 * UP_BUF_BYTES : TRANS_OUT ? 0 : EPI_WARPS * STORE_BUF_BYTES;
+  static constexpr int STORE_BYTES = SWIGLU_ROWS ? 2 * UP_BUF_BYTES : TRANS_OUT ? 0 : (PAIRED ? 8 : EPI_WARPS) * STORE_BUF_BYTES;
   static constexpr int BIAS_BYTES = (EPI == EPI_BIAS && !TRANS_OUT) ? 2 * BN * 4 : 0;
   static constexpr int MISC_BYTES = GATED ? 384 : 256;
 #ifdef AYLA_B200_TRACE
@@ -221,6 +229,7 @@ struct GemmTraits {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N extent");
   static_assert(B_BYTES % 1024 == 0, "B slab must keep the 1024-byte swizzle alignment");
   static_assert(!SWIGLU_COLS || BN == 256, "row-major SwiGLU uses the 2x128 layout");
+  static_assert(!PAIRED || (LEAN && !GATED && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
   static_assert(!GATED || (ACT && LEAN && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
   static_assert(TRANS_OUT || BN >= 64, "the TMA-store epilogue writes 64-column boxes");
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared-memory limit");
@@ -568,7 +577,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   // issued, 12 first TMA load issued, 13 epilogue saw the first finished accumulator, 14 the preceding
   // launch is complete (dependency wait returned), 15 split-k parts sent, 16 first accumulator chunk in
   // registers, 17 last output chunk handed to the store path, 18-21 the first warp's 64-column groups done,
-  // 22/23 its first two chunks staged, 24 staging published to the async proxy, 25 bulk store issued,
   // 26 split-k: own partial of the first chunk in registers, 27 that chunk summed.
   long long* stamps = (p.trace != nullptr) ? reinterpret_cast<long long*>(smem_misc + T::MISC_BYTES) : nullptr;
   if (stamps != nullptr && threadIdx.x == 0) {
@@ -940,13 +948,16 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // scheduler is latency-bound on its own dependent instruction stream; two hide
     // each other's TMEM-load, conversion and store latencies.
     const int q = warp & 3;                          // TMEM lane quarter
-    const int wsub = (warp - 2) >> 2;                // which 64-column groups: 0 / 1; GATED: the group
+    // Which 64-column groups: 0 / 1; GATED: the group.
+    const int wsub = T::PAIRED ? (warp - 2) >> 3 : (warp - 2) >> 2;
+    const int half_of_pair = T::PAIRED ? ((warp - 2) >> 2) & 1 : 0;
+    const uint32_t pair_bar = 8 + wsub * 4 + q;
     const int epi_tid = (warp - 2) * 32 + lane;
     const int row_in_tile = q * 32 + lane;
     const bool up_rows = T::SWIGLU_ROWS && q >= 2;  // this warp's accumulator rows belong to the up weight
     const int is_bf16 = p.is_bf16;
     const int act = T::ACT ? p.act : static_cast<int>(ACT_NONE);
-    uint8_t* my_store = smem_store + (warp - 2) * T::STORE_BUF_BYTES;
+    uint8_t* my_store = smem_store + (T::PAIRED ? wsub * 4 + q : warp - 2) * T::STORE_BUF_BYTES;
     uint32_t acc = 0, acc_phase = 0;
     uint32_t bias_buf = 0;
     uint32_t gate_phase = 0;
@@ -962,18 +973,41 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #endif
     AYLA_TRACE_BEGIN
 
+    // Bias (row-major): the four warps of one column group share the groups' columns, a thread reads one of them.
+    // Kernels that take several tiles look one unit ahead and read its slice while this one's tile is on its way
+    // (read at the head of a tile its latency was part of every tile: addmm 5215x1216x320 8.3 -> 7.6 us).
+    constexpr bool ROW_BIAS = T::EPI == EPI_BIAS && !T::TRANS_OUT;
+    constexpr bool AHEAD = ROW_BIAS && T::LEAN && BN >= 128;
+    const int bias_thread = half_of_pair * 128 + q * 32 + lane;
+    const int bias_col = (T::GATED ? wsub * 64 : (bias_thread >> 6) * 128 + wsub * 64) + (bias_thread & 63);
+    const bool bias_reads = T::GATED ? bias_thread < 64 : bias_col < BN;
+    auto load_bias = [&](int n0) {
+      return bias_reads && n0 + bias_col < p.n ? load_elem(p.bias, n0 + bias_col, is_bf16) : 0.0f;
+    };
+    float bias_next = 0.0f;
+
     // No early exit in this loop: the warps meet at named barriers, so after an abort
     // they keep walking the units together (every wait then returns at once) and the
     // results are garbage that the status word disowns.
     UnitCursor<T> cursor(p, first_unit, unit_stride, cta_rank, csk_rank);
-    WorkUnit w;
+    WorkUnit w, next;
+    bool has_next = false;
+    if constexpr (AHEAD) has_next = cursor.next(next);
     grid_dependency_wait();  // these warps read bias / gate operands and write the output
-    while (cursor.next(w)) {
+    if constexpr (AHEAD) {
+      if (has_next) bias_next = load_bias(next.n0);
+    }
+    while (AHEAD ? has_next : cursor.next(w)) {
+      if constexpr (AHEAD) w = next;
       const bool split_k = T::LEAN ? false : w.is_split;
 
-      if constexpr (T::EPI == EPI_BIAS && !T::TRANS_OUT) {
-        // Stage this tile's bias slice as fp32; double buffered so one barrier per
-        // tile is enough.
+      // This tile's bias slice as fp32, double buffered so one meeting per tile is enough.
+      if constexpr (AHEAD) {
+        if (bias_reads) smem_bias[bias_buf * BN + bias_col] = bias_next;
+        named_bar_sync(6 + wsub, T::PAIRED ? 256 : 128);
+        has_next = cursor.next(next);
+        if (has_next) bias_next = load_bias(next.n0);
+      } else if constexpr (ROW_BIAS) {
         float* bdst = smem_bias + bias_buf * BN;
         for (int c = epi_tid; c < BN; c += EPI_THREADS) {
           const int col = w.n0 + c;
@@ -990,6 +1024,14 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         tma_store_wait_read<0>();
         mbar_arrive_expect_tx(my_gate_bar, T::STORE_BUF_BYTES);
         tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, gate_policy);
+      }
+
+      // One factor per output row: read while the MMAs run.
+      float row_factor = 1.0f;
+      if constexpr (T::ACT && !T::TRANS_OUT) {
+        if (p.mul_per_row && w.m0 + row_in_tile < p.m) {
+          row_factor = load_elem(p.mul, w.batch * static_cast<long long>(p.m) + w.m0 + row_in_tile, is_bf16);
+        }
       }
 
       AYLA_TRACE_WAIT(tr_wait, bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL))
@@ -1016,7 +1058,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // a CTA pair they would be remote arrivals still in flight when the leader leaves, so
       // they are not sent.
       static_assert(T::ACC_BUFS <= 2, "UnitCursor::follows looks at most two units ahead");
-      const bool release_awaited = cursor.follows(T::ACC_BUFS);
+      const bool release_awaited = AHEAD ? has_next && cursor.follows(T::ACC_BUFS - 1) : cursor.follows(T::ACC_BUFS);
       auto release_accumulator = [&]() {
         if (!release_awaited) return;
         tc_fence_before_sync();
@@ -1038,9 +1080,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           const int col0 = w.n0 + c32 * 32;
           if (p.mul == nullptr || row >= p.m) return;
           if (p.mul_per_row) {
-            const float g = load_elem(p.mul, w.batch * static_cast<long long>(p.m) + row, is_bf16);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] *= g;
+            for (int j = 0; j < 32; ++j) v[j] *= row_factor;
             return;
           }
           const uint8_t* src = reinterpret_cast<const uint8_t*>(p.mul) +
@@ -1075,6 +1116,47 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           }
         }
         return x;
+      };
+
+      // Row-major output: 32 fp32 values of this thread's row become 16 words of the output type ...
+      auto pack_chunk = [&](float (&v)[32], int c32, uint32_t* pk) {
+        if constexpr (T::EPI == EPI_BIAS) {
+          const float4* b4 = reinterpret_cast<const float4*>(smem_bias + bias_buf * BN + c32 * 32);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 b = b4[j];
+            v[4 * j + 0] += b.x;
+            v[4 * j + 1] += b.y;
+            v[4 * j + 2] += b.z;
+            v[4 * j + 3] += b.w;
+          }
+        }
+        apply_act_chunk<32>(v, act);
+        gate_chunk(v, c32);
+        if (is_bf16) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = pack2(v[2 * j], v[2 * j + 1], 1);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = pack2(v[2 * j], v[2 * j + 1], 0);
+        }
+      };
+      // ... which are one half of this thread's 128-byte row of a 64-column staging box ...
+      auto stage_half = [&](uint8_t* box, int half, const uint32_t* pk) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          *reinterpret_cast<uint4*>(box + lane * 128 + (((half * 4 + j) ^ (lane & 7)) << 4)) =
+              make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+        }
+      };
+      // ... that leaves in one bulk store.
+      auto store_group = [&](uint8_t* box, int group64) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&tm_d, smem_u32(box), w.n0 + group64 * 64, w.m0 + q * 32, w.batch);
+          tma_store_commit();
+        }
       };
 
       // Finish one chunk of up to 32 fp32 values of this thread's row (bias, round,
@@ -1120,63 +1202,16 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
           }
         } else {
-          if constexpr (T::EPI == EPI_BIAS) {
-            const float4* b4 = reinterpret_cast<const float4*>(smem_bias + bias_buf * BN + c32 * 32);
-#pragma unroll
-            for (int j = 0; j < CHUNK_COLS / 4; ++j) {
-              const float4 b = b4[j];
-              v[4 * j + 0] += b.x;
-              v[4 * j + 1] += b.y;
-              v[4 * j + 2] += b.z;
-              v[4 * j + 3] += b.w;
-            }
-          }
-          apply_act_chunk<CHUNK_COLS>(v, act);
-          gate_chunk(v, c32);
-          // Two 32-column chunks fill one 64-column (128-byte) store row.
+          uint32_t pk[16];
+          pack_chunk(v, c32, pk);
           const int half = c32 & 1;
           if (half == 0) {
             // The bulk store this warp issued last must have finished reading the buffer.
             if (lane == 0) tma_store_wait_read<0>();
             __syncwarp();
           }
-          uint32_t pk[CHUNK_COLS / 2];
-          if (is_bf16) {
-#pragma unroll
-            for (int j = 0; j < CHUNK_COLS / 2; ++j) {
-              __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-              pk[j] = *reinterpret_cast<uint32_t*>(&t);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < CHUNK_COLS / 2; ++j) {
-              __half2 t = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
-              pk[j] = *reinterpret_cast<uint32_t*>(&t);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < CHUNK_COLS / 8; ++j) {
-            const int chunk16 = half * 4 + j;  // 16-byte chunk within the 128-byte row
-            *reinterpret_cast<uint4*>(my_store + lane * 128 + ((chunk16 ^ (lane & 7)) << 4)) =
-                make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-          }
-#ifdef AYLA_B200_TRACE
-          if (stamps != nullptr && warp == 2 && lane == 0 && c32 < 2) trace_stamp(stamps, 22 + c32);
-#endif
-          if (half == 1) {
-            fence_proxy_async_smem();
-#ifdef AYLA_B200_TRACE
-            if (stamps != nullptr && warp == 2 && lane == 0 && c32 < 2) trace_stamp(stamps, 24);
-#endif
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_3d(&tm_d, smem_u32(my_store), w.n0 + (c32 >> 1) * 64, w.m0 + q * 32, w.batch);
-              tma_store_commit();
-            }
-#ifdef AYLA_B200_TRACE
-            if (stamps != nullptr && warp == 2 && lane == 0 && c32 < 2) trace_stamp(stamps, 25);
-#endif
-          }
+          stage_half(my_store, half, pk);
+          if (half == 1) store_group(my_store, c32 >> 1);
         }
       };
 
@@ -1469,6 +1504,33 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
               tma_store_commit();
             }
           }
+        } else if constexpr (T::PAIRED) {
+          // Two warps to a 64-column group, each with one 32-column half of it: they fill one box together.
+          if (wsub >= unit_groups) release_accumulator();
+#pragma unroll 1
+          for (int g = wsub; g < unit_groups; g += 2) {
+            const int c32 = 2 * g + half_of_pair;
+            uint32_t r[32];
+            tmem_ld_32x32(t_acc + c32 * 32, r);
+            tmem_ld_wait();
+            if (g + 2 >= unit_groups) release_accumulator();
+            if (!(rows_live && w.n0 + g * 64 < p.n)) continue;
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            uint32_t pk[16];
+            pack_chunk(v, c32, pk);
+            // The bulk store that left from the box last must have finished reading it.
+            if (half_of_pair == 0 && lane == 0) tma_store_wait_read<0>();
+            named_bar_sync(pair_bar, 64);
+            stage_half(my_store, half_of_pair, pk);
+            fence_proxy_async_smem();
+            named_bar_sync(pair_bar, 64);
+            if (half_of_pair == 0 && lane == 0) {
+              tma_store_3d(&tm_d, smem_u32(my_store), w.n0 + g * 64, w.m0 + q * 32, w.batch);
+              tma_store_commit();
+            }
+          }
         } else if constexpr (!T::TRANS_OUT) {
           // This warp's 64-column groups, software-pipelined over 32-column chunks: the
           // TMEM load of the next chunk is in flight while this one is converted,
@@ -1483,9 +1545,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
               tmem_ld_32x32(t_acc + c32 * 32, r);
             }
           };
-          auto consume = [&](int c32, uint32_t (&r)[REGS]) {
-            // Liveness per 64 columns: both halves of a 128-byte store row go together.
-            if (!(rows_live && (w.n0 + (c32 >> 1) * 64) < p.n)) return;
+          auto convert = [&](int c32, const uint32_t (&r)[REGS], uint32_t* pk) {
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -1495,7 +1555,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 v[j] = __uint_as_float(r[j]);
               }
             }
-            finish_chunk(v, c32);
+            pack_chunk(v, c32, pk);
           };
           if (wsub >= unit_groups) {
             release_accumulator();
@@ -1503,19 +1563,31 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             issue(2 * wsub, ra);
 #pragma unroll 1
             for (int g = wsub; g < unit_groups; g += 2) {
+              // Liveness per 64 columns: both halves of a 128-byte store row go together.
+              const bool live = rows_live && w.n0 + g * 64 < p.n;
+              uint32_t pk[16];
               tmem_ld_wait();
 #ifdef AYLA_B200_TRACE
               if (stamps != nullptr && warp == 2 && lane == 0 && g == wsub) trace_stamp(stamps, 16);
 #endif
               issue(2 * g + 1, rb);
-              consume(2 * g, ra);
+              if (live) {
+                convert(2 * g, ra, pk);
+                // The bulk store this warp issued last must have finished reading the box.
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
+                stage_half(my_store, 0, pk);
+              }
               tmem_ld_wait();
               if (g + 2 < unit_groups) {
                 issue(2 * (g + 2), ra);
               } else {
                 release_accumulator();
               }
-              consume(2 * g + 1, rb);
+              if (!live) continue;
+              convert(2 * g + 1, rb, pk);
+              stage_half(my_store, 1, pk);
+              store_group(my_store, g);
 #ifdef AYLA_B200_TRACE
               if (stamps != nullptr && warp == 2 && lane == 0 && (g >> 1) < 4) trace_stamp(stamps, 18 + (g >> 1));
 #endif

@@ -24,7 +24,7 @@ struct KernelEntry {
   int tile_n, cta_group, epilogue, transposed_out, stages, smem_bytes;
   int kb_per_slot;  // k-blocks one ring slot holds
   int activation;  // 1 = the variant whose epilogue applies the launch's activation, 2 = the same for
-                   // launches with a gate operand shaped like the output
+                   // launches with a gate operand shaped like the output, 3 = with sixteen epilogue warps
   int lean;        // 1 = the variant without the k-split epilogues
   const void* func;
   cudaError_t (*launch)(const LaunchArgs&);
@@ -73,7 +73,7 @@ cudaError_t launch_variant(const LaunchArgs& a) {
   return cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<T>, a.tm_a, a.tm_b, a.tm_b2, a.tm_d, a.p);
 }
 
-template <int BN, int CG, int EPI, bool TR, bool ACT = false, bool LEAN = false, bool GATED = false>
+template <int BN, int CG, int EPI, bool TR, int ACT = 0, bool LEAN = false, bool GATED = false>
 KernelEntry make_entry() {
   using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED>(), ACT, LEAN, GATED>;
   KernelEntry e;
@@ -84,7 +84,7 @@ KernelEntry make_entry() {
   e.stages = T::STAGES;
   e.smem_bytes = T::SMEM_BYTES;
   e.kb_per_slot = T::KB_PER_SLOT;
-  e.activation = GATED ? 2 : ACT ? 1 : 0;
+  e.activation = GATED ? 2 : T::PAIRED ? 3 : ACT;
   e.lean = LEAN ? 1 : 0;
   e.func = reinterpret_cast<const void*>(&gemm_sm100_kernel<T>);
   e.launch = &launch_variant<T>;
@@ -105,6 +105,8 @@ void append_variants_lean_cg2(std::vector<KernelEntry>* out);
 void append_variants_lean_trans(std::vector<KernelEntry>* out);
 void append_variants_lean_act_cg1(std::vector<KernelEntry>* out);
 void append_variants_lean_act_cg2(std::vector<KernelEntry>* out);
+void append_variants_paired_cg1(std::vector<KernelEntry>* out);
+void append_variants_paired_cg2(std::vector<KernelEntry>* out);
 void append_variants_gated_cg1(std::vector<KernelEntry>* out);
 void append_variants_gated_cg2(std::vector<KernelEntry>* out);
 void append_variants_lean_act_trans(std::vector<KernelEntry>* out);

@@ -284,8 +284,7 @@ def run_case(args) -> None:
 
 STAMPS = {"entry": 0, "set-up done": 1, "preceding launch complete": 14, "first TMA issued": 12,
           "first operands landed": 2, "last MMA committed": 3, "epilogue saw the accumulator": 13,
-          "first chunk in registers": 16, "first chunk staged": 22, "second chunk staged": 23,
-          "staging published (proxy fence)": 24, "first bulk store issued": 25,
+          "first chunk in registers": 16,
           "split-k: cluster met": 6, "split-k: own part sent": 15, "split-k: peers' parts in": 7,
           "split-k: own partial in registers": 26, "split-k: first chunk summed": 27, 
           "first 64-column group done": 18, "second 64-column group done": 19,
@@ -294,9 +293,6 @@ INTERVALS = (("entry", "set-up done"), ("preceding launch complete", "first TMA 
              ("preceding launch complete", "first operands landed"),
              ("first operands landed", "last MMA committed"), ("last MMA committed", "epilogue saw the accumulator"),
              ("last MMA committed", "first chunk in registers"),
-             ("last MMA committed", "first chunk staged"), ("last MMA committed", "second chunk staged"),
-             ("last MMA committed", "staging published (proxy fence)"),
-             ("last MMA committed", "first bulk store issued"),
              ("last MMA committed", "split-k: cluster met"),
              ("last MMA committed", "split-k: own part sent"), ("last MMA committed", "split-k: peers' parts in"),
              ("last MMA committed", "split-k: own partial in registers"),
