@@ -58,20 +58,23 @@ struct Registry {
     append_variants_lean_act_trans(&entries);
     append_variants_paired_cg1(&entries);
     append_variants_paired_cg2(&entries);
+    append_variants_shared_cg1(&entries);
+    append_variants_shared_cg2(&entries);
+    append_variants_shared_act_cg1(&entries);
+    append_variants_shared_act_cg2(&entries);
     append_variants_gated_cg1(&entries);
     append_variants_gated_cg2(&entries);
   }
   int base_count = 0;  // the variants without the activation epilogue come first
-  // `lean` asks for the variant without the k-split epilogues; where there is none the full
-  // variant serves.
+  // Where there is no variant of the form asked for, the one with all epilogues serves.
   const KernelEntry* find(int tile_n, int cta_group, int epilogue, int transposed, int activation = 0,
-                          int lean = 0) const {
+                          int form = FORM_FULL) const {
     const KernelEntry* full = nullptr;
     for (const KernelEntry& e : entries) {
       if (e.tile_n == tile_n && e.cta_group == cta_group && e.epilogue == epilogue &&
           e.transposed_out == transposed && e.activation == activation) {
-        if (e.lean == lean) return &e;
-        if (e.lean == 0) full = &e;
+        if (e.form == form) return &e;
+        if (e.form == FORM_FULL) full = &e;
       }
     }
     return full;
@@ -83,9 +86,16 @@ const Registry& registry() {
   return r;
 }
 
+// SMs, and how many clusters of four and of eight CTAs with a ring of shared memory each run at the same time: fewer
+// than the SMs would hold, since a cluster lies within one GPC (33 and 15 on a B200 of 148 SMs).
+struct Machine {
+  int sm_count = 148, clusters4 = 33, clusters8 = 15;
+  int clusters(int ctas) const { return ctas >= 8 ? clusters8 : ctas >= 4 ? clusters4 : sm_count / ctas; }
+};
 struct DeviceState {
   std::atomic<bool> ready{false};
   int sm_count = 0;
+  Machine machine;
 };
 DeviceState g_devices[kMaxDevices];
 std::mutex g_init_mutex;
@@ -184,6 +194,7 @@ struct Plan {
   int cluster_split;    // cluster size of the cluster split-K schedule (0 = not used)
   long long slabs;      // fp32 partial-sum slabs of 128 x tile_n the schedule may write
   int row_tiles;  // 128-row x tile_n tiles (split-K counters, slabs)
+  int shared_reduce;  // the CTAs that split a tile's depth through the workspace share the sum
   int tile_rows;  // rows of the row operand per tile (128 unless the swapped form trims it)
 };
 
@@ -290,13 +301,17 @@ int check_config(const ayla_b200_config& c, bool swiglu) {
 constexpr int kMaxSplitKTiles = 16384;
 constexpr size_t kCounterBytes = static_cast<size_t>(kMaxSplitKTiles) * 4;
 
+// How long the owner of a piece of a split tile waits for the other partials before it leaves the piece to the last
+// of them: far above the few microseconds by which CTAs that run together differ, and little where they do not.
+constexpr unsigned kHandoverNs = 20000;
+
 // Fills `plan` for a validated config.  `epilogue` is one of EPI_*.
 int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t rows, int64_t cols,
               int64_t k, int sm_count, Plan* plan, int activation = 0) {
   const int transposed = c.swap_ab ? 1 : 0;
   const bool swiglu_cols = epilogue == EPI_SWIGLU && !c.swap_ab;
   const int tile_n = swiglu_cols ? 256 : c.tile_n;
-  const int lean = (c.split_k <= 1 && c.stream_k == 0) ? 1 : 0;
+  const int form = (c.split_k <= 1 && c.stream_k == 0) ? FORM_LEAN : FORM_FULL;
   // `activation` 3: one that is more than a comparison, for which those launches have kernels with sixteen epilogue
   // warps (see GemmTraits::PAIRED; with a comparison or a row factor alone eight do as well or better: RMS norm and
   // projection 4096x6144x4096 172 against 173 us).
@@ -304,9 +319,9 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   // their own (us per launch, before -> with them: 16384x2048x256 71.4 -> 38.1, 6983x1472x1312 43.8 -> 32.2,
   // 1024x4096x512 15.3 -> 12.0, 64x8192x1024 10.4 -> 8.9); the k-split and swapped forms load it directly.
   const KernelEntry* e = nullptr;
-  if (activation == 2 && lean == 1) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 2, 1);
-  if (activation == 3 && lean == 1) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 3, 1);
-  if (e == nullptr) e = registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, lean);
+  if (activation == 2 && form == FORM_LEAN) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 2, FORM_LEAN);
+  if (activation == 3 && form == FORM_LEAN) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 3, FORM_LEAN);
+  if (e == nullptr) e = registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, form);
   if (e == nullptr) {
     return fail(AYLA_B200_E_UNSUPPORTED, "no kernel variant tile_n=%d cta_group=%d epilogue=%d swap=%d",
                 tile_n, c.cta_group, epilogue, transposed);
@@ -335,6 +350,7 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   plan->stream_k = 0;
   plan->kb_per_cta = 0;
   plan->cluster_split = 0;  // also for the stream-K plan below, which returns before the cluster branch
+  plan->shared_reduce = 0;
   if (c.stream_k) {
     // Equal contiguous shares of the (tile, k-block) sequence; a share is never shorter
     // than four k-blocks so that a segment is worth its epilogue.
@@ -427,6 +443,17 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   plan->group_m = c.group_m;
   if (wave > units) grid = static_cast<int>(units * c.cta_group);
   plan->grid = grid;
+  // At most one split unit per CTA, its last: those of a tile share its sum.  With more of them a CTA would wait for
+  // partials that it, or one that waits as well, has yet to compute; there the last arriver sums.
+  if (plan->splits > 1 && split_from % wave == 0 && (tiles - split_from) * plan->splits <= wave && !transposed &&
+      static_cast<int64_t>(plan->row_tiles) * (tile_n / 32) * 4 <= kMaxSplitKTiles) {
+    const KernelEntry* shared =
+        registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, FORM_SHARED);
+    if (shared != nullptr && shared->form == FORM_SHARED) {
+      plan->kernel = shared;
+      plan->shared_reduce = 1;
+    }
+  }
   return AYLA_B200_OK;
 }
 
@@ -469,16 +496,17 @@ int current_device_state(DeviceState** out, int* device) {
   return AYLA_B200_OK;
 }
 
-// For queries, which need no device: the current device's SM count where it has been set up, else a B200's.
-int current_sm_count() {
+// For queries, which need no device: the current device's where it has been set up, else a B200's.
+Machine current_machine() {
   int dev = -1;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
       g_devices[dev].ready.load(std::memory_order_acquire)) {
-    return g_devices[dev].sm_count;
+    return g_devices[dev].machine;
   }
   (void)cudaGetLastError();
-  return 148;
+  return Machine{};
 }
+int current_sm_count() { return current_machine().sm_count; }
 
 // Whether the tiles chosen for a product of at most four k-blocks are better run by CTA pairs, which read half as much
 // of B.  170 shapes timed in both forms: with this rule the paired ones take 0.946 of the time without an activation
@@ -504,8 +532,9 @@ bool shallow_pairs_pay(int64_t batch, int64_t m, int64_t n, int64_t k, int tile_
   return mid_sector ? waves >= 1.0 : waves >= 2.0 && (tile_n == 256 || k_blocks >= 3);
 }
 
-void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, int sm_count,
+void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, const Machine& machine,
                     ayla_b200_config* c) {
+  const int sm_count = machine.sm_count;
   memset(c, 0, sizeof(*c));
   c->cta_group = 1;
   c->split_k = 1;
@@ -521,11 +550,15 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
     c->swap_ab = 1;
     c->tile_n = m <= 16 ? 16 : (m <= 32 ? 32 : 64);
     const int64_t tiles = batch * ceil_div(n, 128);
-    // Split K across a cluster of 4 or 2 (summed through distributed shared memory) while
-    // the whole grid still runs in one wave and every CTA keeps at least four k-blocks.
-    // (Clusters of 8 measured about twice as slow as clusters of 4 on these shapes.)
-    for (int s = 4; s >= 2; s /= 2) {
-      if (tiles * s <= static_cast<int64_t>(sm_count) && k_blocks >= 4 * s && c->tile_n % (4 * s) == 0) {
+    // Split K across a cluster of 8, 4 or 2 (summed through distributed shared memory) while all the clusters run at
+    // once and every CTA keeps a few k-blocks.  us, all at once -> in two waves: 12x4608x5504, 36 tiles, clusters of
+    // two 12.2, of four 17.0; 17x4568x2520, 36 tiles, 8.9 and 12.7; 2x4160x8704, 33 tiles, clusters of four 13.2, of
+    // two 15.9.  Eight for deep products of the fewest tiles (28x1824x9144, 15 tiles, clusters of eight 9.8, of four
+    // 12.6; 32x2112x2560, 17 tiles, 9.6 and 5.7).
+    for (int s = 8; s >= 2; s /= 2) {
+      const int width = s == 8 && c->tile_n < 32 ? 32 : c->tile_n;
+      if (tiles <= machine.clusters(s) && k_blocks >= (s == 8 ? 140 : 4 * s) && width % (4 * s) == 0) {
+        c->tile_n = width;
         c->split_k = s;
         c->cluster_split = 1;
         break;
@@ -537,11 +570,22 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
       const int64_t share = k_blocks / c->split_k / 2;
       c->early_prefetch = static_cast<int>(share < 16 ? share : 16);
     }
-    if (c->split_k == 1 && m > 16) {
+    // One wave of tiles that would leave SMs idle is cut into as many as there are SMs (3x13056x1728, 102 -> 136 tiles,
+    // 9.7 -> 9.1; 7x13696x5504, 107 -> 143, 24.5 -> 23.6; 44x12216x4760, 96 -> 139, 30.8 -> 27.5), a split one where the
+    // stream is long (2x5888x7200, 46 -> 74, 17.0 -> 16.0; 9x6208x11200, 49 -> 71, 25.6 -> 24.4; but 14x7552x1536,
+    // 59 -> 73, 6.3 -> 6.6).
+    if (c->split_k <= 2 && batch == 1) {
+      const int64_t rows = ceil_div(ceil_div(n, sm_count / c->split_k), 8) * 8;
+      if (rows >= 72 && rows <= 96 && k_blocks / c->split_k >= (c->split_k == 1 ? 20 : 48)) {
+        c->tile_rows = static_cast<int>(rows);
+      }
+    }
+    if (c->split_k == 1 && m > 16 && (c->tile_rows == 0 || k_blocks < 40)) {
       // No room to split K (bt alone fills the SMs): with a few dozen rows of `a` the plain
       // row-major 128-wide tile, its `a` box trimmed to the rows that exist, measures 1.2-1.3x
       // faster than the swapped form (M = 32, 64 at N = 14336).
       c->swap_ab = 0;
+      c->tile_rows = 0;
       c->tile_n = (batch * ceil_div(n, 128) <= static_cast<int64_t>(sm_count)) ? 128 : 256;  // one wave if it fits
       c->group_m = 8;
       c->split_tail = 2;
@@ -606,6 +650,99 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
   if (ceil_div(m, 128 * c->cta_group) > c->group_m) c->l2_hint_b = 2;
 }
 
+// Microseconds that a product without an activation takes where its units run in one wave: a launch, then k-blocks at a
+// rate that falls with the share of the SMs at work, then, for a split depth, the sum.  Fitted to 2600 timings of 310
+// shapes (tile widths of 192 between their neighbours), median error 4 %; k-blocks of rows that start inside a 32-byte
+// sector take about 1.35 times as long.
+struct Rate { double launch, block, block_busy, per_split; };
+enum { RATE_WHOLE = 0, RATE_SHARED = 1, RATE_CLUSTER = 2 };
+double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tiles, int64_t k, const Machine& machine) {
+  static const Rate kRates[3][4][2] = {
+      {{{3.80, .147, .078, 0}, {3.20, .137, .076, 0}}, {{4.05, .221, .081, 0}, {3.80, .163, .073, 0}},
+       {{4.10, .260, .130, 0}, {4.10, .210, .100, 0}}, {{4.25, .298, .180, 0}, {4.35, .256, .131, 0}}},
+      {{{5.24, .156, .068, .30}, {5.16, .127, .097, .32}}, {{5.44, .203, .149, .265}, {5.87, .152, .118, .28}},
+       {{6.50, .250, .210, .20}, {7.00, .200, .130, .20}}, {{7.40, .289, .281, .17}, {8.25, .260, .143, .20}}},
+      {{{5.10, .170, .086, 0}, {5.10, .127, .097, 0}}, {{6.30, .262, .064, 0}, {4.30, .262, .019, 0}},
+       {{6.50, .250, .210, 0}, {7.00, .200, .130, 0}}, {{7.40, .289, .281, 0}, {8.25, .260, .143, 0}}},
+  };
+  const Rate& r = kRates[kind][tile_n / 64 - 1][cta_group - 1];
+  const int64_t at_once = kind == RATE_CLUSTER ? machine.clusters(splits * cta_group) : machine.sm_count / cta_group / splits;
+  const int64_t waves = ceil_div(tiles, at_once < 1 ? 1 : at_once);
+  double busy = static_cast<double>(tiles * splits * cta_group) / static_cast<double>(waves * machine.sm_count);
+  if (busy > 1.0) busy = 1.0;
+  const double blocks = static_cast<double>(waves * ceil_div(ceil_div(k, 64), splits)) * (k % 16 != 0 ? 1.35 : 1.0);
+  return r.launch + blocks * (r.block + r.block_busy * busy) + r.per_split * splits + 4.5 * static_cast<double>(waves - 1);
+}
+
+// Splits the depth where a row-major schedule leaves SMs idle through a long product: the CTAs of a tile share its sum
+// (see the kernel), so any number of them may work on it.  Two places:
+//  * The last, partial wave of tiles.  Splitting its tiles S ways takes 1/S of a tile's time and some 7 us for the sum
+//    instead of a whole tile's time, or three quarters of it where its tiles run at half width (us, whole -> half ->
+//    split: 2744x2112x29248, 1 + 25/74 waves, 332 -> 316 -> 266 with 2; 3024x1856x11776, 1 + 22/74, 120 -> 116 -> 104
+//    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
+//    Rows that start inside a sector are bound by their loads, which a lone pair gets faster: two ways at most
+//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6).  Otherwise half width wherever two halves fit (1260x4480x768
+//    12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
+//  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
+//    take 0.96 of the time for pairs and a deep product, 0.9 otherwise: over 152 shapes it was chosen 38 times and took
+//    0.83 of the time (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29, 175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 ->
+//    18.0, 1024x1024x8192 22.0 -> 20.1; single CTAs by less than that lose: 128x4096x4096 12.1 -> 13.5).
+void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+  if (c->swap_ab || c->stream_k || c->grid_ctas != 0 || c->split_tail == 1) return;
+  if (c->split_k > 1 && !c->cluster_split && c->split_tail != 0) return;
+  const int64_t k_blocks = ceil_div(k, 64);
+  const bool mid_sector = k % 16 != 0;
+  const int64_t wave = machine.sm_count / c->cta_group;
+  const int64_t tiles = batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n);
+  if (tiles > wave) {
+    const int64_t rest = tiles % wave;
+    if (c->split_k > 1 || c->cluster_split || rest == 0) return;
+    const bool halves_fit = c->tile_n % 128 == 0 && rest * 2 <= wave;
+    if (c->tile_n >= 128 && rest * 2 <= wave && k_blocks >= 32) {
+      int64_t splits = wave / rest;
+      if (splits > k_blocks / 8) splits = k_blocks / 8;
+      if (splits > (mid_sector ? 2 : 16)) splits = mid_sector ? 2 : 16;
+      const double block = c->tile_n == 256 ? 0.38 : c->tile_n == 192 ? 0.33 : 0.275;
+      const double now = mid_sector ? 0.7 : halves_fit ? 0.75 : 1.0;  // of a tile: a half runs at three quarters of the rate
+      if (splits >= 2 && static_cast<double>(k_blocks) * (now - 1.0 / static_cast<double>(splits)) * block > 8.5) {
+        c->split_k = static_cast<int>(splits);
+        c->split_tail = 1;
+        return;
+      }
+    }
+    if (halves_fit && !mid_sector) c->split_tail = 2;
+    return;
+  }
+  if (m <= 64 || k_blocks < 16) return;
+  const double now = modelled_us(c->tile_n, c->cta_group, c->split_k,
+                                 c->cluster_split ? RATE_CLUSTER : c->split_k > 1 ? RATE_SHARED : RATE_WHOLE, tiles, k, machine);
+  double best = now;
+  ayla_b200_config chosen = *c;
+  static const int kWidths[3] = {64, 128, 256};
+  for (int tile_n : kWidths) {
+    if (tile_n > 64 && n * 2 <= tile_n) continue;
+    for (int cta_group = 1; cta_group <= 2; ++cta_group) {
+      if (cta_group == 2 && m <= 128) continue;
+      const int64_t there = batch * ceil_div(m, 128 * cta_group) * ceil_div(n, tile_n);
+      int64_t most = machine.sm_count / cta_group / there;
+      if (most > 48) most = 48;
+      if (most > k_blocks / 4) most = k_blocks / 4;
+      for (int64_t splits = most; splits >= 2; --splits) {
+        const double bound = cta_group == 2 && tile_n >= 128 && k_blocks >= 48 ? 0.96 : 0.9;
+        const double us = modelled_us(tile_n, cta_group, static_cast<int>(splits), RATE_SHARED, there, k, machine);
+        if (us >= best || us > bound * now) continue;
+        best = us;
+        chosen.tile_n = tile_n;
+        chosen.cta_group = cta_group;
+        chosen.split_k = static_cast<int>(splits);
+        chosen.split_tail = 0;
+        chosen.cluster_split = 0;
+      }
+    }
+  }
+  *c = chosen;
+}
+
 // The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
 // leave 32 of them working at n = 4096): 64 output columns per tile, M on the narrow accumulator, k split across
 // a cluster, all in one wave.  False where no such schedule exists; where one does it measured the faster in 168
@@ -617,7 +754,7 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
 // 659x896x2432, 38, 16.0 -> 15.2, 374x2944x3200, 50, 21.9 -> 20.7; against single CTAs: 109x6080x960, 15, 10.5 ->
 // 11.4, but 150x3304x1664, 26, 14.0 -> 12.8; with rows that start inside a 32-byte sector 381x3136x3208, 51,
 // 25.1 -> 29.2, but 68x5232x11720, 184, 92.4 -> 72.8.
-bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b200_config* c) {
+bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   // us per k-block and per cluster exchange, fitted to the same measurements.
   struct Width { int tile_n; double per_kb, exchange2, exchange4; };
   static const Width kWidths[4] = {{16, 0.160, 0.9, 1.4}, {32, 0.170, 0.9, 1.4}, {64, 0.20, 1.5, 3.0}, {128, 0.28, 2.7, 4.6}};
@@ -627,7 +764,7 @@ bool swapped_swiglu_config(int64_t m, int64_t n, int64_t k, int sm_count, ayla_b
   for (const Width& w : kWidths) {
     const int64_t tiles = row_tiles * ceil_div(m, w.tile_n);
     for (int split = 1; split <= 4; split *= 2) {
-      if (tiles * split > sm_count || (split > 1 && k_blocks < 4 * split)) break;
+      if (tiles > machine.clusters(split) || (split > 1 && k_blocks < 4 * split)) break;
       if (w.tile_n == 128 && split == 1 && k_blocks < (k % 16 != 0 ? 60 : m < 256 ? 20 : 36)) continue;
       const double cost = static_cast<double>(ceil_div(k_blocks, split)) * w.per_kb +
                           (split == 1 ? 0.0 : split == 2 ? w.exchange2 : w.exchange4);
@@ -783,6 +920,7 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
       p.inbox_in_ring = 1;
     }
   }
+  p.handover_ns = (g_debug_flags.load() & 32) != 0 ? 0u : kHandoverNs;
   p.tile_rows = plan.tile_rows;
   p.act = activation;
   p.mul = mul;
@@ -912,6 +1050,28 @@ int ayla_b200_init(int device) {
       if (rc) break;
     }
     g_devices[device].sm_count = prop.multiProcessorCount;
+    Machine& machine = g_devices[device].machine;
+    machine.sm_count = prop.multiProcessorCount;
+    const KernelEntry* clustered = registry().find(128, 1, EPI_PLAIN, 0);
+    for (int ctas = 4; ctas <= 8; ctas *= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(machine.sm_count / ctas * ctas));
+      cfg.blockDim = dim3(static_cast<unsigned>(clustered->threads));
+      cfg.dynamicSmemBytes = static_cast<size_t>(clustered->smem_bytes);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int at_once = 0;
+      if (cudaOccupancyMaxActiveClusters(&at_once, clustered->func, &cfg) != cudaSuccess || at_once < 1) {
+        (void)cudaGetLastError();
+        continue;  // what a B200 holds stays
+      }
+      (ctas == 4 ? machine.clusters4 : machine.clusters8) = at_once;
+    }
     g_devices[device].ready.store(true, std::memory_order_release);
   } while (false);
   if (prev >= 0 && prev != device) cudaSetDevice(prev);
@@ -931,7 +1091,17 @@ int ayla_b200_default_config_act(int op, int dtype, int activation, int64_t batc
   if (activation < AYLA_B200_ACT_NONE || activation > AYLA_B200_ACT_GELU_TANH) {
     return fail(AYLA_B200_E_INVALID, "unknown activation %d", activation);
   }
-  default_config(batch, m, n, k, activation, current_sm_count(), cfg_out);
+  default_config(batch, m, n, k, activation, current_machine(), cfg_out);
+  return AYLA_B200_OK;
+}
+
+int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k, ayla_b200_config* cfg) {
+  if (cfg == nullptr) return fail(AYLA_B200_E_INVALID, "cfg is null");
+  int rc = check_shape(op, dtype, batch, m, n, k);
+  if (rc) return rc;
+  rc = check_config(*cfg, false);
+  if (rc) return rc;
+  share_depth(batch, m, n, k, current_machine(), cfg);
   return AYLA_B200_OK;
 }
 
@@ -939,7 +1109,7 @@ int ayla_b200_swiglu_default_config(int dtype, int64_t m, int64_t n, int64_t k, 
   if (cfg_out == nullptr) return fail(AYLA_B200_E_INVALID, "cfg_out is null");
   const int rc = check_shape(AYLA_B200_OP_MM, dtype, 1, m, n, k);
   if (rc) return rc;
-  if (!swapped_swiglu_config(m, n, k, current_sm_count(), cfg_out)) *cfg_out = row_major_swiglu_config(m);
+  if (!swapped_swiglu_config(m, n, k, current_machine(), cfg_out)) *cfg_out = row_major_swiglu_config(m);
   return AYLA_B200_OK;
 }
 
@@ -1046,7 +1216,15 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   } else if (activation == AYLA_B200_ACT_NONE && mul == nullptr && packed_preferred(batch, m, n, k, ds->sm_count)) {
     return ayla_b200_gemm_packed(op, dtype, bias, a, bt, out, batch, m, n, k, status, stream);
   } else {
-    default_config(batch, m, n, k, activation, ds->sm_count, &c);
+    default_config(batch, m, n, k, activation, ds->machine, &c);
+    // A gate shaped like the output has kernels of its own, without a k-split; and a caller who lent no workspace, or
+    // too little, gets the schedule as it was.
+    if (mul == nullptr || mul_per_row != 0) {
+      ayla_b200_config shared = c;
+      share_depth(batch, m, n, k, ds->machine, &shared);
+      const size_t need = ayla_b200_workspace_bytes(&shared, op, batch, m, n, k);
+      if (need == 0 || (workspace != nullptr && workspace_bytes >= need)) c = shared;
+    }
   }
   rc = check_config(c, false);
   if (rc) return rc;
@@ -1147,7 +1325,7 @@ int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const voi
   if (cfg != nullptr) {
     c = *cfg;
   } else {
-    default_config(batch, m, n, k, AYLA_B200_ACT_NONE, ds->sm_count, &c);
+    default_config(batch, m, n, k, AYLA_B200_ACT_NONE, ds->machine, &c);
   }
   rc = check_config(c, false);
   if (rc) return rc;
@@ -1176,7 +1354,8 @@ int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const voi
     if (rc) return rc;
     // The array keeps whatever the previous call left behind.  Only the arrival
     // counters must start at zero; partial sums are fully rewritten before they are read.
-    const cudaError_t err = cudaMemsetAsync(scratch, 0, static_cast<size_t>(plan.row_tiles) * 4, s);
+    const int counters = plan.row_tiles * (plan.shared_reduce ? plan.kernel->tile_n / 32 * 4 : 1);
+    const cudaError_t err = cudaMemsetAsync(scratch, 0, static_cast<size_t>(counters) * 4, s);
     if (err != cudaSuccess) {
       return fail(AYLA_B200_E_CUDA, "clearing the split-K counters: %s", cudaGetErrorString(err));
     }
@@ -1201,7 +1380,7 @@ int ayla_b200_swiglu(int dtype, const void* x, const void* w_gate, const void* w
   rc = current_device_state(&ds, &dev);
   if (rc) return rc;
   ayla_b200_config c;
-  const bool swapped = cfg == nullptr && swapped_swiglu_config(m, n, k, ds->sm_count, &c);
+  const bool swapped = cfg == nullptr && swapped_swiglu_config(m, n, k, ds->machine, &c);
   if (!swapped) {
     c = cfg != nullptr ? *cfg : row_major_swiglu_config(m);
     c.tile_n = 256;

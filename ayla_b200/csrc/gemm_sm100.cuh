@@ -38,6 +38,9 @@ namespace ayla_b200 {
 
 enum : int { EPI_PLAIN = 0, EPI_BIAS = 1, EPI_SWIGLU = 2 };
 
+// Which k-split epilogues a kernel is compiled with: all but the shared sum, none, or the shared sum alone.
+enum : int { FORM_FULL = 0, FORM_LEAN = 1, FORM_SHARED = 2 };
+
 // Error codes written to the device status word (first error wins).
 enum : unsigned {
   ST_OK = 0,
@@ -113,6 +116,7 @@ struct KernelParams {
   FastDiv div_last_group_rows;  // by the row tiles of the last, partial raster group (m_tiles % group_m)
   FastDiv div_splits;           // by splits
   int ctas_per_unit_log2;       // log2(CTA_GROUP * cluster_split or 1)
+  unsigned handover_ns; // shared sum: how long the owner of a piece waits before it leaves the piece to the others
   int stages;         // ring slots in use (<= the kernel's STAGES); fewer when the top of the ring region
                       // is set aside as the inbox of a cluster split-K launch
   uint32_t inbox_offset;  // cluster split-K: byte offset of the inbox from the start of shared memory
@@ -156,13 +160,16 @@ __device__ __forceinline__ void trace_stamp(long long* stamps, int slot) {
 #define AYLA_TRACE_END(slot)
 #endif
 
-template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, int ACT_ = 0, bool LEAN_ = false,
+template <int BN_, int CTA_GROUP_, int EPI_, bool TRANS_OUT_, int STAGES_, int ACT_ = 0, int FORM_ = FORM_FULL,
           bool GATED_ = false>
 struct GemmTraits {
   // LEAN: the kernel is compiled without the k-split epilogues (workspace and cluster forms) and
   // serves the launches that do not split k.  The unused code is never executed, yet it costs a
   // single-tile launch up to 1 us (instruction fetch), so those launches get a kernel without it.
-  static constexpr bool LEAN = LEAN_;
+  static constexpr bool LEAN = FORM_ == FORM_LEAN;
+  // SHARED: whole tiles, and k-splits, one unit per CTA, that share their sum through the workspace.
+  static constexpr bool SHARED = FORM_ == FORM_SHARED;
+  static constexpr bool FULL = FORM_ == FORM_FULL;
   // ACT: the epilogue applies the activation named in the launch parameters.  A separate set of
   // instantiations, so that the plain kernels carry none of that code (compiled in as a run-time
   // branch it cost the output-bound bmm 5 %).
@@ -230,6 +237,7 @@ struct GemmTraits {
   static_assert(B_BYTES % 1024 == 0, "B slab must keep the 1024-byte swizzle alignment");
   static_assert(!SWIGLU_COLS || BN == 256, "row-major SwiGLU uses the 2x128 layout");
   static_assert(!PAIRED || (LEAN && !GATED && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
+  static_assert(!SHARED || (!TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches");
   static_assert(!GATED || (ACT && LEAN && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
   static_assert(TRANS_OUT || BN >= 64, "the TMA-store epilogue writes 64-column boxes");
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB shared-memory limit");
@@ -251,6 +259,20 @@ struct BoundedWait {
   __device__ __noinline__ void give_up(unsigned code) const {
     *abort_flag = 1;
     if (status != nullptr) atomicCAS(status, 0u, code | (blockIdx.x << 8));
+  }
+
+  // Whether a counter in global memory reaches `value` within `limit_ns`; if so, what was released with the
+  // increments is visible to this thread.
+  __device__ __forceinline__ bool count_reaches(const unsigned* counter, unsigned value, unsigned limit_ns) const {
+    uint64_t t0 = 0;
+    for (;;) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+      if (seen == value) return true;
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 >= limit_ns || aborted()) return false;
+    }
   }
 
   __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, unsigned code) const {
@@ -599,7 +621,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
   // Cluster split-K: the cluster holds `csk` CTAs (CTA pairs when CG == 2), one per k-split
   // of the cluster's tile.
-  const int csk = (!T::SWIGLU_COLS && !T::LEAN) ? p.cluster_split : 0;
+  const int csk = (!T::SWIGLU_COLS && T::FULL) ? p.cluster_split : 0;
   constexpr int group = T::KB_PER_SLOT;  // k-blocks per ring slot
   const int n_stages = p.stages;         // ring slots in use
 
@@ -977,7 +999,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // Kernels that take several tiles look one unit ahead and read its slice while this one's tile is on its way
     // (read at the head of a tile its latency was part of every tile: addmm 5215x1216x320 8.3 -> 7.6 us).
     constexpr bool ROW_BIAS = T::EPI == EPI_BIAS && !T::TRANS_OUT;
-    constexpr bool AHEAD = ROW_BIAS && T::LEAN && BN >= 128;
+    constexpr bool AHEAD = ROW_BIAS && !T::FULL && BN >= 128;
     const int bias_thread = half_of_pair * 128 + q * 32 + lane;
     const int bias_col = (T::GATED ? wsub * 64 : (bias_thread >> 6) * 128 + wsub * 64) + (bias_thread & 63);
     const bool bias_reads = T::GATED ? bias_thread < 64 : bias_col < BN;
@@ -1004,7 +1026,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // This tile's bias slice as fp32, double buffered so one meeting per tile is enough.
       if constexpr (AHEAD) {
         if (bias_reads) smem_bias[bias_buf * BN + bias_col] = bias_next;
-        named_bar_sync(6 + wsub, T::PAIRED ? 256 : 128);
+        if constexpr (T::LEAN) {
+          named_bar_sync(6 + wsub, T::PAIRED ? 256 : 128);
+        } else {
+          named_bar_sync(1, EPI_THREADS);  // the chunks of a k-split are not dealt by column groups
+        }
         has_next = cursor.next(next);
         if (has_next) bias_next = load_bias(next.n0);
       } else if constexpr (ROW_BIAS) {
@@ -1215,7 +1241,43 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
       };
 
-      if (csk > 0) {
+      // A lone 32-column chunk of summed partials, row-major: bias, activation and gate, then through this warp's
+      // staging rows, so that one store instruction writes eight rows of 64 contiguous bytes instead of 16 bytes of
+      // each of 32 rows (the load/store unit takes a cycle per 128-byte line touched: 0.6 us for the tile the direct
+      // way).  Row r holds its four 16-byte pieces at r * 64, piece c at position c ^ ((r >> 1) & 3).
+      auto write_lone_chunk = [&](float (&v)[32], int c32) {
+        if constexpr (!T::TRANS_OUT && !T::LEAN) {
+          const int col0 = w.n0 + c32 * 32;
+          uint32_t pk[16];
+          if (w.m0 + row_in_tile < row_end) pack_chunk(v, c32, pk);
+          if constexpr (T::SHARED) {
+            if (lane == 0) tma_store_wait_read<0>();  // of a whole tile before this one
+          }
+          __syncwarp();
+          if (w.m0 + row_in_tile < row_end) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              *reinterpret_cast<uint4*>(my_store + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) =
+                  make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+            }
+          }
+          __syncwarp();
+          const int piece = lane & 3;
+          const int col = col0 + piece * 8;
+          uint8_t* dst0 = reinterpret_cast<uint8_t*>(p.out) + 2 * (w.batch * p.out_batch_stride + col);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = i * 8 + (lane >> 2);
+            const int out_row = w.m0 + q * 32 + r;
+            const uint4 x = *reinterpret_cast<const uint4*>(my_store + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4));
+            if (out_row < row_end && col < p.n) {
+              *reinterpret_cast<uint4*>(dst0 + 2 * static_cast<long long>(out_row) * p.out_ld) = x;
+            }
+          }
+        }
+      };
+
+      if (T::FULL && csk > 0) {
         // ---- cluster split-K: S CTAs of the cluster (those with this CTA's place in its
         // pair) hold the S partial sums of this 128-row tile.  Each owns BN / S columns of
         // it: every CTA sends each owner its partial of the owner's columns with asynchronous
@@ -1223,7 +1285,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         // owner's inbox barrier with its bytes; an owner waits for that barrier alone, adds
         // the S partials in split order and stores.  Nobody waits for a sender's stores but
         // their receiver.
-        if constexpr (!T::SWIGLU_COLS) {
+        if constexpr (!T::SWIGLU_COLS && T::FULL) {
           const int slice_cols = BN / csk;
           const int slice_shift = __ffs(slice_cols) - 1;
           const int slice_c4 = slice_cols >> 2;
@@ -1353,42 +1415,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 if (!(rows_live && col0 < p.n)) continue;
                 if constexpr (T::TRANS_OUT) {
                   finish_chunk(v, c32);
-                } else if (row < row_end) {
-                  // A lone 32-column chunk: 64 contiguous bytes of this thread's output row.
-                  if constexpr (T::EPI == EPI_BIAS) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += smem_bias[bias_buf * BN + c32 * 32 + j];
-                  }
-                  apply_act_chunk<32>(v, act);
-                  gate_chunk(v, c32);
-                }
-                // Through this warp's staging rows, so that one store instruction writes eight
-                // rows of 64 contiguous bytes instead of 16 bytes of each of 32 rows (the load/store
-                // unit takes a cycle per 128-byte line touched: 0.6 us for the tile the direct way).
-                // Row r holds its four 16-byte pieces at r * 64, piece c at position c ^ ((r >> 1) & 3).
-                if constexpr (!T::TRANS_OUT) {
-                  __syncwarp();
-                  if (row < row_end) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                      *reinterpret_cast<uint4*>(my_store + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) =
-                          make_uint4(pack2(v[8 * j], v[8 * j + 1], is_bf16), pack2(v[8 * j + 2], v[8 * j + 3], is_bf16),
-                                     pack2(v[8 * j + 4], v[8 * j + 5], is_bf16), pack2(v[8 * j + 6], v[8 * j + 7], is_bf16));
-                    }
-                  }
-                  __syncwarp();
-                  const int piece = lane & 3;
-                  const int col = col0 + piece * 8;
-                  uint8_t* dst0 = reinterpret_cast<uint8_t*>(p.out) + 2 * (w.batch * p.out_batch_stride + col);
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) {
-                    const int r = i * 8 + (lane >> 2);
-                    const int out_row = w.m0 + q * 32 + r;
-                    const uint4 x = *reinterpret_cast<const uint4*>(my_store + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4));
-                    if (out_row < row_end && col < p.n) {
-                      *reinterpret_cast<uint4*>(dst0 + 2 * static_cast<long long>(out_row) * p.out_ld) = x;
-                    }
-                  }
+                } else {
+                  write_lone_chunk(v, c32);
                 }
               }
             }
@@ -1617,12 +1645,132 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           }
           if (wsub >= CHUNKS32) release_accumulator();
         }
+      } else if (T::SHARED) {
+        // ---- split-K, the sum shared by the S CTAs that hold the partials of this 128-row tile (one such unit per
+        // CTA, its last).
+        // Each piece of it, 32 rows x 32 columns, has an owner among them: every CTA writes its partial of the pieces
+        // of others into its slab and counts itself in at the piece's counter; the owner keeps its own in TMEM, waits
+        // for the S - 1 others, adds in split order and stores.  All of it is warp to warp: the sender and the owner
+        // of a piece are the warps of one lane quarter and chunk parity.
+        // The others need not be running (the grid may share the GPU), so the owner's wait is short: when it runs
+        // out, it parks its own partial as well and leaves the piece to whoever counts itself in last.
+        // What bounds it is the SM's store rate (some 28 bytes a clock, 96 KB per CTA of a 256 x 256 pair tile split
+        // four ways) and a chain of fence, atomic, poll and read through L2: 2 us (128-wide tiles) to 4 us (256-wide)
+        // and 0.2 to 0.3 us per split on top of a launch.  Where the last arriver summed S slabs of the tile alone, it
+        // read S - 1 times as much in one CTA; a cluster's exchange through shared memory needs its CTAs to fit one
+        // GPC (mm 1024x1024x8192 in 128-wide pair tiles split in two: through clusters 21.9 us, this way 20.9).
+        if constexpr (T::SHARED) {
+          constexpr unsigned HANDED_OVER = 1u << 16;
+          const int splits = w.nsplit;
+          const float4* slabs = reinterpret_cast<const float4*>(p.ws) + static_cast<size_t>(w.slab0) * (32 * BN);
+          float4* my_slab = reinterpret_cast<float4*>(p.ws) + static_cast<size_t>(w.slab0 + w.split) * (32 * BN);
+          unsigned* counters = p.counters + w.counter * (CHUNKS32 * 4) + q;  // of chunk c32: [c32 * 4]
+          auto owner_of = [&](int c32) {
+            // Up to a chunk per CTA: contiguous chunks each; beyond: the lane quarters of a chunk apart as well.
+            return splits <= CHUNKS32 ? (c32 * splits) / CHUNKS32
+                                      : c32 + CHUNKS32 * ((q * min(splits / CHUNKS32, 4)) >> 2);
+          };
+          auto park = [&](int c32) {
+            uint32_t r[32];
+            tmem_ld_32x32(t_acc + c32 * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              __stcg(my_slab + (c32 * 8 + j) * 128 + row_in_tile,
+                     make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                 __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+            }
+          };
+          // The pieces of others: parked, then counted in with one fence for all of them.
+          int sent = 0, my_piece = -1;  // lane i remembers the i-th piece sent
+#pragma unroll 1
+          for (int c32 = wsub; c32 < CHUNKS32; c32 += 2) {
+            if (!rows_live || w.n0 + c32 * 32 >= p.n || owner_of(c32) == w.split) continue;
+            park(c32);
+            if (lane == sent) my_piece = c32;
+            ++sent;
+          }
+          __syncwarp();
+          unsigned before = 0;
+          if (my_piece >= 0) {
+            __threadfence();
+            before = atomicAdd(counters + my_piece * 4, 1u);
+          }
+          const bool left_to_me = my_piece >= 0 && before == HANDED_OVER + static_cast<unsigned>(splits - 2);
+          // This CTA's own pieces, and those whose owner gave up waiting and whose last partial was this warp's.
+#pragma unroll 1
+          for (int c32 = wsub; c32 < CHUNKS32; c32 += 2) {
+            if (!rows_live || w.n0 + c32 * 32 >= p.n) continue;
+            const bool own = owner_of(c32) == w.split;
+            bool complete;
+            if (own) {
+              complete = true;
+              if (lane == 0) complete = bw.count_reaches(counters + c32 * 4, static_cast<unsigned>(splits - 1), p.handover_ns);
+              if (!__shfl_sync(0xffffffffu, complete ? 1 : 0, 0)) {
+                park(c32);
+                __syncwarp();
+                if (lane == 0) {
+                  __threadfence();
+                  // The others may all have arrived by now: then nobody comes after this.
+                  complete = atomicAdd(counters + c32 * 4, HANDED_OVER) == static_cast<unsigned>(splits - 1);
+                  __threadfence();
+                }
+              }
+              complete = __shfl_sync(0xffffffffu, complete ? 1 : 0, 0) != 0;
+            } else {
+              complete = __any_sync(0xffffffffu, left_to_me && my_piece == c32);
+              if (complete) __threadfence();
+            }
+            if (!complete) continue;
+            __syncwarp();  // what one lane has acquired is there for all
+            // All partials in split order, two of them on their way at a time; an owner's own comes from TMEM.
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0.0f;
+            const float4* at = slabs + c32 * 8 * 128 + row_in_tile;
+            const int in_tmem = own ? w.split : -1;
+            auto fetch = [&](int s, float4 (&x)[8]) {
+              if (s == in_tmem) {
+                tmem_ld_32x32(t_acc + c32 * 32, *reinterpret_cast<uint32_t(*)[32]>(&x[0]));
+                tmem_ld_wait();
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = __ldcg(at + static_cast<size_t>(s) * (32 * BN) + j * 128);
+              }
+            };
+            auto add = [&](const float4 (&x)[8]) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                v[4 * j + 0] += x[j].x;
+                v[4 * j + 1] += x[j].y;
+                v[4 * j + 2] += x[j].z;
+                v[4 * j + 3] += x[j].w;
+              }
+            };
+#pragma unroll 1
+            for (int s = 0; s + 1 < splits; s += 2) {
+              float4 x0[8], x1[8];
+              fetch(s, x0);
+              fetch(s + 1, x1);
+              add(x0);
+              add(x1);
+            }
+            if ((splits & 1) != 0) {
+              float4 x0[8];
+              fetch(splits - 1, x0);
+              add(x0);
+            }
+            write_lone_chunk(v, c32);
+            if (lane == 0) counters[c32 * 4] = 0;  // clean for the next launch
+          }
+          release_accumulator();
+        }
       } else {
         // ---- split-K: park the fp32 partial, last arriver of the tile reduces.
         // Slab layout: float4 index (c4, row) -> c4 * 128 + row, so a warp's
         // 16-byte accesses are contiguous.  64-column groups (32-column chunks in the
         // transposed form) alternate between the two warps of a lane quarter.
-        if constexpr (T::EPI != EPI_SWIGLU) {
+        if constexpr (T::EPI != EPI_SWIGLU && T::FULL) {
           constexpr int STEP = T::TRANS_OUT ? 1 : 2;  // chunks handled back to back
           float4* slab = reinterpret_cast<float4*>(p.ws) +
                          static_cast<size_t>(cursor.slab_of(w, w.split)) * (32 * BN);

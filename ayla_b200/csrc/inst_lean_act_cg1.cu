@@ -4,13 +4,13 @@
 
 namespace ayla_b200 {
 void append_variants_lean_act_cg1(std::vector<KernelEntry>* out) {
-  out->push_back(make_entry<64, 1, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<128, 1, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<192, 1, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<256, 1, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<64, 1, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<128, 1, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<192, 1, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<256, 1, EPI_BIAS, false, true, true>());
+  out->push_back(make_entry<64, 1, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 1, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<192, 1, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<256, 1, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<64, 1, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 1, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<192, 1, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<256, 1, EPI_BIAS, false, true, FORM_LEAN>());
 }
 }  // namespace ayla_b200

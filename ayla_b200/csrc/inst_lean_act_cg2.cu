@@ -4,13 +4,13 @@
 
 namespace ayla_b200 {
 void append_variants_lean_act_cg2(std::vector<KernelEntry>* out) {
-  out->push_back(make_entry<64, 2, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<128, 2, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<192, 2, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<256, 2, EPI_PLAIN, false, true, true>());
-  out->push_back(make_entry<64, 2, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<128, 2, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<192, 2, EPI_BIAS, false, true, true>());
-  out->push_back(make_entry<256, 2, EPI_BIAS, false, true, true>());
+  out->push_back(make_entry<64, 2, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_PLAIN, false, true, FORM_LEAN>());
+  out->push_back(make_entry<64, 2, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_BIAS, false, true, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_BIAS, false, true, FORM_LEAN>());
 }
 }  // namespace ayla_b200

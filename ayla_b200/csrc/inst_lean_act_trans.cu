@@ -4,13 +4,13 @@
 
 namespace ayla_b200 {
 void append_variants_lean_act_trans(std::vector<KernelEntry>* out) {
-  out->push_back(make_entry<16, 1, EPI_PLAIN, true, true, true>());
-  out->push_back(make_entry<32, 1, EPI_PLAIN, true, true, true>());
-  out->push_back(make_entry<64, 1, EPI_PLAIN, true, true, true>());
-  out->push_back(make_entry<128, 1, EPI_PLAIN, true, true, true>());
-  out->push_back(make_entry<16, 1, EPI_BIAS, true, true, true>());
-  out->push_back(make_entry<32, 1, EPI_BIAS, true, true, true>());
-  out->push_back(make_entry<64, 1, EPI_BIAS, true, true, true>());
-  out->push_back(make_entry<128, 1, EPI_BIAS, true, true, true>());
+  out->push_back(make_entry<16, 1, EPI_PLAIN, true, true, FORM_LEAN>());
+  out->push_back(make_entry<32, 1, EPI_PLAIN, true, true, FORM_LEAN>());
+  out->push_back(make_entry<64, 1, EPI_PLAIN, true, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 1, EPI_PLAIN, true, true, FORM_LEAN>());
+  out->push_back(make_entry<16, 1, EPI_BIAS, true, true, FORM_LEAN>());
+  out->push_back(make_entry<32, 1, EPI_BIAS, true, true, FORM_LEAN>());
+  out->push_back(make_entry<64, 1, EPI_BIAS, true, true, FORM_LEAN>());
+  out->push_back(make_entry<128, 1, EPI_BIAS, true, true, FORM_LEAN>());
 }
 }  // namespace ayla_b200

@@ -4,13 +4,13 @@
 
 namespace ayla_b200 {
 void append_variants_lean_cg2(std::vector<KernelEntry>* out) {
-  out->push_back(make_entry<64, 2, EPI_PLAIN, false, false, true>());
-  out->push_back(make_entry<128, 2, EPI_PLAIN, false, false, true>());
-  out->push_back(make_entry<192, 2, EPI_PLAIN, false, false, true>());
-  out->push_back(make_entry<256, 2, EPI_PLAIN, false, false, true>());
-  out->push_back(make_entry<64, 2, EPI_BIAS, false, false, true>());
-  out->push_back(make_entry<128, 2, EPI_BIAS, false, false, true>());
-  out->push_back(make_entry<192, 2, EPI_BIAS, false, false, true>());
-  out->push_back(make_entry<256, 2, EPI_BIAS, false, false, true>());
+  out->push_back(make_entry<64, 2, EPI_PLAIN, false, false, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_PLAIN, false, false, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_PLAIN, false, false, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_PLAIN, false, false, FORM_LEAN>());
+  out->push_back(make_entry<64, 2, EPI_BIAS, false, false, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_BIAS, false, false, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_BIAS, false, false, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_BIAS, false, false, FORM_LEAN>());
 }
 }  // namespace ayla_b200

@@ -4,13 +4,13 @@
 
 namespace ayla_b200 {
 void append_variants_paired_cg2(std::vector<KernelEntry>* out) {
-  out->push_back(make_entry<64, 2, EPI_PLAIN, false, 2, true>());
-  out->push_back(make_entry<128, 2, EPI_PLAIN, false, 2, true>());
-  out->push_back(make_entry<192, 2, EPI_PLAIN, false, 2, true>());
-  out->push_back(make_entry<256, 2, EPI_PLAIN, false, 2, true>());
-  out->push_back(make_entry<64, 2, EPI_BIAS, false, 2, true>());
-  out->push_back(make_entry<128, 2, EPI_BIAS, false, 2, true>());
-  out->push_back(make_entry<192, 2, EPI_BIAS, false, 2, true>());
-  out->push_back(make_entry<256, 2, EPI_BIAS, false, 2, true>());
+  out->push_back(make_entry<64, 2, EPI_PLAIN, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_PLAIN, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_PLAIN, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_PLAIN, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<64, 2, EPI_BIAS, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<128, 2, EPI_BIAS, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<192, 2, EPI_BIAS, false, 2, FORM_LEAN>());
+  out->push_back(make_entry<256, 2, EPI_BIAS, false, 2, FORM_LEAN>());
 }
 }  // namespace ayla_b200

@@ -23,9 +23,10 @@ struct LaunchArgs {
 struct KernelEntry {
   int tile_n, cta_group, epilogue, transposed_out, stages, smem_bytes;
   int kb_per_slot;  // k-blocks one ring slot holds
+  int threads;
   int activation;  // 1 = the variant whose epilogue applies the launch's activation, 2 = the same for
                    // launches with a gate operand shaped like the output, 3 = with sixteen epilogue warps
-  int lean;        // 1 = the variant without the k-split epilogues
+  int form;        // FORM_*: the k-split epilogues it is compiled with
   const void* func;
   cudaError_t (*launch)(const LaunchArgs&);
 };
@@ -34,7 +35,7 @@ constexpr int kMaxSmem = 232448;
 
 template <int BN, int CG, int EPI, bool TR, bool GATED = false>
 constexpr int max_stages() {
-  using T1 = GemmTraits<BN, CG, EPI, TR, 1, GATED, GATED, GATED>;
+  using T1 = GemmTraits<BN, CG, EPI, TR, 1, GATED, GATED ? FORM_LEAN : FORM_FULL, GATED>;
   const int fixed = T1::STORE_BYTES + T1::BIAS_BYTES + T1::MISC_BYTES;
   const int s = (kMaxSmem - fixed) / T1::SLOT_BYTES;
 #ifdef AYLA_B200_STAGE_CAP
@@ -73,9 +74,9 @@ cudaError_t launch_variant(const LaunchArgs& a) {
   return cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<T>, a.tm_a, a.tm_b, a.tm_b2, a.tm_d, a.p);
 }
 
-template <int BN, int CG, int EPI, bool TR, int ACT = 0, bool LEAN = false, bool GATED = false>
+template <int BN, int CG, int EPI, bool TR, int ACT = 0, int FORM = FORM_FULL, bool GATED = false>
 KernelEntry make_entry() {
-  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED>(), ACT, LEAN, GATED>;
+  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED>(), ACT, FORM, GATED>;
   KernelEntry e;
   e.tile_n = BN;
   e.cta_group = CG;
@@ -84,8 +85,9 @@ KernelEntry make_entry() {
   e.stages = T::STAGES;
   e.smem_bytes = T::SMEM_BYTES;
   e.kb_per_slot = T::KB_PER_SLOT;
+  e.threads = T::THREADS;
   e.activation = GATED ? 2 : T::PAIRED ? 3 : ACT;
-  e.lean = LEAN ? 1 : 0;
+  e.form = FORM;
   e.func = reinterpret_cast<const void*>(&gemm_sm100_kernel<T>);
   e.launch = &launch_variant<T>;
   return e;
@@ -110,5 +112,9 @@ void append_variants_paired_cg2(std::vector<KernelEntry>* out);
 void append_variants_gated_cg1(std::vector<KernelEntry>* out);
 void append_variants_gated_cg2(std::vector<KernelEntry>* out);
 void append_variants_lean_act_trans(std::vector<KernelEntry>* out);
+void append_variants_shared_cg1(std::vector<KernelEntry>* out);
+void append_variants_shared_cg2(std::vector<KernelEntry>* out);
+void append_variants_shared_act_cg1(std::vector<KernelEntry>* out);
+void append_variants_shared_act_cg2(std::vector<KernelEntry>* out);
 
 }  // namespace ayla_b200

@@ -20,7 +20,7 @@ from __future__ import annotations
 
 import math
 import os
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from functools import cache
 
 import torch
@@ -104,6 +104,8 @@ def _seed(captured: dict[str, object], operation: str, dtype: str, m: int, n: in
 
 
 _SM_COUNT = 148
+# Clusters of this many CTAs that run at the same time on a B200: each lies within one GPC.
+_CLUSTERS_AT_ONCE = {1: 148, 2: 74, 4: 33, 8: 15}
 
 
 def _waves(config: dict[str, object], batch: int, m: int, n: int) -> int:
@@ -117,7 +119,7 @@ def _waves(config: dict[str, object], batch: int, m: int, n: int) -> int:
     split = int(config["split_k"])
     if config["cluster_split"]:
         cluster = split * pair
-        return -(-tiles // max(1, _SM_COUNT // cluster))
+        return -(-tiles // _CLUSTERS_AT_ONCE.get(cluster, max(1, _SM_COUNT // cluster)))
     units = tiles * (1 if config["split_tail"] else split)
     return -(-units // (_SM_COUNT // pair))
 
@@ -139,14 +141,36 @@ def measured_gemm_configs(operation: str, dtype: str, m: int, n: int, k: int,
     return tuple({**_DEFAULTS, **CONFIGS[index]} for index in indices)
 
 
+def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int,
+                  batch: int) -> GemmScheduleSeed | None:
+    """The schedule with its depth split where it leaves SMs idle (``ayla_b200_share_depth``)."""
+    if seed is None or seed.builder_config is None:
+        return seed
+    shared = _lib.share_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
+    if shared == seed.builder_config:
+        return seed
+    captured = {**seed.captured_config, **shared}
+    return replace(seed, captured_config=captured, builder_config=_builder_config(captured),
+                   adaptations=(*seed.adaptations, "depth split where SMs would idle"))
+
+
+def _streams_weights(operation: str, batch: int, m: int, n: int, k: int) -> bool:
+    """A few rows against a large weight: the library's rule (one wave of clusters that run at once, as many tiles as
+    SMs) is the better guess there than a neighbour's schedule (us, neighbour -> rule: 12x4608x5504 17.2 -> 12.2,
+    17x4568x2520 12.8 -> 8.9, 7x13696x5504 26.1 -> 23.6, 10x7424x3968 12.7 -> 11.7)."""
+    return operation != "bmm" and batch == 1 and m <= 64 and n >= 1024 and k >= 1024
+
+
 def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
-                         batch: int = 1, activation: str = "none") -> GemmScheduleSeed | None:
+                         batch: int = 1, activation: str = "none", share_depth: bool = True) -> GemmScheduleSeed | None:
     """The schedule a launch of this shape uses, or ``None`` if the shape is unsupported.
 
     An exact table hit has empty ``adaptations``; a schedule transferred from a
     nearby measured shape names that shape; otherwise the library's shape-aware
     default, which takes the fused ``activation`` into account, is returned with
-    ``source_shape`` ``None``.  It is a schedule of the general
+    ``source_shape`` ``None``.  Any of them has its depth split further where that is faster, which its
+    adaptations then say, unless ``share_depth`` is false (for a gate shaped like the output, whose kernels do not
+    split, and for launches that leave SMs to others).  It is a schedule of the general
     kernel: plain products that ``packed_serves`` run on the packed kernel, which takes none.
     """
     if min(batch, m, n, k) <= 0 or operation not in _OPERATIONS:
@@ -163,6 +187,11 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
     def distance(shape: tuple[int, int, int, int]) -> float:
         return sum(abs(math.log2(a) - math.log2(b)) for a, b in zip(shape, query, strict=True))
 
+    def finished(seed: GemmScheduleSeed | None) -> GemmScheduleSeed | None:
+        return _shared_depth(seed, operation, dtype, m, n, k, batch) if share_depth else seed
+
+    if query not in table and _streams_weights(operation, batch, m, n, k):
+        return finished(_fallback_schedule(operation, dtype, m, n, k, batch, activation))
     for shape in sorted(table, key=distance):
         if distance(shape) > _MAX_TRANSFER_DISTANCE:
             break
@@ -180,8 +209,8 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
                     seed = GemmScheduleSeed(seed.captured_config, seed.builder_config,
                                             (*seed.adaptations, f"measured in {other}"), seed.source_shape,
                                             seed.source_percentage_of_torch)
-                return seed
-    return _fallback_schedule(operation, dtype, m, n, k, batch, activation)
+                return finished(seed)
+    return finished(_fallback_schedule(operation, dtype, m, n, k, batch, activation))
 
 
 def _fallback_schedule(operation: str, dtype: str, m: int, n: int, k: int,
@@ -405,7 +434,7 @@ def gemm_jit_compiler(operation: str, dtype: str, activation: str = "none",
         if gated is True and tuple(mul) != tuple(out):
             raise ValueError(f"{bound.name}: mul must have the shape of out {tuple(out)}, got {tuple(mul)}")
         count = batch[0] if batch else 1
-        schedule = select_gemm_schedule(operation, dtype, m, n, k, count, activation)
+        schedule = select_gemm_schedule(operation, dtype, m, n, k, count, activation, gated is not True)
         if schedule is None:
             raise ValueError(f"{bound.name}: no schedule for {operation} {lead}x{m}x{n}x{k}")
         return GemmLauncher(operation, dtype, count, m, n, k, schedule, device, activation, gated,

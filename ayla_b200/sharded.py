@@ -247,7 +247,7 @@ class NShardedMM:
         self.cfgs: dict[int, object] = {}
         need = 16
         for height in sorted({p.rows for p in self.panels}):
-            seed = select_gemm_schedule("mm", dtype, height, self.width, k)
+            seed = select_gemm_schedule("mm", dtype, height, self.width, k, share_depth=False)
             if seed is None:
                 raise ValueError(f"no schedule for panel {height}x{self.width}x{k}")
             cfg = dict(seed.builder_config)

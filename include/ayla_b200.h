@@ -255,6 +255,15 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
                                                int64_t n, int64_t k, ayla_b200_config* cfg_out);
 
 /*
+ * Rewrites a schedule that leaves SMs idle through a deep product (a thin last wave of tiles, or too few tiles) into
+ * one whose k-splits share their sum through the workspace, where that is the faster one; others stay as they are.
+ * Ask ayla_b200_workspace_bytes afterwards.  With cfg == NULL ayla_b200_gemm* do the same to the default schedule when
+ * the workspace they are given suffices.
+ */
+AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
+                                        ayla_b200_config* cfg);
+
+/*
  * The schedule ayla_b200_swiglu uses when cfg == NULL: row-major (swap_ab == 0), or with the weights on the row
  * side (swap_ab == 1), a form that cannot be asked for by a cfg.
  */

@@ -185,3 +185,26 @@ def test_swiglu_of_few_rows_is_swapped_where_it_measured_faster(m, n, k, tile_n,
         assert (cfg.swap_ab, cfg.tile_n, cfg.split_k, cfg.cta_group) == (0, 256, 1, 2 if m >= 256 else 1)
     else:
         assert (cfg.swap_ab, cfg.tile_n, cfg.split_k, cfg.cluster_split) == (1, tile_n, split, int(split > 1))
+
+
+def test_depth_is_shared_where_sms_would_idle():
+    def shared(m, n, k, **config):
+        cfg = _lib.Config.from_dict(dict(group_m=8, **config))
+        out = _lib.share_depth(cfg, "mm", "bfloat16", 1, m, n, k)
+        assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
+        return (out.tile_n, out.cta_group, out.split_k, out.split_tail, out.cluster_split), out.to_dict() == cfg.to_dict()
+
+    pairs = dict(tile_n=256, cta_group=2, split_k=1)
+    # a thin last wave: split where a tile is long, run at half width where it is not, left alone where it is full
+    assert shared(2744, 2112, 29248, **pairs)[0] == (256, 2, 2, 1, 0)
+    assert shared(4451, 2240, 7040, **pairs)[0] == (256, 2, 5, 1, 0)
+    assert shared(1260, 4480, 768, **pairs)[0] == (256, 2, 1, 2, 0)
+    assert shared(8192, 1024, 8192, **pairs)[1]
+    # a deep product on a few SMs, and clusters that do not all run at once
+    assert shared(536, 896, 59968, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0][1:] == (2, 6, 0, 0)
+    assert shared(175, 2304, 8000, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0] == (128, 2, 4, 0, 0)
+    # neither: shallow, few rows, swapped, or a grid of its own
+    assert shared(256, 1024, 1024, tile_n=64, cta_group=2, split_k=1)[1]
+    assert shared(128, 4096, 4096, tile_n=64, cta_group=1, split_k=2, cluster_split=1)[1]
+    assert shared(8, 4096, 4096, tile_n=16, cta_group=1, split_k=4, cluster_split=1, swap_ab=1)[1]
+    assert shared(4451, 2240, 7040, grid_ctas=140, **pairs)[1]

@@ -159,6 +159,47 @@ def test_row_major_variants(tile_n, cta_group, split_k, dtype, device_state):
         assert_parity(out, O.gemm_ref32(operation, *tensors), f"{operation} {batch}x{m}x{n}x{k} {cfg}")
 
 
+# (batch, m, n, k): one tile and several, extents inside a chunk and a lane quarter, depths that the splits do not share
+# evenly; the last three fill whole waves first and split the depth of the tiles left over.
+@pytest.mark.parametrize("batch, m, n, k, config", [
+    (1, 128, 64, 1000, dict(tile_n=64, cta_group=1, split_k=7)),
+    (1, 130, 136, 2056, dict(tile_n=64, cta_group=1, split_k=8)),
+    (3, 257, 200, 1024, dict(tile_n=128, cta_group=2, split_k=4)),
+    (1, 40, 128, 8192, dict(tile_n=128, cta_group=1, split_k=48)),
+    (1, 300, 264, 3000, dict(tile_n=192, cta_group=2, split_k=5)),
+    (1, 600, 520, 4096, dict(tile_n=256, cta_group=2, split_k=2)),
+    (1, 512, 256, 4096, dict(tile_n=256, cta_group=1, split_k=32)),
+    (2, 1024, 1000, 512, dict(tile_n=256, cta_group=1, split_k=3, split_tail=1, grid_ctas=54)),
+    (1, 2100, 1000, 640, dict(tile_n=128, cta_group=2, split_k=2, split_tail=1, grid_ctas=60)),
+    (1, 520, 520, 1032, dict(tile_n=64, cta_group=1, split_k=5, split_tail=1, grid_ctas=40)),
+])
+@pytest.mark.parametrize("bias", [False, True])
+def test_shared_sum_of_a_split_depth(batch, m, n, k, config, bias, device_state):
+    """The k-splits of a tile share its sum; an owner that does not wait leaves its pieces to the last of the others.
+    Both add in split order, so they agree bit for bit."""
+    lib = _lib.load()
+    operation = "bmm" if batch > 1 else "addmm" if bias else "mm"
+    g = torch.Generator().manual_seed(m + n + k)
+    lead = (batch,) if batch > 1 else ()
+    a = torch.randn((*lead, m, k), generator=g).bfloat16()
+    bt = (torch.randn((*lead, n, k), generator=g) * k ** -0.5).bfloat16()
+    tensors = [a, bt] if operation != "addmm" else [torch.randn(n, generator=g).bfloat16(), a, bt]
+    out, status = run_abi(operation, "bfloat16", tensors, config, device_state)
+    assert status == 0
+    assert_parity(out, O.gemm_ref32(operation, *tensors), config)
+    lib.ayla_b200_debug_set_flags(32)  # owners hand their pieces over at once unless all partials are there
+    try:
+        for _ in range(3):
+            handed, status = run_abi(operation, "bfloat16", tensors, config, device_state)
+            assert status == 0
+            assert torch.equal(handed, out)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+    again, _ = run_abi(operation, "bfloat16", tensors, config, device_state)  # the counters were left clean
+    assert torch.equal(again, out)
+    assert not bool(device_state[1][:65536].any())
+
+
 @pytest.mark.parametrize("tile_n", [16, 32, 64, 128])
 @pytest.mark.parametrize("split_k", [1, 4])
 def test_swapped_variants(tile_n, split_k, device_state):
