@@ -674,6 +674,12 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
   return r.launch + blocks * (r.block + r.block_busy * busy) + r.per_split * splits + 4.5 * static_cast<double>(waves - 1);
 }
 
+// What a schedule measured elsewhere, or here by bursts, is corrected in.
+//
+// Shallow products of 256-wide tiles become pairs where no rows are padded: they read B half as often, and under the
+// power cap, which a burst does not reach, that is time (bmm 64 x 2048x2048x128 121.9 -> 110.9, 106 x 1872x1456x96 152.7 ->
+// 142.1, 35 x 1219x1960x128 50.0 -> 45.4; of one k-block they do not gain: 55 x 2043x1208x64 80.1 -> 81.1).
+//
 // Splits the depth where a row-major schedule leaves SMs idle through a long product: the CTAs of a tile share its sum
 // (see the kernel), so any number of them may work on it.  Two places:
 //  * The last, partial wave of tiles.  Splitting its tiles S ways takes 1/S of a tile's time and some 7 us for the sum
@@ -684,14 +690,20 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6).  Otherwise half width wherever two halves fit (1260x4480x768
 //    12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
-//    take 0.96 of the time for pairs and a deep product, 0.9 otherwise: over 152 shapes it was chosen 38 times and took
-//    0.83 of the time (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29, 175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 ->
-//    18.0, 1024x1024x8192 22.0 -> 20.1; single CTAs by less than that lose: 128x4096x4096 12.1 -> 13.5).
+//    take 0.97 of the time for pairs and a deep product, 0.9 otherwise: over 152 shapes 0.9 chose it 34 times, and it took
+//    0.81 of the time (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29, 175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 ->
+//    18.0, 1024x1024x8192 22.0 -> 20.1; by less than that others lose: 128x4096x4096 12.1 -> 13.5, 433x1280x3584 with
+//    row factors 12.9 -> 13.7).
 void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   if (c->swap_ab || c->stream_k || c->grid_ctas != 0 || c->split_tail == 1) return;
   if (c->split_k > 1 && !c->cluster_split && c->split_tail != 0) return;
   const int64_t k_blocks = ceil_div(k, 64);
   const bool mid_sector = k % 16 != 0;
+  if (c->cta_group == 1 && c->split_k == 1 && c->tile_n == 256 && k_blocks >= 2 &&
+      shallow_pairs_pay(batch, m, n, k, 256, AYLA_B200_ACT_RELU, machine.sm_count)) {
+    c->cta_group = 2;
+    c->split_tail = 0;
+  }
   const int64_t wave = machine.sm_count / c->cta_group;
   const int64_t tiles = batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n);
   if (tiles > wave) {
@@ -728,7 +740,7 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
       if (most > 48) most = 48;
       if (most > k_blocks / 4) most = k_blocks / 4;
       for (int64_t splits = most; splits >= 2; --splits) {
-        const double bound = cta_group == 2 && tile_n >= 128 && k_blocks >= 48 ? 0.96 : 0.9;
+        const double bound = cta_group == 2 && tile_n >= 128 && k_blocks >= 96 ? 0.97 : 0.9;
         const double us = modelled_us(tile_n, cta_group, static_cast<int>(splits), RATE_SHARED, there, k, machine);
         if (us >= best || us > bound * now) continue;
         best = us;
