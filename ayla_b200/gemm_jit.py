@@ -67,6 +67,7 @@ class GemmScheduleSeed:
     source_shape: tuple[int, int, int] | None
     source_percentage_of_torch: float | None = None
     post_builder_passes: tuple[str, ...] = ()
+    unsplit_config: dict[str, object] | None = None  # the schedule before its depth was split further
 
 
 def _builder_config(captured: dict[str, object]) -> dict[str, object]:
@@ -151,6 +152,7 @@ def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: 
         return seed
     captured = {**seed.captured_config, **shared}
     return replace(seed, captured_config=captured, builder_config=_builder_config(captured),
+                   unsplit_config=seed.builder_config,
                    adaptations=(*seed.adaptations, "depth split where SMs would idle"))
 
 
@@ -251,7 +253,8 @@ class GemmLauncher:
     stream gets a workspace of its own the first time that stream is used (two launches
     of one shape that overlap on different streams would otherwise sum into each other's
     partial tiles); that first use allocates, so it must happen outside graph capture --
-    inside capture it raises ``RuntimeError`` as a first call of a new shape does.
+    inside capture a schedule without a workspace runs instead, or, where a k-split was measured
+    for the shape itself, it raises ``RuntimeError`` as a first call of a new shape does.
 
     The status word lives in pinned host memory (``_lib.StatusWord``): every call reads it
     before launching, without synchronising, and raises ``RuntimeError`` if an earlier
@@ -263,6 +266,9 @@ class GemmLauncher:
     It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the launch goes to the
     packed kernel instead, and ``seed`` and ``config`` are not used.
     """
+
+    _unsplit_config: _lib.Config | None = None
+    _unsplit_tail: tuple | None = None
 
     def __init__(self, operation: str, dtype: str, batch: int, m: int, n: int, k: int,
                  seed: GemmScheduleSeed, device: torch.device, activation: str = "none",
@@ -298,6 +304,19 @@ class GemmLauncher:
                       self.workspace.numel() if self.workspace is not None else 0, self._status_ptr)
         self._has_bias = operation == "addmm"
         self._device_index = index
+        if need and seed.adaptations:
+            # What a capture on a stream without a workspace records, unless this schedule was measured for the shape:
+            # the one before its depth was split, the library's, or this one with its depth whole.
+            whole = {**seed.builder_config, "split_k": 1, "split_tail": 0, "cluster_split": 0}
+            library = _lib.default_config(operation, dtype, batch, m, n, k, activation).to_dict()
+            for candidate in (seed.unsplit_config, library, whole):
+                if candidate is None or not _legal(candidate, operation, dtype, m, n, k, batch):
+                    continue
+                unsplit = _lib.Config.from_dict(candidate)
+                if not _lib.workspace_bytes(unsplit, operation, batch, m, n, k):
+                    self._unsplit_config = unsplit
+                    self._unsplit_tail = (batch, m, n, k, ctypes.byref(unsplit), None, 0, self._status_ptr)
+                    break
 
     def __call__(self, *tensors: torch.Tensor) -> None:
         bias_ptr = mul_ptr = None
@@ -352,6 +371,8 @@ class GemmLauncher:
         entry = self._per_stream.get(stream)
         if entry is None:
             if torch.cuda.is_current_stream_capturing():
+                if self._unsplit_tail is not None:
+                    return self._unsplit_tail
                 raise RuntimeError(
                     f"jit_{self.operation}: the first launch of this k-split shape on a new stream allocates its "
                     "workspace and cannot happen during CUDA graph capture; run it once on that stream before capturing")
