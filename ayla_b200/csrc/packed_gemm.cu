@@ -35,6 +35,14 @@ constexpr int kStages = 2;
 constexpr int kMaxCtasPerSm = 4;  // each may hold 128 of the 512 TMEM columns
 constexpr int kRows = 128;        // accumulator rows
 
+// The piped kernel: a CTA of its own warps for the loads, the MMAs and the epilogue.
+constexpr int kLoadThreads = 128;
+constexpr int kEpilogueSets = 1;   // of four warps; a set takes every other unit
+constexpr int kPipedThreads = kEpilogueSets * 128 + kLoadThreads + 32;
+constexpr int kPipedMaxStages = 4;
+constexpr int kPipedCtasPerSm = 2;
+constexpr int kAccs = 2;              // accumulators in TMEM: the MMAs of a unit run under the epilogue of the one before
+
 struct PackedParams {
   const uint8_t* a;
   const uint8_t* b;
@@ -48,6 +56,7 @@ struct PackedParams {
   int narrow;     // operand rows of 128 >> narrow bytes per block (a depth of at most 64 >> narrow)
   int mma_n;      // accumulator columns
   int shared_b;   // 1: every unit multiplies by the same B, loaded once
+  int stages;     // ring slots of the piped kernel
   int tmem_cols;
   uint32_t idesc;
   uint32_t staging_pitch;
@@ -96,6 +105,158 @@ template <bool BF16>
 __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
   return pack2(lo, hi, BF16 ? 1 : 0);
 }
+
+// Loads of one unit's operands by a group of threads, each keeping to one 16-byte piece of its rows.
+struct UnitLoader {
+  const PackedParams& p;
+  const int tid, load_row, load_c;
+  const bool loads;
+  const uint32_t a_block, b_block;
+
+  __device__ UnitLoader(const PackedParams& p_, int tid_, uint32_t a_block_, uint32_t b_block_)
+      : p(p_), tid(tid_), load_row(p_.div_k_chunks.div(tid_)), load_c(tid_ - load_row * p_.k_chunks),
+        loads(tid_ < p_.load_threads), a_block(a_block_), b_block(b_block_) {}
+
+  __device__ __forceinline__ void load_operand(uint32_t dst, const uint8_t* src, int rows, uint32_t block_bytes,
+                                               int rows_per_matrix, int gap) const {
+    src += static_cast<uint32_t>(tid) * 16u;
+    const uint32_t step = static_cast<uint32_t>(p.load_threads) * 16u;
+    int slot_row = load_row, left = rows_per_matrix - load_row;  // rows of this matrix still ahead
+    for (int row = load_row; row < rows; row += p.load_rows) {
+      while (left <= 0) {
+        left += rows_per_matrix;
+        slot_row += gap;
+      }
+      cp_async_16(dst + piece_offset(slot_row, load_c, block_bytes, p.narrow), src);
+      src += step;
+      slot_row += p.load_rows;
+      left -= p.load_rows;
+    }
+  }
+
+  // `first`: also the B that all units share.
+  __device__ __forceinline__ void load(int unit, uint32_t dst_a, uint32_t dst_b, bool first) const {
+    if (!loads) return;
+    int first_matrix, matrices, row0, rows;  // rows: of A, over all of the unit's matrices
+    if (p.matrices == 1) {
+      first_matrix = p.div_row_tiles.div(unit);
+      matrices = 1;
+      row0 = (unit - first_matrix * p.row_tiles) * kRows;
+      rows = min(kRows, p.m - row0);
+    } else {
+      first_matrix = unit * p.matrices;
+      matrices = min(p.matrices, p.batch - first_matrix);
+      row0 = 0;
+      rows = matrices * p.m;
+    }
+    load_operand(dst_a, p.a + (static_cast<size_t>(first_matrix) * p.m + row0) * p.k_chunks * 16, rows, a_block,
+                 p.matrices == 1 ? kRows : p.m, p.slot_rows - p.m);
+    if (!p.shared_b || first) {
+      load_operand(dst_b, p.b + static_cast<size_t>(first_matrix) * p.n * p.k_chunks * 16, matrices * p.n, b_block,
+                   kPackedMaxN, 0);
+    }
+  }
+};
+
+// A warp's share of one unit's results: a quarter of the accumulator's rows, through its staging rows into `out`.
+template <bool BF16>
+struct UnitWriter {
+  const PackedParams& p;
+  const int quarter, lane, my_matrix, my_row, n_chunks;
+  uint8_t* const staging;
+  const float* const smem_bias;
+  // This lane's first piece of the warp's staged rows, and the steps to the one 32 pieces on.
+  int out_c, out_c_step;
+  uint32_t out_offset, out_step, out_wrap;
+  mutable int matrix = 0, row0 = 0, rows = 0;
+
+  __device__ UnitWriter(const PackedParams& p_, int quarter_, int lane_, uint8_t* staging_, const float* smem_bias_)
+      : p(p_), quarter(quarter_), lane(lane_), my_matrix(quarter_ / (p_.slot_rows / 32)),
+        my_row((quarter_ % (p_.slot_rows / 32)) * 32), n_chunks(p_.n >> 3),
+        staging(staging_ + quarter_ * 32 * p_.staging_pitch), smem_bias(smem_bias_) {
+    const int out_row = p.div_n_chunks.div(lane), out_row_step = p.div_n_chunks.div(32);
+    out_c = lane - out_row * n_chunks;
+    out_c_step = 32 - out_row_step * n_chunks;
+    out_offset = static_cast<uint32_t>(out_row) * p.staging_pitch + static_cast<uint32_t>(out_c) * 16u;
+    out_step = static_cast<uint32_t>(out_row_step) * p.staging_pitch + static_cast<uint32_t>(out_c_step) * 16u;
+    out_wrap = p.staging_pitch - static_cast<uint32_t>(n_chunks) * 16u;
+  }
+
+  // Matrix `my_matrix` of the unit, from its row `my_row` on; false where there is none.
+  __device__ __forceinline__ bool locate(int unit) const {
+    if (p.matrices == 1) {
+      matrix = p.div_row_tiles.div(unit);
+      row0 = (unit - matrix * p.row_tiles) * kRows + my_row;
+    } else {
+      matrix = unit * p.matrices + my_matrix;
+      row0 = my_row;
+    }
+    rows = matrix < p.batch ? min(32, p.m - row0) : 0;
+    return rows > 0;
+  }
+
+  __device__ __forceinline__ void stage(uint32_t accumulator) const {
+    const uint32_t t = accumulator + (static_cast<uint32_t>(quarter * 32) << 16) +
+                       static_cast<uint32_t>(p.matrices > 1 ? my_matrix * p.n : 0);
+    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
+      uint32_t r[32];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c0 + j < n_chunks) tmem_ld_32x8(t + (c0 + j) * 8, r + 8 * j);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c0 + j < n_chunks) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
+          if (p.bias != nullptr) {
+            const float4* b4 = reinterpret_cast<const float4*>(smem_bias + (c0 + j) * 8);
+            const float4 lo = b4[0], hi = b4[1];
+            v[0] += lo.x;
+            v[1] += lo.y;
+            v[2] += lo.z;
+            v[3] += lo.w;
+            v[4] += hi.x;
+            v[5] += hi.y;
+            v[6] += hi.z;
+            v[7] += hi.w;
+          }
+          *reinterpret_cast<uint4*>(staging + lane * p.staging_pitch + (c0 + j) * 16) =
+              make_uint4(pack_pair<BF16>(v[0], v[1]), pack_pair<BF16>(v[2], v[3]), pack_pair<BF16>(v[4], v[5]),
+                         pack_pair<BF16>(v[6], v[7]));
+        }
+      }
+    }
+  }
+
+  // The staged rows follow one another in `out` without a gap.
+  __device__ __forceinline__ void copy_out() const {
+    uint8_t* dst = p.out + ((static_cast<size_t>(matrix) * p.m + row0) * n_chunks + lane) * 16;
+    const int pieces = rows * n_chunks;
+    int c = out_c;
+    const uint8_t* src = staging + out_offset;
+    for (int j = lane; j < pieces; j += 128) {
+      uint4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j + 32 * u < pieces) x[u] = *reinterpret_cast<const uint4*>(src);
+        src += out_step;
+        c += out_c_step;
+        if (c >= n_chunks) {
+          c -= n_chunks;
+          src += out_wrap;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j + 32 * u < pieces) *reinterpret_cast<uint4*>(dst + 512 * u) = x[u];
+      }
+      dst += 2048;
+    }
+  }
+};
 
 template <bool BF16>
 __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(const PackedParams p) {
@@ -155,135 +316,20 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
   const int count = (p.units - first + stride - 1) / stride;  // the grid is no larger than `units`
 
   // Loads of this CTA's i-th unit into ring slot `s`: one commit group per unit, empty past the last.
-  const int load_row = p.div_k_chunks.div(tid);
-  const int load_c = tid - load_row * p.k_chunks;
-  const bool loads = tid < p.load_threads;
-  auto load_operand = [&](uint32_t dst, const uint8_t* src, int rows, uint32_t block_bytes, int rows_per_matrix,
-                          int gap) {
-    src += static_cast<uint32_t>(tid) * 16u;
-    const uint32_t step = static_cast<uint32_t>(p.load_threads) * 16u;
-    int slot_row = load_row, left = rows_per_matrix - load_row;  // rows of this matrix still ahead
-    for (int row = load_row; row < rows; row += p.load_rows) {
-      while (left <= 0) {
-        left += rows_per_matrix;
-        slot_row += gap;
-      }
-      cp_async_16(dst + piece_offset(slot_row, load_c, block_bytes, narrow), src);
-      src += step;
-      slot_row += p.load_rows;
-      left -= p.load_rows;
-    }
-  };
+  const UnitLoader loader(p, tid, a_block, b_block);
   auto load_unit = [&](int i, int s) {
-    if (i < count && loads) {
-      const int unit = first + i * stride;
-      int first_matrix, matrices, row0, rows;  // rows: of A, over all of the unit's matrices
-      if (p.matrices == 1) {
-        first_matrix = p.div_row_tiles.div(unit);
-        matrices = 1;
-        row0 = (unit - first_matrix * p.row_tiles) * kRows;
-        rows = min(kRows, p.m - row0);
-      } else {
-        first_matrix = unit * p.matrices;
-        matrices = min(p.matrices, p.batch - first_matrix);
-        row0 = 0;
-        rows = matrices * p.m;
-      }
-      load_operand(smem_u32(packed_smem) + static_cast<uint32_t>(s) * a_bytes,
-                   p.a + (static_cast<size_t>(first_matrix) * p.m + row0) * p.k_chunks * 16, rows, a_block,
-                   p.matrices == 1 ? kRows : p.m, p.slot_rows - p.m);
-      if (!p.shared_b || i == 0) {
-        load_operand(smem_u32(smem_b) + (p.shared_b ? 0u : static_cast<uint32_t>(s) * b_bytes),
-                     p.b + static_cast<size_t>(first_matrix) * p.n * p.k_chunks * 16, matrices * p.n, b_block,
-                     kPackedMaxN, 0);
-      }
+    if (i < count) {
+      loader.load(first + i * stride, smem_u32(packed_smem) + static_cast<uint32_t>(s) * a_bytes,
+                  smem_u32(smem_b) + (p.shared_b ? 0u : static_cast<uint32_t>(s) * b_bytes), i == 0);
     }
     cp_async_commit();
   };
-
-  // Rows of this warp's accumulator quarter: matrix `my_matrix` of the unit, from its row `my_row` on.
-  const int warps_per_slot = p.slot_rows / 32;
-  const int my_matrix = warp / warps_per_slot;
-  const int my_row = (warp % warps_per_slot) * 32;
-  const int n_chunks = p.n >> 3;
-  uint8_t* staging = smem_staging + warp * 32 * p.staging_pitch;
-  // This lane's first piece of the warp's staged rows, and the steps to the one 32 pieces on.
-  const int out_row = p.div_n_chunks.div(lane), out_c = lane - out_row * n_chunks;
-  const int out_row_step = p.div_n_chunks.div(32), out_c_step = 32 - out_row_step * n_chunks;
-  const uint32_t out_offset = static_cast<uint32_t>(out_row) * p.staging_pitch + static_cast<uint32_t>(out_c) * 16u;
-  const uint32_t out_step =
-      static_cast<uint32_t>(out_row_step) * p.staging_pitch + static_cast<uint32_t>(out_c_step) * 16u;
-  const uint32_t out_wrap = p.staging_pitch - static_cast<uint32_t>(n_chunks) * 16u;
-
+  const UnitWriter<BF16> writer(p, warp, lane, smem_staging, smem_bias);
   auto epilogue = [&](int i) {
-    const int unit = first + i * stride;
-    int matrix, row0;
-    if (p.matrices == 1) {
-      matrix = p.div_row_tiles.div(unit);
-      row0 = (unit - matrix * p.row_tiles) * kRows + my_row;
-    } else {
-      matrix = unit * p.matrices + my_matrix;
-      row0 = my_row;
-    }
-    const int rows = matrix < p.batch ? min(32, p.m - row0) : 0;
-    if (rows <= 0) return;
-    const uint32_t t = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) +
-                       static_cast<uint32_t>(p.matrices > 1 ? my_matrix * p.n : 0);
-    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
-      uint32_t r[32];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (c0 + j < n_chunks) tmem_ld_32x8(t + (c0 + j) * 8, r + 8 * j);
-      }
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (c0 + j < n_chunks) {
-          float v[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
-          if (p.bias != nullptr) {
-            const float4* b4 = reinterpret_cast<const float4*>(smem_bias + (c0 + j) * 8);
-            const float4 lo = b4[0], hi = b4[1];
-            v[0] += lo.x;
-            v[1] += lo.y;
-            v[2] += lo.z;
-            v[3] += lo.w;
-            v[4] += hi.x;
-            v[5] += hi.y;
-            v[6] += hi.z;
-            v[7] += hi.w;
-          }
-          *reinterpret_cast<uint4*>(staging + lane * p.staging_pitch + (c0 + j) * 16) =
-              make_uint4(pack_pair<BF16>(v[0], v[1]), pack_pair<BF16>(v[2], v[3]), pack_pair<BF16>(v[4], v[5]),
-                         pack_pair<BF16>(v[6], v[7]));
-        }
-      }
-    }
+    if (!writer.locate(first + i * stride)) return;
+    writer.stage(tmem_base);
     __syncwarp();
-    // The rows follow one another in `out` without a gap.
-    uint8_t* dst = p.out + ((static_cast<size_t>(matrix) * p.m + row0) * n_chunks + lane) * 16;
-    const int pieces = rows * n_chunks;
-    int c = out_c;
-    const uint8_t* src = staging + out_offset;
-    for (int j = lane; j < pieces; j += 128) {
-      uint4 x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (j + 32 * u < pieces) x[u] = *reinterpret_cast<const uint4*>(src);
-        src += out_step;
-        c += out_c_step;
-        if (c >= n_chunks) {
-          c -= n_chunks;
-          src += out_wrap;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (j + 32 * u < pieces) *reinterpret_cast<uint4*>(dst + 512 * u) = x[u];
-      }
-      dst += 2048;
-    }
+    writer.copy_out();
   };
 
 #pragma unroll
@@ -333,6 +379,184 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
 #endif
 }
 
+// The same units through a pipeline inside each CTA: four warps load, one issues MMAs, the others write results, and
+// they meet at mbarriers only, so that the loads run several units ahead and the MMAs and the epilogue of consecutive
+// units overlap.  In the kernel above a unit is a chain (load, MMA, epilogue, 5000 cycles) that only other CTAs of the SM
+// hide: with units of 24 KB and more fewer of those fit, and the chain shows; with small ones its smaller CTAs win.
+// us per launch, the kernel above -> this one: mm 200704x96x24 16.3 -> 14.3, 171761x24x40 11.0 -> 8.2, 131072x64x8 13.9 ->
+// 8.8, 250000x128x40 25.7 -> 20.5, bmm 3000 x 128x64x40 21.3 -> 19.3, 5332 x 45x16x120 22.3 -> 18.9.  What is left is
+// the epilogue's chain (a second set of epilogue warps made no more than 3 %, or lost as much to its staging rows) and,
+// from 30 KB a unit on, the SM's store rate.
+template <bool BF16>
+__global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_kernel(const PackedParams p) {
+#if defined(__CUDA_ARCH_FEAT_SM100_ALL) || defined(__CUDA_ARCH_FEAT_SM101_ALL)
+  extern __shared__ __align__(1024) uint8_t packed_smem[];
+  const int narrow = p.narrow;
+  const uint32_t a_block = static_cast<uint32_t>(kRows * 128) >> narrow;
+  const uint32_t a_bytes = static_cast<uint32_t>(p.k_blocks) * a_block;
+  const uint32_t b_block = static_cast<uint32_t>(p.mma_n * 128) >> narrow;
+  const uint32_t b_bytes = static_cast<uint32_t>(p.k_blocks) * b_block;
+  const int b_copies = p.shared_b ? 1 : p.stages;
+  uint8_t* smem_b = packed_smem + p.stages * a_bytes;
+  uint8_t* smem_staging = smem_b + b_copies * b_bytes;
+  float* smem_bias = reinterpret_cast<float*>(smem_staging + kEpilogueSets * kRows * p.staging_pitch);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_bias + kPackedMaxN);
+  // full[kPipedMaxStages], empty[kPipedMaxStages], acc_full[kAccs], acc_empty[kAccs]
+  const uint32_t bar_full = smem_u32(bars);
+  const uint32_t bar_empty = bar_full + kPipedMaxStages * 8;
+  const uint32_t bar_acc_full = bar_empty + kPipedMaxStages * 8;
+  const uint32_t bar_acc_empty = bar_acc_full + kAccs * 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kPipedMaxStages + 2 * kAccs);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+  constexpr int kFirstLoadWarp = kEpilogueSets * 4, kMmaWarp = kFirstLoadWarp + kLoadThreads / 32;
+  const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    if ((smem_u32(packed_smem) & 1023u) != 0) bw.give_up(ST_BAD_SMEM_ALIGN);
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(bar_full + s * 8, kLoadThreads);
+      mbar_init(bar_empty + s * 8, 1);
+    }
+    for (int i = 0; i < kAccs; ++i) {
+      mbar_init(bar_acc_full + i * 8, 1);
+      mbar_init(bar_acc_empty + i * 8, 4);
+    }
+    fence_mbar_init();
+  }
+  if (warp == kMmaWarp) {
+    tmem_alloc<1>(smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
+    tmem_relinquish<1>();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+
+  const int first = static_cast<int>(blockIdx.x), stride = static_cast<int>(gridDim.x);
+  const int count = (p.units - first + stride - 1) / stride;  // the grid is no larger than `units`
+
+  if (warp >= kFirstLoadWarp && warp < kMmaWarp) {
+    // ---------------------------------------------------------------- loads
+    const int tid = static_cast<int>(threadIdx.x) - kFirstLoadWarp * 32;
+    // A depth that is an odd number of pieces is read one piece further by the MMAs: zero in both operands.
+    if ((p.k_chunks & 1) != 0) {
+      for (int s = 0; s < p.stages; ++s) {
+        *reinterpret_cast<uint4*>(packed_smem + s * a_bytes + piece_offset(tid, p.k_chunks, a_block, narrow)) =
+            make_uint4(0, 0, 0, 0);
+      }
+      for (int s = 0; s < b_copies; ++s) {
+        if (tid < p.mma_n) {
+          *reinterpret_cast<uint4*>(smem_b + s * b_bytes + piece_offset(tid, p.k_chunks, b_block, narrow)) =
+              make_uint4(0, 0, 0, 0);
+        }
+      }
+    }
+    grid_dependency_wait();
+    const bool loads = (p.debug_flags & 1) == 0;
+    const UnitLoader loader(p, tid, a_block, b_block);
+    // A unit is announced once this thread's pieces of it have landed, when the loads of the next `behind` units have
+    // been issued: commit groups complete in order.
+    const int behind = p.stages - 1;
+    int slot = 0, done_slot = 0;
+    uint32_t phase = 1;
+    for (int i = 0; i < count + behind; ++i) {
+      if (i < count) {
+        bw.wait(bar_empty + slot * 8, phase, ST_TIMEOUT_EMPTY);
+        if (loads && !bw.aborted()) {
+          loader.load(first + i * stride, smem_u32(packed_smem) + static_cast<uint32_t>(slot) * a_bytes,
+                      smem_u32(smem_b) + (p.shared_b ? 0u : static_cast<uint32_t>(slot) * b_bytes), i == 0);
+        }
+        if (++slot == p.stages) {
+          slot = 0;
+          phase ^= 1;
+        }
+      }
+      cp_async_commit();
+      if (i >= behind) {
+        switch (behind) {
+          case 1: cp_async_wait<1>(); break;
+          case 2: cp_async_wait<2>(); break;
+          default: cp_async_wait<3>(); break;
+        }
+        fence_proxy_async_smem();
+        if (loads) mbar_arrive(bar_full + done_slot * 8);
+        if (++done_slot == p.stages) done_slot = 0;
+      }
+    }
+    cp_async_wait<0>();
+  } else if (warp == kMmaWarp) {
+    // ----------------------------------------------------------------- MMAs
+    const bool issuer = elect_one();
+    const uint64_t desc_a0 = operand_desc(smem_u32(packed_smem), narrow);
+    const uint64_t desc_b0 = operand_desc(smem_u32(smem_b), narrow);
+    const int steps = (p.k_chunks + 1) >> 1;
+    int slot = 0;
+    uint32_t phase = 0, acc = 0, acc_phase = 1;
+    for (int i = 0; i < count; ++i) {
+      bw.wait(bar_acc_empty + acc * 8, acc_phase, ST_TIMEOUT_ACC_EMPTY);
+      bw.wait(bar_full + slot * 8, phase, ST_TIMEOUT_FULL);
+      if (bw.aborted()) break;
+      tc_fence_after_sync();
+      if (issuer) {
+        const uint64_t desc_a = desc_a0 + static_cast<uint32_t>(slot) * (a_bytes >> 4);
+        const uint64_t desc_b = desc_b0 + (p.shared_b ? 0u : static_cast<uint32_t>(slot) * (b_bytes >> 4));
+        for (int ks = 0; ks < steps; ++ks) {
+          const uint32_t kb = static_cast<uint32_t>(ks >> 2), in_block = 2u * static_cast<uint32_t>(ks & 3);
+          umma_f16<1>(tmem_base + acc * static_cast<uint32_t>(p.mma_n), desc_a + kb * (a_block >> 4) + in_block,
+                      desc_b + kb * (b_block >> 4) + in_block, p.idesc, ks > 0 ? 1u : 0u);
+        }
+        umma_commit_1cta(bar_empty + slot * 8);
+        umma_commit_1cta(bar_acc_full + acc * 8);
+      }
+      __syncwarp();
+      if (++slot == p.stages) {
+        slot = 0;
+        phase ^= 1;
+      }
+      if (++acc == kAccs) {
+        acc = 0;
+        acc_phase ^= 1;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------- epilogue
+    grid_dependency_wait();
+    if (p.bias != nullptr) {
+      if (static_cast<int>(threadIdx.x) < p.n) smem_bias[threadIdx.x] = load_elem(p.bias, threadIdx.x, BF16 ? 1 : 0);
+      named_bar_sync(1, kEpilogueSets * 128);
+    }
+    const int set = warp >> 2;
+    const UnitWriter<BF16> writer(p, warp & 3, lane, smem_staging + set * kRows * p.staging_pitch, smem_bias);
+    for (int i = set; i < count; i += kEpilogueSets) {
+      const uint32_t acc = static_cast<uint32_t>(i) & 1u, acc_phase = (static_cast<uint32_t>(i) >> 1) & 1u;
+      bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL);
+      tc_fence_after_sync();
+      const bool live = writer.locate(first + i * stride) && !bw.aborted();
+      if (live) writer.stage(tmem_base + acc * static_cast<uint32_t>(p.mma_n));
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_acc_empty + acc * 8);
+      if (live) writer.copy_out();
+      __syncwarp();  // the staging rows are free again
+    }
+  }
+
+  if (bw.aborted()) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // MMAs still in flight
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    tc_fence_after_sync();
+    tmem_dealloc<1>(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+  }
+#endif
+}
+
 constexpr int kSmemPerSm = 233472, kSmemPerCta = 232448, kCtaReserve = 1024;
 
 // How a problem lies in shared memory and how many CTAs of it an SM holds.
@@ -341,7 +565,20 @@ struct Footprint {
   int mma_n, narrow, k_blocks;
   int staging_pitch;
   int smem, ctas;
+  bool piped;     // the piped kernel
+  int stages, piped_smem, piped_ctas, piped_tmem_cols;
 };
+
+// Where the piped kernel is the faster one, by how many CTAs of the other an SM would hold (58 shapes timed on both;
+// over those it takes, 0.87 of the time, the slowest 1.01): at two and fewer nothing hides a unit's chain there; at three
+// single matrices gain (57501x72x56 8.7 -> 7.6), pairs of small ones do not (8192 x 56x32x56 22.8 -> 24.0); at four, one
+// B for all units and rows that start inside a 32-byte sector, whose loads take longest (52640x88x24 10.0 -> 7.7, but
+// 146105x56x64 8.7 -> 9.5).  Fewer units than it has CTAs gain nothing from a pipeline (28625x80x24, 224 units, 5.6 ->
+// 5.9).
+bool piped_pays(int64_t units, int64_t k, int matrices, bool shared_b, int chained_ctas) {
+  if (units < 256) return false;
+  return chained_ctas <= 2 || (chained_ctas == 3 && matrices == 1) || (shared_b && k % 16 != 0);
+}
 
 Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
   Footprint f;
@@ -356,17 +593,39 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
   f.smem = kStages * a_bytes + (batch == 1 ? 1 : kStages) * b_bytes + kRows * f.staging_pitch + kPackedMaxN * 4 + 64;
   f.ctas = kSmemPerSm / (f.smem + kCtaReserve);
   if (f.ctas > kMaxCtasPerSm) f.ctas = kMaxCtasPerSm;
+
+  // Two CTAs, or one, and then as many ring slots as still fit.
+  const bool shared_b = batch == 1;
+  auto piped_smem = [&](int stages) {
+    return stages * a_bytes + (shared_b ? 1 : stages) * b_bytes + kEpilogueSets * kRows * f.staging_pitch + kPackedMaxN * 4 + 128;
+  };
+  f.piped_tmem_cols = 32;
+  while (f.piped_tmem_cols < kAccs * f.mma_n) f.piped_tmem_cols *= 2;
+  f.piped_ctas = kPipedCtasPerSm;
+  while (f.piped_ctas > 1 && kSmemPerSm / (piped_smem(2) + kCtaReserve) < f.piped_ctas) --f.piped_ctas;
+  f.stages = 2;
+  while (f.stages < kPipedMaxStages && piped_smem(f.stages + 1) <= kSmemPerCta &&
+         kSmemPerSm / (piped_smem(f.stages + 1) + kCtaReserve) >= f.piped_ctas) {
+    ++f.stages;
+  }
+  f.piped_smem = piped_smem(f.stages);
+  const int64_t units = f.matrices == 1 ? batch * ((m + kRows - 1) / kRows) : (batch + f.matrices - 1) / f.matrices;
+  f.piped = piped_pays(units, k, f.matrices, shared_b, f.ctas);
   return f;
 }
 
 }  // namespace
 
 cudaError_t init_packed_gemm() {
-  const cudaError_t err = cudaFuncSetAttribute(reinterpret_cast<const void*>(&packed_gemm_kernel<false>),
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
-  if (err != cudaSuccess) return err;
-  return cudaFuncSetAttribute(reinterpret_cast<const void*>(&packed_gemm_kernel<true>),
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+  const void* const kernels[4] = {reinterpret_cast<const void*>(&packed_gemm_kernel<false>),
+                                  reinterpret_cast<const void*>(&packed_gemm_kernel<true>),
+                                  reinterpret_cast<const void*>(&packed_piped_kernel<false>),
+                                  reinterpret_cast<const void*>(&packed_piped_kernel<true>)};
+  for (const void* kernel : kernels) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+    if (err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
 }
 
 // Where this kernel is the faster one.  1606 shapes of up to 128 columns and a depth of up to 128 were timed on both
@@ -443,19 +702,22 @@ cudaError_t launch_packed_gemm(const PackedProblem& pr) {
   p.debug_flags = pr.debug_flags;
   p.tmem_cols = 32;
   while (p.tmem_cols < p.mma_n) p.tmem_cols *= 2;
+  if (f.piped) p.tmem_cols = f.piped_tmem_cols;
+  p.stages = f.stages;
 
-  const int64_t room = static_cast<int64_t>(f.ctas) * pr.sm_count;
+  const int64_t room = static_cast<int64_t>(f.piped ? f.piped_ctas : f.ctas) * pr.sm_count;
 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.units < room ? p.units : room));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(f.smem);
+  cfg.blockDim = dim3(f.piped ? kPipedThreads : kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(f.piped ? f.piped_smem : f.smem);
   cfg.stream = pr.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pr.overlap ? 1 : 0;
+  if (f.piped) return cudaLaunchKernelEx(&cfg, pr.is_bf16 ? packed_piped_kernel<true> : packed_piped_kernel<false>, p);
   return cudaLaunchKernelEx(&cfg, pr.is_bf16 ? packed_gemm_kernel<true> : packed_gemm_kernel<false>, p);
 }
 

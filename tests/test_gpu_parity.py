@@ -697,6 +697,61 @@ def test_packed_kernel_equals_the_general_one(operation, batch, m, n, k, dtype):
     assert bool((out[-guard:] == 7.0).all())
 
 
+def test_a_capture_on_a_new_stream_records_the_schedule_without_a_workspace():
+    """A product whose depth is split where SMs would idle needs a workspace per stream; a capture cannot allocate one."""
+    m, n, k = 175, 2304, 8000
+    g = torch.Generator().manual_seed(5)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+    want = O.mm_ref32(a, bt)
+    compiler = gemm_jit_compiler("mm", "bfloat16")
+    a, bt, out = a.to(DEV), bt.to(DEV), torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    compiler(a, bt, out)
+    assert next(iter(compiler._cache.values())).workspace is not None
+    assert_parity(out, want, "split")
+    out.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        compiler(a, bt, out)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_parity(out, want, "captured")
+
+
+# The packed kernel's piped form: one B and many, a depth of one piece and of an odd number, units with rows and matrices
+# missing at the end, one ring slot more or less, units enough to use every slot and accumulator again.
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("operation, batch, m, n, k", [
+    ("mm", 1, 32769, 8, 8), ("addmm", 1, 70000, 96, 24), ("addmm", 1, 40003, 128, 120), ("mm", 1, 90001, 16, 40),
+    ("mm", 1, 33000, 128, 128), ("bmm", 260, 129, 72, 104), ("bmm", 301, 128, 128, 64), ("bmm", 1030, 17, 24, 88),
+    ("bmm", 2055, 45, 16, 120), ("bmm", 600, 1, 96, 72),
+])
+def test_piped_packed_kernel_equals_the_general_one(operation, batch, m, n, k, dtype, device_state):
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    lead = (batch,) if operation == "bmm" else ()
+    a = torch.randn((*lead, m, k), device=DEV, generator=g).to(TD[dtype])
+    bt = (torch.randn((*lead, n, k), device=DEV, generator=g) * k ** -0.5).to(TD[dtype])
+    bias = torch.randn(n, device=DEV, generator=g).to(TD[dtype])
+    status, workspace = device_state
+    status.zero_()
+    outs = [torch.full((batch * m + 4, n), float("nan"), dtype=TD[dtype], device=DEV) for _ in range(2)]
+    stream = torch.cuda.current_stream().cuda_stream
+    bias_ptr = bias.data_ptr() if operation == "addmm" else 0
+    for _ in range(2):
+        _lib.gemm_packed(operation, dtype, bias_ptr, a.data_ptr(), bt.data_ptr(), outs[0].data_ptr(), batch, m, n, k,
+                         status.data_ptr(), stream)
+    cfg = _lib.Config.from_dict(dict(tile_n=64, cta_group=1, split_k=1, group_m=8))
+    _lib.gemm(operation, dtype, bias_ptr, a.data_ptr(), bt.data_ptr(), outs[1].data_ptr(), batch, m, n, k, cfg,
+              workspace.data_ptr(), workspace.numel(), status.data_ptr(), stream)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    # the same products summed in the same order of 16-deep steps; nothing past the output
+    assert torch.equal(outs[0][:batch * m], outs[1][:batch * m])
+    assert bool(torch.isnan(outs[0][batch * m:]).all())
+
+
 def test_packed_kernel_through_the_ops_and_its_limits():
     a = torch.randn(300, 32, 24, device=DEV).half()
     bt = torch.randn(300, 16, 24, device=DEV).half()
