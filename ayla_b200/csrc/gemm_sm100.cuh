@@ -791,11 +791,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (issuer && mine) {
           const uint32_t full_bar = full_bar0 + stage * 8;
           const int blocks = min(group, w.kb1 - kb);  // a unit may end in the middle of a slot
-#ifdef AYLA_B200_TUNE
-          if (p.debug_flags & 4) {  // tuning builds: hand the slot over without loading anything
-            if (is_leader) mbar_arrive(bar_full + stage * 8);
-          } else
-#endif
           {
             if (is_leader) mbar_arrive_expect_tx(bar_full + stage * 8, p.stage_tx * static_cast<uint32_t>(blocks));
 #pragma unroll
@@ -892,9 +887,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             // 16-byte address units.
             const uint32_t slot_off = stage * (T::SLOT_BYTES >> 4);
             const int blocks = min(group, nkb - i);  // a unit may end in the middle of a slot
-#ifdef AYLA_B200_TUNE
-            if ((p.debug_flags & 8) == 0)
-#endif
             {
 #pragma unroll
               for (int g = 0; g < group; ++g) {
@@ -910,11 +902,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #ifdef AYLA_B200_TRACE
             const long long tr_c = clock64();
             tr_issue += tr_c - tr_b;
-#endif
-#ifdef AYLA_B200_TUNE
-            if (p.debug_flags & 16) {
-              mbar_arrive(bar_empty + stage * 8);
-            } else
 #endif
             if constexpr (CG == 1) {
               umma_commit_1cta(bar_empty + stage * 8);
