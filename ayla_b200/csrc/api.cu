@@ -568,7 +568,10 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
     // Weight streaming is what early_prefetch is for: half of the CTA's share of K, 16 k-blocks at most.
     {
       const int64_t share = k_blocks / c->split_k / 2;
-      c->early_prefetch = static_cast<int>(share < 16 ? share : 16);
+      // (Eight blocks of a wider accumulator's, whose loads come with more of `a`: 62x6656x5440 with a gate 16 blocks 27.0,
+      // 12 24.9, 8 24.1; without 17.0, 16.8, 16.9.)
+      const int64_t most = c->tile_n >= 64 ? 8 : 16;
+      c->early_prefetch = static_cast<int>(share < most ? share : most);
     }
     // One wave of tiles that would leave SMs idle is cut into as many as there are SMs (3x13056x1728, 102 -> 136 tiles,
     // 9.7 -> 9.1; 7x13696x5504, 107 -> 143, 24.5 -> 23.6; 44x12216x4760, 96 -> 139, 30.8 -> 27.5), a split one where the
@@ -685,7 +688,8 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //  * The last, partial wave of tiles.  Splitting its tiles S ways takes 1/S of a tile's time and some 7 us for the sum
 //    instead of a whole tile's time, or three quarters of it where its tiles run at half width (us, whole -> half ->
 //    split: 2744x2112x29248, 1 + 25/74 waves, 332 -> 316 -> 266 with 2; 3024x1856x11776, 1 + 22/74, 120 -> 116 -> 104
-//    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
+//    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 2129x4608x5248, 2 + 14/74, 84 -> 80 -> 77 with 5; but
+//    4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
 //    Rows that start inside a sector are bound by their loads, which a lone pair gets faster: two ways at most
 //    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6).  Otherwise half width wherever two halves fit (1260x4480x768
 //    12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
@@ -716,7 +720,8 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
       if (splits > (mid_sector ? 2 : 16)) splits = mid_sector ? 2 : 16;
       const double block = c->tile_n == 256 ? 0.38 : c->tile_n == 192 ? 0.33 : 0.275;
       const double now = mid_sector ? 0.7 : halves_fit ? 0.75 : 1.0;  // of a tile: a half runs at three quarters of the rate
-      if (splits >= 2 && static_cast<double>(k_blocks) * (now - 1.0 / static_cast<double>(splits)) * block > 8.5) {
+      if (splits >= 2 && static_cast<double>(k_blocks) * (now - 1.0 / static_cast<double>(splits)) * block >
+                             (mid_sector ? 8.5 : 14.0)) {
         c->split_k = static_cast<int>(splits);
         c->split_tail = 1;
         return;

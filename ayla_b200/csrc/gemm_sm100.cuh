@@ -1235,8 +1235,14 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       auto write_lone_chunk = [&](float (&v)[32], int c32) {
         if constexpr (!T::TRANS_OUT && !T::LEAN) {
           const int col0 = w.n0 + c32 * 32;
-          uint32_t pk[16];
-          if (w.m0 + row_in_tile < row_end) pack_chunk(v, c32, pk);
+          if (w.m0 + row_in_tile < row_end) {
+            if constexpr (T::EPI == EPI_BIAS) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] += smem_bias[bias_buf * BN + c32 * 32 + j];
+            }
+            apply_act_chunk<32>(v, act);
+            gate_chunk(v, c32);
+          }
           if constexpr (T::SHARED) {
             if (lane == 0) tma_store_wait_read<0>();  // of a whole tile before this one
           }
@@ -1245,7 +1251,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               *reinterpret_cast<uint4*>(my_store + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) =
-                  make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+                  make_uint4(pack2(v[8 * j], v[8 * j + 1], is_bf16), pack2(v[8 * j + 2], v[8 * j + 3], is_bf16),
+                             pack2(v[8 * j + 4], v[8 * j + 5], is_bf16), pack2(v[8 * j + 6], v[8 * j + 7], is_bf16));
             }
           }
           __syncwarp();
