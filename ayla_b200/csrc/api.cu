@@ -1234,14 +1234,6 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
     return ayla_b200_gemm_packed(op, dtype, bias, a, bt, out, batch, m, n, k, status, stream);
   } else {
     default_config(batch, m, n, k, activation, ds->machine, &c);
-    // A gate shaped like the output has kernels of its own, without a k-split; and a caller who lent no workspace, or
-    // too little, gets the schedule as it was.
-    if (mul == nullptr || mul_per_row != 0) {
-      ayla_b200_config shared = c;
-      share_depth(batch, m, n, k, ds->machine, &shared);
-      const size_t need = ayla_b200_workspace_bytes(&shared, op, batch, m, n, k);
-      if (need == 0 || (workspace != nullptr && workspace_bytes >= need)) c = shared;
-    }
   }
   rc = check_config(c, false);
   if (rc) return rc;

@@ -257,8 +257,8 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
 /*
  * Rewrites a schedule that leaves SMs idle through a deep product (a thin last wave of tiles, or too few tiles) into
  * one whose k-splits share their sum through the workspace, where that is the faster one; others stay as they are.
- * Ask ayla_b200_workspace_bytes afterwards.  With cfg == NULL ayla_b200_gemm* do the same to the default schedule when
- * the workspace they are given suffices.
+ * Ask ayla_b200_workspace_bytes afterwards.  cfg == NULL never means such a schedule: it runs the one that
+ * ayla_b200_default_config reports, and of a lent workspace uses what ayla_b200_workspace_bytes says of that one.
  */
 AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                         ayla_b200_config* cfg);

@@ -966,6 +966,27 @@ def test_op_level_validation():
         gemm_op("addmm", "bfloat16")(torch.empty(32, device=DEV, dtype=torch.bfloat16), a, a, out)
 
 
+@pytest.mark.parametrize("m, n, k", [(1024, 1024, 8192), (175, 2304, 8000), (4451, 2240, 7040)])
+def test_no_schedule_leaves_a_workspace_alone_that_the_default_does_not_need(m, n, k, device_state):
+    """cfg == NULL is the schedule that ayla_b200_default_config reports: where that one asks for no workspace, a lent
+    one need not be clean, and two streams may lend the same."""
+    status, _ = device_state
+    status.zero_()
+    assert _lib.workspace_bytes(_lib.default_config("mm", "bfloat16", 1, m, n, k), "mm", 1, m, n, k) == 0
+    g = torch.Generator(device=DEV).manual_seed(m)
+    a = torch.randn(m, k, device=DEV, generator=g).bfloat16()
+    bt = (torch.randn(n, k, device=DEV, generator=g) * k ** -0.5).bfloat16()
+    lent = torch.full((64 << 20,), 7, dtype=torch.uint8, device=DEV)
+    out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    _lib.gemm("mm", "bfloat16", 0, a.data_ptr(), bt.data_ptr(), out.data_ptr(), 1, m, n, k, None, lent.data_ptr(),
+              lent.numel(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert bool((lent == 7).all())
+    # fp32 sums in another order than the reference's, then one rounding to bfloat16
+    torch.testing.assert_close(out.float(), a.float() @ bt.float().T, atol=0.02, rtol=2.0 ** -8)
+
+
 def test_abi_workspace_and_init_errors(device_state):
     status, workspace = device_state
     a = torch.randn(256, 1024, device=DEV, dtype=torch.bfloat16)
