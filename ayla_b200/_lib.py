@@ -37,6 +37,7 @@ EXPORTS = (
     "ayla_b200_config_valid",
     "ayla_b200_workspace_bytes",
     "ayla_b200_workspace_counter_bytes",
+    "ayla_b200_capture_workspace",
     "ayla_b200_copy_2d",
     "ayla_b200_kernel_count",
     "ayla_b200_kernel_info",
@@ -153,6 +154,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_workspace_bytes.restype = sz
         lib.ayla_b200_workspace_counter_bytes.argtypes = [cfgp, i32, i64, i64, i64, i64]
         lib.ayla_b200_workspace_counter_bytes.restype = sz
+        lib.ayla_b200_capture_workspace.argtypes = [vp, sz, ctypes.POINTER(vp)]
+        lib.ayla_b200_capture_workspace.restype = i32
         lib.ayla_b200_copy_2d.argtypes = [vp, sz, vp, sz, sz, sz, vp]
         lib.ayla_b200_copy_2d.restype = i32
         lib.ayla_b200_kernel_count.argtypes = []
@@ -268,6 +271,17 @@ def workspace_bytes(cfg: Config, op: str, batch: int, m: int, n: int, k: int) ->
 
 def workspace_counter_bytes(cfg: Config, op: str, batch: int, m: int, n: int, k: int) -> int:
     return int(load().ayla_b200_workspace_counter_bytes(ctypes.byref(cfg), OP_CODES[op], batch, m, n, k))
+
+
+def capture_workspace(stream: int, size: int) -> int | None:
+    """Pointer to the workspace of launches captured on ``stream``, which the graph under capture keeps; ``None`` where
+    there is no memory for it."""
+    pointer = ctypes.c_void_p()
+    code = load().ayla_b200_capture_workspace(stream or None, size, ctypes.byref(pointer))
+    if code == E_CUDA:
+        return None
+    check(code)
+    return pointer.value
 
 
 def gemm(op: str, dtype: str, bias_ptr: int, a_ptr: int, bt_ptr: int, out_ptr: int, batch: int,

@@ -1,7 +1,7 @@
 // C ABI of the sm_100a GEMM backend: argument checks, schedule choice, tensor-map
 // encoding and the kernel launch.  Nothing here allocates device memory or
-// synchronises, so every entry point except ayla_b200_init can run inside CUDA
-// graph capture.
+// synchronises but ayla_b200_capture_workspace, which is for captures, so every entry
+// point except ayla_b200_init can run inside CUDA graph capture.
 #include "../../include/ayla_b200.h"
 
 #include <cuda.h>
@@ -17,6 +17,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "capture_workspace.h"
 #include "kernel_registry.h"
 #include "packed_gemm.h"
 #include "rms_factors.h"
@@ -1160,6 +1161,19 @@ size_t ayla_b200_workspace_counter_bytes(const ayla_b200_config* cfg, int op, in
   const int epi = (op == AYLA_B200_OP_ADDMM) ? EPI_BIAS : EPI_PLAIN;
   if (make_plan(*cfg, epi, batch, cfg->swap_ab ? n : m, cfg->swap_ab ? m : n, k, 148, &plan)) return 0;
   return counter_bytes_for(plan);
+}
+
+int ayla_b200_capture_workspace(void* stream, size_t bytes, void** workspace) {
+  if (workspace == nullptr || bytes < kCounterBytes) {
+    return fail(AYLA_B200_E_INVALID, "a workspace has at least its %zu bytes of counters", kCounterBytes);
+  }
+  const cudaError_t err =
+      capture_workspace(reinterpret_cast<cudaStream_t>(stream), bytes, kCounterBytes, workspace);
+  if (err != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(AYLA_B200_E_CUDA, "a workspace for the graph being captured: %s", cudaGetErrorString(err));
+  }
+  return AYLA_B200_OK;
 }
 
 int ayla_b200_gemm(int op, int dtype, const void* bias, const void* a, const void* bt, void* out,

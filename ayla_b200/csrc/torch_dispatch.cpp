@@ -7,8 +7,9 @@
 // the launch included.
 //
 // Everything that is not the plain repeated call stays in Python: an unseen shape, operands the op refuses, a
-// launch reported as timed out by its status word, a stream other than the one the workspace belongs to, another
-// current device, a launch the library refuses.  Those go to the fallback with nothing done yet.
+// launch reported as timed out by its status word, a stream other than the one the workspace belongs to, a capture of a
+// launch with a workspace, another current device, a launch the library refuses.  Those go to the fallback with nothing
+// done yet.
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
@@ -20,6 +21,7 @@
 
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
@@ -68,6 +70,16 @@ void call_python(PyObject* function, c10::ArrayRef<c10::IValue> args) {
   Py_DECREF(result);
 }
 
+// A captured launch gets a workspace of its graph's.
+bool capturing(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &status) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
 constexpr size_t kMaxOperands = 5;
 constexpr size_t kMaxKey = 1 + kMaxOperands * 4;  // the device, and of each operand its rank and up to three sizes
 
@@ -102,7 +114,7 @@ class Dispatcher {
     if (*static_cast<volatile const uint32_t*>(l->status) != 0) return false;
     if (c10::cuda::current_device() != l->device) return false;
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(l->device)).stream();
-    if (l->workspace_bytes != 0 && reinterpret_cast<uintptr_t>(stream) != l->home_stream) return false;
+    if (l->workspace_bytes != 0 && (reinterpret_cast<uintptr_t>(stream) != l->home_stream || capturing(stream))) return false;
     const void* p[kMaxOperands];
     for (size_t i = 0; i + 1 < operands_; ++i) p[i] = args[i].toTensor().const_data_ptr();
     p[operands_ - 1] = args[operands_ - 1].toTensor().mutable_data_ptr();  // the last operand is written

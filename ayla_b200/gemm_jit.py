@@ -252,9 +252,11 @@ class GemmLauncher:
     itself allocates nothing and can be captured in a CUDA graph.  A launch on another
     stream gets a workspace of its own the first time that stream is used (two launches
     of one shape that overlap on different streams would otherwise sum into each other's
-    partial tiles); that first use allocates, so it must happen outside graph capture --
-    inside capture a schedule without a workspace runs instead, or, where a k-split was measured
-    for the shape itself, it raises ``RuntimeError`` as a first call of a new shape does.
+    partial tiles).  A captured launch gets the workspace of its graph
+    (``ayla_b200_capture_workspace``), since the graph may be replayed beside eager launches and
+    other graphs; without memory for one it runs a schedule that needs none.  Where a k-split was
+    measured for the shape itself, its first call on a stream must happen outside capture:
+    inside it raises ``RuntimeError`` as a first call of a new shape does.
 
     The status word lives in pinned host memory (``_lib.StatusWord``): every call reads it
     before launching, without synchronising, and raises ``RuntimeError`` if an earlier
@@ -267,6 +269,7 @@ class GemmLauncher:
     packed kernel instead, and ``seed`` and ``config`` are not used.
     """
 
+    _captured_only_where_run = True  # a capture on a stream where this launcher has not run is refused
     _unsplit_config: _lib.Config | None = None
     _unsplit_tail: tuple | None = None
 
@@ -304,9 +307,10 @@ class GemmLauncher:
                       self.workspace.numel() if self.workspace is not None else 0, self._status_ptr)
         self._has_bias = operation == "addmm"
         self._device_index = index
+        self._captured_only_where_run = not seed.adaptations
         if need and seed.adaptations:
-            # What a capture on a stream without a workspace records, unless this schedule was measured for the shape:
-            # the one before its depth was split, the library's, or this one with its depth whole.
+            # What a capture without memory for a workspace records, unless this schedule was measured for the shape: the
+            # one before its depth was split, the library's, or this one with its depth whole.
             whole = {**seed.builder_config, "split_k": 1, "split_tail": 0, "cluster_split": 0}
             library = _lib.default_config(operation, dtype, batch, m, n, k, activation).to_dict()
             for candidate in (seed.unsplit_config, library, whole):
@@ -332,7 +336,7 @@ class GemmLauncher:
             self._report_timeout()
         stream = torch.cuda.current_stream(self._device_index).cuda_stream
         tail = self._tail
-        if self._ws_bytes and stream != self._home_stream:
+        if self._ws_bytes:
             tail = self._tail_for_stream(stream)
         # The library launches on the current device (the reference's launcher guards the device
         # the same way, ayla/ptx_runtime.py:268-275).
@@ -367,20 +371,36 @@ class GemmLauncher:
         }
 
     def _tail_for_stream(self, stream: int) -> tuple:
-        """The call arguments with the workspace that belongs to ``stream`` (allocated on first use)."""
+        """The call arguments with the workspace that belongs to ``stream`` (allocated on first use), or to the graph
+        under capture there."""
         entry = self._per_stream.get(stream)
+        with torch.cuda.device(self._device_index):
+            capturing = torch.cuda.is_current_stream_capturing()
+            if capturing:
+                if self._captured_only_where_run and entry is None and stream != self._home_stream:
+                    raise RuntimeError(
+                        f"jit_{self.operation}: the first launch of this k-split shape on a stream cannot happen during "
+                        "CUDA graph capture; run it once on that stream before capturing")
+                return self._captured_tail(stream)
+        if stream == self._home_stream:
+            return self._tail
         if entry is None:
-            if torch.cuda.is_current_stream_capturing():
-                if self._unsplit_tail is not None:
-                    return self._unsplit_tail
-                raise RuntimeError(
-                    f"jit_{self.operation}: the first launch of this k-split shape on a new stream allocates its "
-                    "workspace and cannot happen during CUDA graph capture; run it once on that stream before capturing")
             workspace = torch.zeros(self._ws_bytes, dtype=torch.uint8, device=self.device)
-            batch, m, n, k, cfg, _, size, status = self._tail
-            entry = (workspace, (batch, m, n, k, cfg, workspace.data_ptr(), size, status))
+            entry = (workspace, self._tail_with(workspace.data_ptr()))
             self._per_stream[stream] = entry
         return entry[1]
+
+    def _tail_with(self, workspace: int) -> tuple:
+        batch, m, n, k, cfg, _, _, status = self._tail
+        return (batch, m, n, k, cfg, workspace, self._ws_bytes, status)
+
+    def _captured_tail(self, stream: int) -> tuple:
+        workspace = _lib.capture_workspace(stream, self._ws_bytes)
+        if workspace is not None:
+            return self._tail_with(workspace)
+        if self._unsplit_tail is None:
+            raise RuntimeError(f"jit_{self.operation}: no memory for the workspace of a captured launch")
+        return self._unsplit_tail
 
     def _report_timeout(self) -> None:
         code = self.status.peek()

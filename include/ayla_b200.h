@@ -290,6 +290,15 @@ AYLA_B200_API size_t ayla_b200_workspace_counter_bytes(const ayla_b200_config* c
                                          int64_t m, int64_t n, int64_t k);
 
 /*
+ * A workspace for launches captured on `stream`, which is capturing and belongs to the current device: `bytes` bytes,
+ * the counters zero, held by the graph under capture and by every executable made from it, and given back by a later
+ * call once they are gone.  Launches captured on one stream get the same one.  A captured launch should use no other:
+ * its graph may be replayed beside eager launches and other graphs, and two launches that share a workspace must not
+ * overlap.  AYLA_B200_E_CUDA where there is no memory, or no capture.  (No counterpart in the reference.)
+ */
+AYLA_B200_API int ayla_b200_capture_workspace(void* stream, size_t bytes, void** workspace);
+
+/*
  * Strided device-to-device copy on the copy engines (no SMs): `rows` rows of `width_bytes`,
  * source rows `src_pitch` apart, destination rows `dst_pitch` apart.  Used by the N-sharded
  * multi-GPU mm to put gathered column blocks of `out` in place while the GEMM of the next

@@ -697,8 +697,9 @@ def test_packed_kernel_equals_the_general_one(operation, batch, m, n, k, dtype):
     assert bool((out[-guard:] == 7.0).all())
 
 
-def test_a_capture_on_a_new_stream_records_the_schedule_without_a_workspace():
-    """A product whose depth is split where SMs would idle needs a workspace per stream; a capture cannot allocate one."""
+def test_a_capture_without_memory_for_a_workspace_records_a_schedule_that_needs_none(monkeypatch):
+    """A product whose depth is split where SMs would idle needs a workspace, which its graph may not get."""
+    monkeypatch.setattr(_lib, "capture_workspace", lambda stream, size: None)
     m, n, k = 175, 2304, 8000
     g = torch.Generator().manual_seed(5)
     a = torch.randn(m, k, generator=g).bfloat16()
@@ -718,6 +719,110 @@ def test_a_capture_on_a_new_stream_records_the_schedule_without_a_workspace():
         graph.replay()
         torch.cuda.synchronize()
         assert_parity(out, want, "captured")
+
+
+def _split_product(m=175, n=2304, k=8000):
+    """A specialised mm whose depth is split through a workspace, its operands and its eager result."""
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    a = torch.randn(m, k, device=DEV, generator=g).bfloat16()
+    bt = (torch.randn(n, k, device=DEV, generator=g) * k ** -0.5).bfloat16()
+    compiler = gemm_jit_compiler("mm", "bfloat16")
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    compiler(a, bt, out)
+    launcher = next(iter(compiler._cache.values()))
+    assert launcher.workspace is not None
+    return compiler, launcher, a, bt, out
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_captured_launches_have_a_workspace_of_their_graph(warm):
+    """Whether or not the stream they were captured on has one: a replay touches no stream's workspace, and gives what
+    the eager launch gives, bit for bit."""
+    compiler, launcher, a, bt, want = _split_product()
+    stream = torch.cuda.Stream()
+    out = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    if warm:
+        with torch.cuda.stream(stream):
+            compiler(a, bt, out)
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        compiler(a, bt, out)
+        compiler(a, bt, out)
+    spaces = [launcher.workspace, *(workspace for workspace, _ in launcher._per_stream.values())]
+    assert len(spaces) == 1 + warm
+    header = _lib.workspace_counter_bytes(launcher.config, "mm", 1, *want.shape, a.shape[1])
+    for workspace in spaces:
+        workspace[header:] = 7
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    for workspace in spaces:
+        assert not bool(workspace[:header].any()) and bool((workspace[header:] == 7).all())
+
+
+def test_graphs_and_eager_launches_of_a_split_product_overlap():
+    compiler, _, a, bt, want = _split_product()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    outs = [torch.zeros_like(want) for _ in streams]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        compiler(a, bt, outs[0])
+    torch.cuda.synchronize()
+    graphs = []
+    for out in outs[1:]:  # both captured on the stream that the eager launches use
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            for _ in range(4):
+                compiler(a, bt, out)
+        graphs.append(graph)
+    for _ in range(25):
+        for stream, graph in zip(streams[1:], graphs):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        with torch.cuda.stream(streams[0]):
+            for _ in range(4):
+                compiler(a, bt, outs[0])
+        torch.cuda.synchronize()
+        for out in outs:
+            assert torch.equal(out, want)
+            out.zero_()
+        torch.cuda.synchronize()
+
+
+def test_workspaces_of_graphs_are_shared_along_a_stream_and_given_back():
+    size = 8 << 20
+    stream = torch.cuda.current_stream().cuda_stream
+    assert _lib.capture_workspace(stream, size) is None  # not capturing
+    with pytest.raises(ValueError, match="counters"):
+        _lib.capture_workspace(stream, 1024)
+    x = torch.zeros(8, device=DEV)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    here, other = torch.cuda.Stream(), torch.cuda.Stream()
+    for i in range(40):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=here):
+            first = _lib.capture_workspace(here.cuda_stream, size)
+            assert first is not None
+            assert _lib.capture_workspace(here.cuda_stream, size // 2) == first
+            other.wait_stream(here)
+            second = _lib.capture_workspace(other.cuda_stream, size)
+            with torch.cuda.stream(other):
+                x.add_(1)
+            here.wait_stream(other)
+            larger = _lib.capture_workspace(here.cuda_stream, 2 * size)
+            assert len({first, second, larger}) == 3
+            assert _lib.capture_workspace(here.cuda_stream, size) in (first, larger)
+        graph.replay()
+        torch.cuda.synchronize()
+        del graph
+    # 40 graphs of 32 MB each; the last one or two may still be held
+    assert before - torch.cuda.mem_get_info()[0] < 256 << 20
+    assert bool((x == 40).all())
 
 
 # The packed kernel's piped form: one B and many, a depth of one piece and of an odd number, units with rows and matrices
