@@ -20,6 +20,8 @@ from __future__ import annotations
 
 import math
 import os
+import threading
+import weakref
 from dataclasses import dataclass, replace
 from functools import cache
 
@@ -244,15 +246,39 @@ def packed_serves(operation: str, batch: int, m: int, n: int, k: int, device: to
         return _lib.packed_preferred(operation, batch, m, n, k)
 
 
+class _StreamWorkspace:
+    """Memory that the k-split launches of one stream take in turn: each leaves its arrival counters at zero, wherever
+    the next one's partial sums lie."""
+
+    def __init__(self, size: int, device: torch.device):
+        self.size = size
+        self.tensor = torch.zeros(size, dtype=torch.uint8, device=device)
+
+
+_WORKSPACES: weakref.WeakValueDictionary[tuple[int, int], _StreamWorkspace] = weakref.WeakValueDictionary()
+_WORKSPACES_LOCK = threading.Lock()
+
+
+def _stream_workspace(index: int, stream: int, size: int, device: torch.device) -> _StreamWorkspace:
+    """The workspace of ``stream``, the current one, with at least ``size`` bytes.  All shapes share it (one each, for a
+    thousand token counts through one layer, had taken ten gigabytes).  It grows by a factor of two or more; a launcher
+    keeps what it was given, so a stream holds less than four times its largest need, and the memory goes with the last
+    launcher that has it."""
+    with _WORKSPACES_LOCK:
+        workspace = _WORKSPACES.get((index, stream))
+        if workspace is None or workspace.size < size:
+            workspace = _StreamWorkspace(size if workspace is None else max(size, 2 * workspace.size), device)
+            _WORKSPACES[index, stream] = workspace
+        return workspace
+
+
 class GemmLauncher:
     """One specialised ``(operation, dtype, shape, device)`` launch.
 
-    Owns the split-K workspaces and the status word of its shape.  The workspace of the
-    stream that is current at specialisation time is allocated here, so that a launch
-    itself allocates nothing and can be captured in a CUDA graph.  A launch on another
-    stream gets a workspace of its own the first time that stream is used (two launches
-    of one shape that overlap on different streams would otherwise sum into each other's
-    partial tiles).  A captured launch gets the workspace of its graph
+    Owns the status word of its shape and holds the split-K workspace of every stream it is used on
+    (``_stream_workspace``; two launches that overlap on different streams would otherwise sum into
+    each other's partial tiles): that of the stream which is current at specialisation time from then on,
+    so that a launch there allocates nothing, another stream's from its first use.  A captured launch gets the workspace of its graph
     (``ayla_b200_capture_workspace``), since the graph may be replayed beside eager launches and
     other graphs; without memory for one it runs a schedule that needs none.  Where a k-split was
     measured for the shape itself, its first call on a stream must happen outside capture:
@@ -288,13 +314,18 @@ class GemmLauncher:
         self._packed = packed  # the library takes that kernel where it is given no schedule
         need = 0 if self._packed else _lib.workspace_bytes(self.config, operation, batch, m, n, k)
         self._ws_bytes = need
-        self.workspace = torch.zeros(need, dtype=torch.uint8, device=device) if need else None
+        self.workspace = None
+        self._home_stream = None
+        self._held: list[_StreamWorkspace] = []
+        if need:
+            with torch.cuda.device(index):
+                self._home_stream = torch.cuda.current_stream().cuda_stream
+                self._held.append(_stream_workspace(index, self._home_stream, need, device))
+            self.workspace = self._held[0].tensor
         self.status = _lib.StatusWord()
         self._ws_ptr = self.workspace.data_ptr() if self.workspace is not None else 0
         self._status_ptr = self.status.ptr
-        # stream handle -> (workspace tensor, argument tail); the first entry serves the stream current now
-        with torch.cuda.device(index):
-            self._home_stream = torch.cuda.current_stream().cuda_stream if need else None
+        # stream handle -> (workspace tensor, argument tail), other than the stream current now
         self._per_stream: dict[int, tuple[torch.Tensor, tuple]] = {}
         self._debug = bool(os.environ.get("AYLA_B200_DEBUG"))
         # Everything that does not change from call to call, converted for the C call once.
@@ -304,7 +335,7 @@ class GemmLauncher:
         self._entry = lib.ayla_b200_gemm_act_rowmul if gated == "row" else lib.ayla_b200_gemm_act_mul
         self._head = (_lib.OP_CODES[operation], _lib.DTYPE_CODES[dtype], _lib.ACT_CODES[activation])
         self._tail = (batch, m, n, k, None if self._packed else ctypes.byref(self.config), self._ws_ptr or None,
-                      self.workspace.numel() if self.workspace is not None else 0, self._status_ptr)
+                      self._ws_bytes, self._status_ptr)
         self._has_bias = operation == "addmm"
         self._device_index = index
         self._captured_only_where_run = not seed.adaptations
@@ -385,8 +416,10 @@ class GemmLauncher:
         if stream == self._home_stream:
             return self._tail
         if entry is None:
-            workspace = torch.zeros(self._ws_bytes, dtype=torch.uint8, device=self.device)
-            entry = (workspace, self._tail_with(workspace.data_ptr()))
+            with torch.cuda.device(self._device_index):
+                space = _stream_workspace(self._device_index, stream, self._ws_bytes, self.device)
+            self.__dict__.setdefault("_held", []).append(space)
+            entry = (space.tensor, self._tail_with(space.tensor.data_ptr()))
             self._per_stream[stream] = entry
         return entry[1]
 
@@ -406,10 +439,17 @@ class GemmLauncher:
         code = self.status.peek()
         with torch.cuda.device(self._device_index):
             torch.cuda.current_stream().synchronize()  # nothing of the failed launch is still running
-            if self.workspace is not None:
-                self.workspace.zero_()  # arrival counters a timed-out k-split leaves behind
-            for workspace, _ in self._per_stream.values():
-                workspace.zero_()
+            # Arrival counters a timed-out k-split leaves behind: behind the launches of the stream that uses them.
+            here = torch.cuda.current_stream().cuda_stream
+            spaces = [(stream, workspace) for stream, (workspace, _) in self._per_stream.items()]
+            for stream, workspace in [(self._home_stream, self.workspace), *spaces]:
+                if workspace is None:
+                    continue
+                if stream is None or stream == here:
+                    workspace.zero_()
+                else:
+                    with torch.cuda.stream(torch.cuda.ExternalStream(stream)):
+                        workspace.zero_()
         self.status.clear()
         raise RuntimeError(
             f"jit_{self.operation}: device wait timed out (code {code & 0xFF}, CTA {code >> 8})"

@@ -300,6 +300,26 @@ def test_launcher_gives_every_stream_its_own_k_split_workspace(monkeypatch):
         launcher(tensor, tensor, tensor)
 
 
+def test_launchers_of_one_stream_share_a_workspace_that_grows(monkeypatch):
+    """One per stream for all shapes, at least doubled when it grows, given back with the last launcher that has it."""
+    import types
+
+    from ayla_b200 import gemm_jit
+
+    allocated = []
+    monkeypatch.setattr(torch, "zeros", lambda size, dtype=None, device=None: allocated.append(size) or
+                        types.SimpleNamespace(size=size))
+    held = [gemm_jit._stream_workspace(63, 5, size, "cuda:63") for size in (1000, 900, 1000, 1001, 2000, 1500, 9000)]
+    assert allocated == [1000, 2000, 9000]
+    assert held[0] is held[1] is held[2] and held[3] is held[4] is held[5] and held[6] is not held[5]
+    other = gemm_jit._stream_workspace(63, 6, 10, "cuda:63")
+    assert other is not held[0] and allocated[-1] == 10
+    assert (63, 5) in gemm_jit._WORKSPACES
+    del held
+    assert (63, 5) not in gemm_jit._WORKSPACES
+    assert gemm_jit._stream_workspace(63, 6, 5, "cuda:63") is other
+
+
 def test_a_schedule_is_not_transferred_to_a_shape_where_its_tiles_are_mostly_padding():
     from ayla_b200 import gemm_jit
 

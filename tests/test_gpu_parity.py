@@ -793,6 +793,30 @@ def test_graphs_and_eager_launches_of_a_split_product_overlap():
         torch.cuda.synchronize()
 
 
+def test_many_row_counts_share_a_workspace():
+    """A layer called with any number of tokens: every second count has a k-split schedule, all on one workspace."""
+    n, k = 1024, 8192
+    g = torch.Generator(device=DEV).manual_seed(2)
+    a = torch.randn(1024, k, device=DEV, generator=g).bfloat16()
+    bt = (torch.randn(n, k, device=DEV, generator=g) * k ** -0.5).bfloat16()
+    out = torch.empty(1024, n, dtype=torch.bfloat16, device=DEV)
+    want = a.float() @ bt.float().T
+    compiler = gemm_jit_compiler("mm", "bfloat16")
+    compiler(a, bt, out)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    counts = list(range(70, 1024, 9))
+    for m in counts:
+        compiler(a[:m], bt, out[:m])
+    for m in counts[::10]:
+        compiler(a[:m], bt, out[:m])
+        # fp32 sums in another order than the reference's, then one rounding to bfloat16
+        torch.testing.assert_close(out[:m].float(), want[:m], atol=0.02, rtol=2.0 ** -8)
+    launchers = compiler._cache.values()
+    assert sum(launcher.workspace is not None for launcher in launchers) > len(counts) // 2
+    assert torch.cuda.memory_allocated() - before < 64 << 20
+
+
 def test_workspaces_of_graphs_are_shared_along_a_stream_and_given_back():
     size = 8 << 20
     stream = torch.cuda.current_stream().cuda_stream
