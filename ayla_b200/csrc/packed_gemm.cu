@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
     for (int i = 0; i < count; ++i) {
       bw.wait(bar_acc_empty + acc * 8, acc_phase, ST_TIMEOUT_ACC_EMPTY);
       bw.wait(bar_full + slot * 8, phase, ST_TIMEOUT_FULL);
-      if (bw.aborted()) break;
+      if (__any_sync(0xffffffffu, bw.aborted())) break;  // lanes whose wait ran out, and the others with them
       tc_fence_after_sync();
       if (issuer) {
         const uint64_t desc_a = desc_a0 + static_cast<uint32_t>(slot) * (a_bytes >> 4);
@@ -534,8 +534,10 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
     for (int i = set; i < count; i += kEpilogueSets) {
       const uint32_t acc = static_cast<uint32_t>(i) & 1u, acc_phase = (static_cast<uint32_t>(i) >> 1) & 1u;
       bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL);
+      // TMEM is read by whole warps: a wait that ran out for some lanes ends the unit for all.
+      const bool aborted = __any_sync(0xffffffffu, bw.aborted());
       tc_fence_after_sync();
-      const bool live = writer.locate(first + i * stride) && !bw.aborted();
+      const bool live = writer.locate(first + i * stride) && !aborted;
       if (live) writer.stage(tmem_base + acc * static_cast<uint32_t>(p.mma_n));
       tc_fence_before_sync();
       __syncwarp();

@@ -881,6 +881,43 @@ def test_piped_packed_kernel_equals_the_general_one(operation, batch, m, n, k, d
     assert bool(torch.isnan(outs[0][batch * m:]).all())
 
 
+@pytest.mark.parametrize("batch, m, n, k", [(1, 70000, 96, 24), (2055, 45, 16, 120), (600, 128, 64, 40)])
+def test_piped_packed_kernel_reports_a_timeout_and_keeps_infinities_apart(batch, m, n, k):
+    """One B and many, several units per CTA and one."""
+    operation = "bmm" if batch > 1 else "mm"
+    lead = (batch,) if batch > 1 else ()
+    g = torch.Generator(device=DEV).manual_seed(m)
+    a = torch.randn((*lead, m, k), device=DEV, generator=g).half()
+    bt = (torch.randn((*lead, n, k), device=DEV, generator=g) * k ** -0.5).half()
+    out = torch.empty((*lead, m, n), device=DEV, dtype=torch.float16)
+    compiler = gemm_jit_compiler(operation, "float16")
+    compiler(a, bt, out)
+    launcher = next(iter(compiler._cache.values()))
+    assert launcher._packed
+    want = out.clone()
+    a.view(-1, k)[m - 1, 5] = float("inf")
+    compiler(a, bt, out)
+    bad = ~torch.isfinite(out.view(-1, n))
+    assert bool(bad[m - 1].all()) and int(bad.sum()) == n
+    a.view(-1, k)[m - 1] = 1.0
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(30)
+        lib.ayla_b200_debug_set_flags(1)
+        launcher(a, bt, out)  # no operand arrives: the waits run out
+        torch.cuda.synchronize()
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    with pytest.raises(RuntimeError, match="timed out"):
+        launcher(a, bt, out)
+    out.zero_()
+    launcher(a, bt, out)
+    launcher.check_status()
+    rows = torch.arange(out.numel() // n, device=DEV) != m - 1
+    assert torch.equal(out.view(-1, n)[rows], want.view(-1, n)[rows])
+
+
 def test_packed_kernel_through_the_ops_and_its_limits():
     a = torch.randn(300, 32, 24, device=DEV).half()
     bt = torch.randn(300, 16, 24, device=DEV).half()
