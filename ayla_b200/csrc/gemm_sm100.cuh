@@ -116,7 +116,7 @@ struct KernelParams {
   FastDiv div_last_group_rows;  // by the row tiles of the last, partial raster group (m_tiles % group_m)
   FastDiv div_splits;           // by splits
   int ctas_per_unit_log2;       // log2(CTA_GROUP * cluster_split or 1)
-  unsigned handover_ns; // shared sum: how long the owner of a piece waits before it leaves the piece to the others
+  unsigned handover_ns; // shared sum: how long the owner of a piece waits before it hands it over (0: it does so at once)
   int stages;         // ring slots in use (<= the kernel's STAGES); fewer when the top of the ring region
                       // is set aside as the inbox of a cluster split-K launch
   uint32_t inbox_offset;  // cluster split-K: byte offset of the inbox from the start of shared memory
@@ -1699,7 +1699,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             bool complete;
             if (own) {
               complete = true;
-              if (lane == 0) complete = bw.count_reaches(counters + c32 * 4, static_cast<unsigned>(splits - 1), p.handover_ns);
+              if (lane == 0) {
+                complete = p.handover_ns != 0 &&
+                           bw.count_reaches(counters + c32 * 4, static_cast<unsigned>(splits - 1), p.handover_ns);
+              }
               if (!__shfl_sync(0xffffffffu, complete ? 1 : 0, 0)) {
                 park(c32);
                 __syncwarp();

@@ -325,7 +325,9 @@ AYLA_B200_API void ayla_b200_set_wait_timeout_ms(int64_t ms);
  * normally with code 2 in `status` and garbage in `out`; the context stays usable.
  * Bit 1: cluster split-K launches keep all their ring slots and let the inbox of partial sums
  * overlay them (the form used when the ring could not spare the slots), so that both forms of
- * the exchange can be compared on one shape.  0 restores normal operation.
+ * the exchange can be compared on one shape.  Bit 5: where the CTAs that split a tile's depth share
+ * its sum, the owner of a piece hands it over without waiting for the others, even if they are all
+ * there.  0 restores normal operation.
  */
 AYLA_B200_API void ayla_b200_debug_set_flags(int flags);
 

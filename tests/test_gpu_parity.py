@@ -187,7 +187,7 @@ def test_shared_sum_of_a_split_depth(batch, m, n, k, config, bias, device_state)
     out, status = run_abi(operation, "bfloat16", tensors, config, device_state)
     assert status == 0
     assert_parity(out, O.gemm_ref32(operation, *tensors), config)
-    lib.ayla_b200_debug_set_flags(32)  # owners hand their pieces over at once unless all partials are there
+    lib.ayla_b200_debug_set_flags(32)  # owners hand every piece over, to whoever is last or back to themselves
     try:
         for _ in range(3):
             handed, status = run_abi(operation, "bfloat16", tensors, config, device_state)
@@ -198,6 +198,48 @@ def test_shared_sum_of_a_split_depth(batch, m, n, k, config, bias, device_state)
     again, _ = run_abi(operation, "bfloat16", tensors, config, device_state)  # the counters were left clean
     assert torch.equal(again, out)
     assert not bool(device_state[1][:65536].any())
+
+
+@pytest.mark.parametrize("tile_n,cta_group", ROW_MAJOR)
+def test_split_depths_summed_by_the_last_arriver(tile_n, cta_group, device_state):
+    """More split units than the grid runs at once (few CTAs asked for), so that a CTA has several: the last to arrive
+    sums a tile.  With a bias, an activation, factors per row, a gate and batches."""
+    status, workspace = device_state
+    config = dict(tile_n=tile_n, cta_group=cta_group, split_k=3, grid_ctas=6)
+    torch.manual_seed(tile_n + cta_group)
+    for operation, activation, gate, batch, m, n, k in (
+            ("mm", "none", None, 1, 333, 520, 520), ("addmm", "none", None, 1, 300, 776, 264), ("bmm", "none", None, 4, 200, 136, 712),
+            ("addmm", "gelu", None, 1, 520, 520, 200), ("mm", "relu", "row", 1, 300, 1032, 320), ("addmm", "silu", "full", 1, 700, 264, 392)):
+        lead = (batch,) if operation == "bmm" else ()
+        a = torch.randn((*lead, m, k)).bfloat16()
+        bt = (torch.randn((*lead, n, k)) * k ** -0.5).bfloat16()
+        tensors = (a, bt) if operation != "addmm" else (torch.randn(n).bfloat16(), a, bt)
+        assert -(-m // (128 * cta_group)) * -(-n // tile_n) * batch * 3 > 6 // cta_group
+        want = O.gemm_ref32(operation, *tensors)
+        if activation == "none" and gate is None:
+            out, code = run_abi(operation, "bfloat16", tensors, config, device_state)
+            out = out.cpu()
+        else:
+            want = O.act_ref32(activation, want)
+            dev = [t.to(DEV) for t in tensors]
+            out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+            status.zero_()
+            mul = (torch.rand(m, 1 if gate == "row" else n) + 0.5).bfloat16()
+            head = (operation, "bfloat16", activation, dev[0].data_ptr() if operation == "addmm" else 0, dev[-2].data_ptr(),
+                    dev[-1].data_ptr())
+            tail = (out.data_ptr(), 1, m, n, k, _lib.Config.from_dict(config), workspace.data_ptr(), workspace.numel(),
+                    status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            if gate is None:
+                _lib.gemm_act(*head, *tail)
+            else:
+                want = want * mul.float()
+                held = mul.to(DEV)
+                (_lib.gemm_act_rowmul if gate == "row" else _lib.gemm_act_mul)(*head, held.data_ptr(), *tail)
+            torch.cuda.synchronize()
+            out, code = out.cpu(), int(status.item())
+        assert code == 0
+        assert_parity(out, want, f"{operation} {activation} {gate} {batch}x{m}x{n}x{k} {config}")
+    assert not bool(workspace[:65536].any())
 
 
 @pytest.mark.parametrize("tile_n", [16, 32, 64, 128])
