@@ -159,10 +159,43 @@ def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: 
 
 
 def _streams_weights(operation: str, batch: int, m: int, n: int, k: int) -> bool:
-    """A few rows against a large weight: the library's rule (one wave of clusters that run at once, as many tiles as
-    SMs) is the better guess there than a neighbour's schedule (us, neighbour -> rule: 12x4608x5504 17.2 -> 12.2,
-    17x4568x2520 12.8 -> 8.9, 7x13696x5504 26.1 -> 23.6, 10x7424x3968 12.7 -> 11.7)."""
+    """A few rows against a large weight."""
     return operation != "bmm" and batch == 1 and m <= 64 and n >= 1024 and k >= 1024
+
+
+def _ctas(config: dict[str, object], m: int, n: int) -> int:
+    """CTAs that a schedule puts to work, cluster members included."""
+    pair = int(config["cta_group"])
+    rows, cols = (n, m) if config["swap_ab"] else (m, n)
+    height = (int(config["tile_rows"]) or 128) if config["swap_ab"] else 128 * pair
+    return -(-rows // height) * -(-cols // int(config["tile_n"])) * int(config["split_k"]) * pair
+
+
+def _rule_streams_better(neighbour: dict[str, object], rule: dict[str, object], activation: str, m: int, n: int,
+                         k: int) -> bool:
+    """Whether the library's rule for a stream of weights is the better guess than a neighbour's schedule.
+
+    Over 483 shapes of up to 64 rows timed with both, the rule is taken for 297: the geometric mean of the times is 0.938
+    of the neighbours', two are slower by 2 to 3 %; with the rule always it is 0.948 and 58 are slower, up to 1.66 times.
+    It is better (us, neighbour -> rule)
+     * where it puts more SMs to work, a short product against whole rows of the weight aside (32x8192x1856 20.4 -> 10.4,
+       30x4928x4608 18.6 -> 13.0; but of 20 k-blocks or fewer 45x2752x1088 7.2 -> 7.6);
+     * against clusters that tile the rows, from 24 k-blocks on and with nothing fused (58x1152x2816 8.7 -> 6.9; with a
+       gate 41x9216x3840 18.1 -> 23.3, of 18 k-blocks 53x1560x1112 6.0 -> 6.6);
+     * against the same tiles without a hint that the weight leaves L2 first (4x2752x1280 5.9 -> 5.3).
+    Not against whole rows of the weight on as many SMs (63x7232x1280 8.4 -> 10.7, gated 41x4416x1728 9.2 -> 15.3), and not
+    with clusters of four against eight that run at once (2x1408x7680 7.6 -> 8.7)."""
+    waves, rule_waves = _waves(neighbour, 1, m, n), _waves(rule, 1, m, n)
+    if waves != rule_waves:
+        return rule_waves < waves
+    k_blocks = -(-k // 64)
+    share = _ctas(rule, m, n) / _ctas(neighbour, m, n)
+    if not neighbour["swap_ab"]:
+        if int(neighbour["split_k"]) == 1:
+            return share > 1.05 and k_blocks > 20
+        return share > 1.1 or (activation == "none" and k_blocks >= 24)
+    unhinted = not neighbour["l2_hint_b"] and neighbour["tile_n"] == rule["tile_n"] and int(neighbour["split_k"]) < 8
+    return share > 1.05 or unhinted
 
 
 def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
@@ -194,8 +227,9 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
     def finished(seed: GemmScheduleSeed | None) -> GemmScheduleSeed | None:
         return _shared_depth(seed, operation, dtype, m, n, k, batch) if share_depth else seed
 
+    rule = None
     if query not in table and _streams_weights(operation, batch, m, n, k):
-        return finished(_fallback_schedule(operation, dtype, m, n, k, batch, activation))
+        rule = _fallback_schedule(operation, dtype, m, n, k, batch, activation)
     for shape in sorted(table, key=distance):
         if distance(shape) > _MAX_TRANSFER_DISTANCE:
             break
@@ -209,6 +243,8 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
                     continue  # its tiles would be a third or more padding here and were not where it was measured
             seed = _seed(captured, operation, dtype, m, n, k, batch, shape, exact=shape == query)
             if seed is not None:
+                if rule is not None and _rule_streams_better(captured, rule.captured_config, activation, m, n, k):
+                    return finished(rule)
                 if shape not in SCHEDULES.get((operation, dtype), {}):
                     seed = GemmScheduleSeed(seed.captured_config, seed.builder_config,
                                             (*seed.adaptations, f"measured in {other}"), seed.source_shape,

@@ -119,6 +119,22 @@ def test_meta_dispatch_allocates_nothing_and_returns_none():
         assert gemm_op(operation, "bfloat16")(*args) is None
 
 
+@pytest.mark.parametrize("operation, activation, m, n, k, ruled", [
+    ("mm", "none", 17, 4568, 2520, True), ("mm", "none", 7, 13696, 5504, True), ("mm", "sigmoid", 32, 8192, 1856, True),
+    ("mm", "none", 58, 1152, 2816, True), ("mm", "none", 30, 4928, 4608, True), ("mm", "none", 3, 13056, 1728, True),
+    ("mm", "none", 63, 7232, 1280, False), ("mm", "sigmoid", 41, 4416, 1728, False), ("mm", "sigmoid", 41, 9216, 3840, False),
+    ("mm", "none", 2, 1408, 7680, False), ("mm", "none", 45, 1088, 1280, False), ("addmm", "none", 47, 1344, 8128, False),
+    ("mm", "none", 5, 5136, 2800, False), ("mm", "none", 53, 1560, 1112, False),
+])
+def test_streams_of_weights_go_by_the_rule_where_it_measured_faster(operation, activation, m, n, k, ruled):
+    gated = activation != "none"
+    seed = select_gemm_schedule(operation, "float16", m, n, k, 1, activation, not gated)
+    assert seed is not None and (seed.source_shape is None) == ruled
+    if ruled:
+        rule = _lib.default_config(operation, "float16", 1, m, n, k, activation).to_dict()
+        assert seed.builder_config == rule
+
+
 def test_transferred_schedules_keep_their_wave_count():
     """A schedule measured on a neighbouring shape is not used where it would need more passes of
     the persistent grid than on the shape it was measured on (a fused QKV projection, n = 6144,
