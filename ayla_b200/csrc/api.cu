@@ -584,10 +584,14 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
         c->tile_rows = static_cast<int>(rows);
       }
     }
-    if (c->split_k == 1 && m > 16 && (c->tile_rows == 0 || k_blocks < 40)) {
+    if (c->split_k == 1 && m > 16 && (c->tile_rows == 0 || k_blocks < 40 || (activation != AYLA_B200_ACT_NONE && m > 32))) {
       // No room to split K (bt alone fills the SMs): with a few dozen rows of `a` the plain
       // row-major 128-wide tile, its `a` box trimmed to the rows that exist, measures 1.2-1.3x
-      // faster than the swapped form (M = 32, 64 at N = 14336).
+      // faster than the swapped form (M = 32, 64 at N = 14336).  Trimmed tiles are faster still for deep
+      // products (above), but not over a 64-wide accumulator before a gate, which the swapped form reads
+      // with direct loads and the row-major kernels through their staging rows (38x11512x2952 row-major
+      // 22.0, swapped 25.7; 40x10752x8704 39.8 and 41.6; of 32 rows and fewer 20x11136x5312 27.1 and 25.9).
+      // Gates come with an activation.
       c->swap_ab = 0;
       c->tile_rows = 0;
       c->tile_n = (batch * ceil_div(n, 128) <= static_cast<int64_t>(sm_count)) ? 128 : 256;  // one wave if it fits

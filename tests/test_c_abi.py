@@ -98,6 +98,15 @@ def test_default_schedules_for_the_benchmark_shapes():
         assert _lib.config_valid(cfg, "mm", "bfloat16", *shape)
 
 
+@pytest.mark.parametrize("activation, m, n, k, swapped", [
+    ("sigmoid", 38, 11512, 2952, False), ("silu", 40, 10752, 8704, False), ("sigmoid", 20, 11136, 5312, True),
+    ("none", 38, 13376, 3136, True), ("none", 44, 12216, 4760, True), ("sigmoid", 8, 14336, 4096, True)])
+def test_long_streams_behind_an_activation_are_row_major_from_33_rows_on(activation, m, n, k, swapped):
+    cfg = _lib.default_config("mm", "bfloat16", 1, m, n, k, activation)
+    assert cfg.swap_ab == int(swapped) and cfg.split_k == 1
+    assert swapped or (cfg.tile_n, cfg.tile_rows, cfg.split_tail) == (128, 0, 2)
+
+
 def test_config_validation():
     ok = _lib.Config.from_dict(dict(tile_n=128, cta_group=2))
     assert _lib.config_valid(ok, "mm", "bfloat16", 1, 512, 512, 512)
