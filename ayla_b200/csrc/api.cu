@@ -696,8 +696,12 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 2129x4608x5248, 2 + 14/74, 84 -> 80 -> 77 with 5; but
 //    4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
 //    Rows that start inside a sector are bound by their loads, which a lone pair gets faster: two ways at most
-//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6).  Otherwise half width wherever two halves fit (1260x4480x768
-//    12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
+//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6), behind one whole wave (25 shapes, 0.80 to 0.96 of the time
+//    whole), behind two with a quarter of a wave left (3766x2624x14424, 2 + 17/74, 373 -> 407 -> 356), or where a
+//    schedule has halves (45 shapes of two waves and more, 0.88 to 1.07 of the time in halves, mostly below 0.98);
+//    elsewhere whole tiles stay (4846x3968x12696, 4 + 8/74, 476 -> 561; 6658x2304x12136, 3 + 21/74, 384 -> 431).
+//    Otherwise half width wherever two halves fit (1260x4480x768 12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside
+//    a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
 //    take 0.97 of the time for pairs and a deep product, 0.9 otherwise: over 152 shapes 0.9 chose it 34 times, and it took
 //    0.81 of the time (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29, 175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 ->
@@ -719,7 +723,8 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
     const int64_t rest = tiles % wave;
     if (c->split_k > 1 || c->cluster_split || rest == 0) return;
     const bool halves_fit = c->tile_n % 128 == 0 && rest * 2 <= wave;
-    if (c->tile_n >= 128 && rest * 2 <= wave && k_blocks >= 32) {
+    const bool lone = !mid_sector || tiles < 2 * wave || (tiles < 3 * wave && rest * 4 <= wave) || c->split_tail == 2;
+    if (c->tile_n >= 128 && rest * 2 <= wave && k_blocks >= 32 && lone) {
       int64_t splits = wave / rest;
       if (splits > k_blocks / 8) splits = k_blocks / 8;
       if (splits > (mid_sector ? 2 : 16)) splits = mid_sector ? 2 : 16;

@@ -209,6 +209,13 @@ def test_depth_is_shared_where_sms_would_idle():
     assert shared(4451, 2240, 7040, **pairs)[0] == (256, 2, 5, 1, 0)
     assert shared(1260, 4480, 768, **pairs)[0] == (256, 2, 1, 2, 0)
     assert shared(8192, 1024, 8192, **pairs)[1]
+    # rows that start inside a sector: behind one wave, two with little left, or instead of halves
+    halves = dict(pairs, split_tail=2)
+    assert shared(785, 5056, 8456, **pairs)[0] == (256, 2, 2, 1, 0)
+    assert shared(4096, 2560, 8008, **pairs)[0] == (256, 2, 2, 1, 0)
+    assert shared(4527, 3200, 10792, **halves)[0] == (256, 2, 2, 1, 0)
+    for m, n, k in ((4846, 3968, 12696), (6658, 2304, 12136), (4619, 4992, 11400), (3790, 5568, 7608), (3296, 3136, 8488)):
+        assert shared(m, n, k, **pairs)[1]
     # a deep product on a few SMs, and clusters that do not all run at once
     assert shared(536, 896, 59968, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0][1:] == (2, 6, 0, 0)
     assert shared(175, 2304, 8000, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0] == (128, 2, 4, 0, 0)
