@@ -703,10 +703,13 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    Otherwise half width wherever two halves fit (1260x4480x768 12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside
 //    a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
-//    take 0.97 of the time for pairs and a deep product, 0.9 otherwise: over 152 shapes 0.9 chose it 34 times, and it took
-//    0.81 of the time (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29, 175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 ->
-//    18.0, 1024x1024x8192 22.0 -> 20.1; by less than that others lose: 128x4096x4096 12.1 -> 13.5, 433x1280x3584 with
-//    row factors 12.9 -> 13.7).
+//    take 0.97 of the time for pairs and a deep product, 0.9 otherwise (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29,
+//    175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 -> 18.0, 1024x1024x8192 24.1 -> 22.5; by less than that others lose:
+//    128x4096x4096 12.1 -> 13.5, 433x1280x3584 with row factors 12.9 -> 13.7).  Not 0.97 where the pairs pad a row tile
+//    that single CTAs did not (296x1088x14016 22.6 -> 24.2, 288x576x37248 36.8 -> 40.2), 0.85 for short products whose
+//    rows start inside a sector (332x960x2568 11.8 -> 12.6), and never single CTAs for pairs there, which read B twice as
+//    often (524x3200x13656 88 -> 99).  Over 191 shapes that are split by these bounds it takes 0.81 of the time, the slowest
+//    1.02.
 void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   if (c->swap_ab || c->stream_k || c->grid_ctas != 0 || c->split_tail == 1) return;
   if (c->split_k > 1 && !c->cluster_split && c->split_tail != 0) return;
@@ -749,13 +752,16 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
   for (int tile_n : kWidths) {
     if (tile_n > 64 && n * 2 <= tile_n) continue;
     for (int cta_group = 1; cta_group <= 2; ++cta_group) {
-      if (cta_group == 2 && m <= 128) continue;
+      if ((cta_group == 2 && m <= 128) || (mid_sector && cta_group < c->cta_group)) continue;
       const int64_t there = batch * ceil_div(m, 128 * cta_group) * ceil_div(n, tile_n);
       int64_t most = machine.sm_count / cta_group / there;
       if (most > 48) most = 48;
       if (most > k_blocks / 4) most = k_blocks / 4;
       for (int64_t splits = most; splits >= 2; --splits) {
-        const double bound = cta_group == 2 && tile_n >= 128 && k_blocks >= 96 ? 0.97 : 0.9;
+        const bool pads = cta_group > c->cta_group && ceil_div(m, 128) % 2 != 0;
+        const double bound = cta_group == 2 && tile_n >= 128 && k_blocks >= 96 && !pads ? 0.97
+                             : mid_sector && k_blocks < 48                               ? 0.85
+                                                                                         : 0.9;
         const double us = modelled_us(tile_n, cta_group, static_cast<int>(splits), RATE_SHARED, there, k, machine);
         if (us >= best || us > bound * now) continue;
         best = us;

@@ -219,6 +219,10 @@ def test_depth_is_shared_where_sms_would_idle():
     # a deep product on a few SMs, and clusters that do not all run at once
     assert shared(536, 896, 59968, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0][1:] == (2, 6, 0, 0)
     assert shared(175, 2304, 8000, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[0] == (128, 2, 4, 0, 0)
+    # not for a little in the model where pairs pad, or where rows start inside a sector; no single CTAs for pairs there
+    assert shared(296, 1088, 14016, tile_n=128, cta_group=1, split_k=4, cluster_split=1)[1]
+    assert shared(332, 960, 2568, tile_n=64, cta_group=1, split_k=2, cluster_split=1)[1]
+    assert shared(524, 3200, 13656, **pairs)[0][1] == 2
     # neither: shallow, few rows, swapped, or a grid of its own
     assert shared(256, 1024, 1024, tile_n=64, cta_group=2, split_k=1)[1]
     assert shared(128, 4096, 4096, tile_n=64, cta_group=1, split_k=2, cluster_split=1)[1]
