@@ -701,7 +701,10 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    schedule has halves (45 shapes of two waves and more, 0.88 to 1.07 of the time in halves, mostly below 0.98);
 //    elsewhere whole tiles stay (4846x3968x12696, 4 + 8/74, 476 -> 561; 6658x2304x12136, 3 + 21/74, 384 -> 431).
 //    Otherwise half width wherever two halves fit (1260x4480x768 12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside
-//    a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2).
+//    a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2), in shallow products where the rest is below three tenths of
+//    a wave: there the results that the SMs write set the pace, not their number (bmm 71 x 324x128x272, 0.44 waves, 8.3 ->
+//    8.8; mm 4546x1408x256, 0.46, 7.5 -> 7.8; but 3266x1600x512, 0.23, 9.7 -> 8.6).  192 shapes timed with whole tiles and
+//    halves: 154 take them by this, the geometric mean is 0.963 of the time, three are slower, by 4 to 5 %.
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
 //    take 0.97 of the time for pairs and a deep product, 0.9 otherwise (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29,
 //    175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 -> 18.0, 1024x1024x8192 24.1 -> 22.5; by less than that others lose:
@@ -740,7 +743,7 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
         return;
       }
     }
-    if (halves_fit && !mid_sector) c->split_tail = 2;
+    if (halves_fit && !mid_sector && (k_blocks > 8 || rest * 10 <= wave * 3)) c->split_tail = 2;
     return;
   }
   if (m <= 64 || k_blocks < 16) return;

@@ -209,6 +209,8 @@ def test_depth_is_shared_where_sms_would_idle():
     assert shared(4451, 2240, 7040, **pairs)[0] == (256, 2, 5, 1, 0)
     assert shared(1260, 4480, 768, **pairs)[0] == (256, 2, 1, 2, 0)
     assert shared(8192, 1024, 8192, **pairs)[1]
+    assert shared(3266, 1600, 512, **pairs)[0] == (256, 2, 1, 2, 0)
+    assert shared(4546, 1408, 256, **pairs)[1] and shared(2348, 1408, 448, tile_n=128, cta_group=2)[1]
     # rows that start inside a sector: behind one wave, two with little left, or instead of halves
     halves = dict(pairs, split_tail=2)
     assert shared(785, 5056, 8456, **pairs)[0] == (256, 2, 2, 1, 0)
