@@ -571,15 +571,15 @@ struct Footprint {
   int stages, piped_smem, piped_ctas, piped_tmem_cols;
 };
 
-// Where the piped kernel is the faster one, by how many CTAs of the other an SM would hold (58 shapes timed on both;
-// over those it takes, 0.87 of the time, the slowest 1.01): at two and fewer nothing hides a unit's chain there; at three
-// single matrices gain (57501x72x56 8.7 -> 7.6), pairs of small ones do not (8192 x 56x32x56 22.8 -> 24.0); at four, one
-// B for all units and rows that start inside a 32-byte sector, whose loads take longest (52640x88x24 10.0 -> 7.7, but
-// 146105x56x64 8.7 -> 9.5).  Fewer units than it has CTAs gain nothing from a pipeline (28625x80x24, 224 units, 5.6 ->
-// 5.9).
-bool piped_pays(int64_t units, int64_t k, int matrices, bool shared_b, int chained_ctas) {
-  if (units < 256) return false;
-  return chained_ctas <= 2 || (chained_ctas == 3 && matrices == 1) || (shared_b && k % 16 != 0);
+// Where the piped kernel is the faster one (350 shapes timed on both; over the 67 of the packed kernel's that it takes, 0.911
+// of the time, the slowest 1.04): with rows that start inside a 32-byte sector and one B for all units, whose loads take
+// longest (247747x48x24 18.5 -> 14.0, 33392x64x24 6.7 -> 5.7); otherwise where an SM would hold two CTAs of the other or
+// fewer, which leaves a unit's chain bare (204363x40x88 17.0 -> 14.9), and every CTA has a unit at least (36745x32x128, 288
+// units, 5.0 -> 5.2).  Three CTAs hide it as well or better, far better with few rows to a unit (2984 x 19x112x32 15.1 ->
+// 17.4, 2099 x 10x104x24 11.0 -> 12.7, 381 x 1239x64x56 25.1 -> 26.0).
+bool piped_pays(int64_t units, int64_t k, bool shared_b, int chained_ctas) {
+  if (shared_b && k % 16 != 0) return units >= 256;
+  return chained_ctas <= 2 && units >= 300;
 }
 
 Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
@@ -612,7 +612,7 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
   }
   f.piped_smem = piped_smem(f.stages);
   const int64_t units = f.matrices == 1 ? batch * ((m + kRows - 1) / kRows) : (batch + f.matrices - 1) / f.matrices;
-  f.piped = piped_pays(units, k, f.matrices, shared_b, f.ctas);
+  f.piped = piped_pays(units, k, shared_b, f.ctas);
   return f;
 }
 

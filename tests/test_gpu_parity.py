@@ -923,6 +923,25 @@ def test_piped_packed_kernel_equals_the_general_one(operation, batch, m, n, k, d
     assert bool(torch.isnan(outs[0][batch * m:]).all())
 
 
+@pytest.mark.parametrize("batch, m, n, k, piped", [
+    (1, 70000, 96, 24, True), (2055, 45, 16, 120, True), (2984, 19, 112, 32, False), (381, 1239, 64, 56, False),
+    (1, 36745, 32, 128, False), (5332, 56, 32, 56, False)])
+def test_the_packed_kernels_form_is_the_faster_one(batch, m, n, k, piped):
+    lead = (batch,) if batch > 1 else ()
+    a = torch.zeros((*lead, m, k), device=DEV, dtype=torch.float16)
+    bt = torch.zeros((*lead, n, k), device=DEV, dtype=torch.float16)
+    out = torch.empty((*lead, m, n), device=DEV, dtype=torch.float16)
+    _lib.init(0)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        _lib.gemm_packed("bmm" if batch > 1 else "mm", "float16", 0, a.data_ptr(), bt.data_ptr(), out.data_ptr(), batch, m,
+                         n, k, 0, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+    names = [event.name for event in profile.events() if "packed" in event.name]
+    if not names:
+        pytest.skip("no kernel names from the profiler")
+    assert len(names) == 1 and ("packed_piped_kernel" in names[0]) == piped, names
+
+
 @pytest.mark.parametrize("batch, m, n, k", [(1, 70000, 96, 24), (2055, 45, 16, 120), (600, 128, 64, 40)])
 def test_piped_packed_kernel_reports_a_timeout_and_keeps_infinities_apart(batch, m, n, k):
     """One B and many, several units per CTA and one."""
