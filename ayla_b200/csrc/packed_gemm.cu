@@ -571,7 +571,7 @@ struct Footprint {
   int stages, piped_smem, piped_ctas, piped_tmem_cols;
 };
 
-// Where the piped kernel is the faster one (350 shapes timed on both; over the 67 of the packed kernel's that it takes, 0.911
+// Where the piped kernel is the faster one (350 shapes timed on both; over the 64 of the packed kernel's that it takes, 0.914
 // of the time, the slowest 1.04): with rows that start inside a 32-byte sector and one B for all units, whose loads take
 // longest (247747x48x24 18.5 -> 14.0, 33392x64x24 6.7 -> 5.7); otherwise where an SM would hold two CTAs of the other or
 // fewer, which leaves a unit's chain bare (204363x40x88 17.0 -> 14.9), and every CTA has a unit at least (36745x32x128, 288
