@@ -791,27 +791,25 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (issuer && mine) {
           const uint32_t full_bar = full_bar0 + stage * 8;
           const int blocks = min(group, w.kb1 - kb);  // a unit may end in the middle of a slot
-          {
-            if (is_leader) mbar_arrive_expect_tx(bar_full + stage * 8, p.stage_tx * static_cast<uint32_t>(blocks));
+          if (is_leader) mbar_arrive_expect_tx(bar_full + stage * 8, p.stage_tx * static_cast<uint32_t>(blocks));
 #pragma unroll
-            for (int g = 0; g < group; ++g) {
-              if (g < blocks) {
-                const uint32_t sa = smem_base + stage * T::SLOT_BYTES + g * T::STAGE_BYTES;
-                const uint32_t sb = sa + T::A_BYTES;
-                const int k0 = (kb + g) * T::BK;
-                tma_load_3d<CG>(sa, &tm_a, full_bar, k0, w.m0, w.batch, pol_a);
-                // Rows [0, 64) of the slab = gate, [64, 128) = up.
-                if constexpr (T::SWIGLU_ROWS) tma_load_3d<CG>(sa + T::A_BYTES / 2, &tm_b2, full_bar, k0, w.m0, 0, pol_a);
-                if constexpr (T::SWIGLU_COLS && CG == 1) {
-                  // Accumulator columns [0,128) = gate, [128,256) = up.
-                  tma_load_3d<CG>(sb, &tm_b, full_bar, k0, b_row, 0, pol_b);
-                  tma_load_3d<CG>(sb + T::B_BYTES / 2, &tm_b2, full_bar, k0, b_row, 0, pol_b);
-                } else {
-                  // Pair + SwiGLU: the leader's half of the B tile is gate, the peer's half is up.
-                  tma_load_3d<CG>(sb, tm_b_mine, full_bar, k0, b_row, b_batch, pol_b);
-                }
-                if (pf > 0 && kb + g + pf < w.kb1) prefetch_l2(kb + g + pf);
+          for (int g = 0; g < group; ++g) {
+            if (g < blocks) {
+              const uint32_t sa = smem_base + stage * T::SLOT_BYTES + g * T::STAGE_BYTES;
+              const uint32_t sb = sa + T::A_BYTES;
+              const int k0 = (kb + g) * T::BK;
+              tma_load_3d<CG>(sa, &tm_a, full_bar, k0, w.m0, w.batch, pol_a);
+              // Rows [0, 64) of the slab = gate, [64, 128) = up.
+              if constexpr (T::SWIGLU_ROWS) tma_load_3d<CG>(sa + T::A_BYTES / 2, &tm_b2, full_bar, k0, w.m0, 0, pol_a);
+              if constexpr (T::SWIGLU_COLS && CG == 1) {
+                // Accumulator columns [0,128) = gate, [128,256) = up.
+                tma_load_3d<CG>(sb, &tm_b, full_bar, k0, b_row, 0, pol_b);
+                tma_load_3d<CG>(sb + T::B_BYTES / 2, &tm_b2, full_bar, k0, b_row, 0, pol_b);
+              } else {
+                // Pair + SwiGLU: the leader's half of the B tile is gate, the peer's half is up.
+                tma_load_3d<CG>(sb, tm_b_mine, full_bar, k0, b_row, b_batch, pol_b);
               }
+              if (pf > 0 && kb + g + pf < w.kb1) prefetch_l2(kb + g + pf);
             }
           }
         }
@@ -887,15 +885,13 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             // 16-byte address units.
             const uint32_t slot_off = stage * (T::SLOT_BYTES >> 4);
             const int blocks = min(group, nkb - i);  // a unit may end in the middle of a slot
-            {
 #pragma unroll
-              for (int g = 0; g < group; ++g) {
-                if (g < blocks) {
+            for (int g = 0; g < group; ++g) {
+              if (g < blocks) {
 #pragma unroll
-                  for (int k4 = 0; k4 < T::BK / 16; ++k4) {
-                    const uint32_t off = slot_off + g * (T::STAGE_BYTES >> 4) + 2 * k4;
-                    umma_f16<CG>(tmem_d, desc_a0 + off, desc_b0 + off, unit_idesc, (i + g > 0 || k4 > 0) ? 1u : 0u);
-                  }
+                for (int k4 = 0; k4 < T::BK / 16; ++k4) {
+                  const uint32_t off = slot_off + g * (T::STAGE_BYTES >> 4) + 2 * k4;
+                  umma_f16<CG>(tmem_d, desc_a0 + off, desc_b0 + off, unit_idesc, (i + g > 0 || k4 > 0) ? 1u : 0u);
                 }
               }
             }

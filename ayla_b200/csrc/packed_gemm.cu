@@ -10,16 +10,16 @@
 //    along and dropped, a tcgen05.mma of 128 rows takes the same 39 cycles up to 32 columns);
 //  * operands come through cp.async in 16-byte pieces, which read the contiguous rows as one stream whatever
 //    their length and put each piece where the swizzle wants it;
-//  * the accumulator leaves through shared memory as one contiguous run of 16-byte pieces;
-//  * two to four CTAs share an SM and hide each other's waits; inside one, the next unit's loads run under the
-//    MMAs and the epilogue.
-// us per launch (graph replay, operands past L2), general kernel -> this one: bmm 8192 x 56x32x56 45.9 -> 22.4
-// (110 MB: 16.8 at the copy peak), 8192 x 16x16x16 44.9 -> 7.1, mm 200704x96x24 37.3 -> 16.3 (7.4 at the peak),
-// 153718x32x16 18.5 -> 6.2.  What is left is latency: with two or three units per CTA a unit takes some 5000 cycles
-// from its load to its last store, over half of them in the epilogue's chain of TMEM load, conversion, staging and
-// copy.  Measured and left out: 256 threads per CTA (bmm 22.4 -> 35.8), a third ring slot (25.6, it costs a resident
-// CTA), two accumulators per CTA with the MMAs of a unit under the epilogue of the one before (25.5: half the CTAs
-// find room in TMEM).
+//  * the accumulator leaves through shared memory as one contiguous run of 16-byte pieces.
+// Two kernels do this.  In the chained one two to four CTAs share an SM and hide each other's waits; inside one, the next
+// unit's loads run under the MMAs and the epilogue.  In the piped one, for units too large for that (piped_pays), the
+// stages overlap inside a CTA.
+// us per launch (graph replay, operands past L2), general kernel -> this: chained, bmm 8192 x 56x32x56 45.9 -> 22.4
+// (110 MB: 16.8 at the copy peak), 8192 x 16x16x16 44.9 -> 7.1, mm 153718x32x16 18.5 -> 6.2; piped, mm 200704x96x24 37.3 ->
+// 14.3 (chained 16.3, 7.4 at the peak).  What is left is latency: in the chained form a unit takes some 5000 cycles from its
+// load to its last store, over half of them in the epilogue's chain of TMEM load, conversion, staging and copy.  Measured
+// and left out there: 256 threads per CTA (bmm 22.4 -> 35.8), a third ring slot (25.6, it costs a resident CTA), two
+// accumulators per CTA (25.5: half the CTAs find room in TMEM).
 #include "packed_gemm.h"
 
 #include <cuda_bf16.h>
@@ -30,15 +30,15 @@
 namespace ayla_b200 {
 namespace {
 
-constexpr int kThreads = 128;     // a warp per quarter of the accumulator's rows
+constexpr int kThreads = 128;     // the chained kernel: a warp per quarter of the accumulator's rows
 constexpr int kStages = 2;
 constexpr int kMaxCtasPerSm = 4;  // each may hold 128 of the 512 TMEM columns
 constexpr int kRows = 128;        // accumulator rows
 
-// The piped kernel: a CTA of its own warps for the loads, the MMAs and the epilogue.
+// The piped kernel: warps of its own for the epilogue (one per quarter), the loads and the MMAs.
+constexpr int kEpilogueThreads = 128;
 constexpr int kLoadThreads = 128;
-constexpr int kEpilogueSets = 1;   // of four warps; a set takes every other unit
-constexpr int kPipedThreads = kEpilogueSets * 128 + kLoadThreads + 32;
+constexpr int kPipedThreads = kEpilogueThreads + kLoadThreads + 32;
 constexpr int kPipedMaxStages = 4;
 constexpr int kPipedCtasPerSm = 2;
 constexpr int kAccs = 2;              // accumulators in TMEM: the MMAs of a unit run under the epilogue of the one before
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
   const int b_copies = p.shared_b ? 1 : p.stages;
   uint8_t* smem_b = packed_smem + p.stages * a_bytes;
   uint8_t* smem_staging = smem_b + b_copies * b_bytes;
-  float* smem_bias = reinterpret_cast<float*>(smem_staging + kEpilogueSets * kRows * p.staging_pitch);
+  float* smem_bias = reinterpret_cast<float*>(smem_staging + kRows * p.staging_pitch);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_bias + kPackedMaxN);
   // full[kPipedMaxStages], empty[kPipedMaxStages], acc_full[kAccs], acc_empty[kAccs]
   const uint32_t bar_full = smem_u32(bars);
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-  constexpr int kFirstLoadWarp = kEpilogueSets * 4, kMmaWarp = kFirstLoadWarp + kLoadThreads / 32;
+  constexpr int kFirstLoadWarp = kEpilogueThreads / 32, kMmaWarp = kFirstLoadWarp + kLoadThreads / 32;
   const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
 
   if (threadIdx.x == 0) {
@@ -527,11 +527,10 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
     grid_dependency_wait();
     if (p.bias != nullptr) {
       if (static_cast<int>(threadIdx.x) < p.n) smem_bias[threadIdx.x] = load_elem(p.bias, threadIdx.x, BF16 ? 1 : 0);
-      named_bar_sync(1, kEpilogueSets * 128);
+      named_bar_sync(1, kEpilogueThreads);
     }
-    const int set = warp >> 2;
-    const UnitWriter<BF16> writer(p, warp & 3, lane, smem_staging + set * kRows * p.staging_pitch, smem_bias);
-    for (int i = set; i < count; i += kEpilogueSets) {
+    const UnitWriter<BF16> writer(p, warp, lane, smem_staging, smem_bias);
+    for (int i = 0; i < count; ++i) {
       const uint32_t acc = static_cast<uint32_t>(i) & 1u, acc_phase = (static_cast<uint32_t>(i) >> 1) & 1u;
       bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL);
       // TMEM is read by whole warps: a wait that ran out for some lanes ends the unit for all.
@@ -599,7 +598,7 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
   // Two CTAs, or one, and then as many ring slots as still fit.
   const bool shared_b = batch == 1;
   auto piped_smem = [&](int stages) {
-    return stages * a_bytes + (shared_b ? 1 : stages) * b_bytes + kEpilogueSets * kRows * f.staging_pitch + kPackedMaxN * 4 + 128;
+    return stages * a_bytes + (shared_b ? 1 : stages) * b_bytes + kRows * f.staging_pitch + kPackedMaxN * 4 + 128;
   };
   f.piped_tmem_cols = 32;
   while (f.piped_tmem_cols < kAccs * f.mma_n) f.piped_tmem_cols *= 2;
@@ -630,10 +629,11 @@ cudaError_t init_packed_gemm() {
   return cudaSuccess;
 }
 
-// Where this kernel is the faster one.  1606 shapes of up to 128 columns and a depth of up to 128 were timed on both
-// (graph replay, operands past L2): by this rule the geometric mean is 0.726 of the general kernel's time, 22 shapes
-// are slower by 3 to 14 %, 20 that this kernel would do in less than 0.9 stay with the general one; choosing the
-// faster one every time would give 0.722.  What it goes by (us, general -> packed; or packed over general):
+// Where these kernels are faster than the general one.  The edges come from 1606 shapes of up to 128 columns and a depth of
+// up to 128, timed with the chained form alone (0.726 of the general kernel's time).  With the form that runs now, over 350
+// others: 276 are taken, in 0.575 of the time, five of them slower by 4 to 20 % (285 x 422x128x32 10.4 -> 12.1); of the 74
+// left, 28 would take less than 0.9, most of them piped with one or two CTAs per SM (103219x88x80 16.9, 11.1 piped).
+// What it goes by (us, general -> chained; or chained over general):
 //  * a 128-row tile for every SM; below, both are a launch and one pass (bmm 8 x 1024x64x64 2.8 -> 3.5).
 //  * Small matrices that share an accumulator gain most (1024 x 64x64x64 8.7 -> 7.3, 574 x 15x16x32 5.4 -> 2.6), as
 //    long as two CTAs fit an SM or four matrices a unit (7467 x 17x48x104, one CTA: 42.5 -> 47.9).
