@@ -170,10 +170,12 @@ struct UnitWriter {
   uint32_t out_offset, out_step, out_wrap;
   mutable int matrix = 0, row0 = 0, rows = 0;
 
+  // `staging_`: the warp's own rows (their offset added up in here, the piped kernel took 15.5 us instead of 14.2 for mm
+  // 200704x96x24).
   __device__ UnitWriter(const PackedParams& p_, int quarter_, int lane_, uint8_t* staging_, const float* smem_bias_)
       : p(p_), quarter(quarter_), lane(lane_), my_matrix(quarter_ / (p_.slot_rows / 32)),
         my_row((quarter_ % (p_.slot_rows / 32)) * 32), n_chunks(p_.n >> 3),
-        staging(staging_ + quarter_ * 32 * p_.staging_pitch), smem_bias(smem_bias_) {
+        staging(staging_), smem_bias(smem_bias_) {
     const int out_row = p.div_n_chunks.div(lane), out_row_step = p.div_n_chunks.div(32);
     out_c = lane - out_row * n_chunks;
     out_c_step = 32 - out_row_step * n_chunks;
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
     }
     cp_async_commit();
   };
-  const UnitWriter<BF16> writer(p, warp, lane, smem_staging, smem_bias);
+  const UnitWriter<BF16> writer(p, warp, lane, smem_staging + warp * 32 * p.staging_pitch, smem_bias);
   auto epilogue = [&](int i) {
     if (!writer.locate(first + i * stride)) return;
     writer.stage(tmem_base);
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
       if (static_cast<int>(threadIdx.x) < p.n) smem_bias[threadIdx.x] = load_elem(p.bias, threadIdx.x, BF16 ? 1 : 0);
       named_bar_sync(1, kEpilogueThreads);
     }
-    const UnitWriter<BF16> writer(p, warp, lane, smem_staging, smem_bias);
+    const UnitWriter<BF16> writer(p, warp, lane, smem_staging + warp * 32 * p.staging_pitch, smem_bias);
     for (int i = 0; i < count; ++i) {
       const uint32_t acc = static_cast<uint32_t>(i) & 1u, acc_phase = (static_cast<uint32_t>(i) >> 1) & 1u;
       bw.wait(bar_acc_full + acc * 8, acc_phase, ST_TIMEOUT_ACC_FULL);
