@@ -445,7 +445,8 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   if (wave > units) grid = static_cast<int>(units * c.cta_group);
   plan->grid = grid;
   // At most one split unit per CTA, its last: those of a tile share its sum.  With more of them a CTA would wait for
-  // partials that it, or one that waits as well, has yet to compute; there the last arriver sums.
+  // partials that it, or one that waits as well, has yet to compute; there the last arriver sums.  (320 schedules timed
+  // both ways, two to sixteen splits: 0.74 of the last arriver's time, none slower; 0.99 to 0.78 with two.)
   if (plan->splits > 1 && split_from % wave == 0 && (tiles - split_from) * plan->splits <= wave && !transposed &&
       static_cast<int64_t>(plan->row_tiles) * (tile_n / 32) * 4 <= kMaxSplitKTiles) {
     const KernelEntry* shared =
@@ -661,7 +662,8 @@ void default_config(int64_t batch, int64_t m, int64_t n, int64_t k, int activati
 // Microseconds that a product without an activation takes where its units run in one wave: a launch, then k-blocks at a
 // rate that falls with the share of the SMs at work, then, for a split depth, the sum.  Fitted to 2600 timings of 310
 // shapes (tile widths of 192 between their neighbours), median error 4 %; k-blocks of rows that start inside a 32-byte
-// sector take about 1.35 times as long.
+// sector take about 1.35 times as long.  One rate per tile stands for all depths: 256-wide pairs split four ways take 0.31
+// us a k-block from 4096 to 8192 deep at 1024x1024 and 0.49 from there to 16384, the model 0.38.
 struct Rate { double launch, block, block_busy, per_split; };
 enum { RATE_WHOLE = 0, RATE_SHARED = 1, RATE_CLUSTER = 2 };
 double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tiles, int64_t k, const Machine& machine) {
@@ -685,8 +687,9 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 // What a schedule measured elsewhere, or here by bursts, is corrected in.
 //
 // Shallow products of 256-wide tiles become pairs where no rows are padded: they read B half as often, and under the
-// power cap, which a burst does not reach, that is time (bmm 64 x 2048x2048x128 121.9 -> 110.9, 106 x 1872x1456x96 152.7 ->
-// 142.1, 35 x 1219x1960x128 50.0 -> 45.4; of one k-block they do not gain: 55 x 2043x1208x64 80.1 -> 81.1).
+// power cap, which a burst does not reach, that is time (us per call, bmm 64 x 2048x2048x128 133.2 -> 122.7, 106 x
+// 1872x1456x96 152.7 -> 142.1, 35 x 1219x1960x128 50.0 -> 45.4; of one k-block they do not gain: 55 x 2043x1208x64 80.1 ->
+// 81.1).
 //
 // Splits the depth where a row-major schedule leaves SMs idle through a long product: the CTAs of a tile share its sum
 // (see the kernel), so any number of them may work on it.  Two places:
@@ -696,7 +699,7 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 2129x4608x5248, 2 + 14/74, 84 -> 80 -> 77 with 5; but
 //    4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
 //    Rows that start inside a sector are bound by their loads, which a lone pair gets faster: two ways at most
-//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6), behind one whole wave (25 shapes, 0.80 to 0.96 of the time
+//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6; in calls one after another 210 -> 200), behind one whole wave (25 shapes, 0.80 to 0.96 of the time
 //    whole), behind two with a quarter of a wave left (3766x2624x14424, 2 + 17/74, 373 -> 407 -> 356), or where a
 //    schedule has halves (45 shapes of two waves and more, 0.88 to 1.07 of the time in halves, mostly below 0.98);
 //    elsewhere whole tiles stay (4846x3968x12696, 4 + 8/74, 476 -> 561; 6658x2304x12136, 3 + 21/74, 384 -> 431).
@@ -707,7 +710,7 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    halves: 154 take them by this, the geometric mean is 0.963 of the time, three are slower, by 4 to 5 %.
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
 //    take 0.97 of the time for pairs and a deep product, 0.9 otherwise (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29,
-//    175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 -> 18.0, 1024x1024x8192 24.1 -> 22.5; by less than that others lose:
+//    175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 -> 18.0, 1024x1024x8192 23.8 -> 22.4; by less than that others lose:
 //    128x4096x4096 12.1 -> 13.5, 433x1280x3584 with row factors 12.9 -> 13.7).  Not 0.97 where the pairs pad a row tile
 //    that single CTAs did not (296x1088x14016 22.6 -> 24.2, 288x576x37248 36.8 -> 40.2), 0.85 for short products whose
 //    rows start inside a sector (332x960x2568 11.8 -> 12.6), and never single CTAs for pairs there, which read B twice as

@@ -211,11 +211,12 @@ struct GemmTraits {
   // One staging box per warp; at 256 columns the sixteen of them cost a ring slot.
   static constexpr bool GATED = GATED_;
   // PAIRED (ACT_ 2): sixteen epilogue warps, two to a 64-column group and lane quarter, one staging box between them.
-  // For the activations that are more than a comparison: a GELU takes 4000 cycles of an SM's multiply-adds per 128 x 256 tile, and with eight warps they came
-  // on top of the 5000 that loads from TMEM, staging and stores take; with sixteen they run under them.  us per launch,
-  // eight -> sixteen: addmm 12095x5824x256 + GELU fp16 81.4 -> 78.3, mm 16384x2048x512 + SiLU 44.3 -> 42.6, addmm
-  // 8192x3072x768 + GELU 45.3 -> 44.1 (the power cap takes back more than half of the cycles saved).  Without one
-  // there is nothing to hide (bmm 54x553x1880x64 31.0 -> 32.2, mm 2589x6016x320 15.2 -> 15.7).
+  // For the activations that are more than a comparison: a GELU takes 4000 cycles of an SM's multiply-adds per 128 x 256
+  // tile, and with eight warps they came on top of the 5000 that loads from TMEM, staging and stores take; with sixteen
+  // they run under them.  us per call, eight -> sixteen: addmm 12095x5824x256 + GELU fp16 80.8 -> 77.9, 15000x1000x320
+  // 21.5 -> 20.8, 16384x2048x512 + SiLU 46.2 -> 45.0, 512x4096x1024 + SiLU 9.0 -> 8.8; nothing where the MMAs or the power
+  // cap set the pace (8192x3072x768 + GELU 45.8 -> 45.4 and 2048x8192x2048 63.7 -> 63.8, within the noise).  Without an
+  // activation there is nothing to hide (bmm 54x553x1880x64 31.0 -> 32.2, mm 2589x6016x320 15.2 -> 15.7).
   static constexpr bool PAIRED = ACT_ == 2;
   static constexpr int EPI_WARPS = GATED ? BN / 16 : PAIRED ? 16 : 8;
   static constexpr int STORE_BUF_BYTES = 32 * 128;  // 32 rows x 64 columns of 16-bit
