@@ -1334,6 +1334,31 @@ def test_timed_out_split_k_launch_is_reported_by_the_next_call_without_the_debug
 
 
 @pytest.mark.parametrize("config", [
+    dict(tile_n=128, cta_group=1, split_k=4), dict(tile_n=256, cta_group=2, split_k=3),  # the shared sum
+    dict(tile_n=64, cta_group=1, split_k=3, grid_ctas=6)])                               # the last arriver's
+def test_timed_out_k_splits_leave_their_counters_at_zero(config, device_state):
+    """Nobody can clear the workspace of a captured launch: the launch after one whose waits ran out finds it clean."""
+    m, n, k = 500, 520, 2048
+    g = torch.Generator().manual_seed(6)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+    lib = _lib.load()
+    assert _lib.workspace_bytes(_lib.Config.from_dict(config), "mm", 1, m, n, k) > 0
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(20)
+        lib.ayla_b200_debug_set_flags(1)
+        _, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    assert status & 0xFF != 0
+    assert not bool(device_state[1][:65536].any())
+    out, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    assert status == 0
+    assert_parity(out, O.mm_ref32(a, bt), f"after a timed-out k-split {config}")
+
+
+@pytest.mark.parametrize("config", [
     dict(tile_n=64, cta_group=1, split_k=2), dict(tile_n=128, cta_group=1, split_k=4),
     dict(tile_n=64, cta_group=2, split_k=2), dict(tile_n=16, cta_group=1, swap_ab=1, split_k=4, group_m=1)])
 def test_timed_out_cluster_split_leaves_the_context_usable(config, device_state):
