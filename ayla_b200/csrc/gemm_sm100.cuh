@@ -95,7 +95,7 @@ struct KernelParams {
   int group_m;        // raster: m-tiles per group
   int is_bf16;        // output / operand type: 1 bf16, 0 fp16
   uint32_t idesc;     // tcgen05 instruction descriptor
-  uint32_t l2_hint_a; // 0 normal, 1 evict_first, 2 evict_last
+  uint32_t l2_hint_a; // 0 none, 1 evict_first, 2 evict_last
   uint32_t l2_hint_b;
   const void* bias;   // [n] (or [m] when the output is transposed)
   void* out;          // used by the direct-store epilogues
@@ -559,10 +559,11 @@ __device__ __forceinline__ void apply_act_chunk(float (&v)[N], int act) {
   }
 }
 
+// 0 for no hint.
 __device__ __forceinline__ uint64_t make_policy(uint32_t hint) {
   if (hint == 1) return policy_evict_first();
   if (hint == 2) return policy_evict_last();
-  return policy_evict_normal();
+  return 0;
 }
 
 template <class T>
@@ -968,7 +969,6 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     uint32_t bias_buf = 0;
     uint32_t gate_phase = 0;
     const uint32_t my_gate_bar = bar_gate + (warp - 2) * 8;
-    const uint64_t gate_policy = make_policy(0);
     constexpr int CHUNKS32 = T::OUT_BN / 32 > 0 ? T::OUT_BN / 32 : 1;  // 32-column chunks
     constexpr int CHUNK_COLS = T::OUT_BN < 32 ? T::OUT_BN : 32;
     constexpr int EPI_THREADS = T::EPI_WARPS * 32;
@@ -1033,7 +1033,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       if (gate_live && lane == 0 && !bw.aborted()) {
         tma_store_wait_read<0>();
         mbar_arrive_expect_tx(my_gate_bar, T::STORE_BUF_BYTES);
-        tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, gate_policy);
+        tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, 0);
       }
 
       // One factor per output row: read while the MMAs run.

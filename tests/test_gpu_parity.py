@@ -159,6 +159,23 @@ def test_row_major_variants(tile_n, cta_group, split_k, dtype, device_state):
         assert_parity(out, O.gemm_ref32(operation, *tensors), f"{operation} {batch}x{m}x{n}x{k} {cfg}")
 
 
+@pytest.mark.parametrize("cta_group", [1, 2])
+@pytest.mark.parametrize("k", [1024, 1016, 1000])  # rows of whole lines, starting inside a line, inside a sector
+def test_cache_hints_change_no_bit(cta_group, k, device_state):
+    g = torch.Generator().manual_seed(k)
+    a = torch.randn(520, k, generator=g).bfloat16()
+    bt = (torch.randn(264, k, generator=g) * k ** -0.5).bfloat16()
+    outs = []
+    for hint_a in (0, 1, 2):
+        for hint_b in (0, 1, 2):
+            cfg = dict(tile_n=128, cta_group=cta_group, l2_hint_a=hint_a, l2_hint_b=hint_b)
+            out, status = run_abi("mm", "bfloat16", (a, bt), cfg, device_state)
+            assert status == 0
+            outs.append(out)
+    assert_parity(outs[0], O.mm_ref32(a, bt))
+    assert all(torch.equal(outs[0], out) for out in outs)
+
+
 # (batch, m, n, k): one tile and several, extents inside a chunk and a lane quarter, depths that the splits do not share
 # evenly; the last three fill whole waves first and split the depth of the tiles left over.
 @pytest.mark.parametrize("batch, m, n, k, config", [
