@@ -33,6 +33,7 @@ EXPORTS = (
     "ayla_b200_default_config",
     "ayla_b200_default_config_act",
     "ayla_b200_share_depth",
+    "ayla_b200_fit_depth",
     "ayla_b200_swiglu_default_config",
     "ayla_b200_config_valid",
     "ayla_b200_workspace_bytes",
@@ -146,6 +147,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_default_config_act.restype = i32
         lib.ayla_b200_share_depth.argtypes = [i32, i32, i64, i64, i64, i64, cfgp]
         lib.ayla_b200_share_depth.restype = i32
+        lib.ayla_b200_fit_depth.argtypes = [i32, i32, i64, i64, i64, i64, cfgp]
+        lib.ayla_b200_fit_depth.restype = i32
         lib.ayla_b200_swiglu_default_config.argtypes = [i32, i64, i64, i64, cfgp]
         lib.ayla_b200_swiglu_default_config.restype = i32
         lib.ayla_b200_config_valid.argtypes = [cfgp, i32, i32, i64, i64, i64, i64]
@@ -251,6 +254,13 @@ def share_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k:
     """``cfg``, or what it becomes where splitting the depth shares out SMs that it leaves idle."""
     out = Config.from_dict(cfg.to_dict())
     check(load().ayla_b200_share_depth(OP_CODES[op], DTYPE_CODES[dtype], batch, m, n, k, ctypes.byref(out)))
+    return out
+
+
+def fit_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k: int) -> Config:
+    """As ``share_depth``, and last waves whose rows start inside a sector are split like any others."""
+    out = Config.from_dict(cfg.to_dict())
+    check(load().ayla_b200_fit_depth(OP_CODES[op], DTYPE_CODES[dtype], batch, m, n, k, ctypes.byref(out)))
     return out
 
 

@@ -693,21 +693,16 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //
 // Splits the depth where a row-major schedule leaves SMs idle through a long product: the CTAs of a tile share its sum
 // (see the kernel), so any number of them may work on it.  Two places:
-//  * The last, partial wave of tiles.  Splitting its tiles S ways takes 1/S of a tile's time and some 7 us for the sum
-//    instead of a whole tile's time, or three quarters of it where its tiles run at half width (us, whole -> half ->
-//    split: 2744x2112x29248, 1 + 25/74 waves, 332 -> 316 -> 266 with 2; 3024x1856x11776, 1 + 22/74, 120 -> 116 -> 104
-//    with 3; 4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; 2129x4608x5248, 2 + 14/74, 84 -> 80 -> 77 with 5; but
-//    4096x6144x4096, 5 + 14/74, 152 -> 152 -> 152 with 5).
-//    Rows that start inside a sector are bound by their loads, which a lone pair gets faster: two ways at most
-//    (4096x2560x8008 188 -> 199 -> 180 with 2, 191 with 6; in calls one after another 210 -> 200), behind one whole wave (25 shapes, 0.80 to 0.96 of the time
-//    whole), behind two with a quarter of a wave left (3766x2624x14424, 2 + 17/74, 373 -> 407 -> 356), or where a
-//    schedule has halves (45 shapes of two waves and more, 0.88 to 1.07 of the time in halves, mostly below 0.98);
-//    elsewhere whole tiles stay (4846x3968x12696, 4 + 8/74, 476 -> 561; 6658x2304x12136, 3 + 21/74, 384 -> 431).
-//    Otherwise half width wherever two halves fit (1260x4480x768 12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; rows inside
-//    a sector: 4096x2560x8008, 7960x312x616 11.8 -> 12.2), in shallow products where the rest is below three tenths of
-//    a wave: there the results that the SMs write set the pace, not their number (bmm 71 x 324x128x272, 0.44 waves, 8.3 ->
-//    8.8; mm 4546x1408x256, 0.46, 7.5 -> 7.8; but 3266x1600x512, 0.23, 9.7 -> 8.6).  192 shapes timed with whole tiles and
-//    halves: 154 take them by this, the geometric mean is 0.963 of the time, three are slower, by 4 to 5 %.
+//  * The last, partial wave of tiles, see last_wave: its tiles whole, as two halves each, or split S ways (us, whole -> half
+//    -> split: 2744x2112x29248, 1 + 25/74 waves, 332 -> 316 -> 266 with 2; 4156x1088x3712, 1 + 11/74, 46 -> 40 -> 34 with 6;
+//    4451x2240x7040, 2 + 14/74, 124 -> 112 -> 103 with 5; rows inside a sector: 1128x7488x7928, 2 + 2/74, 176 -> 175 ->
+//    139 with 6; 3915x1088x5032, 1 + 6/74, 70 -> 70 -> 52 with 8).
+//    Otherwise half width where two halves fit (1260x4480x768 12.0 -> 10.6, 1221x4160x1728 21.5 -> 18.8; nothing with rows
+//    inside a sector), in shallow products where the rest is below three tenths of a wave: there the results that the SMs
+//    write set the pace, not their number (bmm 71 x 324x128x272, 0.44 waves, 8.3 -> 8.8; mm 4546x1408x256, 0.46, 7.5 -> 7.8;
+//    but 3266x1600x512, 0.23, 9.7 -> 8.6).  192 shapes timed with whole tiles and halves: 154 take them by this, the
+//    geometric mean is 0.963 of the time, three are slower, by 4 to 5 %.  Where two do not fit, halves take two rounds:
+//    whole instead (37 shapes, 0.74 to 1.0 of the time, all but three below 0.97: 1647x7520x1352, 2 + 62/74, 47 -> 37).
 //  * A single wave with SMs to spare, or with clusters that do not all run at once.  By the model the shared sum has to
 //    take 0.97 of the time for pairs and a deep product, 0.9 otherwise (536x896x59968 132 -> 67, 1064x192x38720 53 -> 29,
 //    175x2304x8000 28.7 -> 16.2, 1896x320x8576 23.0 -> 18.0, 1024x1024x8192 23.8 -> 22.4; by less than that others lose:
@@ -716,7 +711,38 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    rows start inside a sector (332x960x2568 11.8 -> 12.6), and never single CTAs for pairs there, which read B twice as
 //    often (524x3200x13656 88 -> 99).  Over 191 shapes that are split by these bounds it takes 0.81 of the time, the slowest
 //    1.02.
-void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+// Microseconds that a product of more than one wave of 128- to 256-wide tiles takes, launch aside, and the number of ways its
+// last wave's tiles are best split (1: not at all).  A k-block of 256-wide pairs takes 0.39 us, of 192 and 128 columns 0.87
+// and 0.72 of that; tiles of half the width two thirds of a whole one's time, as long as it where rows start inside a
+// sector; the sum of S parts 4.8 us (5.8 of 192 columns) and 0.4 per part.  Fitted to 330 timings of 110 shapes.  A split has to
+// gain 1 us, and 4.5 % or 3 us, by this (by 3.5 %: addmm 640x8160x3968, 1 + 22/74, halves 43.9 -> 47.0 with 3; not without the
+// 3 us: 8071x2944x4480, 5 + 14/74, split five ways 171 -> halves 189).  Of 1000 shapes drawn over all kinds 61 get another
+// schedule than by the bounds before, half of them whole tiles for halves that did not fit; they take 0.91 of the time.
+struct LastWave { double us; int splits; };
+LastWave last_wave(int64_t tiles, int64_t wave, int64_t k, int tile_n) {
+  const int64_t k_blocks = ceil_div(k, 64), whole = tiles / wave, rest = tiles % wave;
+  const double tile = static_cast<double>(k_blocks) * (tile_n == 256 ? 0.39 : tile_n == 192 ? 0.34 : 0.28);
+  LastWave best{static_cast<double>(whole) * tile, 1};
+  if (rest == 0) return best;
+  const double unsplit = tile_n % 128 == 0 && rest * 2 <= wave && k % 16 == 0 ? 0.66 * tile : tile;
+  const double bound = 0.045 * static_cast<double>(whole + 1) * tile;
+  const double sum = tile_n == 192 ? 5.8 : 4.8;
+  double least = unsplit - (bound > 3.0 ? 3.0 : bound > 1.0 ? bound : 1.0);
+  double last = unsplit;
+  for (int s = 2; s <= 16 && s * rest <= wave && s * 5 <= k_blocks; ++s) {
+    const double us = tile / s + sum + 0.4 * s;
+    if (us >= least) continue;
+    least = last = us;
+    best.splits = s;
+  }
+  best.us += last;
+  return best;
+}
+
+//
+// `cautious`: ayla_b200_share_depth keeps the bounds that it has for last waves whose rows start inside a sector: two ways at
+// most, behind one whole wave, behind two with a quarter of a wave left, or where the schedule has halves.
+void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, bool cautious, ayla_b200_config* c) {
   if (c->swap_ab || c->stream_k || c->grid_ctas != 0 || c->split_tail == 1) return;
   if (c->split_k > 1 && !c->cluster_split && c->split_tail != 0) return;
   const int64_t k_blocks = ceil_div(k, 64);
@@ -727,26 +753,41 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
     c->split_tail = 0;
   }
   const int64_t wave = machine.sm_count / c->cta_group;
-  const int64_t tiles = batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n);
+  int64_t tiles = batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n);
   if (tiles > wave) {
-    const int64_t rest = tiles % wave;
-    if (c->split_k > 1 || c->cluster_split || rest == 0) return;
-    const bool halves_fit = c->tile_n % 128 == 0 && rest * 2 <= wave;
-    const bool lone = !mid_sector || tiles < 2 * wave || (tiles < 3 * wave && rest * 4 <= wave) || c->split_tail == 2;
-    if (c->tile_n >= 128 && rest * 2 <= wave && k_blocks >= 32 && lone) {
-      int64_t splits = wave / rest;
-      if (splits > k_blocks / 8) splits = k_blocks / 8;
-      if (splits > (mid_sector ? 2 : 16)) splits = mid_sector ? 2 : 16;
+    if (c->split_k > 1 || c->cluster_split || tiles % wave == 0 || c->tile_n < 128) return;
+    LastWave last = last_wave(tiles, wave, k, c->tile_n);
+    if (cautious && mid_sector) {
+      const int64_t rest = tiles % wave;
+      const bool lone = tiles < 2 * wave || (tiles < 3 * wave && rest * 4 <= wave) || c->split_tail == 2;
       const double block = c->tile_n == 256 ? 0.38 : c->tile_n == 192 ? 0.33 : 0.275;
-      const double now = mid_sector ? 0.7 : halves_fit ? 0.75 : 1.0;  // of a tile: a half runs at three quarters of the rate
-      if (splits >= 2 && static_cast<double>(k_blocks) * (now - 1.0 / static_cast<double>(splits)) * block >
-                             (mid_sector ? 8.5 : 14.0)) {
-        c->split_k = static_cast<int>(splits);
+      if (lone && rest * 2 <= wave && k_blocks >= 32 && static_cast<double>(k_blocks) * 0.2 * block > 8.5) {
+        c->split_k = 2;
         c->split_tail = 1;
-        return;
+      }
+      return;
+    }
+    if (c->tile_n == 192 && c->cta_group == 2) {
+      // 256-wide tiles may leave a thinner last wave, and a split one (2100x2368x7824 90 -> 67, 7328x640x5168 60 -> 50; by
+      // less than 7 % of the model's time the 192-wide ones stay: 6690x1408x3200 0.99, 53 -> 56).
+      const int64_t wider = batch * ceil_div(m, 256) * ceil_div(n, 256);
+      const LastWave there = wider > wave ? last_wave(wider, wave, k, 256) : last;
+      if (there.splits > 1 && there.us < 0.93 * last.us) {
+        c->tile_n = 256;
+        tiles = wider;
+        last = there;
       }
     }
-    if (halves_fit && !mid_sector && (k_blocks > 8 || rest * 10 <= wave * 3)) c->split_tail = 2;
+    const int64_t rest = tiles % wave;
+    const bool halves_fit = c->tile_n % 128 == 0 && rest * 2 <= wave;
+    if (last.splits > 1) {
+      c->split_k = last.splits;
+      c->split_tail = 1;
+    } else if (!halves_fit) {
+      c->split_tail = 0;
+    } else if (!mid_sector && (k_blocks > 8 || rest * 10 <= wave * 3)) {
+      c->split_tail = 2;
+    }
     return;
   }
   if (m <= 64 || k_blocks < 16) return;
@@ -1140,7 +1181,17 @@ int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n
   if (rc) return rc;
   rc = check_config(*cfg, false);
   if (rc) return rc;
-  share_depth(batch, m, n, k, current_machine(), cfg);
+  share_depth(batch, m, n, k, current_machine(), true, cfg);
+  return AYLA_B200_OK;
+}
+
+int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k, ayla_b200_config* cfg) {
+  if (cfg == nullptr) return fail(AYLA_B200_E_INVALID, "cfg is null");
+  int rc = check_shape(op, dtype, batch, m, n, k);
+  if (rc) return rc;
+  rc = check_config(*cfg, false);
+  if (rc) return rc;
+  share_depth(batch, m, n, k, current_machine(), false, cfg);
   return AYLA_B200_OK;
 }
 

@@ -146,10 +146,10 @@ def measured_gemm_configs(operation: str, dtype: str, m: int, n: int, k: int,
 
 def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int,
                   batch: int) -> GemmScheduleSeed | None:
-    """The schedule with its depth split where it leaves SMs idle (``ayla_b200_share_depth``)."""
+    """The schedule with its depth split where it leaves SMs idle (``ayla_b200_fit_depth``)."""
     if seed is None or seed.builder_config is None:
         return seed
-    shared = _lib.share_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
+    shared = _lib.fit_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
     if shared == seed.builder_config:
         return seed
     captured = {**seed.captured_config, **shared}

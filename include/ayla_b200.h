@@ -263,6 +263,11 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
 AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                         ayla_b200_config* cfg);
 
+/* The same, which splits last waves of operand rows that start inside a 32-byte sector (k % 16 != 0) like any others:
+ * ayla_b200_share_depth splits those two ways at most. */
+AYLA_B200_API int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
+                                      ayla_b200_config* cfg);
+
 /*
  * The schedule ayla_b200_swiglu uses when cfg == NULL: row-major (swap_ab == 0), or with the weights on the row
  * side (swap_ab == 1), a form that cannot be asked for by a cfg.

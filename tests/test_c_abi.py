@@ -196,6 +196,26 @@ def test_swiglu_of_few_rows_is_swapped_where_it_measured_faster(m, n, k, tile_n,
         assert (cfg.swap_ab, cfg.tile_n, cfg.split_k, cfg.cluster_split) == (1, tile_n, split, int(split > 1))
 
 
+# (m, n, k), tile width, the schedule's last wave -> width, splits and last wave that are fitted
+@pytest.mark.parametrize("shape, tile_n, tail, expected", [
+    ((4156, 1088, 3712), 256, 0, (256, 6, 1)),  # 1 + 11/74 waves of 58 k-blocks
+    ((783, 4672, 2368), 256, 0, (256, 1, 2)),  # 1 + 2/74 of 37: halves
+    ((1128, 7488, 7928), 256, 0, (256, 11, 1)),  # rows inside a sector
+    ((2920, 2568, 3832), 256, 2, (256, 1, 0)),  # 1 + 58/74: two halves of a tile do not fit
+    ((9874, 640, 832), 256, 2, (256, 1, 0)),
+    ((1260, 4480, 768), 256, 2, (256, 1, 2)),
+    ((7328, 640, 5168), 192, 0, (256, 5, 1)),  # a thinner last wave of wider tiles
+    ((6690, 1408, 3200), 192, 0, (192, 1, 0)),
+    ((4096, 4096, 4096), 256, 2, (256, 1, 2)),
+])
+def test_last_waves_are_fitted_by_their_length(shape, tile_n, tail, expected):
+    m, n, k = shape
+    cfg = _lib.Config.from_dict(dict(group_m=8, tile_n=tile_n, cta_group=2, split_k=1, split_tail=tail))
+    out = _lib.fit_depth(cfg, "mm", "bfloat16", 1, m, n, k)
+    assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
+    assert (out.tile_n, out.split_k, out.split_tail) == expected
+
+
 def test_depth_is_shared_where_sms_would_idle():
     def shared(m, n, k, **config):
         cfg = _lib.Config.from_dict(dict(group_m=8, **config))
