@@ -10,13 +10,13 @@
 //    along and dropped, a tcgen05.mma of 128 rows takes the same 39 cycles up to 32 columns);
 //  * operands come through cp.async in 16-byte pieces, which read the contiguous rows as one stream whatever
 //    their length and put each piece where the swizzle wants it;
-//  * the accumulator leaves through shared memory as one contiguous run of 16-byte pieces.
+//  * the accumulator leaves through shared memory as one contiguous run of 16-byte pieces, or row by row (writes_rows).
 // Two kernels do this.  In the chained one two to four CTAs share an SM and hide each other's waits; inside one, the next
 // unit's loads run under the MMAs and the epilogue.  In the piped one, for units too large for that (piped_pays), the
 // stages overlap inside a CTA.
 // us per launch (graph replay, operands past L2), general kernel -> this: chained, bmm 8192 x 56x32x56 45.9 -> 22.4
 // (110 MB: 16.8 at the copy peak), 8192 x 16x16x16 44.9 -> 7.1, mm 153718x32x16 18.5 -> 6.2; piped, mm 200704x96x24 37.3 ->
-// 14.3 (chained 16.3, 7.4 at the peak).  What is left is latency: in the chained form a unit takes some 5000 cycles from its
+// 13.4 (7.4 at the peak).  What is left is latency: in the chained form a unit takes some 5000 cycles from its
 // load to its last store, over half of them in the epilogue's chain of TMEM load, conversion, staging and copy.  Measured
 // and left out there: 256 threads per CTA (bmm 22.4 -> 35.8), a third ring slot (25.6, it costs a resident CTA), two
 // accumulators per CTA (25.5: half the CTAs find room in TMEM).
@@ -81,6 +81,12 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr)
+               : "memory");
+}
+
+__device__ __forceinline__ void store_32_bytes(void* dst, const uint32_t (&x)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(x[0]), "r"(x[1]), "r"(x[2]),
+               "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7])
                : "memory");
 }
 
@@ -158,7 +164,8 @@ struct UnitLoader {
   }
 };
 
-// A warp's share of one unit's results: a quarter of the accumulator's rows, through its staging rows into `out`.
+// A warp's share of one unit's results: a quarter of the accumulator's rows, through its staging rows into `out` or straight
+// (DIRECT kernels, see writes_rows).
 template <bool BF16>
 struct UnitWriter {
   const PackedParams& p;
@@ -233,6 +240,39 @@ struct UnitWriter {
     }
   }
 
+  // Without staging: each lane writes its row, two pieces (a 32-byte sector) an instruction.
+  __device__ __forceinline__ void write(uint32_t accumulator) const {
+    const uint32_t t = accumulator + (static_cast<uint32_t>(quarter * 32) << 16) +
+                       static_cast<uint32_t>(p.matrices > 1 ? my_matrix * p.n : 0);
+    uint8_t* dst = p.out + ((static_cast<size_t>(matrix) * p.m + row0 + lane) * n_chunks) * 16;
+    const bool mine = lane < rows;
+    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
+      uint32_t r[32];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c0 + j < n_chunks) tmem_ld_32x8(t + (c0 + j) * 8, r + 8 * j);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        if (c0 + j < n_chunks) {
+          uint32_t x[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            float lo = __uint_as_float(r[8 * j + 2 * e]), hi = __uint_as_float(r[8 * j + 2 * e + 1]);
+            if (p.bias != nullptr) {
+              const float2 b = *reinterpret_cast<const float2*>(smem_bias + (c0 + j) * 8 + 2 * e);
+              lo += b.x;
+              hi += b.y;
+            }
+            x[e] = pack_pair<BF16>(lo, hi);
+          }
+          if (mine) store_32_bytes(dst + (c0 + j) * 16, x);
+        }
+      }
+    }
+  }
+
   // The staged rows follow one another in `out` without a gap.
   __device__ __forceinline__ void copy_out() const {
     uint8_t* dst = p.out + ((static_cast<size_t>(matrix) * p.m + row0) * n_chunks + lane) * 16;
@@ -260,7 +300,7 @@ struct UnitWriter {
   }
 };
 
-template <bool BF16>
+template <bool BF16, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(const PackedParams p) {
 #if defined(__CUDA_ARCH_FEAT_SM100_ALL) || defined(__CUDA_ARCH_FEAT_SM101_ALL)
   extern __shared__ __align__(1024) uint8_t packed_smem[];
@@ -329,9 +369,13 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
   const UnitWriter<BF16> writer(p, warp, lane, smem_staging + warp * 32 * p.staging_pitch, smem_bias);
   auto epilogue = [&](int i) {
     if (!writer.locate(first + i * stride)) return;
-    writer.stage(tmem_base);
-    __syncwarp();
-    writer.copy_out();
+    if constexpr (DIRECT) {
+      writer.write(tmem_base);
+    } else {
+      writer.stage(tmem_base);
+      __syncwarp();
+      writer.copy_out();
+    }
   };
 
 #pragma unroll
@@ -389,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, kMaxCtasPerSm) packed_gemm_kernel(co
 // 8.8, 250000x128x40 25.7 -> 20.5, bmm 3000 x 128x64x40 21.3 -> 19.3, 5332 x 45x16x120 22.3 -> 18.9.  What is left is
 // the epilogue's chain (a second set of epilogue warps made no more than 3 %, or lost as much to its staging rows) and,
 // from 30 KB a unit on, the SM's store rate.
-template <bool BF16>
+template <bool BF16, bool DIRECT>
 __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_kernel(const PackedParams p) {
 #if defined(__CUDA_ARCH_FEAT_SM100_ALL) || defined(__CUDA_ARCH_FEAT_SM101_ALL)
   extern __shared__ __align__(1024) uint8_t packed_smem[];
@@ -539,12 +583,20 @@ __global__ void __launch_bounds__(kPipedThreads, kPipedCtasPerSm) packed_piped_k
       const bool aborted = __any_sync(0xffffffffu, bw.aborted());
       tc_fence_after_sync();
       const bool live = writer.locate(first + i * stride) && !aborted;
-      if (live) writer.stage(tmem_base + acc * static_cast<uint32_t>(p.mma_n));
+      if (live) {
+        if constexpr (DIRECT) {
+          writer.write(tmem_base + acc * static_cast<uint32_t>(p.mma_n));
+        } else {
+          writer.stage(tmem_base + acc * static_cast<uint32_t>(p.mma_n));
+        }
+      }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_acc_empty + acc * 8);
-      if (live) writer.copy_out();
-      __syncwarp();  // the staging rows are free again
+      if constexpr (!DIRECT) {
+        if (live) writer.copy_out();
+        __syncwarp();  // the staging rows are free again
+      }
     }
   }
 
@@ -568,6 +620,7 @@ struct Footprint {
   int mma_n, narrow, k_blocks;
   int staging_pitch;
   int smem, ctas;
+  int64_t units;
   bool piped;     // the piped kernel
   int stages, piped_smem, piped_ctas, piped_tmem_cols;
 };
@@ -583,7 +636,21 @@ bool piped_pays(int64_t units, int64_t k, bool shared_b, int chained_ctas) {
   return chained_ctas <= 2 && units >= 300;
 }
 
-Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
+// Where the lanes write their rows themselves, without staging: rows of whole sectors, but not of whole lines, whose stores
+// meet in one another's way.  What it saves is the way through shared memory, and its rows there, which makes room for more
+// CTAs.  Over 140 shapes of 16 to 112 columns timed both ways it takes 0.90 of the time (us, staged -> direct: mm 200704x96x24
+// 14.6 -> 13.7, 262144x48x32 11.7 -> 8.9, bmm 3194 x 13x80x112 25.6 -> 16.8, 8149 x 32x48x8 12.3 -> 10.8); of 64 and 128
+// columns 1.0 to 1.2 (mm 121018x64x32 7.0 -> 8.3).  Rows of 64 bytes are half lines, which only shallow products make up for
+// (bmm 2500 x 100x32x32 10.0 -> 9.0, x40 10.6 -> 11.1, x56 12.5 -> 13.5, 8192 x 56x32x56 21.1 -> 21.8), and those of 192 are a
+// line and a half (bmm 2500 x 100x96x56 20.4 -> 21.5, x40 18.1 -> 18.5; with one B or another depth they gain).
+bool writes_rows(int64_t n, int64_t k, bool shared_b) {
+  if (n % 16 != 0 || n % 64 == 0) return false;
+  if (n == 32) return k <= 32;
+  return n != 96 || shared_b || k <= 32 || k > 64;
+}
+
+// `staged`: with room for the results on their way out.
+Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k, bool staged = true) {
   Footprint f;
   f.matrices = 1;
   while (batch > 1 && f.matrices < 4 && m * f.matrices * 2 <= kRows && n * f.matrices * 2 <= kPackedMaxN) f.matrices *= 2;
@@ -591,7 +658,7 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
   f.narrow = k <= 16 ? 2 : k <= 32 ? 1 : 0;
   f.k_blocks = static_cast<int>((k + 63) / 64);
   // An odd number of 16-byte pieces per staging row: eight lanes writing a piece of eight rows meet eight banks.
-  f.staging_pitch = 16 * static_cast<int>((n / 8) | 1);
+  f.staging_pitch = staged ? 16 * static_cast<int>((n / 8) | 1) : 0;
   const int a_bytes = (f.k_blocks * kRows * 128) >> f.narrow, b_bytes = (f.k_blocks * f.mma_n * 128) >> f.narrow;
   f.smem = kStages * a_bytes + (batch == 1 ? 1 : kStages) * b_bytes + kRows * f.staging_pitch + kPackedMaxN * 4 + 64;
   f.ctas = kSmemPerSm / (f.smem + kCtaReserve);
@@ -612,18 +679,24 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k) {
     ++f.stages;
   }
   f.piped_smem = piped_smem(f.stages);
-  const int64_t units = f.matrices == 1 ? batch * ((m + kRows - 1) / kRows) : (batch + f.matrices - 1) / f.matrices;
-  f.piped = piped_pays(units, k, shared_b, f.ctas);
+  f.units = f.matrices == 1 ? batch * ((m + kRows - 1) / kRows) : (batch + f.matrices - 1) / f.matrices;
+  f.piped = piped_pays(f.units, k, shared_b, f.ctas);
   return f;
 }
 
 }  // namespace
 
 cudaError_t init_packed_gemm() {
-  const void* const kernels[4] = {reinterpret_cast<const void*>(&packed_gemm_kernel<false>),
-                                  reinterpret_cast<const void*>(&packed_gemm_kernel<true>),
-                                  reinterpret_cast<const void*>(&packed_piped_kernel<false>),
-                                  reinterpret_cast<const void*>(&packed_piped_kernel<true>)};
+  const void* const kernels[] = {
+      reinterpret_cast<const void*>(&packed_gemm_kernel<false, false>),
+      reinterpret_cast<const void*>(&packed_gemm_kernel<true, false>),
+      reinterpret_cast<const void*>(&packed_gemm_kernel<false, true>),
+      reinterpret_cast<const void*>(&packed_gemm_kernel<true, true>),
+      reinterpret_cast<const void*>(&packed_piped_kernel<false, false>),
+      reinterpret_cast<const void*>(&packed_piped_kernel<true, false>),
+      reinterpret_cast<const void*>(&packed_piped_kernel<false, true>),
+      reinterpret_cast<const void*>(&packed_piped_kernel<true, true>),
+  };
   for (const void* kernel : kernels) {
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
     if (err != cudaSuccess) return err;
@@ -676,7 +749,19 @@ bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_cou
 }
 
 cudaError_t launch_packed_gemm(const PackedProblem& pr) {
-  const Footprint f = footprint(pr.batch, pr.m, pr.n, pr.k);
+  Footprint f = footprint(pr.batch, pr.m, pr.n, pr.k);
+  const bool direct = writes_rows(pr.n, pr.k, pr.batch == 1) && (reinterpret_cast<uintptr_t>(pr.out) & 31) == 0;
+  if (direct) {
+    const Footprint staged = f;
+    f = footprint(pr.batch, pr.m, pr.n, pr.k, false);
+    f.piped = staged.piped;  // by the CTAs that staging leaves: the form was chosen between with them
+    if (f.units <= static_cast<int64_t>(staged.ctas) * pr.sm_count) {
+      // A single round as it was: the room would let some SMs take more units than others (see below; mm 56229x80x48 5.4 ->
+      // 6.3, 28359x112x40 6.5 -> 7.3).
+      f.smem = staged.smem;
+      f.ctas = staged.ctas;
+    }
+  }
   PackedParams p = {};
   p.a = static_cast<const uint8_t*>(pr.a);
   p.b = static_cast<const uint8_t*>(pr.b);
@@ -715,14 +800,30 @@ cudaError_t launch_packed_gemm(const PackedProblem& pr) {
   cfg.gridDim = dim3(static_cast<unsigned>(p.units < room ? p.units : room));
   cfg.blockDim = dim3(f.piped ? kPipedThreads : kThreads);
   cfg.dynamicSmemBytes = static_cast<size_t>(f.piped ? f.piped_smem : f.smem);
+  // The launch hardware deals CTAs out by shared memory, registers and threads: with little of them an SM may get five and
+  // another three, and TMEM, which it does not count, may hold only four, so that the fifth starts when another has done all
+  // its units.  From 1.6 rounds on each takes its share of the SM's shared memory, and no SM gets more (us: bmm 5400 x
+  // 26x96x8 23.8 -> 17.4, 2500 x 64x96x16 14.2 -> 11.6, mm 262144x48x32 11.7 -> 10.5, 125610x80x16 8.2 -> 7.3).  With fewer
+  // units the next launch's CTAs better set up beside them (mm 21517x72x24 5.0 -> 5.6, bmm 444 x 31x88x8 3.3 -> 4.0, 1776 x
+  // 15x48x8 4.1 -> 4.5), and accumulators of 32 columns are too small to matter (4576 x 47x16x16 6.9 -> 7.0).
+  if (!f.piped && p.tmem_cols >= 64 && f.units * 5 >= room * 8) {
+    const size_t share = kSmemPerSm / f.ctas - kCtaReserve;
+    if (cfg.dynamicSmemBytes < share) cfg.dynamicSmemBytes = share < kSmemPerCta ? share : kSmemPerCta;
+  }
   cfg.stream = pr.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pr.overlap ? 1 : 0;
-  if (f.piped) return cudaLaunchKernelEx(&cfg, pr.is_bf16 ? packed_piped_kernel<true> : packed_piped_kernel<false>, p);
-  return cudaLaunchKernelEx(&cfg, pr.is_bf16 ? packed_gemm_kernel<true> : packed_gemm_kernel<false>, p);
+  using Kernel = void (*)(PackedParams);
+  static const Kernel kernels[2][2][2] = {  // [piped][direct][bf16]
+      {{packed_gemm_kernel<false, false>, packed_gemm_kernel<true, false>},
+       {packed_gemm_kernel<false, true>, packed_gemm_kernel<true, true>}},
+      {{packed_piped_kernel<false, false>, packed_piped_kernel<true, false>},
+       {packed_piped_kernel<false, true>, packed_piped_kernel<true, true>}},
+  };
+  return cudaLaunchKernelEx(&cfg, kernels[f.piped ? 1 : 0][direct ? 1 : 0][pr.is_bf16 ? 1 : 0], p);
 }
 
 }  // namespace ayla_b200

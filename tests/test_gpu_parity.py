@@ -756,6 +756,39 @@ def test_packed_kernel_equals_the_general_one(operation, batch, m, n, k, dtype):
     assert bool((out[-guard:] == 7.0).all())
 
 
+@pytest.mark.parametrize("offset", [0, 8])  # results on whole sectors (written by row where that is faster), or inside them
+@pytest.mark.parametrize(
+    "operation,batch,m,n,k",
+    [
+        # rows of one sector, of a half line, of others; the last rows of a quarter and a tile; a matrix per unit, two, four
+        ("mm", 1, 1, 16, 8), ("addmm", 1, 130, 32, 32), ("addmm", 1, 20001, 48, 24), ("mm", 1, 257, 112, 128),
+        ("mm", 1, 90003, 80, 88), ("bmm", 3, 33, 96, 72), ("bmm", 5, 64, 48, 40), ("bmm", 3, 31, 32, 16), ("bmm", 7, 1, 16, 24),
+        # as many units as the SMs take at a time and more, in the chained form
+        ("bmm", 700, 40, 80, 16), ("mm", 1, 76000, 48, 32), ("mm", 1, 75700, 72, 16), ("bmm", 1300, 20, 40, 24),
+    ])
+def test_packed_kernels_results_by_row(operation, batch, m, n, k, offset):
+    _lib.init(0)
+    g = torch.Generator(device=DEV).manual_seed(m * n + k)
+    lead = (batch,) if operation == "bmm" else ()
+    a = torch.randn(*lead, m, k, device=DEV, generator=g).bfloat16()
+    bt = torch.randn(*lead, n, k, device=DEV, generator=g).bfloat16()
+    bias = torch.randn(n, device=DEV, generator=g).bfloat16()
+    store = torch.full((batch * m * n + 64 + offset,), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = store[offset:-64]
+    want = torch.empty(*lead, m, n, dtype=torch.bfloat16, device=DEV)
+    status = _lib.StatusWord()
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(2):
+        _lib.gemm_packed(operation, "bfloat16", bias.data_ptr(), a.data_ptr(), bt.data_ptr(), out.data_ptr(), batch, m, n, k,
+                         status.ptr, stream)
+    _lib.gemm(operation, "bfloat16", bias.data_ptr(), a.data_ptr(), bt.data_ptr(), want.data_ptr(), batch, m, n, k,
+              _lib.Config.from_dict(dict(tile_n=64)), 0, 0, status.ptr, stream)
+    torch.cuda.synchronize()
+    assert status.peek() == 0
+    assert torch.equal(out.view_as(want), want)
+    assert bool((store[:offset] == 7.0).all()) and bool((store[-64:] == 7.0).all())
+
+
 def test_a_capture_without_memory_for_a_workspace_records_a_schedule_that_needs_none(monkeypatch):
     """A product whose depth is split where SMs would idle needs a workspace, which its graph may not get."""
     monkeypatch.setattr(_lib, "capture_workspace", lambda stream, size: None)
