@@ -684,6 +684,30 @@ Footprint footprint(int64_t batch, int64_t m, int64_t n, int64_t k, bool staged 
   return f;
 }
 
+bool one_piece_round(int64_t k, int64_t n, bool shared_b, const Footprint& f, int64_t tiles, int sm_count) {
+  const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);
+  return f.ctas >= 4 && shared_b && k < 16 && n > 40 && n <= 64 && rounds > 0.5 && rounds < 1.35;
+}
+
+bool preferred_by_rounds(int64_t batch, int64_t n, int64_t k, int64_t tiles, const Footprint& f, int sm_count) {
+  if (f.matrices > 1) return f.matrices == 4 || f.ctas >= 2;
+  if (f.ctas < 2) return false;
+  const bool shared_b = batch == 1, mid_sector = k % 16 != 0;
+  if (n <= 32) return shared_b || f.ctas >= 3 || mid_sector;
+  const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);
+  if (k >= 48 && rounds < 0.5) return false;
+  if (f.ctas >= 4) return !one_piece_round(k, n, shared_b, f, tiles, sm_count);
+  const bool settled = rounds <= 0.95 || rounds >= 1.35;
+  if (f.ctas == 3) {
+    if (n <= 64) return settled || k < 48;
+    if (shared_b) return rounds >= 1.25 || (mid_sector && k < 48);
+    return settled && (mid_sector || (n <= 80 && rounds >= 1.35) || (k <= 32 && rounds >= 2.0));
+  }
+  if (!shared_b) return n <= 64 ? settled && mid_sector : k < 64 && rounds <= 0.95;
+  if (mid_sector) return (k > 64 && n <= 96) || (settled && (n <= 96 || rounds >= 1.35 || k < 64));
+  return n <= 64 ? rounds >= 2.4 : k < 64 && n % 16 != 0 && rounds >= 1.35;
+}
+
 }  // namespace
 
 cudaError_t init_packed_gemm() {
@@ -725,27 +749,29 @@ cudaError_t init_packed_gemm() {
 //    473x56x40 0.81, 512 x 128x48x40 0.83).
 //  * A product of one 16-byte piece in depth with shared B, in a single round (60000x64x8 8.6 -> 10.8; 131072x64x8, in
 //    two, 16.0 -> 13.7).
+//
+// Where two CTAs and more of the form that runs fit an SM (without staging rows where the lanes write their own), these
+// besides, from 1100 shapes timed on both kernels:
+//  * up to a depth of 40, from 64 tiles on: 98 shapes, 0.80 of the time, the slowest 1.01 (the widest outputs, where every SM
+//    has a tile: bmm 73 x 72x120x40 3.4 -> 3.6, mm 11964x128x40 4.6 -> 4.9);
+//  * deeper, with few rows to a unit or one B, from 950 tiles on: 13 shapes, 0.78, 0.93 (1226 x 26x80x80 10.7 -> 8.5, mm
+//    246943x72x96 0.54);
+//  * up to 80 columns and a depth of 88, with a tile for every SM: 41 shapes, 0.88, 1.06 (59 x 635x80x64 0.75, but 24 x
+//    1677x80x120 1.24), four tenths of a round and thin second rounds aside.
 bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count) {
   if (n > kPackedMaxN || k > kPackedMaxK) return false;
   const int64_t tiles = batch * ((m + kRows - 1) / kRows);
-  if (tiles < sm_count || tiles > 0x7FFFFFFF) return false;
+  if (tiles > 0x7FFFFFFF) return false;
   const Footprint f = footprint(batch, m, n, k);
-  if (f.matrices > 1) return f.matrices == 4 || f.ctas >= 2;
-  if (f.ctas < 2) return false;
-  const bool shared_b = batch == 1, mid_sector = k % 16 != 0;
-  if (n <= 32) return shared_b || f.ctas >= 3 || mid_sector;
+  if (tiles >= sm_count && preferred_by_rounds(batch, n, k, tiles, f, sm_count)) return true;
+  if (f.matrices > 1 && f.matrices < 4 && f.ctas < 2) return false;
+  const bool shared_b = batch == 1, direct = writes_rows(n, k, shared_b);
+  if ((direct ? footprint(batch, m, n, k, false).ctas : f.ctas) < 2 || one_piece_round(k, n, shared_b, f, tiles, sm_count)) return false;
+  if (k <= 40) return tiles >= 64 && (n <= 112 || (n < 128 && tiles >= sm_count));
+  if (tiles > 950) return m <= 65 || (shared_b && n <= 112);
+  if (tiles < sm_count || n > 80 || k > 88) return false;
   const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);
-  if (k >= 48 && rounds < 0.5) return false;
-  if (f.ctas >= 4) return !(shared_b && k < 16 && n > 40 && n <= 64 && rounds > 0.5 && rounds < 1.35);
-  const bool settled = rounds <= 0.95 || rounds >= 1.35;
-  if (f.ctas == 3) {
-    if (n <= 64) return settled || k < 48;
-    if (shared_b) return rounds >= 1.25 || (mid_sector && k < 48);
-    return settled && (mid_sector || (n <= 80 && rounds >= 1.35) || (k <= 32 && rounds >= 2.0));
-  }
-  if (!shared_b) return n <= 64 ? settled && mid_sector : k < 64 && rounds <= 0.95;
-  if (mid_sector) return (k > 64 && n <= 96) || (settled && (n <= 96 || rounds >= 1.35 || k < 64));
-  return n <= 64 ? rounds >= 2.4 : k < 64 && n % 16 != 0 && rounds >= 1.35;
+  return direct || (rounds >= 0.4 && (rounds <= 0.95 || rounds >= 1.35));
 }
 
 cudaError_t launch_packed_gemm(const PackedProblem& pr) {
@@ -806,9 +832,8 @@ cudaError_t launch_packed_gemm(const PackedProblem& pr) {
   // 26x96x8 23.8 -> 17.4, 2500 x 64x96x16 14.2 -> 11.6, mm 262144x48x32 11.7 -> 10.5, 125610x80x16 8.2 -> 7.3).  With fewer
   // units the next launch's CTAs better set up beside them (mm 21517x72x24 5.0 -> 5.6, bmm 444 x 31x88x8 3.3 -> 4.0, 1776 x
   // 15x48x8 4.1 -> 4.5), and accumulators of 32 columns are too small to matter (4576 x 47x16x16 6.9 -> 7.0).
-  if (!f.piped && p.tmem_cols >= 64 && f.units * 5 >= room * 8) {
-    const size_t share = kSmemPerSm / f.ctas - kCtaReserve;
-    if (cfg.dynamicSmemBytes < share) cfg.dynamicSmemBytes = share < kSmemPerCta ? share : kSmemPerCta;
+  if (!f.piped && p.tmem_cols >= 64 && f.units * 5 >= room * 8 && kSmemPerSm / (f.smem + kCtaReserve) > f.ctas) {
+    cfg.dynamicSmemBytes = static_cast<size_t>(kSmemPerSm / f.ctas - kCtaReserve);
   }
   cfg.stream = pr.stream;
   cudaLaunchAttribute attr[1];

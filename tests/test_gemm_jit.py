@@ -407,3 +407,13 @@ def test_the_suite_times_the_kernel_the_ops_run(packed, monkeypatch):
 ])
 def test_the_packed_kernel_is_preferred_where_it_measured_faster(operation, batch, m, n, k, packed):
     assert _lib.packed_preferred(operation, batch, m, n, k) is packed
+
+
+@pytest.mark.parametrize("operation, batch, m, n, k, packed", [
+    # Shallow ones from 64 tiles on, deeper ones with few rows or one B, narrow ones with a tile for every SM.
+    ("bmm", 64, 128, 64, 40, True), ("bmm", 63, 128, 64, 40, False), ("bmm", 73, 72, 120, 40, False),
+    ("bmm", 1226, 26, 80, 80, True), ("mm", 1, 182773, 112, 112, True), ("bmm", 80, 1923, 80, 128, False),
+    ("bmm", 59, 635, 80, 64, True), ("bmm", 24, 1677, 80, 120, False), ("bmm", 53, 298, 112, 128, False),
+])
+def test_the_packed_kernel_is_preferred_where_two_ctas_fit(operation, batch, m, n, k, packed):
+    assert _lib.packed_preferred(operation, batch, m, n, k) is packed
