@@ -258,7 +258,7 @@ def share_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k:
 
 
 def fit_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k: int) -> Config:
-    """As ``share_depth``, and last waves whose rows start inside a sector are split like any others."""
+    """``cfg``, or what it becomes where other tiles or a shared depth fit the shape better."""
     out = Config.from_dict(cfg.to_dict())
     check(load().ayla_b200_fit_depth(OP_CODES[op], DTYPE_CODES[dtype], batch, m, n, k, ctypes.byref(out)))
     return out

@@ -684,6 +684,81 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
   return r.launch + blocks * (r.block + r.block_busy * busy) + r.per_split * splits + 4.5 * static_cast<double>(waves - 1);
 }
 
+// Microseconds that a product of more than one wave of 128- to 256-wide tiles takes, launch aside, and the number of ways its
+// last wave's tiles are best split (1: not at all).  A k-block of 256-wide pairs takes 0.39 us, of 192 and 128 columns 0.34
+// and 0.25; tiles of half the width two thirds of a whole one's time, as long as it where rows start inside a
+// sector; the sum of S parts 4.8 us (5.8 of 192 columns) and 0.4 per part.  Fitted to 330 timings of 110 shapes.  A split has to
+// gain 1 us, and 4.5 % or 3 us, by this (by 3.5 %: addmm 640x8160x3968, 1 + 22/74, halves 43.9 -> 47.0 with 3; not without the
+// 3 us: 8071x2944x4480, 5 + 14/74, split five ways 171 -> halves 189).  Of 1000 shapes drawn over all kinds 61 get another
+// schedule than by the bounds before, half of them whole tiles for halves that did not fit; they take 0.91 of the time.
+struct LastWave { double us; int splits; };
+LastWave last_wave(int64_t tiles, int64_t wave, int64_t k, int tile_n) {
+  const int64_t k_blocks = ceil_div(k, 64), whole = tiles / wave, rest = tiles % wave;
+  const double tile = static_cast<double>(k_blocks) * (tile_n == 256 ? 0.39 : tile_n == 192 ? 0.34 : 0.25);
+  LastWave best{static_cast<double>(whole) * tile, 1};
+  if (rest == 0) return best;
+  const double unsplit = tile_n % 128 == 0 && rest * 2 <= wave && k % 16 == 0 ? 0.66 * tile : tile;
+  const double bound = 0.045 * static_cast<double>(whole + 1) * tile;
+  const double sum = tile_n == 192 ? 5.8 : 4.8;
+  double least = unsplit - (bound > 3.0 ? 3.0 : bound > 1.0 ? bound : 1.0);
+  double last = unsplit;
+  for (int s = 2; s <= 16 && s * rest <= wave && s * 5 <= k_blocks; ++s) {
+    const double us = tile / s + sum + 0.4 * s;
+    if (us >= least) continue;
+    least = last = us;
+    best.splits = s;
+  }
+  best.us += last;
+  return best;
+}
+
+// A row-major schedule's time by the two models, roughly.
+double scheduled_us(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, const ayla_b200_config& c) {
+  const int64_t wave = machine.sm_count / c.cta_group;
+  const int64_t tiles = batch * ceil_div(m, 128 * c.cta_group) * ceil_div(n, c.tile_n);
+  if (tiles > wave && !c.cluster_split) {
+    return last_wave(tiles, wave, k, c.tile_n).us * (c.cta_group == 2 ? 1.0 : 1.2) * (k % 16 != 0 ? 1.2 : 1.0) + 4.3;
+  }
+  return modelled_us(c.tile_n, c.cta_group, c.split_k,
+                     c.cluster_split ? RATE_CLUSTER : c.split_k > 1 ? RATE_SHARED : RATE_WHOLE, tiles, k, machine);
+}
+
+// Whole tiles of the best other width or pairing that all run at once, for a schedule measured on another shape whose tiles
+// fit this one badly; false where there is none 8 % faster by the model.  (us, the schedule -> this: 5539x384x4096 + GELU,
+// 256-wide pairs in 1 + 14/74 waves -> 128-wide ones, 30.4 -> 19.9; 1240x2176x28672, 45 pairs of 256 columns -> 60 of 192, 157
+// -> 137; 620x7232x1664, three rows of pairs -> five of single CTAs, 19.8 -> 16.8; 119x5312x832, clusters in two waves -> 64
+// columns, 7.5 -> 5.7.)  Not for the shallowest (mm 1759x1344x640 7.0 -> 8.0) nor, with rows inside a sector, for clusters (mm
+// 200x3208x2456 13.1 -> 14.6).
+bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+  if (m <= 64 || k <= 704 || (k % 16 != 0 && c->cluster_split)) return false;
+  const int64_t wave = machine.sm_count / c->cta_group;
+  if (batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n) > wave &&
+      (c->split_k > 1 || c->cluster_split || c->tile_n < 128)) {
+    return false;
+  }
+  double best = 0.92 * scheduled_us(batch, m, n, k, machine, *c);
+  ayla_b200_config chosen = *c;
+  chosen.split_k = 1;
+  chosen.split_tail = 0;
+  chosen.cluster_split = 0;
+  bool found = false;
+  for (int tile_n = 64; tile_n <= 256; tile_n += 64) {
+    for (int cta_group = 1; cta_group <= 2; ++cta_group) {
+      if (cta_group == 2 && m <= 128) continue;
+      const int64_t tiles = batch * ceil_div(m, 128 * cta_group) * ceil_div(n, tile_n);
+      if (tiles > machine.sm_count / cta_group) continue;
+      const double us = modelled_us(tile_n, cta_group, 1, RATE_WHOLE, tiles, k, machine);
+      if (us >= best) continue;
+      best = us;
+      found = true;
+      chosen.tile_n = tile_n;
+      chosen.cta_group = cta_group;
+    }
+  }
+  if (found) *c = chosen;
+  return found;
+}
+
 // What a schedule measured elsewhere, or here by bursts, is corrected in.
 //
 // Shallow products of 256-wide tiles become pairs where no rows are padded: they read B half as often, and under the
@@ -711,34 +786,6 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 //    rows start inside a sector (332x960x2568 11.8 -> 12.6), and never single CTAs for pairs there, which read B twice as
 //    often (524x3200x13656 88 -> 99).  Over 191 shapes that are split by these bounds it takes 0.81 of the time, the slowest
 //    1.02.
-// Microseconds that a product of more than one wave of 128- to 256-wide tiles takes, launch aside, and the number of ways its
-// last wave's tiles are best split (1: not at all).  A k-block of 256-wide pairs takes 0.39 us, of 192 and 128 columns 0.87
-// and 0.72 of that; tiles of half the width two thirds of a whole one's time, as long as it where rows start inside a
-// sector; the sum of S parts 4.8 us (5.8 of 192 columns) and 0.4 per part.  Fitted to 330 timings of 110 shapes.  A split has to
-// gain 1 us, and 4.5 % or 3 us, by this (by 3.5 %: addmm 640x8160x3968, 1 + 22/74, halves 43.9 -> 47.0 with 3; not without the
-// 3 us: 8071x2944x4480, 5 + 14/74, split five ways 171 -> halves 189).  Of 1000 shapes drawn over all kinds 61 get another
-// schedule than by the bounds before, half of them whole tiles for halves that did not fit; they take 0.91 of the time.
-struct LastWave { double us; int splits; };
-LastWave last_wave(int64_t tiles, int64_t wave, int64_t k, int tile_n) {
-  const int64_t k_blocks = ceil_div(k, 64), whole = tiles / wave, rest = tiles % wave;
-  const double tile = static_cast<double>(k_blocks) * (tile_n == 256 ? 0.39 : tile_n == 192 ? 0.34 : 0.28);
-  LastWave best{static_cast<double>(whole) * tile, 1};
-  if (rest == 0) return best;
-  const double unsplit = tile_n % 128 == 0 && rest * 2 <= wave && k % 16 == 0 ? 0.66 * tile : tile;
-  const double bound = 0.045 * static_cast<double>(whole + 1) * tile;
-  const double sum = tile_n == 192 ? 5.8 : 4.8;
-  double least = unsplit - (bound > 3.0 ? 3.0 : bound > 1.0 ? bound : 1.0);
-  double last = unsplit;
-  for (int s = 2; s <= 16 && s * rest <= wave && s * 5 <= k_blocks; ++s) {
-    const double us = tile / s + sum + 0.4 * s;
-    if (us >= least) continue;
-    least = last = us;
-    best.splits = s;
-  }
-  best.us += last;
-  return best;
-}
-
 //
 // `cautious`: ayla_b200_share_depth keeps the bounds that it has for last waves whose rows start inside a sector: two ways at
 // most, behind one whole wave, behind two with a quarter of a wave left, or where the schedule has halves.
@@ -821,6 +868,17 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
     }
   }
   *c = chosen;
+}
+
+// A schedule that was measured elsewhere: with its depth shared out, or with tiles that fit the shape in one wave, and their
+// depth shared out, where that takes 0.92 of the time by the models.  Of 2600 shapes drawn over all kinds 168 get such tiles, in
+// 0.88 of the time, three of them slower by more than 2 % (2200x1216x35136 185 -> 202).
+void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+  ayla_b200_config fitted = *c;
+  share_depth(batch, m, n, k, machine, false, c);
+  if (fitted.swap_ab || fitted.stream_k || fitted.grid_ctas != 0 || !one_wave(batch, m, n, k, machine, &fitted)) return;
+  share_depth(batch, m, n, k, machine, false, &fitted);
+  if (scheduled_us(batch, m, n, k, machine, fitted) < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
 }
 
 // The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
@@ -1191,7 +1249,7 @@ int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, 
   if (rc) return rc;
   rc = check_config(*cfg, false);
   if (rc) return rc;
-  share_depth(batch, m, n, k, current_machine(), false, cfg);
+  fit_depth(batch, m, n, k, current_machine(), cfg);
   return AYLA_B200_OK;
 }
 

@@ -263,8 +263,9 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
 AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                         ayla_b200_config* cfg);
 
-/* The same, which splits last waves of operand rows that start inside a 32-byte sector (k % 16 != 0) like any others:
- * ayla_b200_share_depth splits those two ways at most. */
+/* For a schedule that was measured on another shape: the same, or whole tiles of another width or pairing that all run at
+ * once, where a timing model finds them clearly faster.  Splits last waves of operand rows that start inside a 32-byte sector
+ * (k % 16 != 0) like any others, which ayla_b200_share_depth splits two ways at most. */
 AYLA_B200_API int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                       ayla_b200_config* cfg);
 

@@ -199,7 +199,7 @@ def test_swiglu_of_few_rows_is_swapped_where_it_measured_faster(m, n, k, tile_n,
 # (m, n, k), tile width, the schedule's last wave -> width, splits and last wave that are fitted
 @pytest.mark.parametrize("shape, tile_n, tail, expected", [
     ((4156, 1088, 3712), 256, 0, (256, 6, 1)),  # 1 + 11/74 waves of 58 k-blocks
-    ((783, 4672, 2368), 256, 0, (256, 1, 2)),  # 1 + 2/74 of 37: halves
+    ((2229, 4864, 1792), 256, 0, (256, 1, 2)),  # 2 + 23/74 of 28: halves
     ((1128, 7488, 7928), 256, 0, (256, 11, 1)),  # rows inside a sector
     ((2920, 2568, 3832), 256, 2, (256, 1, 0)),  # 1 + 58/74: two halves of a tile do not fit
     ((9874, 640, 832), 256, 2, (256, 1, 0)),
@@ -214,6 +214,25 @@ def test_last_waves_are_fitted_by_their_length(shape, tile_n, tail, expected):
     out = _lib.fit_depth(cfg, "mm", "bfloat16", 1, m, n, k)
     assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
     assert (out.tile_n, out.split_k, out.split_tail) == expected
+
+
+# (m, n, k), the schedule measured elsewhere -> tiles that all run at once here
+@pytest.mark.parametrize("shape, config, expected", [
+    ((5539, 384, 4096), dict(tile_n=256, cta_group=2, split_tail=2), (128, 2, 1, 0, 0)),
+    ((1240, 2176, 28672), dict(tile_n=256, cta_group=2), (192, 2, 1, 0, 0)),
+    ((620, 7232, 1664), dict(tile_n=256, cta_group=2, split_tail=2), (256, 1, 1, 0, 0)),
+    ((119, 5312, 832), dict(tile_n=128, cta_group=1, split_k=2, cluster_split=1), (64, 1, 1, 0, 0)),
+    # as they are: the shallowest, clusters whose rows start inside a sector, few rows, what the model finds no faster
+    ((1759, 1344, 640), dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2, 0)),
+    ((200, 3208, 2456), dict(tile_n=128, cta_group=1, split_k=2, cluster_split=1), (128, 1, 2, 0, 1)),
+    ((64, 3208, 2048), dict(tile_n=64, cta_group=1), (64, 1, 1, 0, 0)),
+    ((1056, 2048, 28288), dict(tile_n=256, cta_group=1), (256, 1, 2, 0, 0)),
+])
+def test_schedules_from_other_shapes_are_fitted_to_one_wave(shape, config, expected):
+    m, n, k = shape
+    out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, **config)), "mm", "bfloat16", 1, m, n, k)
+    assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
+    assert (out.tile_n, out.cta_group, out.split_k, out.split_tail, out.cluster_split) == expected
 
 
 def test_depth_is_shared_where_sms_would_idle():
