@@ -42,6 +42,7 @@ def load() -> ModuleType | None:
 
 
 _MAX_OPERANDS = 5  # kMaxOperands of the compiled dispatcher
+_DISPATCHERS: dict[tuple[str, str], object] = {}  # those of the ops registered here
 
 
 def serves(launcher, kinds: list[OperandKind]) -> bool:
@@ -74,9 +75,16 @@ def register(namespace: str, name: str, compiler: ShapeSpecializingJITCompiler) 
             dispatcher.insert(list(tensors), launcher, fields)
 
     dispatcher = load().register_op(namespace, name, len(compiler.signature), dtype, fallback)
+    _DISPATCHERS[namespace, name] = dispatcher
 
 
 def register_rms_factors(namespace: str, name: str, dtype: str, torch_dtype: torch.dtype, fallback) -> None:
     """Register the CUDA kernel of the row-factors op ``(x, eps, factors) -> ()``."""
     entry = ctypes.cast(_lib.load().ayla_b200_rms_factors, ctypes.c_void_p).value
     load().register_rms_factors(namespace, name, entry, _lib.DTYPE_CODES[dtype], torch_dtype, fallback)
+
+
+def register_rms_linear(namespace: str, name: str, projection: str, fallback) -> None:
+    """Register the CUDA kernel of ``(x, eps, weight, out) -> ()``, whose projection is the op ``projection``."""
+    entry = ctypes.cast(_lib.load().ayla_b200_rms_factors, ctypes.c_void_p).value
+    load().register_rms_linear(namespace, name, entry, _DISPATCHERS[namespace, projection], fallback)

@@ -56,6 +56,30 @@ def _row_factors_op(dtype: str) -> torch._ops.OpOverload:
     return getattr(getattr(torch.ops, DEFAULT_NAMESPACE), name).default
 
 
+@cache
+def _rms_linear_op(dtype: str, activation: str) -> torch._ops.OpOverload:
+    """Torch op ``(x, eps, weight, out) -> ()``: the row factors of ``x``, then ``out = activation(x @ weight^T)`` times
+    them.  Shapes that have not been specialised go through the two ops one after the other."""
+    row_factors = _row_factors_op(dtype)
+    projection = gemm_act_rowmul_op("mm", activation, dtype)
+    projection_name = projection._schema.name.split("::")[1]
+    name = projection_name.replace("jit_mm", "rms_linear").replace("_rowmul", "")
+
+    def cuda_impl(x: torch.Tensor, eps: float, weight: torch.Tensor, out: torch.Tensor) -> None:
+        factors = torch.empty(x.shape[0], 1, dtype=x.dtype, device=x.device)
+        row_factors(x, eps, factors)
+        projection(x, weight, factors, out)
+
+    lib = _library(DEFAULT_NAMESPACE)
+    lib.define(f"{name}(Tensor arg0, float eps, Tensor arg1, Tensor(a2!) arg2) -> ()")
+    if native_dispatch.load() is not None:
+        native_dispatch.register_rms_linear(DEFAULT_NAMESPACE, name, projection_name, cuda_impl)
+    else:
+        lib.impl(name, cuda_impl, "CUDA")
+    lib.impl(name, lambda x, eps, weight, out: None, "Meta")
+    return getattr(getattr(torch.ops, DEFAULT_NAMESPACE), name).default
+
+
 def rms_norm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float = 1e-5, activation: str = "none",
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """``activation(rmsnorm(x) @ W.T)`` for ``x`` of shape ``[tokens, in_features]`` and
@@ -70,7 +94,5 @@ def rms_norm_linear(x: torch.Tensor, folded_weight: torch.Tensor, eps: float = 1
     if out is None:
         out = torch.empty(tokens, folded_weight.shape[0], dtype=x.dtype, device=x.device)
     dtype = _DTYPE_NAMES[x.dtype]
-    factors = torch.empty(tokens, 1, dtype=x.dtype, device=x.device)
-    _row_factors_op(dtype)(x, eps, factors)
-    gemm_act_rowmul_op("mm", activation, dtype)(x, folded_weight, factors, out)
+    _rms_linear_op(dtype, activation)(x, eps, folded_weight, out)
     return out

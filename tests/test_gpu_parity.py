@@ -687,6 +687,40 @@ def test_rms_norm_linear_behind_the_launch_that_writes_its_input(m, k):
     assert_parity(serial[-1].cpu(), (x32 @ weight.cpu().float().T) * factors, f"rms_norm_linear {m}x192x{k}")
 
 
+@pytest.mark.parametrize("m, n, k", [(20, 1216, 1408), (300, 520, 1024), (130, 1536, 4104), (2048, 1024, 512)])
+def test_rms_norm_linear_between_launches_that_write_its_operands_and_read_its_result(m, n, k):
+    """Weight and input are rewritten in front of every call, its result is read behind it and then overwritten, the row
+    factors' memory is given back with the call: the same bits as with serialised launches."""
+    from ayla_b200.rmsnorm_linear import rms_norm_linear
+
+    g = torch.Generator().manual_seed(m + n + k)
+    rand = lambda *shape: (torch.randn(*shape, generator=g) * 64 ** -0.25).bfloat16().to(DEV)
+    xs, ws = [rand(m, 64) for _ in range(4)], [rand(n, 64) for _ in range(4)]
+    up, down = rand(k, 64), rand(136, n)
+    x, w = torch.empty(m, k, dtype=torch.bfloat16, device=DEV), torch.empty(n, k, dtype=torch.bfloat16, device=DEV)
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    mm = gemm_op("mm", "bfloat16")
+
+    def chain():
+        results = []
+        for i in range(16):
+            mm(ws[i % 4], up, w)
+            mm(xs[(i + i // 4) % 4], up, x)
+            rms_norm_linear(x, w, out=out)
+            results.append(torch.empty(m, 136, dtype=torch.bfloat16, device=DEV))
+            mm(out, down, results[-1])
+        torch.cuda.synchronize()
+        return torch.stack(results)
+
+    try:
+        _lib.set_launch_overlap(False)
+        serial = chain()
+    finally:
+        _lib.set_launch_overlap(True)
+    for _ in range(3):
+        assert torch.equal(chain(), serial)
+
+
 def test_rms_norm_linear_refuses_what_the_projection_refuses():
     from ayla_b200.rmsnorm_linear import rms_norm_linear
 
