@@ -65,6 +65,7 @@ struct Registry {
     append_variants_shared_act_cg2(&entries);
     append_variants_gated_cg1(&entries);
     append_variants_gated_cg2(&entries);
+    append_variants_flat(&entries);
   }
   int base_count = 0;  // the variants without the activation epilogue come first
   // Where there is no variant of the form asked for, the one with all epilogues serves.
@@ -321,7 +322,14 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   // 1024x4096x512 15.3 -> 12.0, 64x8192x1024 10.4 -> 8.9); the k-split and swapped forms load it directly.
   const KernelEntry* e = nullptr;
   if (activation == 2 && form == FORM_LEAN) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 2, FORM_LEAN);
-  if (activation == 3 && form == FORM_LEAN) e = registry().find(tile_n, c.cta_group, epilogue, transposed, 3, FORM_LEAN);
+  if (e == nullptr && rows <= 128 && c.cta_group == 2 && !transposed && c.stream_k == 0 && c.split_tail == 0 &&
+      (c.split_k <= 1 || c.cluster_split)) {
+    const KernelEntry* flat = registry().find(tile_n, 2, epilogue, transposed, activation != 0 ? 1 : 0, FORM_FLAT);
+    if (flat != nullptr && flat->form == FORM_FLAT) e = flat;
+  }
+  if (e == nullptr && activation == 3 && form == FORM_LEAN) {
+    e = registry().find(tile_n, c.cta_group, epilogue, transposed, 3, FORM_LEAN);
+  }
   if (e == nullptr) e = registry().find(tile_n, c.cta_group, epilogue, transposed, activation != 0 ? 1 : 0, form);
   if (e == nullptr) {
     return fail(AYLA_B200_E_UNSUPPORTED, "no kernel variant tile_n=%d cta_group=%d epilogue=%d swap=%d",
@@ -330,7 +338,7 @@ int make_plan(const ayla_b200_config& c, int epilogue, int64_t batch, int64_t ro
   const int out_tile_n = swiglu_cols ? 128 : tile_n;
   plan->kernel = e;
   plan->tile_rows = (c.swap_ab && c.tile_rows > 0) ? c.tile_rows : 128;
-  plan->m_tiles = static_cast<int>(ceil_div(rows, c.swap_ab ? plan->tile_rows : 128 * c.cta_group));
+  plan->m_tiles = static_cast<int>(ceil_div(rows, c.swap_ab ? plan->tile_rows : e->cta_rows * c.cta_group));
   plan->n_tiles = static_cast<int>(ceil_div(cols, out_tile_n));
   plan->k_blocks = static_cast<int>(ceil_div(k, 64));
   int splits = c.split_k;
@@ -870,15 +878,73 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
   *c = chosen;
 }
 
+// Products of 65 to 128 rows on pairs (FORM_FLAT) instead, where by the models they take 0.95 of the schedule's time; all of
+// their tiles at once.  Their times are a launch and the k-blocks, at rates fitted to 1340 timings of 730 shapes (6 % rms); rows
+// that start inside a sector take 1.4 times as long.  The factors on the schedule's own model are what it lacks for 128 rows: a
+// pair's rates do not change with the tile's height, and wide tiles read 128 rows per 128 or 256 columns.  Of those shapes, drawn
+// over mm, addmm with activations, RMS norm and bmm, 391 are taken, in 0.89 of the time, three slower by more than 2.1 % (bmm
+// 32x96x344x872 8.7 -> 9.2, whose columns pad worse in 256); the best pair would give the others 0.97.  us, before -> with it: mm
+// 128x4096x4096 11.8 -> 10.4, 128x8192x2048 11.4 -> 9.5, addmm 100x3584x2560 9.3 -> 7.8, 128x1024x1024 6.1 -> 5.4.  Not below 65
+// rows, where the swapped form reads no more (64x4096x4096 10.2 -> 10.2), and not where depth is short and tiles are narrow already.
+bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+  const int64_t k_blocks = ceil_div(k, 64);
+  if (m <= 64 || m > 128 || c->swap_ab || c->stream_k || c->grid_ctas != 0 || k_blocks < (c->tile_n == 64 ? 12 : 7)) return false;
+  const int64_t own_tiles = batch * ceil_div(n, c->tile_n);
+  if (c->split_tail != 0 && own_tiles > machine.sm_count) return false;
+  const bool mid_sector = k % 16 != 0;
+  double own = modelled_us(c->tile_n, c->cta_group, c->split_k,
+                           c->cluster_split ? RATE_CLUSTER : c->split_k > 1 ? RATE_SHARED : RATE_WHOLE, own_tiles, k, machine);
+  if (c->split_k == 1) {
+    own *= c->tile_n != 128 || c->cta_group != 1 ? 1.0 : mid_sector ? 1.25 : k_blocks < 20 ? 1.05 : 1.2;
+  } else if (c->tile_n == 256) {
+    own *= mid_sector ? 1.06 : 1.24;
+  } else if (c->tile_n == 64) {
+    own *= 1.05;
+  } else if (c->tile_n == 128) {
+    own *= c->cluster_split ? (c->split_k == 2 ? 1.02 : 1.0) : mid_sector ? 1.0 : 1.05;
+  }
+  struct Flat { int tile_n, split; double launch, block, block_busy; };
+  static const Flat kFlat[5] = {{128, 1, 4.17, .099, .077}, {128, 2, 4.85, .105, .082}, {128, 4, 5.69, .095, .091},
+                                {256, 1, 4.44, .126, .227}, {256, 2, 5.08, .163, .247}};
+  const int64_t pairs = machine.sm_count / 2;
+  double best = 0.95 * own;
+  const Flat* chosen = nullptr;
+  for (const Flat& f : kFlat) {
+    const int64_t tiles = batch * ceil_div(n, f.tile_n);
+    if (tiles > machine.clusters(2 * f.split) || (f.split > 1 && k_blocks < 4 * f.split)) continue;
+    const double busy = static_cast<double>(tiles * f.split) / static_cast<double>(pairs);
+    const double us = f.launch + static_cast<double>(ceil_div(k_blocks, f.split)) * (mid_sector ? 1.4 : 1.0) *
+                                     (f.block + f.block_busy * busy);
+    if (us >= best) continue;
+    best = us;
+    chosen = &f;
+  }
+  if (chosen == nullptr) return false;
+  c->tile_n = chosen->tile_n;
+  c->cta_group = 2;
+  c->split_k = chosen->split;
+  c->cluster_split = chosen->split > 1 ? 1 : 0;
+  c->split_tail = 0;
+  c->group_m = 8;
+  // Of 730 schedules faster than before: 1.009 of the best pair of hints with these, 1.013 with none; 1.019 without a prefetch.
+  c->l2_hint_a = 2;
+  c->l2_hint_b = 1;
+  const int64_t share = k_blocks / chosen->split / 2;
+  c->early_prefetch = static_cast<int>(share < 8 ? share : 8);
+  return true;
+}
+
 // A schedule that was measured elsewhere: with its depth shared out, or with tiles that fit the shape in one wave, and their
-// depth shared out, where that takes 0.92 of the time by the models.  Of 2600 shapes drawn over all kinds 168 get such tiles, in
-// 0.88 of the time, three of them slower by more than 2 % (2200x1216x35136 185 -> 202).
+// depth shared out, where that takes 0.92 of the time by the models; or on flat pairs.  Of 2600 shapes drawn over all kinds 168
+// get other whole tiles, in 0.88 of the time, three of them slower by more than 2 % (2200x1216x35136 185 -> 202).
 void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   ayla_b200_config fitted = *c;
   share_depth(batch, m, n, k, machine, false, c);
-  if (fitted.swap_ab || fitted.stream_k || fitted.grid_ctas != 0 || !one_wave(batch, m, n, k, machine, &fitted)) return;
-  share_depth(batch, m, n, k, machine, false, &fitted);
-  if (scheduled_us(batch, m, n, k, machine, fitted) < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
+  if (!fitted.swap_ab && !fitted.stream_k && fitted.grid_ctas == 0 && one_wave(batch, m, n, k, machine, &fitted)) {
+    share_depth(batch, m, n, k, machine, false, &fitted);
+    if (scheduled_us(batch, m, n, k, machine, fitted) < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
+  }
+  flat_pairs(batch, m, n, k, machine, c);
 }
 
 // The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
@@ -950,7 +1016,7 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
   const bool swiglu_rows = e.epilogue == EPI_SWIGLU && e.transposed_out;
   int b_box_rows = swiglu_cols ? 128 : e.tile_n / e.cta_group;
   int b_stage_rows = e.tile_n / e.cta_group;  // rows of the column operand one CTA receives per stage
-  int a_box_rows = plan.tile_rows;
+  int a_box_rows = e.cta_rows < plan.tile_rows ? e.cta_rows : plan.tile_rows;
   // An operand that fits in a single tile is loaded with a box of just its own rows (rounded
   // up to the 8-row swizzle atom): rows of the box that lie outside the tensor are zero-filled
   // by TMA at a cost comparable to real rows, and a GEMM with a handful of rows would spend
@@ -1001,11 +1067,11 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
   p.cluster_split = plan.cluster_split;
   p.stream_k = plan.stream_k;
   p.kb_per_cta = plan.kb_per_cta;
-  p.idesc_narrow = make_idesc(is_bf16, 128 * e.cta_group, e.tile_n / 2);
+  p.idesc_narrow = make_idesc(is_bf16, e.cta_rows * e.cta_group, e.tile_n / 2);
   p.total_units = plan.total_units;
   p.group_m = plan.group_m;
   p.is_bf16 = is_bf16;
-  p.idesc = make_idesc(is_bf16, 128 * e.cta_group, e.tile_n);
+  p.idesc = make_idesc(is_bf16, e.cta_rows * e.cta_group, e.tile_n);
   // Hints are given for a/bt as the caller passed them.
   p.l2_hint_a = static_cast<uint32_t>(c.swap_ab ? c.l2_hint_b : c.l2_hint_a);
   p.l2_hint_b = static_cast<uint32_t>(c.swap_ab ? c.l2_hint_a : c.l2_hint_b);
@@ -1038,11 +1104,11 @@ int launch_plan(const Plan& plan, const ayla_b200_config& c, const Problem& pr, 
     // slots it covers as long as three remain, otherwise the inbox overlays live slots and the
     // kernel holds the partials back until the whole cluster is done with its MMAs.
     const int csk = plan.cluster_split;
-    const int slice_cols = e.tile_n / csk;
-    const int chunk_cols = e.tile_n < 32 ? e.tile_n : 32;
+    const int slice_cols = e.acc_cols / csk;
+    const int chunk_cols = e.acc_cols < 32 ? e.acc_cols : 32;
     const int slots = (slice_cols >= chunk_cols) ? csk - 1 : csk;
     const int inbox_bytes = slots * 128 * slice_cols * 4;
-    const int stage_bytes = e.kb_per_slot * (128 * 64 * 2 + (e.tile_n / e.cta_group) * 64 * 2);  // one ring slot
+    const int stage_bytes = e.kb_per_slot * (e.cta_rows * 64 * 2 + (e.tile_n / e.cta_group) * 64 * 2);  // one ring slot
     const int ring_bytes = e.stages * stage_bytes;
     if (inbox_bytes > ring_bytes) {
       return fail(AYLA_B200_E_UNSUPPORTED, "cluster_split: the %d-byte inbox does not fit the %d-byte ring", inbox_bytes,

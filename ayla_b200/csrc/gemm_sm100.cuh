@@ -38,8 +38,9 @@ namespace ayla_b200 {
 
 enum : int { EPI_PLAIN = 0, EPI_BIAS = 1, EPI_SWIGLU = 2 };
 
-// Which k-split epilogues a kernel is compiled with: all but the shared sum, none, or the shared sum alone.
-enum : int { FORM_FULL = 0, FORM_LEAN = 1, FORM_SHARED = 2 };
+// Which k-split epilogues a kernel is compiled with: all but the shared sum, none, or the shared sum alone; FLAT: pairs on
+// tiles of 128 rows, with the k-split through clusters alone.
+enum : int { FORM_FULL = 0, FORM_LEAN = 1, FORM_SHARED = 2, FORM_FLAT = 3 };
 
 // Error codes written to the device status word (first error wins).
 enum : unsigned {
@@ -170,6 +171,12 @@ struct GemmTraits {
   // SHARED: whole tiles, and k-splits, one unit per CTA, that share their sum through the workspace.
   static constexpr bool SHARED = FORM_ == FORM_SHARED;
   static constexpr bool FULL = FORM_ == FORM_FULL;
+  // FLAT: a CTA pair on a tile of 128 rows, 64 per CTA, for products of at most 128 rows; whole tiles and clusters.  What
+  // bounds those is the rate at which an SM takes operands (some 57 bytes a clock): a pair reads half of the rows and half
+  // of the columns per CTA where a single CTA of the same share of the result reads all rows.  The accumulator lies in
+  // BN / 2 columns: TMEM lanes 0..63 hold the left half of the tile's columns, lanes 64..127 the right one.
+  static constexpr bool FLAT = FORM_ == FORM_FLAT;
+  static constexpr bool CLUSTERS = FULL || FLAT;  // has the k-split through clusters
   // ACT: the epilogue applies the activation named in the launch parameters.  A separate set of
   // instantiations, so that the plain kernels carry none of that code (compiled in as a run-time
   // branch it cost the output-bound bmm 5 %).
@@ -179,7 +186,7 @@ struct GemmTraits {
   static constexpr int EPI = EPI_;
   static constexpr bool TRANS_OUT = TRANS_OUT_;
   static constexpr int STAGES = STAGES_;
-  static constexpr int BM = 128;                // rows per CTA
+  static constexpr int BM = FLAT ? 64 : 128;    // rows per CTA
   static constexpr int BK = 64;                 // one 128-byte swizzle atom of 16-bit elements
   // SwiGLU: row-major, gate and up share the accumulator's columns (2 x 128); swapped, its rows (2 x 64),
   // `tm_a` then being the gate and `tm_b2` the up weight.
@@ -195,10 +202,11 @@ struct GemmTraits {
   // holds; the MMAs of one k-block of a tile narrower than 256 columns take less than that, so
   // those tiles move two k-blocks per slot (measured on B200: M = 512, N = K = 4096 on 256 x 128
   // pair tiles 20.7 -> 17.9 us; M = 8, N = 14336 21.5 -> 19.3 us; four per slot gained nothing more).
-  static constexpr int KB_PER_SLOT = (BN >= 256 || (BN == 192 && CTA_GROUP == 1)) ? 1 : 2;  // at least three slots
+  static constexpr int ACC_COLS = FLAT ? BN / 2 : BN;  // TMEM columns of an accumulator
+  static constexpr int KB_PER_SLOT = ((BN >= 256 && !FLAT) || (BN == 192 && CTA_GROUP == 1)) ? 1 : 2;  // at least three slots
   static constexpr int SLOT_BYTES = KB_PER_SLOT * STAGE_BYTES;
   static constexpr int ACC_BUFS = 2;
-  static constexpr int TMEM_COLS_NEEDED = ACC_BUFS * BN;
+  static constexpr int TMEM_COLS_NEEDED = ACC_BUFS * ACC_COLS;
   static constexpr int TMEM_COLS = TMEM_COLS_NEEDED <= 32    ? 32
                                    : TMEM_COLS_NEEDED <= 64  ? 64
                                    : TMEM_COLS_NEEDED <= 128 ? 128
@@ -237,6 +245,7 @@ struct GemmTraits {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "tcgen05 N extent");
   static_assert(B_BYTES % 1024 == 0, "B slab must keep the 1024-byte swizzle alignment");
   static_assert(!SWIGLU_COLS || BN == 256, "row-major SwiGLU uses the 2x128 layout");
+  static_assert(!FLAT || (CTA_GROUP == 2 && BN >= 128 && !TRANS_OUT && !GATED && EPI != EPI_SWIGLU), "row-major pairs");
   static_assert(!PAIRED || (LEAN && !GATED && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
   static_assert(!SHARED || (!TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches");
   static_assert(!GATED || (ACT && LEAN && !TRANS_OUT && EPI != EPI_SWIGLU), "row-major launches without a k-split");
@@ -623,7 +632,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   const BoundedWait bw{abort_flag, p.status, p.timeout_ns};
   // Cluster split-K: the cluster holds `csk` CTAs (CTA pairs when CG == 2), one per k-split
   // of the cluster's tile.
-  const int csk = (!T::SWIGLU_COLS && T::FULL) ? p.cluster_split : 0;
+  const int csk = (!T::SWIGLU_COLS && T::CLUSTERS) ? p.cluster_split : 0;
   constexpr int group = T::KB_PER_SLOT;  // k-blocks per ring slot
   const int n_stages = p.stages;         // ring slots in use
 
@@ -855,7 +864,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (bw.aborted()) break;
         AYLA_TRACE_WAIT(tr_wait2, bw.wait(bar_acc_empty + acc * 8, acc_phase ^ 1, ST_TIMEOUT_ACC_EMPTY))
         tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * BN;
+        const uint32_t tmem_d = tmem_base + acc * T::ACC_COLS;
         const uint32_t unit_idesc = w.is_narrow ? p.idesc_narrow : idesc;
         const int nkb = w.kb1 - w.kb0;
         for (int i = 0; i < nkb; i += group) {
@@ -960,7 +969,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int half_of_pair = T::PAIRED ? ((warp - 2) >> 2) & 1 : 0;
     const uint32_t pair_bar = 8 + wsub * 4 + q;
     const int epi_tid = (warp - 2) * 32 + lane;
-    const int row_in_tile = q * 32 + lane;
+    const int tmem_lane = q * 32 + lane;
+    const int row0 = (T::FLAT ? q & 1 : q) * 32;  // of this warp's rows among the CTA's, and of its columns in the tile
+    const int col0_in_tile = T::FLAT ? (q >> 1) * T::ACC_COLS : 0;
+    const int row_in_tile = row0 + lane;
     const bool up_rows = T::SWIGLU_ROWS && q >= 2;  // this warp's accumulator rows belong to the up weight
     const int is_bf16 = p.is_bf16;
     const int act = T::ACT ? p.act : static_cast<int>(ACT_NONE);
@@ -969,7 +981,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     uint32_t bias_buf = 0;
     uint32_t gate_phase = 0;
     const uint32_t my_gate_bar = bar_gate + (warp - 2) * 8;
-    constexpr int CHUNKS32 = T::OUT_BN / 32 > 0 ? T::OUT_BN / 32 : 1;  // 32-column chunks
+    constexpr int OUT_COLS = T::FLAT ? T::ACC_COLS : T::OUT_BN;
+    constexpr int CHUNKS32 = OUT_COLS / 32 > 0 ? OUT_COLS / 32 : 1;  // 32-column chunks
     constexpr int CHUNK_COLS = T::OUT_BN < 32 ? T::OUT_BN : 32;
     constexpr int EPI_THREADS = T::EPI_WARPS * 32;
     const uint32_t acc_empty_leader =
@@ -983,7 +996,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // Kernels that take several tiles look one unit ahead and read its slice while this one's tile is on its way
     // (read at the head of a tile its latency was part of every tile: addmm 5215x1216x320 8.3 -> 7.6 us).
     constexpr bool ROW_BIAS = T::EPI == EPI_BIAS && !T::TRANS_OUT;
-    constexpr bool AHEAD = ROW_BIAS && !T::FULL && BN >= 128;
+    constexpr bool AHEAD = ROW_BIAS && !T::CLUSTERS && BN >= 128;
     const int bias_thread = half_of_pair * 128 + q * 32 + lane;
     const int bias_col = (T::GATED ? wsub * 64 : (bias_thread >> 6) * 128 + wsub * 64) + (bias_thread & 63);
     const bool bias_reads = T::GATED ? bias_thread < 64 : bias_col < BN;
@@ -1052,13 +1065,14 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
 #endif
       tc_fence_after_sync();
-      const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+      const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * T::ACC_COLS;
 
       // Rows of the tile that exist: the matrix may end inside it, and the swapped form may
       // give a tile fewer than 128 rows.
       const int row_end = T::TRANS_OUT ? min(p.m, w.m0 + p.tile_rows) : p.m;
       // Swapped SwiGLU: the warps of one chunk meet at a barrier, so they go through it together.
-      const bool rows_live = T::SWIGLU_ROWS || (w.m0 + q * 32) < row_end;
+      const bool rows_live = T::SWIGLU_ROWS || (w.m0 + row0) < row_end;
+      const int n0 = w.n0 + col0_in_tile;  // of this warp's columns
       const int unit_chunks = w.is_narrow ? CHUNKS32 / 2 : CHUNKS32;
       const int unit_groups = (unit_chunks + 1) / 2;
 
@@ -1087,7 +1101,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       auto gate_chunk = [&](float (&v)[32], int c32) {
         if constexpr (T::ACT && !T::TRANS_OUT) {
           const int row = w.m0 + row_in_tile;
-          const int col0 = w.n0 + c32 * 32;
+          const int col0 = n0 + c32 * 32;
           if (p.mul == nullptr || row >= p.m) return;
           if (p.mul_per_row) {
 #pragma unroll
@@ -1131,7 +1145,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // Row-major output: 32 fp32 values of this thread's row become 16 words of the output type ...
       auto pack_chunk = [&](float (&v)[32], int c32, uint32_t* pk) {
         if constexpr (T::EPI == EPI_BIAS) {
-          const float4* b4 = reinterpret_cast<const float4*>(smem_bias + bias_buf * BN + c32 * 32);
+          const float4* b4 = reinterpret_cast<const float4*>(smem_bias + bias_buf * BN + col0_in_tile + c32 * 32);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float4 b = b4[j];
@@ -1164,7 +1178,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_3d(&tm_d, smem_u32(box), w.n0 + group64 * 64, w.m0 + q * 32, w.batch);
+          tma_store_3d(&tm_d, smem_u32(box), n0 + group64 * 64, w.m0 + row0, w.batch);
           tma_store_commit();
         }
       };
@@ -1231,11 +1245,11 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // way).  Row r holds its four 16-byte pieces at r * 64, piece c at position c ^ ((r >> 1) & 3).
       auto write_lone_chunk = [&](float (&v)[32], int c32) {
         if constexpr (!T::TRANS_OUT && !T::LEAN) {
-          const int col0 = w.n0 + c32 * 32;
+          const int col0 = n0 + c32 * 32;
           if (w.m0 + row_in_tile < row_end) {
             if constexpr (T::EPI == EPI_BIAS) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += smem_bias[bias_buf * BN + c32 * 32 + j];
+              for (int j = 0; j < 32; ++j) v[j] += smem_bias[bias_buf * BN + col0_in_tile + c32 * 32 + j];
             }
             apply_act_chunk<32>(v, act);
             gate_chunk(v, c32);
@@ -1259,7 +1273,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int r = i * 8 + (lane >> 2);
-            const int out_row = w.m0 + q * 32 + r;
+            const int out_row = w.m0 + row0 + r;
             const uint4 x = *reinterpret_cast<const uint4*>(my_store + r * 64 + ((piece ^ ((r >> 1) & 3)) << 4));
             if (out_row < row_end && col < p.n) {
               *reinterpret_cast<uint4*>(dst0 + 2 * static_cast<long long>(out_row) * p.out_ld) = x;
@@ -1268,7 +1282,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
       };
 
-      if (T::FULL && csk > 0) {
+      if (T::CLUSTERS && csk > 0) {
         // ---- cluster split-K: S CTAs of the cluster (those with this CTA's place in its
         // pair) hold the S partial sums of this 128-row tile.  Each owns BN / S columns of
         // it: every CTA sends each owner its partial of the owner's columns with asynchronous
@@ -1276,8 +1290,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         // owner's inbox barrier with its bytes; an owner waits for that barrier alone, adds
         // the S partials in split order and stores.  Nobody waits for a sender's stores but
         // their receiver.
-        if constexpr (!T::SWIGLU_COLS && T::FULL) {
-          const int slice_cols = BN / csk;
+        if constexpr (!T::SWIGLU_COLS && T::CLUSTERS) {
+          const int slice_cols = T::ACC_COLS / csk;
           const int slice_shift = __ffs(slice_cols) - 1;
           const int slice_c4 = slice_cols >> 2;
           const uint32_t exch = smem_u32(smem) + p.inbox_offset;
@@ -1305,7 +1319,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
               // An owner that keeps its own partial in TMEM has no inbox slot for itself.
               const int slot = (own_in_tmem && csk_rank > owner) ? csk_rank - 1 : csk_rank;
               const uint32_t dst =
-                  map_to_cta(exch + ((slot * slice_c4 + c4) * 128 + row_in_tile) * 16, owner_cta);
+                  map_to_cta(exch + ((slot * slice_c4 + c4) * 128 + tmem_lane) * 16, owner_cta);
               st_async_v4(dst, __uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
                           __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]),
                           map_to_cta(bar_inbox, owner_cta));
@@ -1371,7 +1385,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
                   for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(own[j]);
                 } else {
-                  const float4* src = mine + ((s > csk_rank ? s - 1 : s) * slice_c4 + lc * 8) * 128 + row_in_tile;
+                  const float4* src = mine + ((s > csk_rank ? s - 1 : s) * slice_c4 + lc * 8) * 128 + tmem_lane;
                   float4 x[8];
 #pragma unroll
                   for (int j = 0; j < 8; ++j) x[j] = src[j * 128];
@@ -1402,7 +1416,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #ifdef AYLA_B200_TRACE
                 if (stamps != nullptr && warp == 2 && lane == 0 && lc == wsub) trace_stamp(stamps, 27);
 #endif
-                const int col0 = w.n0 + c32 * 32;
+                const int col0 = n0 + c32 * 32;
                 if (!(rows_live && col0 < p.n)) continue;
                 if constexpr (T::TRANS_OUT) {
                   finish_chunk(v, c32);
@@ -1418,20 +1432,20 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             for (int c4 = wsub; c4 < slice_c4; c4 += 2) {
               float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
               for (int s = 0; s < csk; ++s) {
-                const float4 x = mine[(s * slice_c4 + c4) * 128 + row_in_tile];
+                const float4 x = mine[(s * slice_c4 + c4) * 128 + tmem_lane];
                 sum.x += x.x;
                 sum.y += x.y;
                 sum.z += x.z;
                 sum.w += x.w;
               }
-              const int col = w.n0 + csk_rank * slice_cols + c4 * 4;
+              const int col = n0 + csk_rank * slice_cols + c4 * 4;
               if (col < p.n) {
                 float v4[4] = {sum.x, sum.y, sum.z, sum.w};
                 if constexpr (T::SWIGLU_ROWS) {
                   // The up partials are in the exchange area as well, 64 rows further on.
                   float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
                   for (int s = 0; s < csk; ++s) {
-                    const float4 x = mine[(s * slice_c4 + c4) * 128 + row_in_tile + 64];
+                    const float4 x = mine[(s * slice_c4 + c4) * 128 + tmem_lane + 64];
                     up.x += x.x;
                     up.y += x.y;
                     up.z += x.z;
@@ -1583,7 +1597,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll 1
             for (int g = wsub; g < unit_groups; g += 2) {
               // Liveness per 64 columns: both halves of a 128-byte store row go together.
-              const bool live = rows_live && w.n0 + g * 64 < p.n;
+              const bool live = rows_live && n0 + g * 64 < p.n;
               uint32_t pk[16];
               tmem_ld_wait();
 #ifdef AYLA_B200_TRACE

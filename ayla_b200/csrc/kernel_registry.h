@@ -23,6 +23,8 @@ struct LaunchArgs {
 struct KernelEntry {
   int tile_n, cta_group, epilogue, transposed_out, stages, smem_bytes;
   int kb_per_slot;  // k-blocks one ring slot holds
+  int cta_rows;     // rows of a tile one CTA holds
+  int acc_cols;     // TMEM columns of an accumulator: tile_n, half of it where a CTA holds 64 rows
   int threads;
   int activation;  // 1 = the variant whose epilogue applies the launch's activation, 2 = the same for
                    // launches with a gate operand shaped like the output, 3 = with sixteen epilogue warps
@@ -33,9 +35,9 @@ struct KernelEntry {
 
 constexpr int kMaxSmem = 232448;
 
-template <int BN, int CG, int EPI, bool TR, bool GATED = false>
+template <int BN, int CG, int EPI, bool TR, bool GATED = false, bool FLAT = false>
 constexpr int max_stages() {
-  using T1 = GemmTraits<BN, CG, EPI, TR, 1, GATED, GATED ? FORM_LEAN : FORM_FULL, GATED>;
+  using T1 = GemmTraits<BN, CG, EPI, TR, 1, GATED, GATED ? FORM_LEAN : FLAT ? FORM_FLAT : FORM_FULL, GATED>;
   const int fixed = T1::STORE_BYTES + T1::BIAS_BYTES + T1::MISC_BYTES;
   const int s = (kMaxSmem - fixed) / T1::SLOT_BYTES;
 #ifdef AYLA_B200_STAGE_CAP
@@ -76,7 +78,7 @@ cudaError_t launch_variant(const LaunchArgs& a) {
 
 template <int BN, int CG, int EPI, bool TR, int ACT = 0, int FORM = FORM_FULL, bool GATED = false>
 KernelEntry make_entry() {
-  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED>(), ACT, FORM, GATED>;
+  using T = GemmTraits<BN, CG, EPI, TR, max_stages<BN, CG, EPI, TR, GATED, FORM == FORM_FLAT>(), ACT, FORM, GATED>;
   KernelEntry e;
   e.tile_n = BN;
   e.cta_group = CG;
@@ -86,6 +88,8 @@ KernelEntry make_entry() {
   e.smem_bytes = T::SMEM_BYTES;
   e.kb_per_slot = T::KB_PER_SLOT;
   e.threads = T::THREADS;
+  e.cta_rows = T::BM;
+  e.acc_cols = T::ACC_COLS;
   e.activation = GATED ? 2 : T::PAIRED ? 3 : ACT;
   e.form = FORM;
   e.func = reinterpret_cast<const void*>(&gemm_sm100_kernel<T>);
@@ -116,5 +120,6 @@ void append_variants_shared_cg1(std::vector<KernelEntry>* out);
 void append_variants_shared_cg2(std::vector<KernelEntry>* out);
 void append_variants_shared_act_cg1(std::vector<KernelEntry>* out);
 void append_variants_shared_act_cg2(std::vector<KernelEntry>* out);
+void append_variants_flat(std::vector<KernelEntry>* out);
 
 }  // namespace ayla_b200

@@ -153,9 +153,11 @@ def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: 
     if shared == seed.builder_config:
         return seed
     captured = {**seed.captured_config, **shared}
+    flat = m <= 128 and shared["cta_group"] == 2 and seed.builder_config["cta_group"] == 1
     return replace(seed, captured_config=captured, builder_config=_builder_config(captured),
                    unsplit_config=seed.builder_config,
-                   adaptations=(*seed.adaptations, "depth split where SMs would idle"))
+                   adaptations=(*seed.adaptations,
+                                "pairs on 128 rows" if flat else "depth split where SMs would idle"))
 
 
 def _streams_weights(operation: str, batch: int, m: int, n: int, k: int) -> bool:

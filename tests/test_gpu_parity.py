@@ -365,6 +365,46 @@ def test_paired_cluster_split_k_variants(split_k, tile_n, device_state):
         assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("split_k", [1, 2, 4])
+@pytest.mark.parametrize("tile_n", [128, 256])
+def test_pairs_on_tiles_of_128_rows(tile_n, split_k, device_state):
+    """Products of at most 128 rows on CTA pairs, whole and split through clusters: the same bits as with single CTAs, and
+    the epilogue's bias, activation, row factors and gate on the half of the columns that each lane has."""
+    torch.manual_seed(tile_n + split_k)
+    status, workspace = device_state
+    cfg = dict(tile_n=tile_n, cta_group=2, split_k=split_k, cluster_split=int(split_k > 1), group_m=8)
+    for operation, dtype, activation, batch, m, n, k in (
+            ("mm", "bfloat16", "none", 1, 128, 256, 512), ("mm", "float16", "none", 1, 65, 520, 1000),
+            ("addmm", "float16", "gelu", 1, 97, 776, 2056), ("addmm", "bfloat16", "none", 1, 127, 136, 640),
+            ("bmm", "float16", "silu", 5, 70, 264, 648), ("bmm", "bfloat16", "none", 40, 128, 392, 512),
+            ("mm", "bfloat16", "relu", 1, 33, 72, 4096), ("mm", "float16", "none", 1, 3, 4096, 584)):
+        lead = (batch,) if operation == "bmm" else ()
+        a = torch.randn((*lead, m, k)).to(TD[dtype])
+        bt = (torch.randn((*lead, n, k)) * k ** -0.5).to(TD[dtype])
+        tensors = (a, bt) if operation != "addmm" else (torch.randn(n).to(TD[dtype]), a, bt)
+        what = f"{operation} {activation} {batch}x{m}x{n}x{k} {cfg}"
+        out, code = run_abi(operation, dtype, tensors, cfg, device_state)
+        assert code == 0
+        ref = O.gemm_ref32(operation, *tensors)
+        assert_parity(out, ref, what)
+        single, code = run_abi(operation, dtype, tensors, dict(cfg, cta_group=1), device_state)
+        assert code == 0 and torch.equal(out, single), what
+        dev = [t.to(DEV) for t in tensors]
+        row = (torch.rand((*lead, m, 1)) + 0.5).to(TD[dtype])
+        gate = torch.randn((*lead, m, n)).to(TD[dtype])
+        for entry, factors in ((_lib.gemm_act_rowmul, row), (_lib.gemm_act_mul, gate)):
+            store = torch.full((batch * m + 4, n), float("nan"), dtype=TD[dtype], device=DEV)
+            status.zero_()
+            entry(operation, dtype, activation, dev[0].data_ptr() if operation == "addmm" else 0, dev[-2].data_ptr(),
+                  dev[-1].data_ptr(), (factors_on_device := factors.to(DEV)).data_ptr(), store.data_ptr(), batch, m, n, k,
+                  _lib.Config.from_dict(cfg), workspace.data_ptr(), workspace.numel(), status.data_ptr(),
+                  torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            assert int(status.item()) == 0 and bool(torch.isnan(store[batch * m:]).all()), what
+            got = store[:batch * m].view(*lead, m, n).cpu()
+            assert_parity(got, O.act_ref32(activation, ref) * factors.float(), f"{what} {entry.__name__}")
+
+
 def test_launch_overlap_keeps_stream_order(device_state):
     """A chain of launches, each reading what the one before wrote, gives the same bits whether
     or not a launch may start its set-up under its predecessor's tail."""
