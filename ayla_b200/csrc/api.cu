@@ -878,30 +878,46 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
   *c = chosen;
 }
 
-// Products of 65 to 128 rows on pairs (FORM_FLAT) instead, where by the models they take 0.95 of the schedule's time; all of
+// Products of 33 to 128 rows on pairs (FORM_FLAT) instead, where by the models they take 0.95 of the schedule's time; all of
 // their tiles at once.  Their times are a launch and the k-blocks, at rates fitted to 1340 timings of 730 shapes (6 % rms); rows
 // that start inside a sector take 1.4 times as long.  The factors on the schedule's own model are what it lacks for 128 rows: a
 // pair's rates do not change with the tile's height, and wide tiles read 128 rows per 128 or 256 columns.  Of those shapes, drawn
 // over mm, addmm with activations, RMS norm and bmm, 391 are taken, in 0.89 of the time, three slower by more than 2.1 % (bmm
 // 32x96x344x872 8.7 -> 9.2, whose columns pad worse in 256); the best pair would give the others 0.97.  us, before -> with it: mm
-// 128x4096x4096 11.8 -> 10.4, 128x8192x2048 11.4 -> 9.5, addmm 100x3584x2560 9.3 -> 7.8, 128x1024x1024 6.1 -> 5.4.  Not below 65
-// rows, where the swapped form reads no more (64x4096x4096 10.2 -> 10.2), and not where depth is short and tiles are narrow already.
+// 128x4096x4096 11.8 -> 10.4, 128x8192x2048 11.4 -> 9.5, addmm 100x3584x2560 9.3 -> 7.8, 128x1024x1024 6.1 -> 5.4.  Not where
+// depth is short and tiles are narrow already.
+// Of 33 to 64 rows only in place of a split depth: single CTAs on whole tiles load just the rows that exist (36x5632x1664 7.7 ->
+// 8.3).  The swapped form's own model is fitted to 200 timings (4 to 6 % rms; eight-way clusters and narrower accumulators stay, pairs
+// take 1.1 to 1.4 of their time).  Of 337 shapes 50 are taken, in 0.90, none slower by more than 0.9 %: 64x8832x2816 12.4 -> 11.4,
+// 53x1344x8448 12.1 -> 10.4, RMS norm and 55x5312x3264 14.1 -> 11.3.
 bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   const int64_t k_blocks = ceil_div(k, 64);
-  if (m <= 64 || m > 128 || c->swap_ab || c->stream_k || c->grid_ctas != 0 || k_blocks < (c->tile_n == 64 ? 12 : 7)) return false;
-  const int64_t own_tiles = batch * ceil_div(n, c->tile_n);
-  if (c->split_tail != 0 && own_tiles > machine.sm_count) return false;
+  if (m <= 32 || m > 128 || c->stream_k || c->grid_ctas != 0) return false;
+  if (m <= 64 ? c->split_k == 1 || k_blocks < 16 : c->swap_ab || k_blocks < (c->tile_n == 64 ? 12 : 7)) return false;
   const bool mid_sector = k % 16 != 0;
-  double own = modelled_us(c->tile_n, c->cta_group, c->split_k,
-                           c->cluster_split ? RATE_CLUSTER : c->split_k > 1 ? RATE_SHARED : RATE_WHOLE, own_tiles, k, machine);
-  if (c->split_k == 1) {
-    own *= c->tile_n != 128 || c->cta_group != 1 ? 1.0 : mid_sector ? 1.25 : k_blocks < 20 ? 1.05 : 1.2;
-  } else if (c->tile_n == 256) {
-    own *= mid_sector ? 1.06 : 1.24;
-  } else if (c->tile_n == 64) {
-    own *= 1.05;
-  } else if (c->tile_n == 128) {
-    own *= c->cluster_split ? (c->split_k == 2 ? 1.02 : 1.0) : mid_sector ? 1.0 : 1.05;
+  const int64_t own_tiles = batch * ceil_div(n, c->swap_ab ? (c->tile_rows > 0 ? c->tile_rows : 128) : c->tile_n);
+  if (c->split_tail != 0 && own_tiles > machine.sm_count) return false;
+  double own;
+  if (c->swap_ab) {
+    if (c->tile_n != 64 || !c->cluster_split || c->split_k > 4) return false;
+    const bool two = c->split_k == 2;
+    const int64_t ctas = own_tiles * c->split_k, waves = ceil_div(ctas, machine.sm_count);
+    const double busy = static_cast<double>(ctas * (c->tile_rows > 0 ? c->tile_rows : 128)) /
+                        static_cast<double>(128 * waves * machine.sm_count);
+    own = (two ? 5.70 : 5.23) + static_cast<double>(waves * ceil_div(k_blocks, c->split_k)) *
+                                    (mid_sector ? (two ? 1.25 : 1.18) : 1.0) * (two ? .136 + .191 * busy : .149 + .172 * busy);
+  } else {
+    own = modelled_us(c->tile_n, c->cta_group, c->split_k,
+                      c->cluster_split ? RATE_CLUSTER : c->split_k > 1 ? RATE_SHARED : RATE_WHOLE, own_tiles, k, machine);
+    if (c->split_k == 1) {
+      own *= c->tile_n != 128 || c->cta_group != 1 ? 1.0 : mid_sector ? 1.25 : k_blocks < 20 ? 1.05 : 1.2;
+    } else if (c->tile_n == 256) {
+      own *= mid_sector ? 1.06 : 1.24;
+    } else if (c->tile_n == 64) {
+      own *= 1.05;
+    } else if (c->tile_n == 128) {
+      own *= c->cluster_split ? (c->split_k == 2 ? 1.02 : 1.0) : mid_sector ? 1.0 : 1.05;
+    }
   }
   struct Flat { int tile_n, split; double launch, block, block_busy; };
   static const Flat kFlat[5] = {{128, 1, 4.17, .099, .077}, {128, 2, 4.85, .105, .082}, {128, 4, 5.69, .095, .091},
@@ -922,6 +938,8 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
   if (chosen == nullptr) return false;
   c->tile_n = chosen->tile_n;
   c->cta_group = 2;
+  c->swap_ab = 0;
+  c->tile_rows = 0;
   c->split_k = chosen->split;
   c->cluster_split = chosen->split > 1 ? 1 : 0;
   c->split_tail = 0;

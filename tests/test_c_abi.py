@@ -241,9 +241,13 @@ def test_schedules_from_other_shapes_are_fitted_to_one_wave(shape, config, expec
     ((65, 8192, 2048), dict(tile_n=128, cta_group=1, split_k=2, cluster_split=1), (128, 2, 1, 0, 0)),
     ((128, 14336, 4096), dict(tile_n=128, cta_group=1, split_tail=2), (256, 2, 1, 0, 0)),
     ((74, 960, 3136), dict(tile_n=64, cta_group=1, split_k=5), (128, 2, 4, 0, 1)),
-    # as they are: the next number of rows, few k-blocks, clusters of eight on the fewest tiles, more than one wave of pairs,
-    # the swapped form, a given grid
-    ((64, 4096, 4096), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (64, 1, 2, 0, 1)),
+    ((64, 8832, 2816), dict(tile_n=64, cta_group=1, swap_ab=1, split_k=2, cluster_split=1), (128, 2, 1, 0, 0)),
+    ((33, 1344, 8448), dict(tile_n=64, cta_group=1, swap_ab=1, split_k=4, cluster_split=1), (128, 2, 4, 0, 1)),
+    # as they are: other numbers of rows, whole tiles of few rows, few k-blocks, clusters of eight on the fewest tiles, more
+    # than one wave of pairs, the swapped form of more rows, a given grid
+    ((32, 1408, 8448), dict(tile_n=64, cta_group=1, swap_ab=1, split_k=4, cluster_split=1), (64, 1, 4, 0, 1)),
+    ((64, 5120, 3328), dict(tile_n=64, cta_group=1), (64, 1, 1, 0, 0)),
+    ((64, 128, 9728), dict(tile_n=64, cta_group=1, swap_ab=1, split_k=8, cluster_split=1), (64, 1, 8, 0, 1)),
     ((129, 4096, 4096), dict(tile_n=128, cta_group=2, split_k=2), (128, 2, 2, 0, 0)),
     ((128, 4096, 704), dict(tile_n=64, cta_group=1), (64, 1, 1, 0, 0)),
     ((128, 256, 9728), dict(tile_n=64, cta_group=1, split_k=8, cluster_split=1), (64, 1, 8, 0, 1)),
@@ -257,6 +261,7 @@ def test_few_rows_are_given_to_pairs(shape, config, expected):
     assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
     assert (out.tile_n, out.cta_group, out.split_k, out.split_tail, out.cluster_split) == expected
     if out.cta_group == 2 and m <= 128:
+        assert out.swap_ab == 0 and out.tile_rows == 0
         assert _lib.workspace_bytes(out, "mm", 1, m, n, k) == 0
 
 
