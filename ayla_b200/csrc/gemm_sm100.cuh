@@ -568,11 +568,10 @@ __device__ __forceinline__ void apply_act_chunk(float (&v)[N], int act) {
   }
 }
 
-// 0 for no hint.
 __device__ __forceinline__ uint64_t make_policy(uint32_t hint) {
   if (hint == 1) return policy_evict_first();
   if (hint == 2) return policy_evict_last();
-  return 0;
+  return policy_evict_unchanged();
 }
 
 template <class T>
@@ -981,6 +980,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     uint32_t bias_buf = 0;
     uint32_t gate_phase = 0;
     const uint32_t my_gate_bar = bar_gate + (warp - 2) * 8;
+    const uint64_t gate_policy = make_policy(0);
     constexpr int OUT_COLS = T::FLAT ? T::ACC_COLS : T::OUT_BN;
     constexpr int CHUNKS32 = OUT_COLS / 32 > 0 ? OUT_COLS / 32 : 1;  // 32-column chunks
     constexpr int CHUNK_COLS = T::OUT_BN < 32 ? T::OUT_BN : 32;
@@ -1046,7 +1046,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       if (gate_live && lane == 0 && !bw.aborted()) {
         tma_store_wait_read<0>();
         mbar_arrive_expect_tx(my_gate_bar, T::STORE_BUF_BYTES);
-        tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, 0);
+        tma_load_3d<1>(smem_u32(my_store), &tm_b2, my_gate_bar, w.n0 + wsub * 64, w.m0 + q * 32, w.batch, gate_policy);
       }
 
       // One factor per output row: read while the MMAs run.

@@ -183,22 +183,10 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm) {
 // Tiled 3-D load global -> this CTA's shared memory.  `bar` is a shared::cluster
 // address; with CTA_GROUP == 2 it may name the barrier of the pair's leader CTA.
 // No multicast: the box lands in the issuing CTA only.
-// `policy` 0: no cache hint.  That is not what an explicit evict_normal policy does, which loses L2 hits where a box's rows
-// end inside a line that the next box reads on: of 41 shapes timed back to back with either, 0.76 to 0.83 of the time
-// without the hint for products of many tiles with k % 64 != 0 (mm 4096x2560x8008 211 -> 164 us, addmm 5000x3000x1000 48.7
-// -> 38.2, mm 14862x5264x720 132 -> 106), 0.90 to 1.0 with whole lines, none slower.  evict_last takes the time of no hint.
 template <int CTA_GROUP>
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
                                             int c0, int c1, int c2, uint64_t policy) {
   if constexpr (CTA_GROUP == 1) {
-    if (policy == 0) {
-      asm volatile(
-          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-          :
-          : "r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-          : "memory");
-      return;
-    }
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
         " [%0], [%1, {%3, %4, %5}], [%2], %6;"
@@ -207,15 +195,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm,
           "l"(policy)
         : "memory");
   } else {
-    if (policy == 0) {
-      asm volatile(
-          "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%3, %4, %5}], [%2];"
-          :
-          : "r"(dst), "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-          : "memory");
-      return;
-    }
     asm volatile(
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
         ".L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
@@ -277,6 +256,18 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// For loads that ask for nothing.  evict_unchanged takes the time of a load without a hint, evict_normal does not: it loses L2
+// hits where a box's rows end inside a line that the next box reads on.  Of 41 shapes timed back to back with either, 0.76 to
+// 0.83 of the time for products of many tiles with k % 64 != 0 (mm 4096x2560x8008 211 -> 164 us, addmm 5000x3000x1000 48.7 ->
+// 38.2, mm 14862x5264x720 132 -> 106), 0.90 to 1.0 with whole lines, none slower.  A policy rather than a second form of the
+// load without one: the choice between the two cost the loading warps up to 5 % of a small product (mm 768x768x2048 start to end
+// 6.50 us with either policy, 6.80 with the choice; 872x576x2176 6.82 and 6.98).
+__device__ __forceinline__ uint64_t policy_evict_unchanged() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_unchanged.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
 // ----------------------------------------------------------------- tcgen05
 
 template <int CTA_GROUP>

@@ -57,7 +57,8 @@ extern "C" {
  */
 typedef struct ayla_b200_config {
   int32_t tile_n;    /* accumulator columns per tile: 16,32,64,128,192,256 (16/32 only with swap_ab, 192 only without) */
-  int32_t cta_group; /* 1, or 2 = two CTAs share one 256-row tile */
+  int32_t cta_group; /* 1, or 2 = two CTAs share one 256-row tile (128 rows, whole or split
+                        through a cluster, where the product has no more and tile_n >= 128) */
   int32_t swap_ab;   /* 1 = compute out^T = bt @ a^T (rows of bt fill the 128-row tile); small M */
   int32_t split_k;   /* >= 1; > 1 needs a workspace */
   int32_t group_m;   /* raster: row tiles per group, >= 1 */
@@ -264,8 +265,9 @@ AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_
                                         ayla_b200_config* cfg);
 
 /* For a schedule that was measured on another shape: the same, or whole tiles of another width or pairing that all run at
- * once, where a timing model finds them clearly faster.  Splits last waves of operand rows that start inside a 32-byte sector
- * (k % 16 != 0) like any others, which ayla_b200_share_depth splits two ways at most. */
+ * once, or for 33 to 128 rows CTA pairs on 128-row tiles, where timing models find them clearly faster.  Splits last waves
+ * of operand rows that start inside a 32-byte sector (k % 16 != 0) like any others, which ayla_b200_share_depth splits two
+ * ways at most. */
 AYLA_B200_API int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                       ayla_b200_config* cfg);
 
