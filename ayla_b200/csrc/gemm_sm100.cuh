@@ -80,7 +80,7 @@ struct FastDiv {
 struct KernelParams {
   int m, n, k;        // extents of the kernel's (row, column, depth) problem
   int batch;
-  int m_tiles;        // tiles of 128*CTA_GROUP rows
+  int m_tiles;        // tiles of 128*CTA_GROUP rows (FLAT: 128)
   int n_tiles;        // tiles of the output tile width
   int k_blocks;       // ceil(k / 64)
   int splits;         // k-splits per split tile (1 = none)
@@ -174,7 +174,9 @@ struct GemmTraits {
   // FLAT: a CTA pair on a tile of 128 rows, 64 per CTA, for products of at most 128 rows; whole tiles and clusters.  What
   // bounds those is the rate at which an SM takes operands (some 57 bytes a clock): a pair reads half of the rows and half
   // of the columns per CTA where a single CTA of the same share of the result reads all rows.  The accumulator lies in
-  // BN / 2 columns: TMEM lanes 0..63 hold the left half of the tile's columns, lanes 64..127 the right one.
+  // BN / 2 columns: TMEM lanes 0..63 hold the left half of the tile's columns, lanes 64..127 the right one.  A k-block takes
+  // 0.176 us with 128 columns and 0.377 with 256, all SMs at work.  us, single CTAs -> pairs: mm 128x4096x4096 (split in two,
+  // 64 -> 128 columns) 11.8 -> 10.3, 128x8192x2048 11.4 -> 9.5, 128x14336x4096 25.0 -> 23.3, addmm 100x3584x2560 9.3 -> 7.8.
   static constexpr bool FLAT = FORM_ == FORM_FLAT;
   static constexpr bool CLUSTERS = FULL || FLAT;  // has the k-split through clusters
   // ACT: the epilogue applies the activation named in the launch parameters.  A separate set of
