@@ -1458,7 +1458,8 @@ static int gemm_fused(int op, int dtype, int activation, const void* bias, const
   ayla_b200_config c;
   if (cfg != nullptr) {
     c = *cfg;
-  } else if (activation == AYLA_B200_ACT_NONE && mul == nullptr && packed_preferred(batch, m, n, k, ds->sm_count)) {
+  } else if (activation == AYLA_B200_ACT_NONE && mul == nullptr &&
+             packed_preferred(batch, m, n, k, ds->sm_count, on_sectors(out))) {
     return ayla_b200_gemm_packed(op, dtype, bias, a, bt, out, batch, m, n, k, status, stream);
   } else {
     default_config(batch, m, n, k, activation, ds->machine, &c);
@@ -1537,7 +1538,7 @@ int ayla_b200_gemm_packed(int op, int dtype, const void* bias, const void* a, co
 
 int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k) {
   if (check_shape(op, AYLA_B200_BF16, batch, m, n, k) != AYLA_B200_OK) return 0;
-  return packed_preferred(batch, m, n, k, current_sm_count()) ? 1 : 0;
+  return packed_preferred(batch, m, n, k, current_sm_count(), true) ? 1 : 0;
 }
 
 int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const void* a, const void* bt,

@@ -28,7 +28,9 @@ constexpr int kPackedMaxN = 128;
 constexpr int kPackedMaxK = 128;
 
 cudaError_t init_packed_gemm();
-bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count);
+// Whether `out` starts on a 32-byte sector: else its rows go through staging, whatever they are.
+inline bool on_sectors(const void* out) { return (reinterpret_cast<uintptr_t>(out) & 31) == 0; }
+bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count, bool on_sectors);
 cudaError_t launch_packed_gemm(const PackedProblem& problem);
 
 }  // namespace ayla_b200

@@ -217,8 +217,9 @@ AYLA_B200_API int ayla_b200_gemm_packed(int op, int dtype, const void* bias, con
                                         void* stream);
 
 /*
- * 1 where ayla_b200_gemm_packed is the faster way to run the problem, else 0: there ayla_b200_gemm takes
- * it by itself when cfg == NULL.
+ * 1 where ayla_b200_gemm_packed is the faster way to run the problem with `out` on a 32-byte boundary, else 0:
+ * there ayla_b200_gemm takes it by itself when cfg == NULL.  For an `out` on 16 bytes alone it looks again, since
+ * the results then need more shared memory, and takes the general kernel where that is the faster one.
  */
 AYLA_B200_API int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k);
 

@@ -1066,6 +1066,33 @@ def test_the_packed_kernels_form_is_the_faster_one(batch, m, n, k, piped):
     assert len(names) == 1 and ("packed_piped_kernel" in names[0]) == piped, names
 
 
+@pytest.mark.parametrize("batch, m, n, k", [(1097, 19, 96, 128), (151, 301, 80, 88), (1, 124739, 112, 112)])
+def test_results_inside_a_sector_take_the_packed_kernel_only_where_their_staging_rows_fit(batch, m, n, k):
+    """Rows written straight from registers make room for a second CTA on an SM; an ``out`` that starts inside a sector
+    needs staging rows, which leave room for one, and the general kernel is the faster one."""
+    operation = "bmm" if batch > 1 else "mm"
+    lead = (batch,) if batch > 1 else ()
+    g = torch.Generator(device=DEV).manual_seed(m)
+    a = torch.randn(*lead, m, k, device=DEV, generator=g).bfloat16()
+    bt = torch.randn(*lead, n, k, device=DEV, generator=g).bfloat16()
+    op = gemm_op(operation, "bfloat16")
+    store = torch.empty(batch * m * n + 8, dtype=torch.bfloat16, device=DEV)
+    results, kernels = [], []
+    for offset in (0, 8):
+        out = store[offset:offset + batch * m * n].view(*lead, m, n)
+        op(a, bt, out)
+        torch.cuda.synchronize()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+            op(a, bt, out)
+            torch.cuda.synchronize()
+        kernels += [event.name for event in profile.events() if "packed" in event.name or "gemm_sm100" in event.name]
+        results.append(out.clone())
+    assert torch.equal(*results)
+    if not kernels:
+        pytest.skip("no kernel names from the profiler")
+    assert len(kernels) == 2 and "packed" in kernels[0] and "gemm_sm100" in kernels[1], kernels
+
+
 @pytest.mark.parametrize("batch, m, n, k", [(1, 70000, 96, 24), (2055, 45, 16, 120), (600, 128, 64, 40)])
 def test_piped_packed_kernel_reports_a_timeout_and_keeps_infinities_apart(batch, m, n, k):
     """One B and many, several units per CTA and one."""
