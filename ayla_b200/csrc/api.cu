@@ -881,15 +881,22 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
 // Products of 33 to 128 rows on pairs (FORM_FLAT) instead, where by the models they take 0.95 of the schedule's time; all of
 // their tiles at once.  Their times are a launch and the k-blocks, at rates fitted to 1340 timings of 730 shapes (6 % rms); rows
 // that start inside a sector take 1.4 times as long.  The factors on the schedule's own model are what it lacks for 128 rows: a
-// pair's rates do not change with the tile's height, and wide tiles read 128 rows per 128 or 256 columns.  Of those shapes, drawn
-// over mm, addmm with activations, RMS norm and bmm, 391 are taken, in 0.89 of the time, three slower by more than 2.1 % (bmm
-// 32x96x344x872 8.7 -> 9.2, whose columns pad worse in 256); the best pair would give the others 0.97.  us, before -> with it: mm
-// 128x4096x4096 11.8 -> 10.4, 128x8192x2048 11.4 -> 9.5, addmm 100x3584x2560 9.3 -> 7.8, 128x1024x1024 6.1 -> 5.4.  Not where
-// depth is short and tiles are narrow already.
+// pair's rates do not change with the tile's height, and wide tiles read 128 rows per 128 or 256 columns.  us, before -> with
+// it: mm 128x4096x4096 11.8 -> 10.4, 128x8192x2048 11.4 -> 9.5, addmm 100x3584x2560 9.3 -> 7.8, 128x1024x1024 6.1 -> 5.4.  Not
+// where depth is short and tiles are narrow already.
 // Of 33 to 64 rows only in place of a split depth: single CTAs on whole tiles load just the rows that exist (36x5632x1664 7.7 ->
 // 8.3).  The swapped form's own model is fitted to 200 timings (4 to 6 % rms; eight-way clusters and narrower accumulators stay, pairs
-// take 1.1 to 1.4 of their time).  Of 337 shapes 50 are taken, in 0.90, none slower by more than 0.9 %: 64x8832x2816 12.4 -> 11.4,
-// 53x1344x8448 12.1 -> 10.4, RMS norm and 55x5312x3264 14.1 -> 11.3.
+// take 1.1 to 1.4 of their time).
+// Timed besides over 2729 shapes that the models alone took, thin and batched ones and every measured schedule that changes
+// among them: the bounds below leave 2308 of those, in 0.893 of the time, 21 slower by 2 % and the slowest by 7 % (addmm
+// 64x312x1872 + ReLU 5.9 -> 6.3); the 416 others took 0.965, up to 1.31.  Of 790 drawn afterwards: 0.889, 12 slower by 2 %, the
+// slowest by 8.5 % (36x1632x1464 5.9 -> 6.4); the 42 measured schedules that change: 0.906, the slowest by 1 %.
+//  * Rows inside a sector cost narrow tiles less than the models say, the more so where the depth is split (mm 64x104x13320, 16
+//    ways, 10.7 -> 14.1; addmm 64x104x10520, eight ways, 10.4 -> 12.3), and batches of whole 128-wide tiles (17 x 78x944x392 5.8
+//    -> 6.5); a pair that has neither rows nor columns for its second CTA stays single there (11 x 37x64x3576 7.7 -> 8.8).
+//  * Tiles with three eighths of their columns past the product: not in place of depths split twelve ways and more (mm 65x32x15984
+//    10.4 -> 11.6) nor with nearly as many clusters as run at once (bmm 33 x 72x72x1512 7.0 -> 7.9, 24 x 64x64x1024 8.5 -> 9.0).
+//  * No split depth in place of whole 64-wide tiles up to 16 k-blocks (mm 128x4096x1024 8.2 -> 8.9, 94x3456x1024 5.3 -> 5.7).
 bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   const int64_t k_blocks = ceil_div(k, 64);
   if (m <= 32 || m > 128 || c->stream_k || c->grid_ctas != 0) return false;
@@ -918,7 +925,11 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
     } else if (c->tile_n == 128) {
       own *= c->cluster_split ? (c->split_k == 2 ? 1.02 : 1.0) : mid_sector ? 1.0 : 1.05;
     }
+    if (mid_sector && c->tile_n == 64) own *= c->split_k == 1 ? 0.95 : c->split_k == 2 ? 0.92 : c->cluster_split ? 0.9 : 0.85;
+    if (mid_sector && c->tile_n == 128 && c->split_k == 1 && batch > 1) own *= 0.86;
   }
+  if (batch > 1) own *= 0.97;
+  if (mid_sector && m <= 64 && n <= 64) return false;
   struct Flat { int tile_n, split; double launch, block, block_busy; };
   static const Flat kFlat[5] = {{128, 1, 4.17, .099, .077}, {128, 2, 4.85, .105, .082}, {128, 4, 5.69, .095, .091},
                                 {256, 1, 4.44, .126, .227}, {256, 2, 5.08, .163, .247}};
@@ -928,6 +939,8 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
   for (const Flat& f : kFlat) {
     const int64_t tiles = batch * ceil_div(n, f.tile_n);
     if (tiles > machine.clusters(2 * f.split) || (f.split > 1 && k_blocks < 4 * f.split)) continue;
+    if (n * 8 <= f.tile_n * 5 && (c->split_k >= 12 || tiles * 3 > machine.clusters4 * 2)) continue;
+    if (f.split > 1 && c->split_k == 1 && k_blocks <= 16 && !mid_sector) continue;
     const double busy = static_cast<double>(tiles * f.split) / static_cast<double>(pairs);
     const double us = f.launch + static_cast<double>(ceil_div(k_blocks, f.split)) * (mid_sector ? 1.4 : 1.0) *
                                      (f.block + f.block_busy * busy);
@@ -952,7 +965,7 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
   return true;
 }
 
-// A schedule that was measured elsewhere: with its depth shared out, or with tiles that fit the shape in one wave, and their
+// A schedule that was measured elsewhere, or here without what this knows: with its depth shared out, or with tiles that fit the shape in one wave, and their
 // depth shared out, where that takes 0.92 of the time by the models; or on flat pairs.  Of 2600 shapes drawn over all kinds 168
 // get other whole tiles, in 0.88 of the time, three of them slower by more than 2 % (2200x1216x35136 185 -> 202).
 void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {

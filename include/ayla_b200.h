@@ -265,8 +265,9 @@ AYLA_B200_API int ayla_b200_default_config_act(int op, int dtype, int activation
 AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                         ayla_b200_config* cfg);
 
-/* For a schedule that was measured on another shape: the same, or whole tiles of another width or pairing that all run at
- * once, or for 33 to 128 rows CTA pairs on 128-row tiles, where timing models find them clearly faster.  Splits last waves
+/* The same for a schedule that was measured on another shape, or on this one without what this knows (the ops hand over
+ * exact hits of their table too): besides, whole tiles of another width or pairing that all run at once, or for 33 to 128
+ * rows CTA pairs on 128-row tiles, where timing models find them clearly faster.  Splits last waves
  * of operand rows that start inside a 32-byte sector (k % 16 != 0) like any others, which ayla_b200_share_depth splits two
  * ways at most. */
 AYLA_B200_API int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,

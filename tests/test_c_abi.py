@@ -265,6 +265,32 @@ def test_few_rows_are_given_to_pairs(shape, config, expected):
         assert _lib.workspace_bytes(out, "mm", 1, m, n, k) == 0
 
 
+# (batch, m, n, k), a schedule that stays one of single CTAs
+@pytest.mark.parametrize("batch, shape, config", [
+    # rows inside a sector: split depths of narrow tiles, whole tiles of a batch, neither rows nor columns for a second CTA
+    (1, (64, 104, 13320), dict(tile_n=64, cta_group=1, split_k=16)),
+    (1, (64, 104, 10520), dict(tile_n=64, cta_group=1, split_k=8)),
+    (17, (78, 944, 392), dict(tile_n=128, cta_group=1)),
+    (11, (37, 64, 3576), dict(tile_n=64, cta_group=1, split_k=4, cluster_split=1)),
+    # mostly padding, in place of 16-way splits or with nearly as many clusters as run at once
+    (1, (65, 32, 15984), dict(tile_n=64, cta_group=1, split_k=16)),
+    (33, (72, 72, 1512), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1)),
+    (24, (64, 64, 1024), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1)),
+])
+def test_few_rows_stay_with_single_ctas_where_those_measured_faster(batch, shape, config):
+    m, n, k = shape
+    operation = "bmm" if batch > 1 else "mm"
+    cfg = _lib.Config.from_dict(dict(group_m=8, l2_hint_a=2, l2_hint_b=1, **config))
+    out = _lib.fit_depth(cfg, operation, "bfloat16", batch, m, n, k)
+    assert _lib.config_valid(out, operation, "bfloat16", batch, m, n, k)
+    assert out.cta_group == 1
+
+
+def test_whole_narrow_tiles_of_few_rows_are_not_given_a_split_depth():
+    out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, tile_n=64, cta_group=1)), "mm", "float16", 1, 94, 3456, 1024)
+    assert out.split_k == 1
+
+
 def test_depth_is_shared_where_sms_would_idle():
     def shared(m, n, k, **config):
         cfg = _lib.Config.from_dict(dict(group_m=8, **config))
