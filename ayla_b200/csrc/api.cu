@@ -694,15 +694,16 @@ double modelled_us(int tile_n, int cta_group, int splits, int kind, int64_t tile
 
 // Microseconds that a product of more than one wave of 128- to 256-wide tiles takes, launch aside, and the number of ways its
 // last wave's tiles are best split (1: not at all).  A k-block of 256-wide pairs takes 0.39 us, of 192 and 128 columns 0.34
-// and 0.25; tiles of half the width two thirds of a whole one's time, as long as it where rows start inside a
+// and 0.25 (0.23 to 0.27 in eleven products 400 to 1000 k-blocks deep); tiles of half the width two thirds of a whole one's time, as long as it where rows start inside a
 // sector; the sum of S parts 4.8 us (5.8 of 192 columns) and 0.4 per part.  Fitted to 330 timings of 110 shapes.  A split has to
 // gain 1 us, and 4.5 % or 3 us, by this (by 3.5 %: addmm 640x8160x3968, 1 + 22/74, halves 43.9 -> 47.0 with 3; not without the
 // 3 us: 8071x2944x4480, 5 + 14/74, split five ways 171 -> halves 189).  Of 1000 shapes drawn over all kinds 61 get another
 // schedule than by the bounds before, half of them whole tiles for halves that did not fit; they take 0.91 of the time.
+double block_us(int tile_n) { return tile_n == 256 ? 0.39 : tile_n == 192 ? 0.34 : 0.25; }
 struct LastWave { double us; int splits; };
 LastWave last_wave(int64_t tiles, int64_t wave, int64_t k, int tile_n) {
   const int64_t k_blocks = ceil_div(k, 64), whole = tiles / wave, rest = tiles % wave;
-  const double tile = static_cast<double>(k_blocks) * (tile_n == 256 ? 0.39 : tile_n == 192 ? 0.34 : 0.25);
+  const double tile = static_cast<double>(k_blocks) * block_us(tile_n);
   LastWave best{static_cast<double>(whole) * tile, 1};
   if (rest == 0) return best;
   const double unsplit = tile_n % 128 == 0 && rest * 2 <= wave && k % 16 == 0 ? 0.66 * tile : tile;
@@ -735,10 +736,20 @@ double scheduled_us(int64_t batch, int64_t m, int64_t n, int64_t k, const Machin
 // fit this one badly; false where there is none 8 % faster by the model.  (us, the schedule -> this: 5539x384x4096 + GELU,
 // 256-wide pairs in 1 + 14/74 waves -> 128-wide ones, 30.4 -> 19.9; 1240x2176x28672, 45 pairs of 256 columns -> 60 of 192, 157
 // -> 137; 620x7232x1664, three rows of pairs -> five of single CTAs, 19.8 -> 16.8; 119x5312x832, clusters in two waves -> 64
-// columns, 7.5 -> 5.7.)  Not for the shallowest (mm 1759x1344x640 7.0 -> 8.0) nor, with rows inside a sector, for clusters (mm
-// 200x3208x2456 13.1 -> 14.6).
+// columns, 7.5 -> 5.7.)  Not for the shallowest (mm 1759x1344x640 7.0 -> 8.0).  With whole sectors not
+//  * with wider tiles in place of 128-wide pairs up to 23 k-blocks, whose several waves take less than the model says (addmm
+//    1147x1920x1408 + GELU, 22, 10.1 -> 11.6; 990x2368x768 6.5 -> 7.2, 8586x448x896 + GELU 11.1 -> 12.0; from 24 on 0.88 to
+//    0.99 in eight shapes);
+//  * with pairs in place of single CTAs of the same 256 columns up to 23 (nine of eleven 1.01 to 1.04: addmm 1722x2560x768
+//    8.2 -> 8.5).
+// Not in place of clusters whose rows start inside a sector (mm 200x3208x2456 13.1 -> 14.6), of one product's 64-wide ones whose rows
+// start inside a 128-byte line from 21 k-blocks on (seven shapes 0.90 to 1.06, whole lines and fewer 0.76 to 0.96: addmm
+// 179x768x1296 + ReLU 6.6 -> 7.0), nor of 256-wide ones of single CTAs (addmm 282x5440x3776 21.3 -> 23.8).
 bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
-  if (m <= 64 || k <= 704 || (k % 16 != 0 && c->cluster_split)) return false;
+  const bool mid_sector = k % 16 != 0;
+  if (m <= 64 || k <= 704) return false;
+  if (c->cluster_split && (mid_sector || (c->tile_n == 256 && c->cta_group == 1))) return false;
+  if (c->cluster_split && c->tile_n == 64 && batch == 1 && k % 64 != 0 && k > 20 * 64) return false;
   const int64_t wave = machine.sm_count / c->cta_group;
   if (batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n) > wave &&
       (c->split_k > 1 || c->cluster_split || c->tile_n < 128)) {
@@ -755,6 +766,8 @@ bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& mac
       if (cta_group == 2 && m <= 128) continue;
       const int64_t tiles = batch * ceil_div(m, 128 * cta_group) * ceil_div(n, tile_n);
       if (tiles > machine.sm_count / cta_group) continue;
+      if (!mid_sector && c->tile_n == 128 && c->cta_group == 2 && tile_n > 128 && k <= 23 * 64) continue;
+      if (!mid_sector && c->tile_n == 256 && c->cta_group == 1 && tile_n == 256 && cta_group == 2 && k <= 23 * 64) continue;
       const double us = modelled_us(tile_n, cta_group, 1, RATE_WHOLE, tiles, k, machine);
       if (us >= best) continue;
       best = us;
@@ -965,15 +978,23 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
   return true;
 }
 
-// A schedule that was measured elsewhere, or here without what this knows: with its depth shared out, or with tiles that fit the shape in one wave, and their
-// depth shared out, where that takes 0.92 of the time by the models; or on flat pairs.  Of 2600 shapes drawn over all kinds 168
-// get other whole tiles, in 0.88 of the time, three of them slower by more than 2 % (2200x1216x35136 185 -> 202).
+// A schedule that was measured elsewhere, or here without what this knows: with its depth shared out, or with tiles that fit
+// the shape in one wave, and their depth shared out, where that takes 0.92 of the time by the models; or on flat pairs.  Beside
+// 128-wide pairs whose last wave is split, whole 192-wide ones count with the k-blocks of a last wave's model: their operands
+// outgrow L2, and by the rate of a single wave mm 2200x1216x35136 took them, 174 -> 191, and 1304x1808x33888, 179 -> 204 (eleven
+// such shapes: the four still taken 0.75 to 0.94, the others 0.97 to 1.13).  Of 954 shapes drawn over all kinds that get whole
+// tiles so, 0.863 of the time, four slower by 2 % (the slowest 186x8008x3992 + SiLU, rows inside a sector, 25 -> 29).
 void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
   ayla_b200_config fitted = *c;
   share_depth(batch, m, n, k, machine, false, c);
   if (!fitted.swap_ab && !fitted.stream_k && fitted.grid_ctas == 0 && one_wave(batch, m, n, k, machine, &fitted)) {
     share_depth(batch, m, n, k, machine, false, &fitted);
-    if (scheduled_us(batch, m, n, k, machine, fitted) < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
+    double us = scheduled_us(batch, m, n, k, machine, fitted);
+    if (c->tile_n == 128 && c->split_tail == 1 && fitted.tile_n == 192 && fitted.split_k == 1) {
+      const double deep = 4.3 + static_cast<double>(ceil_div(k, 64)) * block_us(192) * (k % 16 != 0 ? 1.2 : 1.0);
+      if (us < deep) us = deep;
+    }
+    if (us < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
   }
   flat_pairs(batch, m, n, k, machine, c);
 }
