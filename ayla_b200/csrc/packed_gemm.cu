@@ -753,12 +753,16 @@ cudaError_t init_packed_gemm() {
 // Where two CTAs and more of the form that runs fit an SM (without staging rows where the lanes write their own, for which
 // `out` has to be `on_sectors`: with staging rows and one CTA, bmm 7653 x 22x96x120 general 52.8, packed 74.2; 156 x
 // 726x80x80 11.0 and 14.9), these besides, from 1100 shapes timed on both kernels:
-//  * up to a depth of 40, from 64 tiles on: 98 shapes, 0.80 of the time, the slowest 1.01 (the widest outputs, where every SM
-//    has a tile: bmm 73 x 72x120x40 3.4 -> 3.6, mm 11964x128x40 4.6 -> 4.9);
+//  * up to a depth of 40, from 64 tiles on: 98 shapes, 0.80 of the time, the slowest 1.01; of 120 columns, where every SM has a
+//    tile (bmm 73 x 72x120x40 3.4 -> 3.6), one to a unit with few rows or five tiles to an SM (17 shapes: 283 x 24x120x32 5.5 ->
+//    3.6, 2557 x 186x120x40 55 -> 41, 561 x 661x120x40 30.5 -> 28.6, but in two or three rounds of full tiles 153 x 238x120x40 5.5 ->
+//    6.5, 250 x 174x120x32 8.6 -> 9.4); not of 128 (mm 11964x128x40 4.6 -> 4.9);
 //  * deeper, with few rows to a unit or one B, from 950 tiles on: 13 shapes, 0.78, 0.93 (1226 x 26x80x80 10.7 -> 8.5, mm
 //    246943x72x96 0.54);
 //  * up to 80 columns and a depth of 88, with a tile for every SM: 41 shapes, 0.88, 1.06 (59 x 635x80x64 0.75, but 24 x
 //    1677x80x120 1.24), four tenths of a round and thin second rounds aside.
+// Of 547 shapes drawn afterwards among those that these three take: 0.80 of the time of the general kernel with the ops'
+// schedule, eight slower by 2 %, at most 1.09 (43 x 786x48x80).
 bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_count, bool on_sectors) {
   if (n > kPackedMaxN || k > kPackedMaxK) return false;
   const int64_t tiles = batch * ((m + kRows - 1) / kRows);
@@ -768,7 +772,9 @@ bool packed_preferred(int64_t batch, int64_t m, int64_t n, int64_t k, int sm_cou
   if (f.matrices > 1 && f.matrices < 4 && f.ctas < 2) return false;
   const bool shared_b = batch == 1, direct = on_sectors && writes_rows(n, k, shared_b);
   if ((direct ? footprint(batch, m, n, k, false).ctas : f.ctas) < 2 || one_piece_round(k, n, shared_b, f, tiles, sm_count)) return false;
-  if (k <= 40) return tiles >= 64 && (n <= 112 || (n < 128 && tiles >= sm_count));
+  if (k <= 40) {
+    return tiles >= 64 && (n <= 112 || (n < 128 && tiles >= sm_count && (m <= 65 || tiles >= 5 * sm_count)));
+  }
   if (tiles > 950) return m <= 65 || (shared_b && n <= 112);
   if (tiles < sm_count || n > 80 || k > 88) return false;
   const double rounds = static_cast<double>(tiles) / (static_cast<double>(f.ctas) * sm_count);

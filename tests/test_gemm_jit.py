@@ -417,3 +417,9 @@ def test_the_packed_kernel_is_preferred_where_it_measured_faster(operation, batc
 ])
 def test_the_packed_kernel_is_preferred_where_two_ctas_fit(operation, batch, m, n, k, packed):
     assert _lib.packed_preferred(operation, batch, m, n, k) is packed
+
+
+@pytest.mark.parametrize("batch, m, packed", [(153, 238, False), (250, 174, False), (33, 1590, False), (283, 24, True),
+                                              (711, 9, True), (414, 987, True)])
+def test_packed_products_of_120_columns_have_few_rows_or_many_tiles(batch, m, packed):
+    assert _lib.packed_preferred("bmm", batch, m, 120, 40) is packed
