@@ -144,20 +144,37 @@ def measured_gemm_configs(operation: str, dtype: str, m: int, n: int, k: int,
     return tuple({**_DEFAULTS, **CONFIGS[index]} for index in indices)
 
 
-def _shared_depth(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int,
-                  batch: int) -> GemmScheduleSeed | None:
-    """The schedule with its depth split where it leaves SMs idle (``ayla_b200_fit_depth``)."""
+def _fit_labels(before: dict[str, object], after: dict[str, object], m: int) -> tuple[str, ...]:
+    """What ``ayla_b200_fit_depth`` made of a schedule, in words."""
+    if m <= 128 and after["cta_group"] == 2 and not (before["cta_group"] == 2 and before["tile_n"] == after["tile_n"]):
+        return ("pairs on 128 rows",)
+    labels = []
+    if (after["tile_n"], after["cta_group"]) != (before["tile_n"], before["cta_group"]):
+        labels.append("tiles of another width or pairing")
+    if int(after["split_k"]) > 1:
+        if any(after[key] != before[key] for key in ("split_k", "split_tail", "cluster_split")):
+            labels.append("depth split where SMs would idle")
+    else:
+        if int(before["split_k"]) > 1:
+            labels.append("depth whole")
+        if after["split_tail"] != before["split_tail"]:
+            labels.append("last wave in halves" if after["split_tail"] else "last wave of whole tiles")
+    return tuple(labels) or ("fitted to the shape",)
+
+
+def _fitted(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int,
+            batch: int) -> GemmScheduleSeed | None:
+    """The schedule as ``ayla_b200_fit_depth`` fits it to the shape: its depth split where SMs would idle, its last wave
+    whole, in halves or split, tiles that all run at once, pairs on 128 rows."""
     if seed is None or seed.builder_config is None:
         return seed
-    shared = _lib.fit_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
-    if shared == seed.builder_config:
+    fitted = _lib.fit_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
+    if fitted == seed.builder_config:
         return seed
-    captured = {**seed.captured_config, **shared}
-    flat = m <= 128 and shared["cta_group"] == 2 and seed.builder_config["cta_group"] == 1
+    captured = {**seed.captured_config, **fitted}
     return replace(seed, captured_config=captured, builder_config=_builder_config(captured),
                    unsplit_config=seed.builder_config,
-                   adaptations=(*seed.adaptations,
-                                "pairs on 128 rows" if flat else "depth split where SMs would idle"))
+                   adaptations=(*seed.adaptations, *_fit_labels(seed.builder_config, fitted, m)))
 
 
 def _streams_weights(operation: str, batch: int, m: int, n: int, k: int) -> bool:
@@ -207,8 +224,8 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
     An exact table hit has empty ``adaptations``; a schedule transferred from a
     nearby measured shape names that shape; otherwise the library's shape-aware
     default, which takes the fused ``activation`` into account, is returned with
-    ``source_shape`` ``None``.  Any of them has its depth split further where that is faster, which its
-    adaptations then say, unless ``share_depth`` is false (for a gate shaped like the output, whose kernels do not
+    ``source_shape`` ``None``.  Any of them is fitted to the shape where that is faster (``_fitted``), exact hits too, which
+    its adaptations then say, unless ``share_depth`` is false (for a gate shaped like the output, whose kernels do not
     split, and for launches that leave SMs to others).  It is a schedule of the general
     kernel: plain products that ``packed_serves`` run on the packed kernel, which takes none.
     """
@@ -227,7 +244,7 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
         return sum(abs(math.log2(a) - math.log2(b)) for a, b in zip(shape, query, strict=True))
 
     def finished(seed: GemmScheduleSeed | None) -> GemmScheduleSeed | None:
-        return _shared_depth(seed, operation, dtype, m, n, k, batch) if share_depth else seed
+        return _fitted(seed, operation, dtype, m, n, k, batch) if share_depth else seed
 
     rule = None
     if query not in table and _streams_weights(operation, batch, m, n, k):
@@ -329,8 +346,9 @@ class GemmLauncher:
     error is correct again.  ``check_status()`` does the same after a synchronise, and
     ``AYLA_B200_DEBUG=1`` calls it after every launch.
 
-    It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the launch goes to the
-    packed kernel instead, and ``seed`` and ``config`` are not used.
+    It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the library is given none and
+    takes the packed kernel, or for an ``out`` on 16 bytes alone its default schedule where that is the faster one;
+    ``seed`` and ``config`` are not used.
     """
 
     _captured_only_where_run = True  # a capture on a stream where this launcher has not run is refused
@@ -349,7 +367,7 @@ class GemmLauncher:
         index = device.index if device.index is not None else torch.cuda.current_device()
         with torch.cuda.device(index):
             _lib.init(index)
-        self._packed = packed  # the library takes that kernel where it is given no schedule
+        self._packed = packed  # the library is given no schedule, and takes that kernel
         need = 0 if self._packed else _lib.workspace_bytes(self.config, operation, batch, m, n, k)
         self._ws_bytes = need
         self.workspace = None

@@ -8,6 +8,7 @@ import torch
 from ayla_b200.gemm_jit import (
     _DEFAULTS,
     _fallback_schedule,
+    _fit_labels,
     _seed,
     gemm_jit_compiler,
     gemm_op,
@@ -423,3 +424,27 @@ def test_the_packed_kernel_is_preferred_where_two_ctas_fit(operation, batch, m, 
                                               (711, 9, True), (414, 987, True)])
 def test_packed_products_of_120_columns_have_few_rows_or_many_tiles(batch, m, packed):
     assert _lib.packed_preferred("bmm", batch, m, 120, 40) is packed
+
+
+@pytest.mark.parametrize("operation, batch, m, n, k, labels", [
+    ("addmm", 1, 128, 1000, 2304, ("pairs on 128 rows",)),
+    ("addmm", 1, 2048, 2560, 10240, ("depth split where SMs would idle",)),
+    ("addmm", 1, 256, 1024, 16384, ("tiles of another width or pairing", "depth split where SMs would idle")),
+    ("addmm", 1, 8192, 32000, 1024, ("last wave in halves",)),
+    ("addmm", 1, 32768, 30528, 128, ("last wave of whole tiles",)),
+    ("bmm", 64, 2048, 2048, 128, ("tiles of another width or pairing",)),
+])
+def test_a_fitted_schedule_says_what_was_changed(operation, batch, m, n, k, labels):
+    seed = select_gemm_schedule(operation, "bfloat16", m, n, k, batch)
+    before, after = seed.unsplit_config, seed.builder_config
+    assert seed.adaptations == labels
+    assert ("depth split where SMs would idle" in labels) == (after["split_k"] > 1 and after["cluster_split"] == 0)
+    assert ("tiles of another width or pairing" in labels) == (
+        m > 128 and (after["tile_n"], after["cta_group"]) != (before["tile_n"], before["cta_group"]))
+
+
+def test_labels_of_a_depth_that_is_whole_again():
+    before = dict(tile_n=64, cta_group=1, split_k=2, split_tail=0, cluster_split=1)
+    after = dict(before, split_k=1, cluster_split=0)
+    assert _fit_labels(before, after, 200) == ("depth whole",)
+    assert _fit_labels(before, dict(after, cta_group=2), 200) == ("tiles of another width or pairing", "depth whole")
