@@ -90,6 +90,13 @@ def candidates(op: str, batch: int, m: int, n: int, k: int) -> list[dict]:
             continue
         for cta_group in (1, 2):
             if cta_group == 2 and m <= 128:
+                # Pairs on tiles of 128 rows, whole or split through a cluster, with the hints and the prefetch that
+                # ayla_b200_fit_depth gives them.
+                tiles = batch * -(-n // tile_n)
+                for s in (1, 2, 4) if m > 32 and tile_n in (128, 256) else ():
+                    if s * tile_n <= 512 and tiles * s <= SM_COUNT // 2 and (s == 1 or k_blocks >= 4 * s):
+                        out.append(dict(tile_n=tile_n, cta_group=2, group_m=8, split_k=s, cluster_split=int(s > 1),
+                                        l2_hint_a=2, l2_hint_b=1, early_prefetch=min(8, k_blocks // s // 2)))
                 continue
             base = dict(tile_n=tile_n, cta_group=cta_group, group_m=8)
             out.append(dict(base))

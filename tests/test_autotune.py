@@ -8,7 +8,7 @@ import json
 import pytest
 import torch
 
-from ayla_b200 import autotune
+from ayla_b200 import _lib, autotune
 
 
 def _row(op, dtype, batch, m, n, k, configs, torch_us=10.0):
@@ -33,6 +33,20 @@ def test_candidates_cover_the_regimes_the_table_relies_on():
     large = autotune.candidates("mm", 1, 4096, 4096, 4096)
     assert dict(tile_n=256, cta_group=2, group_m=8) in large and dict(tile_n=256, cta_group=2, group_m=8, split_tail=2) in large
     assert not any(c.get("swap_ab") for c in large)
+
+
+def test_candidates_for_few_rows_have_pairs():
+    def pairs(*shape):
+        found = [c for c in autotune.candidates(*shape) if c["cta_group"] == 2]
+        for c in found:
+            assert _lib.config_valid(_lib.Config.from_dict(c), shape[0], "bfloat16", *shape[1:]), c
+        return {(c["tile_n"], c["split_k"], c["cluster_split"]) for c in found}
+
+    assert pairs("mm", 1, 128, 4096, 4096) == {(128, 1, 0), (128, 2, 1), (256, 1, 0), (256, 2, 1)}
+    assert pairs("addmm", 1, 33, 1024, 4096) == {(128, 1, 0), (128, 2, 1), (128, 4, 1), (256, 1, 0), (256, 2, 1)}
+    assert pairs("mm", 1, 100, 14336, 4096) == {(256, 1, 0)}
+    assert pairs("bmm", 40, 64, 64, 448) == {(128, 1, 0)}
+    assert pairs("mm", 1, 32, 4096, 4096) == set()
 
 
 def test_emit_table_takes_a_shape_from_the_first_file_that_has_it(tmp_path):
