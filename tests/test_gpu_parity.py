@@ -9,6 +9,9 @@ while being the neighbouring representable value of the reference are rounding f
 of the last bit and are counted, not failed (``Parity.ok``).
 """
 
+import json
+import re
+
 import pytest
 import torch
 
@@ -62,6 +65,21 @@ def run_abi(operation, dtype, tensors, cfg, device_state, canary_rows=4):
     # rows past the end of `out` must still hold their poison
     assert bool(torch.isnan(store[store.shape[0] - canary_rows:]).all()), "kernel wrote past the output"
     return out, int(status.item())
+
+
+def launched_kernels(call, tmp_path):
+    """(name, bytes of shared memory) of every kernel that ``call`` launches, as the profiler records them."""
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        call()
+        torch.cuda.synchronize()
+    profile.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    kernels = [(e["name"], e["args"].get("shared memory")) for e in events if e.get("cat") == "kernel"]
+    if not kernels:
+        pytest.skip("no kernels from the profiler")
+    return kernels
 
 
 def assert_parity(out, ref32, what=""):
@@ -403,6 +421,45 @@ def test_pairs_on_tiles_of_128_rows(tile_n, split_k, device_state):
             assert int(status.item()) == 0 and bool(torch.isnan(store[batch * m:]).all()), what
             got = store[:batch * m].view(*lead, m, n).cpu()
             assert_parity(got, O.act_ref32(activation, ref) * factors.float(), f"{what} {entry.__name__}")
+
+
+@pytest.mark.parametrize("m, flat", [(33, True), (128, True), (129, False)])
+@pytest.mark.parametrize("operation, activation, tile_n, split_k", [("mm", "none", 128, 2), ("addmm", "gelu", 128, 1),
+                                                                    ("mm", "silu", 256, 1), ("addmm", "none", 256, 2)])
+def test_pairs_of_few_rows_run_the_kernel_of_64_rows_a_cta(operation, activation, tile_n, split_k, m, flat, device_state,
+                                                           tmp_path):
+    status, _ = device_state
+    a, bt = (torch.zeros(rows, 1024, dtype=torch.bfloat16, device=DEV) for rows in (m, 512))
+    out, bias = torch.empty(m, 512, dtype=torch.bfloat16, device=DEV), torch.zeros(512, dtype=torch.bfloat16, device=DEV)
+    cfg = _lib.Config.from_dict(dict(tile_n=tile_n, cta_group=2, split_k=split_k, cluster_split=int(split_k > 1), group_m=8))
+
+    def call():
+        _lib.gemm_act(operation, "bfloat16", activation, bias.data_ptr(), a.data_ptr(), bt.data_ptr(), out.data_ptr(), 1, m, 512,
+                      1024, cfg, 0, 0, status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+
+    [(name, _)] = launched_kernels(call, tmp_path)
+    traits = re.search(r"GemmTraits<([^>]*)>", name).group(1).split(", ")
+    assert traits[:2] == [str(tile_n), "2"] and (traits[6] == "3") == flat, name
+
+
+@pytest.mark.parametrize("tile_n, split_k", [(128, 2), (128, 4), (256, 2), (256, 4)])
+def test_pairs_of_few_rows_exchange_partial_sums_in_the_ring(tile_n, split_k, device_state):
+    """The exchange area over ring slots that are still in use, which no schedule of theirs needs: all partial sums wait."""
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(tile_n + split_k)
+    cfg = dict(tile_n=tile_n, cta_group=2, split_k=split_k, cluster_split=1)
+    for m, n, k in ((128, 520, 2048), (70, 264, 1992), (33, 136, 4096)):
+        a = torch.randn(m, k, generator=g).bfloat16()
+        bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+        want, code = run_abi("mm", "bfloat16", (a, bt), cfg, device_state)
+        assert code == 0
+        try:
+            lib.ayla_b200_debug_set_flags(2)
+            out, code = run_abi("mm", "bfloat16", (a, bt), cfg, device_state)
+        finally:
+            lib.ayla_b200_debug_set_flags(0)
+        assert code == 0 and torch.equal(out, want)
+        assert_parity(out, O.mm_ref32(a, bt), f"{m}x{n}x{k} {cfg}")
 
 
 def test_launch_overlap_keeps_stream_order(device_state):
@@ -1066,6 +1123,41 @@ def test_the_packed_kernels_form_is_the_faster_one(batch, m, n, k, piped):
     assert len(names) == 1 and ("packed_piped_kernel" in names[0]) == piped, names
 
 
+# (operation, batch, m, n, k), offset of the results in elements, CTAs on an SM whose share of its shared memory each takes (0: no more
+# than it needs)
+@pytest.mark.parametrize("operation, batch, m, n, k, offset, ctas", [
+    ("mm", 1, 125610, 80, 16, 0, 4), ("addmm", 1, 125610, 80, 16, 8, 4), ("bmm", 2500, 64, 96, 16, 0, 4),
+    ("bmm", 2500, 64, 96, 16, 8, 4), ("bmm", 5400, 26, 96, 8, 0, 4),
+    ("mm", 1, 75700, 72, 16, 0, 0), ("bmm", 4576, 47, 16, 16, 0, 0)])
+def test_packed_ctas_take_their_share_of_an_sm_from_one_and_a_half_rounds_on(operation, batch, m, n, k, offset, ctas, tmp_path):
+    _lib.init(0)
+    g = torch.Generator(device=DEV).manual_seed(m)
+    lead = (batch,) if operation == "bmm" else ()
+    a = torch.randn(*lead, m, k, device=DEV, generator=g).half()
+    bt = torch.randn(*lead, n, k, device=DEV, generator=g).half()
+    bias = torch.randn(n, device=DEV, generator=g).half()
+    store = torch.full((batch * m * n + 64 + offset,), 7.0, dtype=torch.float16, device=DEV)
+    out = store[offset:-64]
+    want = torch.empty(*lead, m, n, dtype=torch.float16, device=DEV)
+    status = _lib.StatusWord()
+    stream = torch.cuda.current_stream().cuda_stream
+    [(name, shared)] = launched_kernels(
+        lambda: _lib.gemm_packed(operation, "float16", bias.data_ptr(), a.data_ptr(), bt.data_ptr(), out.data_ptr(), batch, m, n, k,
+                                 status.ptr, stream), tmp_path)
+    _lib.gemm(operation, "float16", bias.data_ptr(), a.data_ptr(), bt.data_ptr(), want.data_ptr(), batch, m, n, k,
+              _lib.Config.from_dict(dict(tile_n=64)), 0, 0, status.ptr, stream)
+    torch.cuda.synchronize()
+    assert status.peek() == 0
+    assert torch.equal(out.view_as(want), want)
+    assert bool((store[:offset] == 7.0).all()) and bool((store[-64:] == 7.0).all())
+    assert "packed_gemm_kernel" in name, name
+    per_sm, reserve = 233472, 1024
+    if ctas:
+        assert shared >= per_sm // ctas - reserve, (shared, per_sm // ctas - reserve)
+    else:
+        assert shared < per_sm // 4 - reserve
+
+
 @pytest.mark.parametrize("batch, m, n, k", [(1097, 19, 96, 128), (151, 301, 80, 88), (1, 124739, 112, 112)])
 def test_results_inside_a_sector_take_the_packed_kernel_only_where_their_staging_rows_fit(batch, m, n, k):
     """Rows written straight from registers make room for a second CTA on an SM; an ``out`` that starts inside a sector
@@ -1532,6 +1624,30 @@ def test_timed_out_cluster_split_leaves_the_context_usable(config, device_state)
     out, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
     assert status == 0
     assert_parity(out, O.mm_ref32(a, bt), f"after a timed-out cluster split {config}")
+
+
+@pytest.mark.parametrize("config", [dict(tile_n=128, split_k=1), dict(tile_n=128, split_k=2), dict(tile_n=128, split_k=4),
+                                    dict(tile_n=256, split_k=1), dict(tile_n=256, split_k=2), dict(tile_n=256, split_k=4)])
+@pytest.mark.parametrize("m", [40, 128])
+def test_timed_out_pairs_of_few_rows_leave_the_context_usable(m, config, device_state):
+    """Pairs on 128-row tiles with their loads withheld, whole and in clusters of two and four pairs."""
+    n, k = 1024, 2048
+    g = torch.Generator().manual_seed(m)
+    a = torch.randn(m, k, generator=g).bfloat16()
+    bt = (torch.randn(n, k, generator=g) * k ** -0.5).bfloat16()
+    config = dict(config, cta_group=2, cluster_split=int(config["split_k"] > 1))
+    lib = _lib.load()
+    try:
+        lib.ayla_b200_set_wait_timeout_ms(20)
+        lib.ayla_b200_debug_set_flags(1)
+        _, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    finally:
+        lib.ayla_b200_debug_set_flags(0)
+        lib.ayla_b200_set_wait_timeout_ms(2000)
+    assert status & 0xFF != 0
+    out, status = run_abi("mm", "bfloat16", (a, bt), config, device_state)
+    assert status == 0
+    assert_parity(out, O.mm_ref32(a, bt), f"after timed-out pairs {config}")
 
 
 @pytest.mark.parametrize("m, n, k", [(8, 1024, 2048), (100, 1024, 1024), (60, 4096, 512)])
