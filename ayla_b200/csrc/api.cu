@@ -809,7 +809,8 @@ bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& mac
 //    1.02.
 //
 // `cautious`: ayla_b200_share_depth keeps the bounds that it has for last waves whose rows start inside a sector: two ways at
-// most, behind one whole wave, behind two with a quarter of a wave left, or where the schedule has halves.
+// most, behind one whole wave, behind two with a quarter of a wave left, or where the schedule has halves.  No op asks for that
+// entry's answers; callers of the library may.
 void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, bool cautious, ayla_b200_config* c) {
   if (c->swap_ab || c->stream_k || c->grid_ctas != 0 || c->split_tail == 1) return;
   if (c->split_k > 1 && !c->cluster_split && c->split_tail != 0) return;

@@ -171,12 +171,16 @@ struct GemmTraits {
   // SHARED: whole tiles, and k-splits, one unit per CTA, that share their sum through the workspace.
   static constexpr bool SHARED = FORM_ == FORM_SHARED;
   static constexpr bool FULL = FORM_ == FORM_FULL;
-  // FLAT: a CTA pair on a tile of 128 rows, 64 per CTA, for products of at most 128 rows; whole tiles and clusters.  What
-  // bounds those is the rate at which an SM takes operands (some 57 bytes a clock): a pair reads half of the rows and half
-  // of the columns per CTA where a single CTA of the same share of the result reads all rows.  The accumulator lies in
-  // BN / 2 columns: TMEM lanes 0..63 hold the left half of the tile's columns, lanes 64..127 the right one.  A k-block takes
-  // 0.176 us with 128 columns and 0.377 with 256, all SMs at work.  us, single CTAs -> pairs: mm 128x4096x4096 (split in two,
-  // 64 -> 128 columns) 11.8 -> 10.3, 128x8192x2048 11.4 -> 9.5, 128x14336x4096 25.0 -> 23.3, addmm 100x3584x2560 9.3 -> 7.8.
+  // FLAT: a CTA pair on a tile of 128 rows, 64 per CTA, for products of at most 128 rows; whole tiles and clusters.  A pair reads
+  // half of the rows and half of the columns per CTA where a single CTA of the same share of the result reads all rows.  The
+  // accumulator lies in BN / 2 columns: TMEM lanes 0..63 hold the left half of the tile's columns, lanes 64..127 the right one.
+  // What bounds them: us a k-block, weights from L2 | from DRAM (slopes from 16 to 32 k-blocks, graph replay, 1.9 GHz):
+  //   128 columns  18 tiles .105 | .109   37 tiles .111 | .120   74 tiles .131 | .163
+  //   256 columns           .143 | .179            .149 | .209            .237 | .345
+  // With all SMs at work the weights' stream, 7.0 to 7.5 TB/s with what L2 still holds of it; from L2 what it sends, 54 to 65
+  // bytes a clock to each SM; with few tiles the MMAs of 256 columns (256 cycles, .135).  us, single CTAs -> pairs: mm
+  // 128x4096x4096 (split in two, 64 -> 128 columns) 11.8 -> 10.3, 128x8192x2048 11.4 -> 9.5, 128x14336x4096 25.0 -> 23.3, addmm
+  // 100x3584x2560 9.3 -> 7.8.
   static constexpr bool FLAT = FORM_ == FORM_FLAT;
   static constexpr bool CLUSTERS = FULL || FLAT;  // has the k-split through clusters
   // ACT: the epilogue applies the activation named in the launch parameters.  A separate set of
