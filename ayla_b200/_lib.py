@@ -28,6 +28,7 @@ EXPORTS = (
     "ayla_b200_gemm_static_scratch",
     "ayla_b200_gemm_packed",
     "ayla_b200_packed_preferred",
+    "ayla_b200_packed_preferred_at",
     "ayla_b200_swiglu",
     "ayla_b200_rms_factors",
     "ayla_b200_default_config",
@@ -137,6 +138,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_gemm_packed.restype = i32
         lib.ayla_b200_packed_preferred.argtypes = [i32, i64, i64, i64, i64]
         lib.ayla_b200_packed_preferred.restype = i32
+        lib.ayla_b200_packed_preferred_at.argtypes = [i32, i64, i64, i64, i64, vp]
+        lib.ayla_b200_packed_preferred_at.restype = i32
         lib.ayla_b200_swiglu.argtypes = [i32, vp, vp, vp, vp, i64, i64, i64, cfgp, vp, vp]
         lib.ayla_b200_swiglu.restype = i32
         lib.ayla_b200_rms_factors.argtypes = [i32, vp, vp, i64, i64, ctypes.c_float, vp]
@@ -338,9 +341,9 @@ def gemm_act_rowmul(op: str, dtype: str, activation: str, bias_ptr: int, a_ptr: 
         workspace_size, status_ptr or None, stream or None))
 
 
-def packed_preferred(op: str, batch: int, m: int, n: int, k: int) -> bool:
-    """Whether ``gemm_packed`` is the faster way to run the problem."""
-    return bool(load().ayla_b200_packed_preferred(OP_CODES[op], batch, m, n, k))
+def packed_preferred(op: str, batch: int, m: int, n: int, k: int, out_ptr: int = 0) -> bool:
+    """Whether ``gemm_packed`` is the faster way to run the problem, with results on 32 bytes or at ``out_ptr``."""
+    return bool(load().ayla_b200_packed_preferred_at(OP_CODES[op], batch, m, n, k, out_ptr or None))
 
 
 def gemm_packed(op: str, dtype: str, bias_ptr: int, a_ptr: int, bt_ptr: int, out_ptr: int, batch: int, m: int,

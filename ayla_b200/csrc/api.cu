@@ -1572,8 +1572,12 @@ int ayla_b200_gemm_packed(int op, int dtype, const void* bias, const void* a, co
 }
 
 int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k) {
+  return ayla_b200_packed_preferred_at(op, batch, m, n, k, nullptr);
+}
+
+int ayla_b200_packed_preferred_at(int op, int64_t batch, int64_t m, int64_t n, int64_t k, const void* out) {
   if (check_shape(op, AYLA_B200_BF16, batch, m, n, k) != AYLA_B200_OK) return 0;
-  return packed_preferred(batch, m, n, k, current_sm_count(), true) ? 1 : 0;
+  return packed_preferred(batch, m, n, k, current_sm_count(), on_sectors(out)) ? 1 : 0;
 }
 
 int ayla_b200_gemm_static_scratch(int op, int dtype, const void* bias, const void* a, const void* bt,

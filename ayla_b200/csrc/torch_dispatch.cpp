@@ -44,6 +44,7 @@ struct Launch {
   bool has_bias = false, gated = false;
   int64_t batch = 0, m = 0, n = 0, k = 0;
   const void* config = nullptr;
+  const void* inside_config = nullptr;  // instead, if given, for results that start inside a 32-byte sector
   void* workspace = nullptr;
   size_t workspace_bytes = 0;
   uint32_t* status = nullptr;
@@ -136,8 +137,9 @@ class Dispatcher {
     const void* a = *next++;
     const void* bt = *next++;
     const void* mul = l->gated ? *next++ : nullptr;
-    return reinterpret_cast<GemmFn>(l->entry)(l->op, l->dtype, l->activation, bias, a, bt, mul,
-                                              const_cast<void*>(*next), l->batch, l->m, l->n, l->k, l->config,
+    const bool inside = l->inside_config != nullptr && (reinterpret_cast<uintptr_t>(*next) & 31) != 0;
+    return reinterpret_cast<GemmFn>(l->entry)(l->op, l->dtype, l->activation, bias, a, bt, mul, const_cast<void*>(*next),
+                                              l->batch, l->m, l->n, l->k, inside ? l->inside_config : l->config,
                                               l->workspace, l->workspace_bytes, l->status, stream) == 0;
   }
 
@@ -162,6 +164,7 @@ class Dispatcher {
     l->n = fields["n"].cast<int64_t>();
     l->k = fields["k"].cast<int64_t>();
     l->config = reinterpret_cast<const void*>(fields["config"].cast<uintptr_t>());
+    if (fields.contains("inside_config")) l->inside_config = reinterpret_cast<const void*>(fields["inside_config"].cast<uintptr_t>());
     l->workspace = reinterpret_cast<void*>(fields["workspace"].cast<uintptr_t>());
     l->workspace_bytes = fields["workspace_bytes"].cast<size_t>();
     l->status = reinterpret_cast<uint32_t*>(fields["status"].cast<uintptr_t>());

@@ -346,14 +346,15 @@ class GemmLauncher:
     error is correct again.  ``check_status()`` does the same after a synchronise, and
     ``AYLA_B200_DEBUG=1`` calls it after every launch.
 
-    It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the library is given none and
-    takes the packed kernel, or for an ``out`` on 16 bytes alone its default schedule where that is the faster one;
-    ``seed`` and ``config`` are not used.
+    It runs the schedule it is given.  With ``packed`` (for what ``packed_serves`` says) the launch goes to the
+    packed kernel instead, and ``seed`` and ``config`` are used for an ``out`` on 16 bytes alone where the general
+    kernel is then the faster one.
     """
 
     _captured_only_where_run = True  # a capture on a stream where this launcher has not run is refused
     _unsplit_config: _lib.Config | None = None
     _unsplit_tail: tuple | None = None
+    _inside_tail: tuple | None = None  # for results that start inside a 32-byte sector
 
     def __init__(self, operation: str, dtype: str, batch: int, m: int, n: int, k: int,
                  seed: GemmScheduleSeed, device: torch.device, activation: str = "none",
@@ -367,7 +368,7 @@ class GemmLauncher:
         index = device.index if device.index is not None else torch.cuda.current_device()
         with torch.cuda.device(index):
             _lib.init(index)
-        self._packed = packed  # the library is given no schedule, and takes that kernel
+        self._packed = packed  # the library takes that kernel where it is given no schedule
         need = 0 if self._packed else _lib.workspace_bytes(self.config, operation, batch, m, n, k)
         self._ws_bytes = need
         self.workspace = None
@@ -392,6 +393,10 @@ class GemmLauncher:
         self._head = (_lib.OP_CODES[operation], _lib.DTYPE_CODES[dtype], _lib.ACT_CODES[activation])
         self._tail = (batch, m, n, k, None if self._packed else ctypes.byref(self.config), self._ws_ptr or None,
                       self._ws_bytes, self._status_ptr)
+        if self._packed and not _lib.workspace_bytes(self.config, operation, batch, m, n, k):
+            with torch.cuda.device(index):
+                if not _lib.packed_preferred(operation, batch, m, n, k, 16):
+                    self._inside_tail = (batch, m, n, k, ctypes.byref(self.config), None, 0, self._status_ptr)
         self._has_bias = operation == "addmm"
         self._device_index = index
         self._captured_only_where_run = not seed.adaptations
@@ -425,6 +430,8 @@ class GemmLauncher:
         tail = self._tail
         if self._ws_bytes:
             tail = self._tail_for_stream(stream)
+        elif self._inside_tail is not None and out.data_ptr() & 31:
+            tail = self._inside_tail
         # The library launches on the current device (the reference's launcher guards the device
         # the same way, ayla/ptx_runtime.py:268-275).
         if torch.cuda.current_device() != self._device_index:
@@ -453,6 +460,7 @@ class GemmLauncher:
             "has_bias": self._has_bias, "gated": bool(self.gated),
             "batch": self.batch, "m": self.m, "n": self.n, "k": self.k,
             "config": 0 if self._packed else ctypes.addressof(self.config),
+            "inside_config": 0 if self._inside_tail is None else ctypes.addressof(self.config),
             "workspace": self._ws_ptr, "workspace_bytes": self._ws_bytes,
             "status": self._status_ptr, "home_stream": self._home_stream or 0, "device": self._device_index,
         }

@@ -219,9 +219,12 @@ AYLA_B200_API int ayla_b200_gemm_packed(int op, int dtype, const void* bias, con
 /*
  * 1 where ayla_b200_gemm_packed is the faster way to run the problem with `out` on a 32-byte boundary, else 0:
  * there ayla_b200_gemm takes it by itself when cfg == NULL.  For an `out` on 16 bytes alone it looks again, since
- * the results then need more shared memory, and takes the general kernel where that is the faster one.
+ * the results then need more shared memory, and takes the general kernel where that is the faster one: what it does
+ * is what the second function says of that `out`, which is not read or written.
  */
 AYLA_B200_API int ayla_b200_packed_preferred(int op, int64_t batch, int64_t m, int64_t n, int64_t k);
+AYLA_B200_API int ayla_b200_packed_preferred_at(int op, int64_t batch, int64_t m, int64_t n, int64_t k,
+                                                const void* out);
 
 /*
  * out[M,N] = silu(x[M,K] @ w_gate[N,K]^T) * (x @ w_up[N,K]^T), both products kept

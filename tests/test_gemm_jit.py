@@ -448,3 +448,38 @@ def test_labels_of_a_depth_that_is_whole_again():
     after = dict(before, split_k=1, cluster_split=0)
     assert _fit_labels(before, after, 200) == ("depth whole",)
     assert _fit_labels(before, dict(after, cta_group=2), 200) == ("tiles of another width or pairing", "depth whole")
+
+
+@pytest.mark.parametrize("operation, batch, m, n, k, own", [
+    ("mm", 1, 186073, 96, 80, True), ("bmm", 1097, 19, 96, 128, True), ("bmm", 151, 301, 80, 88, True),
+    ("mm", 1, 65536, 32, 32, False), ("bmm", 8192, 56, 32, 56, False)])
+def test_results_inside_a_sector_run_the_ops_schedule_where_packed_is_not_preferred(operation, batch, m, n, k, own, monkeypatch):
+    import contextlib
+    import ctypes
+    import types
+
+    from ayla_b200 import gemm_jit
+
+    monkeypatch.setattr(torch.cuda, "device", lambda index: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index=None: types.SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(_lib, "init", lambda index: None)
+    monkeypatch.setattr(_lib, "StatusWord", lambda: types.SimpleNamespace(ptr=16, peek=lambda: 0))
+    monkeypatch.delenv("AYLA_B200_DEBUG", raising=False)
+    assert _lib.packed_preferred(operation, batch, m, n, k)
+    assert _lib.packed_preferred(operation, batch, m, n, k, 1 << 20)
+    assert _lib.packed_preferred(operation, batch, m, n, k, (1 << 20) + 16) is not own
+    seed = select_gemm_schedule(operation, "bfloat16", m, n, k, batch)
+    launcher = gemm_jit.GemmLauncher(operation, "bfloat16", batch, m, n, k, seed, torch.device("cpu"), packed=True)
+    call = launcher.native_call()
+    assert call["config"] == 0 and call["inside_config"] == (ctypes.addressof(launcher.config) if own else 0)
+    assert launcher.config.to_dict() == seed.builder_config
+
+    # ... in the Python dispatcher as well
+    given = []
+    launcher._entry = lambda *args: given.append(args) or 0
+    for address in (1 << 20, (1 << 20) + 16):
+        tensor = types.SimpleNamespace(data_ptr=lambda: 1 << 20)
+        launcher(tensor, tensor, types.SimpleNamespace(data_ptr=lambda: address))
+    configs = [args[12] for args in given]
+    assert configs[0] is None and (configs[1] is not None) is own

@@ -16,7 +16,7 @@ import pytest
 import torch
 
 from ayla_b200 import _lib, gemm_act_op, gemm_op, gemm_op_compiler, swiglu_op, swiglu_op_compiler
-from ayla_b200.gemm_jit import gemm_jit_compiler
+from ayla_b200.gemm_jit import gemm_jit_compiler, select_gemm_schedule
 from oracle import gemm_oracle as O
 from tests.conftest import load_golden_cases
 
@@ -1158,7 +1158,7 @@ def test_packed_ctas_take_their_share_of_an_sm_from_one_and_a_half_rounds_on(ope
         assert shared < per_sm // 4 - reserve
 
 
-@pytest.mark.parametrize("batch, m, n, k", [(1097, 19, 96, 128), (151, 301, 80, 88), (1, 124739, 112, 112)])
+@pytest.mark.parametrize("batch, m, n, k", [(1097, 19, 96, 128), (151, 301, 80, 88), (1, 124739, 112, 112), (1, 186073, 96, 80)])
 def test_results_inside_a_sector_take_the_packed_kernel_only_where_their_staging_rows_fit(batch, m, n, k):
     """Rows written straight from registers make room for a second CTA on an SM; an ``out`` that starts inside a sector
     needs staging rows, which leave room for one, and the general kernel is the faster one."""
@@ -1183,6 +1183,9 @@ def test_results_inside_a_sector_take_the_packed_kernel_only_where_their_staging
     if not kernels:
         pytest.skip("no kernel names from the profiler")
     assert len(kernels) == 2 and "packed" in kernels[0] and "gemm_sm100" in kernels[1], kernels
+    config = select_gemm_schedule(operation, "bfloat16", m, n, k, batch).builder_config  # not the library's default
+    traits = re.search(r"GemmTraits<(\d+), (\d), ", kernels[1]).groups()
+    assert traits == (str(config["tile_n"]), str(config["cta_group"])), kernels
 
 
 @pytest.mark.parametrize("batch, m, n, k", [(1, 70000, 96, 24), (2055, 45, 16, 120), (600, 128, 64, 40)])
