@@ -35,6 +35,7 @@ EXPORTS = (
     "ayla_b200_default_config_act",
     "ayla_b200_share_depth",
     "ayla_b200_fit_depth",
+    "ayla_b200_fit_depth_act",
     "ayla_b200_swiglu_default_config",
     "ayla_b200_config_valid",
     "ayla_b200_workspace_bytes",
@@ -152,6 +153,8 @@ def load() -> ctypes.CDLL:
         lib.ayla_b200_share_depth.restype = i32
         lib.ayla_b200_fit_depth.argtypes = [i32, i32, i64, i64, i64, i64, cfgp]
         lib.ayla_b200_fit_depth.restype = i32
+        lib.ayla_b200_fit_depth_act.argtypes = [i32, i32, i32, i64, i64, i64, i64, cfgp]
+        lib.ayla_b200_fit_depth_act.restype = i32
         lib.ayla_b200_swiglu_default_config.argtypes = [i32, i64, i64, i64, cfgp]
         lib.ayla_b200_swiglu_default_config.restype = i32
         lib.ayla_b200_config_valid.argtypes = [cfgp, i32, i32, i64, i64, i64, i64]
@@ -260,10 +263,11 @@ def share_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k:
     return out
 
 
-def fit_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k: int) -> Config:
+def fit_depth(cfg: Config, op: str, dtype: str, batch: int, m: int, n: int, k: int, activation: str = "none") -> Config:
     """``cfg``, or what it becomes where other tiles or a shared depth fit the shape better."""
     out = Config.from_dict(cfg.to_dict())
-    check(load().ayla_b200_fit_depth(OP_CODES[op], DTYPE_CODES[dtype], batch, m, n, k, ctypes.byref(out)))
+    check(load().ayla_b200_fit_depth_act(OP_CODES[op], DTYPE_CODES[dtype], ACT_CODES[activation], batch, m, n, k,
+                                         ctypes.byref(out)))
     return out
 
 

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -732,29 +733,42 @@ double scheduled_us(int64_t batch, int64_t m, int64_t n, int64_t k, const Machin
                      c.cluster_split ? RATE_CLUSTER : c.split_k > 1 ? RATE_SHARED : RATE_WHOLE, tiles, k, machine);
 }
 
+// Whether wider tiles in one wave pay for 128-wide pairs in more (whole sectors).  Those hide a tile's results under the next one's
+// MMAs, and take less than the model says when shallow; what a lone wide tile shows of its results depends on the activation, and
+// rows that start inside a 128-byte line cost the narrower tiles more.  2873 shapes timed both ways, of their time where taken, and
+// where not (us, 128-wide pairs -> one wave: mm 9457x384x1280 13.7 -> 12.0; addmm 1147x1920x1408 + GELU 10.1 -> 11.6):
+//   none                 578 taken, 0.893, nine of them slower by 2 %; 35 not, 1.01
+//   ReLU or row factors  721, 0.916, 15; 226, 1.04
+//   others               552, 0.916, 12; 761, 1.06
+bool wider_tiles_pay(int64_t tiles, int64_t wave, int64_t k, int activation) {
+  const int64_t k_blocks = ceil_div(k, 64), rest = tiles % wave;
+  const bool lines = k % 64 == 0, many = rest * 10 > wave * 3;
+  if (activation == AYLA_B200_ACT_NONE) return !lines || k_blocks >= 14 || many;
+  if (activation == AYLA_B200_ACT_RELU) return k_blocks >= (lines && !many ? 18 : 15);
+  return k_blocks >= (lines && rest * 2 <= wave ? 33 : 21);
+}
+
 // Whole tiles of the best other width or pairing that all run at once, for a schedule measured on another shape whose tiles
 // fit this one badly; false where there is none 8 % faster by the model.  (us, the schedule -> this: 5539x384x4096 + GELU,
 // 256-wide pairs in 1 + 14/74 waves -> 128-wide ones, 30.4 -> 19.9; 1240x2176x28672, 45 pairs of 256 columns -> 60 of 192, 157
 // -> 137; 620x7232x1664, three rows of pairs -> five of single CTAs, 19.8 -> 16.8; 119x5312x832, clusters in two waves -> 64
-// columns, 7.5 -> 5.7.)  Not for the shallowest (mm 1759x1344x640 7.0 -> 8.0).  With whole sectors not
-//  * with wider tiles in place of 128-wide pairs up to 23 k-blocks, whose several waves take less than the model says (addmm
-//    1147x1920x1408 + GELU, 22, 10.1 -> 11.6; 990x2368x768 6.5 -> 7.2, 8586x448x896 + GELU 11.1 -> 12.0; from 24 on 0.88 to
-//    0.99 in eight shapes);
-//  * with pairs in place of single CTAs of the same 256 columns up to 23 (nine of eleven 1.01 to 1.04: addmm 1722x2560x768
-//    8.2 -> 8.5).
+// columns, 7.5 -> 5.7.)  Not for the shallowest (mm 1759x1344x640 7.0 -> 8.0).  No pairs in place of single CTAs of the same 256
+// columns up to 23 k-blocks of whole lines (182 shapes 1.03 of the time, addmm 1722x2560x768 8.2 -> 8.5; 61 whose rows start inside
+// a 128-byte line 0.93, none slower).
 // Not in place of clusters whose rows start inside a sector (mm 200x3208x2456 13.1 -> 14.6), of one product's 64-wide ones whose rows
-// start inside a 128-byte line from 21 k-blocks on (seven shapes 0.90 to 1.06, whole lines and fewer 0.76 to 0.96: addmm
-// 179x768x1296 + ReLU 6.6 -> 7.0), nor of 256-wide ones of single CTAs (addmm 282x5440x3776 21.3 -> 23.8).
-bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+// start inside a line from 21 k-blocks on (seven shapes 0.90 to 1.06, whole lines and fewer 0.76 to 0.96: addmm 179x768x1296 +
+// ReLU 6.6 -> 7.0), nor of 256-wide ones of single CTAs (addmm 282x5440x3776 21.3 -> 23.8).
+bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, const Machine& machine, ayla_b200_config* c) {
   const bool mid_sector = k % 16 != 0;
   if (m <= 64 || k <= 704) return false;
   if (c->cluster_split && (mid_sector || (c->tile_n == 256 && c->cta_group == 1))) return false;
   if (c->cluster_split && c->tile_n == 64 && batch == 1 && k % 64 != 0 && k > 20 * 64) return false;
   const int64_t wave = machine.sm_count / c->cta_group;
-  if (batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n) > wave &&
-      (c->split_k > 1 || c->cluster_split || c->tile_n < 128)) {
-    return false;
-  }
+  const int64_t own_tiles = batch * ceil_div(m, 128 * c->cta_group) * ceil_div(n, c->tile_n);
+  if (own_tiles > wave && (c->split_k > 1 || c->cluster_split || c->tile_n < 128)) return false;
+  const bool no_wider = !mid_sector && c->tile_n == 128 && c->cta_group == 2 && own_tiles > wave &&
+                        !wider_tiles_pay(own_tiles, wave, k, activation);
+  const bool no_pairs = k % 64 == 0 && c->tile_n == 256 && c->cta_group == 1 && k <= 23 * 64;
   double best = 0.92 * scheduled_us(batch, m, n, k, machine, *c);
   ayla_b200_config chosen = *c;
   chosen.split_k = 1;
@@ -766,8 +780,7 @@ bool one_wave(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& mac
       if (cta_group == 2 && m <= 128) continue;
       const int64_t tiles = batch * ceil_div(m, 128 * cta_group) * ceil_div(n, tile_n);
       if (tiles > machine.sm_count / cta_group) continue;
-      if (!mid_sector && c->tile_n == 128 && c->cta_group == 2 && tile_n > 128 && k <= 23 * 64) continue;
-      if (!mid_sector && c->tile_n == 256 && c->cta_group == 1 && tile_n == 256 && cta_group == 2 && k <= 23 * 64) continue;
+      if ((no_wider && tile_n > 128) || (no_pairs && tile_n == 256 && cta_group == 2)) continue;
       const double us = modelled_us(tile_n, cta_group, 1, RATE_WHOLE, tiles, k, machine);
       if (us >= best) continue;
       best = us;
@@ -901,17 +914,20 @@ void share_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& 
 // Of 33 to 64 rows only in place of a split depth: single CTAs on whole tiles load just the rows that exist (36x5632x1664 7.7 ->
 // 8.3).  The swapped form's own model is fitted to 200 timings (4 to 6 % rms; eight-way clusters and narrower accumulators stay, pairs
 // take 1.1 to 1.4 of their time).
-// Timed besides over 2729 shapes that the models alone took, thin and batched ones and every measured schedule that changes
-// among them: the bounds below leave 2308 of those, in 0.893 of the time, 21 slower by 2 % and the slowest by 7 % (addmm
-// 64x312x1872 + ReLU 5.9 -> 6.3); the 416 others took 0.965, up to 1.31.  Of 790 drawn afterwards: 0.889, 12 slower by 2 %, the
-// slowest by 8.5 % (36x1632x1464 5.9 -> 6.4); the 42 measured schedules that change: 0.906, the slowest by 1 %.
-//  * Rows inside a sector cost narrow tiles less than the models say, the more so where the depth is split (mm 64x104x13320, 16
-//    ways, 10.7 -> 14.1; addmm 64x104x10520, eight ways, 10.4 -> 12.3), and batches of whole 128-wide tiles (17 x 78x944x392 5.8
-//    -> 6.5); a pair that has neither rows nor columns for its second CTA stays single there (11 x 37x64x3576 7.7 -> 8.8).
-//  * Tiles with three eighths of their columns past the product: not in place of depths split twelve ways and more (mm 65x32x15984
-//    10.4 -> 11.6) nor with nearly as many clusters as run at once (bmm 33 x 72x72x1512 7.0 -> 7.9, 24 x 64x64x1024 8.5 -> 9.0).
-//  * No split depth in place of whole 64-wide tiles up to 16 k-blocks (mm 128x4096x1024 8.2 -> 8.9, 94x3456x1024 5.3 -> 5.7).
-bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+// Besides, what the models miss, from 6700 shapes timed both ways, thin and batched ones and every measured schedule that
+// changes among them: `amiss` is how much the log of the modelled ratio falls short, by terms of
+//  * rows: single CTAs load the rows that exist, a pair's second CTA a box of 64 whatever is in it, the more so where rows start
+//    inside a sector (clusters of four pairs for those of four 64-wide CTAs: of 33 to 64 rows 0.93 of the time and of more than 96
+//    0.895, inside a sector 1.00 and 0.91);
+//  * clusters nearly as many as run at once, mostly of padding in particular (bmm 33 x 72x72x1512 7.0 -> 7.9);
+//  * depths split twelve ways and more (mm 65x32x15984 10.4 -> 11.6, 64x104x13320, inside a sector, 10.7 -> 14.1), inside a sector
+//    eight ways (addmm 64x104x10520 10.4 -> 12.3), whole tiles of a batch (17 x 78x944x392 5.8 -> 6.5; but of one product they
+//    gain more than modelled) and whole tiles for clusters;
+//  * an activation (0.04 of the log, no more is known of it).
+// No split depth in place of whole 64-wide tiles up to 16 k-blocks (mm 128x4096x1024 split in two 1.09 of the time, whole 0.85).
+// By them 5724 of those shapes are taken, in 0.90 of the time, 103 slower by 2 %, at most 1.11; the others took 1.02, up to 1.31.  The
+// swapped form needs none (430 shapes 0.87, one slower by 2 %).
+bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, const Machine& machine, ayla_b200_config* c) {
   const int64_t k_blocks = ceil_div(k, 64);
   if (m <= 32 || m > 128 || c->stream_k || c->grid_ctas != 0) return false;
   if (m <= 64 ? c->split_k == 1 || k_blocks < 16 : c->swap_ab || k_blocks < (c->tile_n == 64 ? 12 : 7)) return false;
@@ -939,11 +955,7 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
     } else if (c->tile_n == 128) {
       own *= c->cluster_split ? (c->split_k == 2 ? 1.02 : 1.0) : mid_sector ? 1.0 : 1.05;
     }
-    if (mid_sector && c->tile_n == 64) own *= c->split_k == 1 ? 0.95 : c->split_k == 2 ? 0.92 : c->cluster_split ? 0.9 : 0.85;
-    if (mid_sector && c->tile_n == 128 && c->split_k == 1 && batch > 1) own *= 0.86;
   }
-  if (batch > 1) own *= 0.97;
-  if (mid_sector && m <= 64 && n <= 64) return false;
   struct Flat { int tile_n, split; double launch, block, block_busy; };
   static const Flat kFlat[5] = {{128, 1, 4.17, .099, .077}, {128, 2, 4.85, .105, .082}, {128, 4, 5.69, .095, .091},
                                 {256, 1, 4.44, .126, .227}, {256, 2, 5.08, .163, .247}};
@@ -953,8 +965,7 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
   for (const Flat& f : kFlat) {
     const int64_t tiles = batch * ceil_div(n, f.tile_n);
     if (tiles > machine.clusters(2 * f.split) || (f.split > 1 && k_blocks < 4 * f.split)) continue;
-    if (n * 8 <= f.tile_n * 5 && (c->split_k >= 12 || tiles * 3 > machine.clusters4 * 2)) continue;
-    if (f.split > 1 && c->split_k == 1 && k_blocks <= 16 && !mid_sector) continue;
+    if (f.split > 1 && c->split_k == 1 && c->tile_n == 64 && k_blocks <= 16 && !mid_sector) continue;
     const double busy = static_cast<double>(tiles * f.split) / static_cast<double>(pairs);
     const double us = f.launch + static_cast<double>(ceil_div(k_blocks, f.split)) * (mid_sector ? 1.4 : 1.0) *
                                      (f.block + f.block_busy * busy);
@@ -963,6 +974,20 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
     chosen = &f;
   }
   if (chosen == nullptr) return false;
+  if (!c->swap_ab) {
+    const int64_t tiles = batch * ceil_div(n, chosen->tile_n);
+    const bool shared = c->split_k > 1 && !c->cluster_split;
+    double amiss = (mid_sector ? 0.40 : 0.17) * static_cast<double>(128 - m) / 128.0;
+    if ((chosen->split == 2 && tiles * 3 > machine.clusters4 * 2) || (chosen->split == 4 && tiles * 2 > machine.clusters8)) {
+      amiss += (mid_sector ? 0.085 : 0.05) + (n * 8 <= chosen->tile_n * 5 ? 0.1 : 0.0);
+    }
+    if (shared && c->split_k >= 12) amiss += mid_sector ? 0.31 : k_blocks > 213 ? 0.17 : 0.12;
+    if (mid_sector && shared && c->tile_n == 64 && c->split_k >= 8 && c->split_k < 12) amiss += 0.085;
+    if (mid_sector && c->tile_n == 128 && c->split_k == 1) amiss += batch > 1 ? 0.17 : -0.16;
+    if (mid_sector && c->tile_n == 64 && c->cluster_split && c->split_k == 2 && chosen->split == 1) amiss += 0.12;
+    if (activation != AYLA_B200_ACT_NONE) amiss += 0.04;
+    if (best * std::exp(amiss) >= 1.1 * own) return false;
+  }
   c->tile_n = chosen->tile_n;
   c->cta_group = 2;
   c->swap_ab = 0;
@@ -981,23 +1006,24 @@ bool flat_pairs(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& m
 
 // A schedule that was measured elsewhere, or here without what this knows: with its depth shared out, or with tiles that fit
 // the shape in one wave, and their depth shared out, where that takes 0.92 of the time by the models; or on flat pairs.  Beside
-// 128-wide pairs whose last wave is split, whole 192-wide ones count with the k-blocks of a last wave's model: their operands
-// outgrow L2, and by the rate of a single wave mm 2200x1216x35136 took them, 174 -> 191, and 1304x1808x33888, 179 -> 204 (eleven
-// such shapes: the four still taken 0.75 to 0.94, the others 0.97 to 1.13).  Of 954 shapes drawn over all kinds that get whole
-// tiles so, 0.863 of the time, four slower by 2 % (the slowest 186x8008x3992 + SiLU, rows inside a sector, 25 -> 29).
-void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, const Machine& machine, ayla_b200_config* c) {
+// 128-wide pairs whose last wave is split, whole wider ones count with the k-blocks of a last wave's model: their operands outgrow
+// L2, and by the rate of a single wave mm 2200x1216x35136 took them, 174 -> 191, and 1304x1808x33888, 179 -> 204 (of eleven such
+// shapes the four still taken 0.75 to 0.94, the others 0.97 to 1.13; of 63 that are 64 to 100 k-blocks deep, none of them taken,
+// 1.03).  An activation of RELU stands for row factors too.  Of 12000 shapes drawn over all kinds when these rules stood, 3300 change; 883
+// of them timed take 0.914 of the time, 13 are slower by 2 %, at most 1.06.
+void fit_depth(int64_t batch, int64_t m, int64_t n, int64_t k, int activation, const Machine& machine, ayla_b200_config* c) {
   ayla_b200_config fitted = *c;
   share_depth(batch, m, n, k, machine, false, c);
-  if (!fitted.swap_ab && !fitted.stream_k && fitted.grid_ctas == 0 && one_wave(batch, m, n, k, machine, &fitted)) {
+  if (!fitted.swap_ab && !fitted.stream_k && fitted.grid_ctas == 0 && one_wave(batch, m, n, k, activation, machine, &fitted)) {
     share_depth(batch, m, n, k, machine, false, &fitted);
     double us = scheduled_us(batch, m, n, k, machine, fitted);
-    if (c->tile_n == 128 && c->split_tail == 1 && fitted.tile_n == 192 && fitted.split_k == 1) {
-      const double deep = 4.3 + static_cast<double>(ceil_div(k, 64)) * block_us(192) * (k % 16 != 0 ? 1.2 : 1.0);
+    if (c->tile_n == 128 && c->split_tail == 1 && fitted.tile_n > 128 && fitted.split_k == 1) {
+      const double deep = 4.3 + static_cast<double>(ceil_div(k, 64)) * block_us(fitted.tile_n) * (k % 16 != 0 ? 1.2 : 1.0);
       if (us < deep) us = deep;
     }
     if (us < 0.92 * scheduled_us(batch, m, n, k, machine, *c)) *c = fitted;
   }
-  flat_pairs(batch, m, n, k, machine, c);
+  flat_pairs(batch, m, n, k, activation, machine, c);
 }
 
 // The swapped SwiGLU schedule for a product that does not fill the SMs with 128-column row-major tiles (which
@@ -1363,12 +1389,20 @@ int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n
 }
 
 int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k, ayla_b200_config* cfg) {
+  return ayla_b200_fit_depth_act(op, dtype, AYLA_B200_ACT_NONE, batch, m, n, k, cfg);
+}
+
+int ayla_b200_fit_depth_act(int op, int dtype, int activation, int64_t batch, int64_t m, int64_t n, int64_t k,
+                            ayla_b200_config* cfg) {
   if (cfg == nullptr) return fail(AYLA_B200_E_INVALID, "cfg is null");
   int rc = check_shape(op, dtype, batch, m, n, k);
   if (rc) return rc;
+  if (activation < AYLA_B200_ACT_NONE || activation > AYLA_B200_ACT_GELU_TANH) {
+    return fail(AYLA_B200_E_INVALID, "unknown activation %d", activation);
+  }
   rc = check_config(*cfg, false);
   if (rc) return rc;
-  fit_depth(batch, m, n, k, current_machine(), cfg);
+  fit_depth(batch, m, n, k, activation, current_machine(), cfg);
   return AYLA_B200_OK;
 }
 

@@ -162,13 +162,13 @@ def _fit_labels(before: dict[str, object], after: dict[str, object], m: int) -> 
     return tuple(labels) or ("fitted to the shape",)
 
 
-def _fitted(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int,
-            batch: int) -> GemmScheduleSeed | None:
-    """The schedule as ``ayla_b200_fit_depth`` fits it to the shape: its depth split where SMs would idle, its last wave
+def _fitted(seed: GemmScheduleSeed | None, operation: str, dtype: str, m: int, n: int, k: int, batch: int,
+            activation: str) -> GemmScheduleSeed | None:
+    """The schedule as ``ayla_b200_fit_depth_act`` fits it to the shape: its depth split where SMs would idle, its last wave
     whole, in halves or split, tiles that all run at once, pairs on 128 rows."""
     if seed is None or seed.builder_config is None:
         return seed
-    fitted = _lib.fit_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k).to_dict()
+    fitted = _lib.fit_depth(_lib.Config.from_dict(seed.builder_config), operation, dtype, batch, m, n, k, activation).to_dict()
     if fitted == seed.builder_config:
         return seed
     captured = {**seed.captured_config, **fitted}
@@ -218,7 +218,8 @@ def _rule_streams_better(neighbour: dict[str, object], rule: dict[str, object], 
 
 
 def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
-                         batch: int = 1, activation: str = "none", share_depth: bool = True) -> GemmScheduleSeed | None:
+                         batch: int = 1, activation: str = "none", share_depth: bool = True,
+                         row_factors: bool = False) -> GemmScheduleSeed | None:
     """The schedule a launch of this shape uses, or ``None`` if the shape is unsupported.
 
     An exact table hit has empty ``adaptations``; a schedule transferred from a
@@ -226,7 +227,7 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
     default, which takes the fused ``activation`` into account, is returned with
     ``source_shape`` ``None``.  Any of them is fitted to the shape where that is faster (``_fitted``), exact hits too, which
     its adaptations then say, unless ``share_depth`` is false (for a gate shaped like the output, whose kernels do not
-    split, and for launches that leave SMs to others).  It is a schedule of the general
+    split, and for launches that leave SMs to others), by what their epilogue costs: ``activation`` and ``row_factors``.  It is a schedule of the general
     kernel: plain products that ``packed_serves`` run on the packed kernel, which takes none.
     """
     if min(batch, m, n, k) <= 0 or operation not in _OPERATIONS:
@@ -244,7 +245,8 @@ def select_gemm_schedule(operation: str, dtype: str, m: int, n: int, k: int,
         return sum(abs(math.log2(a) - math.log2(b)) for a, b in zip(shape, query, strict=True))
 
     def finished(seed: GemmScheduleSeed | None) -> GemmScheduleSeed | None:
-        return _fitted(seed, operation, dtype, m, n, k, batch) if share_depth else seed
+        epilogue = "relu" if row_factors and activation == "none" else activation
+        return _fitted(seed, operation, dtype, m, n, k, batch, epilogue) if share_depth else seed
 
     rule = None
     if query not in table and _streams_weights(operation, batch, m, n, k):
@@ -579,7 +581,7 @@ def gemm_jit_compiler(operation: str, dtype: str, activation: str = "none",
         if gated is True and tuple(mul) != tuple(out):
             raise ValueError(f"{bound.name}: mul must have the shape of out {tuple(out)}, got {tuple(mul)}")
         count = batch[0] if batch else 1
-        schedule = select_gemm_schedule(operation, dtype, m, n, k, count, activation, gated is not True)
+        schedule = select_gemm_schedule(operation, dtype, m, n, k, count, activation, gated is not True, gated == "row")
         if schedule is None:
             raise ValueError(f"{bound.name}: no schedule for {operation} {lead}x{m}x{n}x{k}")
         return GemmLauncher(operation, dtype, count, m, n, k, schedule, device, activation, gated,

@@ -276,6 +276,10 @@ AYLA_B200_API int ayla_b200_share_depth(int op, int dtype, int64_t batch, int64_
 AYLA_B200_API int ayla_b200_fit_depth(int op, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                                       ayla_b200_config* cfg);
 
+/* The same for a launch with this fused activation (AYLA_B200_ACT_RELU for one with row factors alone). */
+AYLA_B200_API int ayla_b200_fit_depth_act(int op, int dtype, int activation, int64_t batch, int64_t m, int64_t n,
+                                          int64_t k, ayla_b200_config* cfg);
+
 /*
  * The schedule ayla_b200_swiglu uses when cfg == NULL: row-major (swap_ab == 0), or with the weights on the row
  * side (swap_ab == 1), a form that cannot be asked for by a cfg.

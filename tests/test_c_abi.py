@@ -235,27 +235,34 @@ def test_schedules_from_other_shapes_are_fitted_to_one_wave(shape, config, expec
     assert (out.tile_n, out.cta_group, out.split_k, out.split_tail, out.cluster_split) == expected
 
 
-# (m, n, k), a schedule that measured faster than whole tiles in one wave
-@pytest.mark.parametrize("shape, config, expected", [
-    # 128-wide pairs in more than one wave: few k-blocks, and many with a split last wave
-    ((1147, 1920, 1408), dict(tile_n=128, cta_group=2, split_tail=2), (128, 1, 1, 0)),
-    ((990, 2368, 768), dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2)),
-    ((2200, 1216, 35136), dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 4, 1)),
-    ((1304, 1808, 33888), dict(tile_n=128, cta_group=2), (128, 2, 4, 1)),
-    # single CTAs of the same width, and clusters
-    ((1722, 2560, 768), dict(tile_n=256, cta_group=1), (256, 1, 1, 0)),
-    ((179, 768, 1296), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (64, 1, 2, 0)),
-    ((282, 5440, 3776), dict(tile_n=256, cta_group=1, split_k=2, cluster_split=1), (256, 1, 2, 0)),
-    # taken beside those bounds
-    ((1072, 2240, 1856), dict(tile_n=128, cta_group=2, split_tail=2), (192, 2, 1, 0)),
-    ((1752, 1912, 26640), dict(tile_n=128, cta_group=2), (192, 2, 1, 0)),
-    ((1581, 1712, 760), dict(tile_n=256, cta_group=1), (192, 2, 1, 0)),
-    ((192, 1664, 1152), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (64, 2, 1, 0)),
+# (m, n, k), activation, a schedule -> the one that measured faster of it and whole tiles in one wave
+@pytest.mark.parametrize("shape, activation, config, expected", [
+    # 128-wide pairs in more than one wave: by the activation, the k-blocks and the tiles left over
+    ((9457, 384, 1280), "none", dict(tile_n=128, cta_group=2, split_tail=2), (192, 2, 1, 0)),
+    ((9457, 384, 1280), "relu", dict(tile_n=128, cta_group=2, split_tail=2), (192, 2, 1, 0)),
+    ((9457, 384, 1280), "silu", dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2)),
+    ((990, 2368, 768), "none", dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2)),
+    ((990, 2368, 960), "none", dict(tile_n=128, cta_group=2, split_tail=2), (192, 2, 1, 0)),
+    ((990, 2368, 1088), "relu", dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2)),
+    ((1147, 1920, 1408), "gelu", dict(tile_n=128, cta_group=2, split_tail=2), (128, 1, 1, 0)),
+    ((1072, 2240, 1856), "gelu", dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 1, 2)),
+    ((1072, 2240, 2112), "gelu", dict(tile_n=128, cta_group=2, split_tail=2), (192, 2, 1, 0)),
+    # ... many k-blocks, with a split last wave there
+    ((2200, 1216, 35136), "none", dict(tile_n=128, cta_group=2, split_tail=2), (128, 2, 4, 1)),
+    ((1304, 1808, 33888), "none", dict(tile_n=128, cta_group=2), (128, 2, 4, 1)),
+    ((1752, 1912, 26640), "none", dict(tile_n=128, cta_group=2), (192, 2, 1, 0)),
+    # single CTAs of the same width (whole lines, and others), and clusters
+    ((1722, 2560, 768), "none", dict(tile_n=256, cta_group=1), (256, 1, 1, 0)),
+    ((2188, 1992, 1040), "relu", dict(tile_n=256, cta_group=1), (256, 2, 1, 0)),
+    ((1581, 1712, 760), "none", dict(tile_n=256, cta_group=1), (192, 2, 1, 0)),
+    ((179, 768, 1296), "relu", dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (64, 1, 2, 0)),
+    ((192, 1664, 1152), "none", dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (64, 2, 1, 0)),
+    ((282, 5440, 3776), "none", dict(tile_n=256, cta_group=1, split_k=2, cluster_split=1), (256, 1, 2, 0)),
 ])
-def test_one_wave_only_where_it_measured_faster(shape, config, expected):
+def test_one_wave_only_where_it_measured_faster(shape, activation, config, expected):
     m, n, k = shape
-    out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, **config)), "mm", "bfloat16", 1, m, n, k)
-    assert _lib.config_valid(out, "mm", "bfloat16", 1, m, n, k)
+    out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, **config)), "addmm", "bfloat16", 1, m, n, k, activation)
+    assert _lib.config_valid(out, "addmm", "bfloat16", 1, m, n, k)
     assert (out.tile_n, out.cta_group, out.split_k, out.split_tail) == expected
 
 
