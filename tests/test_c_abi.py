@@ -317,6 +317,22 @@ def test_few_rows_stay_with_single_ctas_where_those_measured_faster(batch, shape
     assert out.cta_group == 1
 
 
+# (batch, m, n, k), a schedule of single CTAs that measured slower than pairs beside the ones above
+@pytest.mark.parametrize("batch, shape, config, expected", [
+    (37, (61, 72, 2240), dict(tile_n=128, cta_group=1, split_k=4, cluster_split=1), (128, 1)),
+    (17, (66, 256, 3136), dict(tile_n=128, cta_group=1, split_k=4), (128, 1)),
+    (33, (89, 56, 1088), dict(tile_n=64, cta_group=1, split_k=2, cluster_split=1), (128, 1)),
+    (1, (128, 192, 760), dict(tile_n=64, cta_group=1, split_k=4, cluster_split=1), (128, 2)),
+    (1, (128, 544, 3464), dict(tile_n=64, cta_group=1, split_k=4, cluster_split=1), (128, 4)),
+])
+def test_few_rows_of_the_same_kinds_go_to_pairs_where_those_measured_faster(batch, shape, config, expected):
+    m, n, k = shape
+    operation = "bmm" if batch > 1 else "mm"
+    out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, **config)), operation, "bfloat16", batch, m, n, k)
+    assert _lib.config_valid(out, operation, "bfloat16", batch, m, n, k)
+    assert out.cta_group == 2 and (out.tile_n, out.split_k) == expected
+
+
 def test_whole_narrow_tiles_of_few_rows_are_not_given_a_split_depth():
     out = _lib.fit_depth(_lib.Config.from_dict(dict(group_m=8, tile_n=64, cta_group=1)), "mm", "float16", 1, 94, 3456, 1024)
     assert out.split_k == 1
